@@ -1,0 +1,70 @@
+"""The substructured solver (shared elimination of the nodes off the mixed
+boundary, one dense root per system) against the oracle's band solution, at
+the sizes where its tiles and chains end: a mesh with a handful of interior
+nodes, electrode counts around the 32-wide tiles, separators beyond one
+front's 64 nodes, jittered triangles, and rectangles of systems cut by the
+memory budget.  Tolerances as in test_gpu_forward.py: complex128 1e-10,
+complex64 + FP64 refinement 1e-6."""
+import numpy as np
+import pytest
+
+from conftest import relerr
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(nx, nz, ne, tri=False, seed=3):
+    from titatest_gb300 import synth
+    rng = np.random.default_rng(seed)
+    grid, surface, _, _ = synth._quad_grid(np.arange(nx + 1, dtype=float), np.arange(nz + 1) * 0.7, triangles=tri,
+                                           jitter=0.2 if tri else 0.0, rng=rng)
+    mag, pha = synth.random_model(grid, rng)
+    enodes = np.linspace(1, nx - 1, ne).astype(int)
+    return synth._finish("sub", grid, surface, enodes, synth.dipole_dipole(ne, [1], [1, 2]), mag, pha, nx, nz)
+
+
+@pytest.mark.parametrize("nx,nz,ne,tri", [(5, 4, 4, False), (24, 9, 16, True), (66, 13, 31, False),
+                                          (67, 20, 33, False), (72, 70, 6, False), (40, 30, 32, True)])
+def test_forward_and_adjoint_match_oracle(gpu_lib, nx, nz, ne, tri):
+    from titatest_gb300 import MIXED, PLAIN, CRMod
+    s = _case(nx, nz, ne, tri)
+    P = O.Problem(s.grid, s.survey)
+    kwn, kwnwi = P.rwaven()
+    kp = P.forward(s.sigma, kwn, kwnwi)
+    volt, _ = P.bvolt(P.rtrafo(kp, kwnwi), 0, None)
+    g = np.random.default_rng(1).normal(size=(s.survey.nanz, 2)) @ np.array([1.0, 1j])
+    grads = {}
+    for prec, tol in ((PLAIN, 1e-10), (MIXED, 1e-6)):
+        with CRMod(s.grid, s.survey, kwn, kwnwi, precision=prec) as m:
+            out = m.forward(s.sigma, kpot=True)
+            grads[prec] = m.adjoint(g)
+            assert relerr(out["kpot"], kp) < tol
+            assert relerr(out["volt"], volt) < tol
+    assert relerr(grads[MIXED], grads[PLAIN]) < 1e-6
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("systems", [5, 33, 70])
+def test_rectangles_of_a_small_memory_budget(gpu_lib, prec, systems):
+    """Fewer systems than one wavenumber has electrodes, and whole
+    wavenumbers that do not divide their count: the same voltages and
+    adjoint as one batch."""
+    from titatest_gb300 import CRMod
+    s = _case(45, 16, 33)
+    g = np.random.default_rng(2).normal(size=(s.survey.nanz, 2)) @ np.array([1.0, 1j])
+    with CRMod(s.grid, s.survey, precision=prec) as m:
+        v1 = m.forward(s.sigma)["volt"]
+        a1 = m.adjoint(g)
+        assert m.stats()["nbatches"] == 1
+    nb = 45 + 2 * 16 + 1
+    mp = (nb + 31) // 32 * 32
+    esz = 16 if prec == 0 else 8
+    per = mp * (mp + 32) * esz + s.grid.sanz * (3 * esz + (32 if prec else 0))
+    with CRMod(s.grid, s.survey, precision=prec) as m:
+        m.set_memory_budget(int(per * systems * 1.35))
+        v2 = m.forward(s.sigma)["volt"]
+        assert m.stats()["nbatches"] > 1
+        a2 = m.adjoint(g)
+    assert relerr(v2, v1) < 1e-12 and relerr(a2, a1) < 1e-12

@@ -103,6 +103,22 @@ void free_batch(crgpu_ctx *c) {
     c->Bmax = DevBatch{};
     c->d_ks = c->d_ls = nullptr;
     c->batch_cap = 0;
+    if (!c->factors_sub) c->factors_resident = false;
+}
+
+void free_sub_batch(crgpu_ctx *c) {
+    drop_graph(c);
+    SubBatch &B = c->SB;
+    void *ptrs[] = {B.C,  c->precision == CRGPU_MIXED ? B.X : nullptr, B.Bt, B.Y, B.W, B.Z, B.U, B.status, B.active,
+                    B.kact, B.mz};
+    for (void *p : ptrs)
+        if (p) {
+            cudaFreeAsync(p, c->st);
+            c->allocs.erase(std::remove(c->allocs.begin(), c->allocs.end(), p), c->allocs.end());
+        }
+    B = SubBatch{};
+    c->sub_cap = 0;
+    if (c->factors_sub) c->factors_resident = false;
 }
 
 // elements between the band factors of consecutive systems (see DevBatch)
@@ -113,6 +129,14 @@ size_t bytes_per_system(const crgpu_ctx *c) {
     size_t esz = c->precision == CRGPU_MIXED ? sizeof(float2) : sizeof(double2);
     return lpitch_of(n, W) * esz + nnz * sizeof(double2) + n * sizeof(double) +
            nr * n * (3 * sizeof(double2) + esz) + 64;
+}
+
+int ensure_refine(crgpu_ctx *c) {
+    if (c->d_refine) return 0;
+    char *cnt = nullptr;  // [kRefineSlots][kRefineCap] steps of {int count, pad, double zmax}
+    int e = dalloc(c, &cnt, kRefineSlots * kRefineCap * sizeof(RefineCount));
+    c->d_refine = cnt;
+    return e;
 }
 
 int ensure_batch(crgpu_ctx *c, int want) {
@@ -132,11 +156,7 @@ int ensure_batch(crgpu_ctx *c, int want) {
     e = e ? e : dalloc(c, &y, (size_t)want * nr * n * esz);
     e = e ? e : dalloc(c, &B.status, (size_t)want);
     e = e ? e : dalloc(c, &B.active, (size_t)want * nr);
-    if (!e && !c->d_refine) {
-        char *cnt = nullptr;  // [kRefineSlots][kRefineCap] steps of {int count, pad, double zmax}
-        e = dalloc(c, &cnt, kRefineSlots * kRefineCap * sizeof(RefineCount));
-        c->d_refine = cnt;
-    }
+    e = e ? e : ensure_refine(c);
     e = e ? e : dalloc(c, &c->d_ks, (size_t)want);
     e = e ? e : dalloc(c, &c->d_ls, (size_t)want);
     if (!e && c->lsr) {
@@ -151,7 +171,7 @@ int ensure_batch(crgpu_ctx *c, int want) {
     return 0;
 }
 
-int check_device_errors(crgpu_ctx *c, const int *d_status, int nsys) {
+int check_device_errors(crgpu_ctx *c, const int *d_status, int nsys, int k0 = -1) {
     int h_err = 0;
     CUCHECK(c, cudaMemcpyAsync(&h_err, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
     std::vector<int> st(nsys > 0 ? nsys : 0);
@@ -160,7 +180,7 @@ int check_device_errors(crgpu_ctx *c, const int *d_status, int nsys) {
     if (h_err) return fail(c, h_err, "device reported error " + std::to_string(h_err));
     for (int s = 0; s < nsys; s++)
         if (st[s]) {
-            int k = c->sys_k.empty() ? 0 : c->sys_k[s];
+            int k = c->sys_k.empty() ? 0 : k0 < 0 ? c->sys_k[s] : std::min(c->K - 1, k0 + s / c->eanz);
             return fail(c, st[s], "system (k=" + std::to_string(k + 1) + ") failed with error " +
                                       std::to_string(st[s]));
         }
@@ -340,36 +360,226 @@ int tail_systems(const crgpu_ctx *c, int ns) {
     return 0;
 }
 
-// the forward block on device-resident sigma
-int run_forward(crgpu_ctx *c, const double2 *d_sigma, int volt_mode, const double *d_kfak, double2 *d_volt,
-                double2 *d_sigmaa) {
-    DevProblem &P = c->P;
-    const bool cap = c->capturing;  // graph capture: no host copies, synchronisation or timing
-    c->stats = crgpu_stats{};
-    c->factors_resident = false;
-    cudaEvent_t ev[4];
-    for (auto &e : ev) cudaEventCreate(&e);
-    if (!cap) cudaEventRecord(ev[0], c->st);
-    CUCHECK(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->st));
-    if (d_sigma != c->d_sigma)  // keep the model of this forward (adjoint, refactorisation)
-        CUCHECK(c, cudaMemcpyAsync(c->d_sigma, d_sigma, sizeof(double2) * c->hg.elanz, cudaMemcpyDeviceToDevice, c->st));
-    d_sigma = c->d_sigma;
-    if (P.ldc) {  // the DC routines take DBLE(sigma) (src/kompadc.f90:114-119, src/bsendc.f90:172)
-        launch_real_part(c->d_sigma, c->hg.elanz, c->st);
-        c->stats.kernel_launches += 1;
+// ---- substructured solver (substruct.cu) ----------------------------------
+
+// Whether this forward runs on it: the problems of the band kernels' own
+// entry points, singularity removal, DC mode (whose pivots are tested one by
+// one, src/choldc.f90:66-70) and valued Dirichlet nodes keep the band.
+bool sub_on(const crgpu_ctx *c) {
+    return c->sub_fits && !c->band_pinned && !c->lsr && !c->P.ldc && !c->P.lrandb2;
+}
+
+size_t sub_bytes_per_system(const crgpu_ctx *c) {
+    const bool mixed = c->precision == CRGPU_MIXED;
+    const size_t n = c->hg.n, esz = mixed ? sizeof(float2) : sizeof(double2);
+    return (size_t)c->D.mp * c->D.ldc * esz + n * ((mixed ? 2 : 0) * sizeof(double2) + 3 * esz) +
+           (size_t)c->D.szU * esz + 64;
+}
+
+// the shared factor's arrays
+int ensure_sub_shared(crgpu_ctx *c) {
+    if (c->sub_shared) return 0;
+    DevSub &D = c->D;
+    const size_t K = c->K, esz = c->precision == CRGPU_MIXED ? sizeof(float2) : sizeof(double2);
+    char *F = nullptr, *G = nullptr, *H = nullptr, *S = nullptr, *R = nullptr;
+    int e = dalloc(c, &D.As, K * c->pat.nnz);
+    e = e ? e : dalloc(c, &D.fk, K * c->hg.n);
+    e = e ? e : dalloc(c, &D.kbad, K);
+    e = e ? e : dalloc(c, &F, K * D.szF * esz);
+    e = e ? e : dalloc(c, &G, K * D.szG * esz);
+    e = e ? e : dalloc(c, &H, K * D.szG * esz);
+    e = e ? e : dalloc(c, &S, K * D.szS * esz);
+    e = e ? e : dalloc(c, &R, K * D.mp * D.ldc * esz);
+    if (e) return e;
+    D.F = F;
+    D.G = G;
+    D.H = H;
+    D.S = S;
+    D.R = R;
+    c->sub_shared = true;
+    return 0;
+}
+
+int ensure_sub_batch(crgpu_ctx *c, int want) {
+    if (c->sub_cap >= want) return 0;
+    free_sub_batch(c);
+    const bool mixed = c->precision == CRGPU_MIXED;
+    const size_t n = c->hg.n, esz = mixed ? sizeof(float2) : sizeof(double2), w = want;
+    SubBatch &B = c->SB;
+    char *C = nullptr, *Y = nullptr, *W = nullptr, *Z = nullptr, *U = nullptr;
+    int e = ensure_refine(c);
+    e = e ? e : dalloc(c, &C, w * c->D.mp * c->D.ldc * esz);
+    B.C = C;
+    if (mixed) {
+        e = e ? e : dalloc(c, &B.X, w * n);
+        e = e ? e : dalloc(c, &B.Bt, w * n);
     }
-    launch_adom(P, d_sigma, c->d_adom, c->st);
+    e = e ? e : dalloc(c, &Y, w * n * esz);
+    B.Y = Y;
+    e = e ? e : dalloc(c, &W, w * n * esz);
+    B.W = W;
+    e = e ? e : dalloc(c, &Z, w * n * esz);
+    B.Z = Z;
+    e = e ? e : dalloc(c, &U, std::max<size_t>(1, w * c->D.szU) * esz);
+    B.U = U;
+    e = e ? e : dalloc(c, &B.status, w);
+    e = e ? e : dalloc(c, &B.active, w);
+    e = e ? e : dalloc(c, &B.kact, (size_t)c->K);
+    e = e ? e : dalloc(c, &B.mz, 2 * w);
+    if (e) return e;
+    B.mx = B.mz + w;
+    if (!mixed) B.X = (double2 *)Z;
+    CUCHECK(c, cudaMemsetAsync(B.mz, 0, 2 * w * sizeof(unsigned long long), c->st));
+    c->sub_cap = want;
+    return 0;
+}
+
+// The rectangles of systems that one batch holds: whole wavenumbers, or some
+// of one wavenumber's electrodes where not even those fit the budget.
+void sub_rect(crgpu_ctx *c, int *kb, int *lb) {
+    const int nsys = (int)c->sys_k.size();
+    const size_t per = sub_bytes_per_system(c);
+    int64_t budget = c->mem_budget;
+    if (budget <= 0) {
+        size_t fr = 0, tot = 0;
+        cudaMemGetInfo(&fr, &tot);
+        budget = (int64_t)(0.6 * (double)(fr + (size_t)c->sub_cap * per));
+    }
+    int bs = (int)std::max<int64_t>(1, std::min<int64_t>(nsys, budget / (int64_t)per));
+    if (c->sub_cap >= nsys) bs = nsys;
+    *kb = bs >= c->eanz ? bs / c->eanz : 1;
+    *lb = bs >= c->eanz ? c->eanz : bs;
+}
+
+int sub_factor_shared(crgpu_ctx *c) {
+    int e = ensure_sub_shared(c);
+    if (e) return e;
+    sub_launch_values(c->P, c->D, c->d_sigma, c->d_adom, c->st);
+    c->stats.kernel_launches += 2;
+    c->stats.kernel_launches += sub_launch_factor(c->P, c->D, c->sp, c->precision == CRGPU_MIXED, c->st);
+    return 0;
+}
+
+int sub_factor_rect(crgpu_ctx *c, const SubBatch &B) {
+    CUCHECK(c, cudaMemsetAsync(B.status, 0, sizeof(int) * B.Kb * B.Lb, c->st));
+    sub_launch_root(c->P, c->D, B, c->d_sigma, c->precision == CRGPU_MIXED, c->st);
     c->stats.kernel_launches += 1;
-    if (c->lsr) {
-        launch_refsig(P, d_sigma, c->d_sigma0, c->st);
-        c->stats.kernel_launches += 1;
+    return 0;
+}
+
+// Solves the rectangle for the right-hand sides of kompab (src null) or for
+// the rows of src; the solution ends in B.X.  Mixed precision refines as
+// solve_view does: every step is launched without waiting for the host.
+int sub_solve_rect(crgpu_ctx *c, const SubBatch &B, const double2 *src) {
+    const bool mixed = c->precision == CRGPU_MIXED;
+    SubBatch B0 = B;
+    B0.kact = nullptr;
+    sub_launch_rhs(c->P, c->D, B, mixed, c->lsink, c->nsink, src, c->st);
+    c->stats.kernel_launches += 1 + sub_launch_apply(c->D, c->sp, B0, mixed, nullptr, c->st);
+    if (!mixed) return 0;
+    RefineCount *cnt = (RefineCount *)c->d_refine;
+    const int steps = std::min(c->refine_maxit, kRefineCap);
+    CUCHECK(c, cudaMemsetAsync(cnt, 0, sizeof(RefineCount) * kRefineCap, c->st));
+    sub_launch_accumulate(c->D, B, true, c->refine_tol, nullptr, nullptr, nullptr, c->st);
+    c->stats.kernel_launches += 2;
+    for (int it = 0; it < steps; it++) {
+        const int *nprev = it > 0 ? &cnt[it - 1].n : nullptr;
+        sub_launch_residual(c->P, c->D, B, c->d_sigma, nprev, c->st);
+        c->stats.kernel_launches += 3 + sub_launch_apply(c->D, c->sp, B, true, nprev, c->st);
+        sub_launch_accumulate(c->D, B, false, c->refine_tol, nprev, &cnt[it].n, &cnt[it].z, c->st);
     }
+    c->refine_used[0] = std::max(c->refine_used[0], steps);
+    return 0;
+}
+
+SubBatch sub_view(const crgpu_ctx *c, int k0, int kb, int l0, int lb) {
+    SubBatch B = c->SB;
+    B.k0 = k0;
+    B.Kb = std::min(kb, c->K - k0);
+    B.l0 = l0;
+    B.Lb = std::min(lb, c->eanz - l0);
+    return B;
+}
+
+// every system of the forward: shared factor, then root factors and solves by
+// rectangles, potentials into d_kpot
+int forward_sub(crgpu_ctx *c, float *t_factor, float *t_solve) {
+    const bool cap = c->capturing;  // recorded, or queued beside other problems: one rectangle, no waiting
+    int kb = c->K, lb = c->eanz;
+    if (!cap) sub_rect(c, &kb, &lb);
+    int e = ensure_sub_batch(c, kb * lb);
+    if (e) return e;
+    c->factors_sub = true;
+    cudaEvent_t ev[4] = {};
+    if (!cap) {
+        for (auto &v : ev) cudaEventCreate(&v);
+        cudaEventRecord(ev[0], c->st);
+    }
+    e = sub_factor_shared(c);
+    if (!cap) cudaEventRecord(ev[1], c->st);
+    float shared = 0.f;
+    for (int k0 = 0; k0 < c->K && !e; k0 += kb)
+        for (int l0 = 0; l0 < c->eanz && !e; l0 += lb) {
+            const SubBatch B = sub_view(c, k0, kb, l0, lb);
+            if (!cap && c->stats.nbatches) cudaEventRecord(ev[1], c->st);
+            e = sub_factor_rect(c, B);
+            if (!cap) cudaEventRecord(ev[2], c->st);
+            if (!e) e = sub_solve_rect(c, B, nullptr);
+            if (e) break;
+            sub_launch_unpack(c->P, c->D, B, -1.0, c->d_kpot, c->d_kpot32, c->st);
+            c->stats.kernel_launches += 1;
+            c->stats.nbatches++;
+            if (cap) continue;
+            cudaEventRecord(ev[3], c->st);
+            e = check_device_errors(c, B.status, B.Kb * B.Lb, k0);
+            float a = 0.f, b = 0.f;
+            if (c->stats.nbatches == 1) cudaEventElapsedTime(&shared, ev[0], ev[1]);
+            cudaEventElapsedTime(&a, ev[1], ev[2]);
+            cudaEventElapsedTime(&b, ev[2], ev[3]);
+            *t_factor += a;
+            *t_solve += b;
+        }
+    *t_factor += shared;
+    if (!cap)
+        for (auto &v : ev) cudaEventDestroy(v);
+    return e;
+}
+
+// lambda_(k,l) of run_adjoint
+int adjoint_sub(crgpu_ctx *c) {
+    const bool have = c->factors_resident && c->factors_sub;
+    int kb = c->K, lb = c->eanz, e = 0;
+    if (!have) {
+        sub_rect(c, &kb, &lb);
+        e = ensure_sub_batch(c, kb * lb);
+        if (!e) e = sub_factor_shared(c);
+        if (e) return e;
+        c->factors_sub = true;
+    }
+    for (int k0 = 0; k0 < c->K; k0 += kb)
+        for (int l0 = 0; l0 < c->eanz; l0 += lb) {
+            const SubBatch B = sub_view(c, k0, kb, l0, lb);
+            if (!have) e = sub_factor_rect(c, B);
+            if (!e) e = sub_solve_rect(c, B, c->d_adjsrc);
+            if (e) return e;
+            sub_launch_unpack(c->P, c->D, B, 1.0, c->d_lambda, nullptr, c->st);
+            c->stats.kernel_launches += 2;
+            e = check_device_errors(c, B.status, B.Kb * B.Lb, k0);
+            if (e) return e;
+        }
+    c->factors_resident = kb == c->K && lb == c->eanz;
+    return 0;
+}
+
+// every system of the forward on its band factor, batch by batch
+int forward_band(crgpu_ctx *c, const double2 *d_sigma, float *t_factor, float *t_solve) {
+    DevProblem &P = c->P;
+    const bool cap = c->capturing;
     const int nsys_total = (int)c->sys_k.size();
     const int bs = cap ? nsys_total : batch_size(c);  // recording: one batch, allocated by the ordinary run
     int e = ensure_batch(c, bs);
     if (e) return e;
-    c->stats.nsystems = nsys_total;
-    float t_factor = 0.f, t_solve = 0.f;
+    c->factors_sub = false;
     cudaEvent_t f0, f1, f2;
     cudaEventCreate(&f0);
     cudaEventCreate(&f1);
@@ -440,12 +650,42 @@ int run_forward(crgpu_ctx *c, const double2 *d_sigma, int volt_mode, const doubl
         float a = 0, b = 0;
         cudaEventElapsedTime(&a, f0, f1);
         cudaEventElapsedTime(&b, f1, f2);
-        t_factor += a;
-        t_solve += b;
+        *t_factor += a;
+        *t_solve += b;
     }
     cudaEventDestroy(f0);
     cudaEventDestroy(f1);
     cudaEventDestroy(f2);
+    return worst;
+}
+
+// the forward block on device-resident sigma
+int run_forward(crgpu_ctx *c, const double2 *d_sigma, int volt_mode, const double *d_kfak, double2 *d_volt,
+                double2 *d_sigmaa) {
+    DevProblem &P = c->P;
+    const bool cap = c->capturing;  // graph capture: no host copies, synchronisation or timing
+    c->stats = crgpu_stats{};
+    c->factors_resident = false;
+    cudaEvent_t ev[4];
+    for (auto &e : ev) cudaEventCreate(&e);
+    if (!cap) cudaEventRecord(ev[0], c->st);
+    CUCHECK(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->st));
+    if (d_sigma != c->d_sigma)  // keep the model of this forward (adjoint, refactorisation)
+        CUCHECK(c, cudaMemcpyAsync(c->d_sigma, d_sigma, sizeof(double2) * c->hg.elanz, cudaMemcpyDeviceToDevice, c->st));
+    d_sigma = c->d_sigma;
+    if (P.ldc) {  // the DC routines take DBLE(sigma) (src/kompadc.f90:114-119, src/bsendc.f90:172)
+        launch_real_part(c->d_sigma, c->hg.elanz, c->st);
+        c->stats.kernel_launches += 1;
+    }
+    launch_adom(P, d_sigma, c->d_adom, c->st);
+    c->stats.kernel_launches += 1;
+    if (c->lsr) {
+        launch_refsig(P, d_sigma, c->d_sigma0, c->st);
+        c->stats.kernel_launches += 1;
+    }
+    c->stats.nsystems = (int)c->sys_k.size();
+    float t_factor = 0.f, t_solve = 0.f;
+    int worst = sub_on(c) ? forward_sub(c, &t_factor, &t_solve) : forward_band(c, d_sigma, &t_factor, &t_solve);
     if (worst) {
         for (auto &ev_ : ev) cudaEventDestroy(ev_);
         return worst;
@@ -499,7 +739,10 @@ int run_adjoint(crgpu_ctx *c, const double2 *d_g, double2 *d_grad) {
     const int nsys_total = (int)c->sys_k.size();
     const int nr = c->nrhs;
     int e = 0;
-    if (c->factors_resident) {
+    if (sub_on(c)) {
+        e = adjoint_sub(c);
+        if (e) return e;
+    } else if (c->factors_resident && !c->factors_sub) {
         DevBatch B = batch_view(c, nsys_total);
         launch_adjoint_rhs(P, B, nr, c->d_adjsrc, c->st);
         e = solve_batch(c, nsys_total, false);
@@ -509,7 +752,10 @@ int run_adjoint(crgpu_ctx *c, const double2 *d_g, double2 *d_grad) {
         e = check_device_errors(c, B.status, nsys_total);
         if (e) return e;
     } else {
+        if (c->batch_cap == 0) e = ensure_batch(c, batch_size(c));
+        if (e) return e;
         const int bs = c->batch_cap;
+        c->factors_sub = false;
         for (int s0 = 0; s0 < nsys_total; s0 += bs) {
             const int ns = std::min(bs, nsys_total - s0);
             DevBatch B = batch_view(c, ns);
@@ -783,6 +1029,48 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
             c->sys_l.push_back(0);
         }
     }
+    if (c->nrhs == 1 && build_sub_plan(hg, c->pat, c->sp)) {
+        const SubPlan &sp = c->sp;
+        DevSub &D = c->D;
+        D.n = sp.n;
+        D.m = sp.m;
+        D.nI = sp.nI;
+        D.mp = (sp.m + 31) & ~31;
+        D.ldc = D.mp + 32;
+        D.szU = sp.szU;
+        D.szF = sp.szF;
+        D.szG = sp.szG;
+        D.szS = sp.szS;
+        D.root_ent0 = sp.root_ent0;
+        D.n_root_ent = (int)sp.ent.size() - sp.root_ent0;
+        D.root_child = sp.root_child;
+        D.root_u0 = sp.fronts[sp.root_child].u0;
+        D.root_r = sp.fronts[sp.root_child].r;
+        D.root_oS = sp.fronts[sp.root_child].oS;
+        std::vector<int32_t> fcolpos(c->pat.fcol.size());
+        for (size_t q = 0; q < fcolpos.size(); q++) fcolpos[q] = sp.pos[c->pat.fcol[q]];
+        e = upload(c, &D.fr, sp.fronts);
+        if (!e) e = upload(c, &D.ent, sp.ent);
+        if (!e) e = upload(c, &D.root_bnd, sp.root_bnd);
+        if (!e) e = upload(c, &D.tG, sp.tG);
+        if (!e) e = upload(c, &D.tS, sp.tS);
+        if (!e) e = upload(c, &D.tU, sp.tU);
+        if (!e) e = upload(c, &D.tD, sp.tD);
+        if (!e) e = upload(c, &D.pos, sp.pos);
+        if (!e) e = upload(c, &D.node, sp.node);
+        if (!e) e = upload(c, &D.rows, sp.rows);
+        if (!e) e = upload(c, &D.inv, sp.inv);
+        if (!e) e = upload(c, &D.root_inv, sp.root_inv);
+        if (!e) e = upload(c, &D.root_bptr, sp.root_bptr);
+        if (!e) e = upload(c, &D.fcolpos, fcolpos);
+        if (e) {
+            *out = c;
+            return e;
+        }
+        const double n = hg.n, mb = hg.mb, band = 0.5 * n * mb * mb + 6.0 * n * mb;
+        const double m = sp.m, sub = m * m * m / 6.0 + 4.0 * sp.c_apply + sp.c_factor / c->eanz;
+        c->sub_fits = sub <= 2.0 * band;
+    }
     if (precision == CRGPU_MIXED && !mixed_window_supported(hg.mb + 1)) {
         c->last_error = "mixed precision supports band widths up to 207";
         *out = c;
@@ -869,6 +1157,7 @@ int crgpu_set_memory_budget(crgpu_ctx *c, int64_t bytes) {
     if (!c) return ERR_ARG;
     c->mem_budget = bytes;
     free_batch(c);
+    free_sub_batch(c);
     return 0;
 }
 
@@ -944,7 +1233,7 @@ int crgpu_forward_sens_graph(crgpu_ctx *c, const void *sigma_device, void *volt_
         cudaEventRecord(a, c->st);
         CUCHECK(c, cudaGraphLaunch(c->graph, c->st));
         cudaEventRecord(b, c->st);
-        int e = check_device_errors(c, c->Bmax.status, (int)c->sys_k.size());
+        int e = check_device_errors(c, c->factors_sub ? c->SB.status : c->Bmax.status, (int)c->sys_k.size());
         c->stats.refine_iterations = 0;
         c->stats.refine_last_correction = 0.0;
         for (int q = 0; q < kRefineSlots; q++) c->refine_used[q] = c->graph_refine_used[q];
@@ -1031,11 +1320,11 @@ int crgpu_memory_need(const crgpu_ctx *c, int64_t *bytes) {
 }
 
 // Forward and Jacobian of several mixed-precision contexts (uneven meshes):
-// each problem is assembled on its own stream, the band factors of all their
-// systems run in one persistent tensor-core launch over a table of (problem,
-// system) items, longest systems first, and each problem's solves,
-// refinement, back-transform, voltages and Jacobian then run on its own
-// stream again.  Every problem must fit one batch (crgpu_memory_need).
+// each problem is assembled on its own stream; those that the substructured
+// solver takes stay there, the band factors of all others' systems run in one
+// persistent tensor-core launch over a table of (problem, system) items,
+// longest systems first, and each problem's solves, refinement,
+// back-transform, voltages and Jacobian then run on its own stream again.  Every problem must fit one batch (crgpu_memory_need).
 int crgpu_forward_sens_batch(crgpu_ctx *const *ctxs, int32_t nprob, const double *const *sigma, int32_t volt_mode,
                              double *const *volt, int32_t sens_mode) {
     if (!ctxs || nprob <= 0 || !sigma || !volt || (sens_mode < -1 || sens_mode > 1)) return ERR_ARG;
@@ -1056,11 +1345,23 @@ int crgpu_forward_sens_batch(crgpu_ctx *const *ctxs, int32_t nprob, const double
         c->stats = crgpu_stats{};
         c->factors_resident = false;
         drop_graph(c);
-        int e = ensure_batch(c, ns);
-        if (e) return e;
         CUCHECK(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->st));
         CUCHECK(c, cudaMemcpyAsync(c->d_sigma, sigma[p], sizeof(double2) * c->hg.elanz, cudaMemcpyHostToDevice, c->st));
         launch_adom(c->P, c->d_sigma, c->d_adom, c->st);
+        order[p] = p;
+        if (sub_on(c)) {  // potentials queued on its own stream; no part in the band launch
+            float t = 0.f;
+            c->capturing = true;
+            const int e = forward_sub(c, &t, &t);
+            c->capturing = false;
+            if (e) return e;
+            c->stats.kernel_launches += 1;
+            c->stats.nsystems = ns;
+            continue;
+        }
+        int e = ensure_batch(c, ns);
+        if (e) return e;
+        c->factors_sub = false;
         e = load_batch(c, 0, ns);
         if (!e) e = assemble_batch(c, c->d_sigma, ns);
         if (e) return e;
@@ -1072,7 +1373,6 @@ int crgpu_forward_sens_batch(crgpu_ctx *const *ctxs, int32_t nprob, const double
         CUCHECK(c, cudaStreamWaitEvent(st0, c->ev_join, 0));
         hp[p] = c->P;
         hb[p] = B;
-        order[p] = p;
     }
     // the item table, longest systems first
     std::sort(order.begin(), order.end(), [&](int a, int b) { return ctxs[a]->hg.n > ctxs[b]->hg.n; });
@@ -1083,21 +1383,26 @@ int crgpu_forward_sens_batch(crgpu_ctx *const *ctxs, int32_t nprob, const double
     DevBatch *dB = nullptr;
     int2 *dI = nullptr;
     crgpu_ctx *c0 = ctxs[0];
-    CUCHECK(c0, cudaMallocAsync((void **)&dP, sizeof(DevProblem) * nprob, st0));
-    CUCHECK(c0, cudaMallocAsync((void **)&dB, sizeof(DevBatch) * nprob, st0));
-    CUCHECK(c0, cudaMallocAsync((void **)&dI, sizeof(int2) * items.size(), st0));
-    CUCHECK(c0, cudaMemcpyAsync(dP, hp.data(), sizeof(DevProblem) * nprob, cudaMemcpyHostToDevice, st0));
-    CUCHECK(c0, cudaMemcpyAsync(dB, hb.data(), sizeof(DevBatch) * nprob, cudaMemcpyHostToDevice, st0));
-    CUCHECK(c0, cudaMemcpyAsync(dI, items.data(), sizeof(int2) * items.size(), cudaMemcpyHostToDevice, st0));
-    launch_factor_tc_multi(dP, dB, dI, (int)items.size(), 1, c0->nsm, st0);
-    CUCHECK(c0, cudaGetLastError());
+    if (!items.empty()) {
+        CUCHECK(c0, cudaMallocAsync((void **)&dP, sizeof(DevProblem) * nprob, st0));
+        CUCHECK(c0, cudaMallocAsync((void **)&dB, sizeof(DevBatch) * nprob, st0));
+        CUCHECK(c0, cudaMallocAsync((void **)&dI, sizeof(int2) * items.size(), st0));
+        CUCHECK(c0, cudaMemcpyAsync(dP, hp.data(), sizeof(DevProblem) * nprob, cudaMemcpyHostToDevice, st0));
+        CUCHECK(c0, cudaMemcpyAsync(dB, hb.data(), sizeof(DevBatch) * nprob, cudaMemcpyHostToDevice, st0));
+        CUCHECK(c0, cudaMemcpyAsync(dI, items.data(), sizeof(int2) * items.size(), cudaMemcpyHostToDevice, st0));
+        launch_factor_tc_multi(dP, dB, dI, (int)items.size(), 1, c0->nsm, st0);
+        CUCHECK(c0, cudaGetLastError());
+    }
     CUCHECK(c0, cudaEventRecord(c0->ev_join, st0));
     for (int p = 0; p < nprob; p++) {  // solves, refinement, voltages and Jacobian, each on its stream
         crgpu_ctx *c = ctxs[p];
-        if (p > 0) CUCHECK(c, cudaStreamWaitEvent(c->st, c0->ev_join, 0));
-        int e = solve_view(c, hb[p], true, c->st, 0);
-        if (e) return e;
-        launch_kpot(c->P, hb[p], 1, c->d_kpot, c->d_kpot32, c->st);
+        int e = 0;
+        if (!sub_on(c)) {
+            if (p > 0) CUCHECK(c, cudaStreamWaitEvent(c->st, c0->ev_join, 0));
+            e = solve_view(c, hb[p], true, c->st, 0);
+            if (e) return e;
+            launch_kpot(c->P, hb[p], 1, c->d_kpot, c->d_kpot32, c->st);
+        }
         launch_rtrafo(c->P, c->d_kpot, c->d_hpot, c->st);
         launch_bvolt(c->P, c->d_hpot, volt_mode, nullptr, c->d_volt, c->d_sigmaa, c->st);
         c->stats.kernel_launches += 4;
@@ -1119,16 +1424,16 @@ int crgpu_forward_sens_batch(crgpu_ctx *const *ctxs, int32_t nprob, const double
         CUCHECK(c, cudaMemcpyAsync(volt[p], volt_mode == 0 ? c->d_volt : c->d_sigmaa, sizeof(double2) * c->nanz,
                                    cudaMemcpyDeviceToHost, c->st));
         c->stats.kernel_launches += p == 0 ? 1 : 0;  // the shared factor launch
-        int e = check_device_errors(c, hb[p].status, hb[p].nsys);
+        const bool sub = sub_on(c);
+        int e = check_device_errors(c, sub ? c->SB.status : hb[p].status, (int)c->sys_k.size());
         if (!e) e = collect_refine_stats(c);
         if (e && !worst) worst = e;
         c->have_forward = !e;
         c->factors_resident = !e;
         c->stats.nbatches = 1;
     }
-    cudaFreeAsync(dP, st0);
-    cudaFreeAsync(dB, st0);
-    cudaFreeAsync(dI, st0);
+    for (void *q : {(void *)dP, (void *)dB, (void *)dI})
+        if (q) cudaFreeAsync(q, st0);
     CUCHECK(c0, cudaStreamSynchronize(st0));
     return worst;
 }
@@ -1421,6 +1726,7 @@ int crgpu_autotune(crgpu_ctx *c, const double *sigma, int32_t flags) {
     P.tune_factor = pick[0];
     P.tune_ctas = pick[1];
     c->factors_resident = false;
+    if (sub_on(c)) free_batch(c);  // the forwards do not run on the band: its buffers go back
     // ---- CRMod Jacobian: tensor cores or SIMT
     if (sens_tc_supported(P, 0)) {
         if (!c->d_sens) {
@@ -1451,6 +1757,7 @@ int crgpu_autotune(crgpu_ctx *c, const double *sigma, int32_t flags) {
 int crgpu_set_tune(crgpu_ctx *c, const int32_t *in) {
     if (!c || !in || in[0] < 0 || in[0] > 4 || in[1] < 0 || in[1] > 8 || in[2] < 0 || in[2] > 2) return ERR_ARG;
     drop_graph(c);
+    c->band_pinned = in[0] != 0;
     c->P.tune_factor = in[0];
     c->P.tune_ctas = in[1];
     c->P.tune_sens = in[2];

@@ -7,6 +7,7 @@
 
 #include "crgpu_internal.h"
 #include "kernels.h"
+#include "substruct.h"
 
 struct crgpu_ctx {
     // everything below is owned by the context
@@ -53,7 +54,16 @@ struct crgpu_ctx {
     int graph_refine_used[2] = {};  // refinement steps recorded in the graph per counter array
     int64_t mem_budget = 0;
     bool have_forward = false;
-    bool factors_resident = false;  // band factors of every system still in Bmax (one batch)
+    bool factors_resident = false;  // factors of every system still on the device (one batch)
+    bool factors_sub = false;       // ... those of the substructured solver (else the band factors in Bmax)
+    // substructured solver (substruct.cu): plan, shared factor, batch rectangle
+    bool sub_fits = false;     // the plan exists and costs less than the band
+    bool band_pinned = false;  // crgpu_set_tune asked for a band kernel
+    crgpu::SubPlan sp;
+    crgpu::DevSub D{};
+    crgpu::SubBatch SB{};
+    bool sub_shared = false;   // D's numeric arrays are allocated
+    int sub_cap = 0;           // systems SB's buffers hold
     // adjoint
     double2 *d_lambda = nullptr, *d_adjsrc = nullptr, *d_adjg = nullptr, *d_adjgrad = nullptr;
     const int32_t *d_ebnd_ptr = nullptr, *d_ebnd_list = nullptr;  // element -> mixed boundary elements

@@ -1,0 +1,61 @@
+// Elimination plan of the substructured solver (substruct.cu): which nodes
+// are eliminated once per wavenumber for all current electrodes, in which
+// order, and where every piece lives.
+#pragma once
+
+#include <cstdint>
+#include <vector>
+
+#include "crgpu_internal.h"
+
+namespace crgpu {
+
+// One front: e nodes eliminated here, r nodes it is coupled to (eliminated
+// later, or root nodes).  Local rows 0..e-1 are positions nd0..nd0+e-1, rows
+// e..e+r-1 the positions rows[rows0 .. rows0+r-1].
+struct SubFront {
+    int32_t e, r, nd0;
+    int32_t ch0, ch1;     // children (-1: none)
+    int32_t ent0, nent;   // matrix entries assembled here
+    int32_t rows0;        // into SubPlan::rows
+    int32_t inv0, inv1;   // into SubPlan::inv: local row -> row of the child's r rows, or -1
+    int32_t u0;           // first row of this front's update vectors
+    int32_t pad;
+    int64_t oF, oG, oS;   // inverse pivot block (e x e), G (e x r), Schur complement (r x r)
+};
+
+struct SubEnt {
+    int32_t p, lr, lc;    // lower-pattern entry and its local row (eliminated) and column
+};
+
+struct SubTile {
+    int32_t front, ti, tj;
+};
+
+constexpr int kSubTile = 32;   // tile edge of the dense kernels
+constexpr int kSubEMax = 64;   // most nodes one front eliminates
+
+struct SubPlan {
+    int n = 0, m = 0, nI = 0, nfront = 0, nlevel = 0;
+    std::vector<int32_t> pos, node;            // node -> position, position -> node
+    std::vector<SubFront> fronts;              // by level
+    std::vector<int32_t> level;                // nlevel + 1: first front of a level
+    std::vector<int32_t> rows, inv;
+    std::vector<SubEnt> ent;                   // of the fronts, then (from root_ent0) of the root
+    int root_ent0 = 0, root_child = -1;
+    std::vector<int32_t> root_inv;             // root row -> row of the last front's r rows, or -1
+    std::vector<int32_t> root_bptr;            // mixed-boundary terms of the root entries, by root column:
+    std::vector<SubEnt> root_bnd;              // (boundary line << 4 | imn, row, column)
+    // tiles of the four dense products, by level
+    std::vector<SubTile> tG, tS, tU, tD;
+    std::vector<int32_t> lG, lS, lU, lD;       // nlevel + 1 each
+    int64_t szF = 0, szG = 0, szS = 0;         // entries per wavenumber
+    int32_t szU = 0;                           // update rows per wavenumber
+    double c_factor = 0, c_apply = 0;          // complex multiply-adds: factor per wavenumber, one solve
+};
+
+// The plan for the grid, or false where it has no root (no mixed boundary)
+// or no interior.
+bool build_sub_plan(const HostGrid &hg, const Pattern &pat, SubPlan &sp);
+
+}  // namespace crgpu

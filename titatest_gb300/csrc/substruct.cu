@@ -1,0 +1,1052 @@
+// Substructured solver of the (wavenumber, electrode) systems of src/fem.f90:
+// 355-397 (src/kompab.f90, src/chol.f90, src/vre.f90).
+//
+// Of a wavenumber's matrix only the entries among the nodes of the mixed
+// boundary depend on the electrode (src/beta.f90).  Every other node is
+// eliminated once per wavenumber, by nested dissection (sub_plan.cpp): a
+// front's pivot block is inverted, G = F11^-1 F12, and S = F22 - F12^T G goes
+// to its parent.  What remains is one dense complex symmetric matrix per
+// system over the m boundary nodes, the wavenumber's Schur complement plus the
+// electrode's boundary terms, which is factored C C^T as src/chol.f90 does.  A
+// solve runs up the tree (all electrodes as columns of dense products),
+// through the root, and down again.
+//
+// Config 2 (12261 nodes, 13 wavenumbers x 96 electrodes, m = 321): 3.9e7
+// complex multiply-adds a wavenumber for the shared part and 5.5e6 a system
+// for the root, against 2.4e7 a system for the band of 62 and 9.0e7 for the
+// grid's band of 121; and 0.4 MB of root factor a system instead of 6.2 (12).
+#include <algorithm>
+#include <mutex>
+
+#include "async.cuh"
+#include "kernels.h"
+#include "substruct.h"
+
+namespace crgpu {
+
+namespace {
+
+// ---------------------------------------------------------------- arithmetic
+__device__ __forceinline__ void fma_(float2 &s, float2 a, float2 b) {
+    s.x = fmaf(a.x, b.x, s.x);
+    s.x = fmaf(-a.y, b.y, s.x);
+    s.y = fmaf(a.x, b.y, s.y);
+    s.y = fmaf(a.y, b.x, s.y);
+}
+__device__ __forceinline__ void fma_(double2 &s, double2 a, double2 b) {
+    s.x = fma(a.x, b.x, s.x);
+    s.x = fma(-a.y, b.y, s.x);
+    s.y = fma(a.x, b.y, s.y);
+    s.y = fma(a.y, b.x, s.y);
+}
+__device__ __forceinline__ void fms_(float2 &s, float2 a, float2 b) { s = cfmsf(s, a, b); }
+__device__ __forceinline__ void fms_(double2 &s, double2 a, double2 b) { s = cfms(s, a, b); }
+__device__ __forceinline__ float2 mul_(float2 a, float2 b) { return cmulf(a, b); }
+__device__ __forceinline__ double2 mul_(double2 a, double2 b) { return cmul(a, b); }
+__device__ __forceinline__ float2 rcp_(float2 a) { return crecipf(a); }
+__device__ __forceinline__ double2 rcp_(double2 a) { return crecip(a); }
+__device__ __forceinline__ float2 sqrt_(float2 a) { return csqrtf_(a); }
+__device__ __forceinline__ double2 sqrt_(double2 a) { return csqrtd(a); }
+__device__ __forceinline__ float2 neg_(float2 a) { return cf(-a.x, -a.y); }
+__device__ __forceinline__ double2 neg_(double2 a) { return cz(-a.x, -a.y); }
+template <typename T>
+__device__ __forceinline__ T from_(double2 v);
+template <>
+__device__ __forceinline__ float2 from_<float2>(double2 v) {
+    return to_f(v);
+}
+template <>
+__device__ __forceinline__ double2 from_<double2>(double2 v) {
+    return v;
+}
+template <typename T>
+__device__ __forceinline__ T shfl_(T v, int src) {
+    v.x = __shfl_sync(0xffffffffu, v.x, src);
+    v.y = __shfl_sync(0xffffffffu, v.y, src);
+    return v;
+}
+template <typename T>
+__device__ __forceinline__ T warp_sum_(T v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+        v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+    }
+    return v;
+}
+template <typename T>
+__device__ __forceinline__ T zero_() {
+    T z;
+    z.x = 0;
+    z.y = 0;
+    return z;
+}
+__device__ __forceinline__ bool is_bad(float2 v) { return !(isfinite(v.x) && isfinite(v.y)) || (v.x == 0.f && v.y == 0.f); }
+__device__ __forceinline__ bool is_bad(double2 v) { return !(isfinite(v.x) && isfinite(v.y)) || (v.x == 0.0 && v.y == 0.0); }
+
+// four consecutive entries at a 16-byte boundary of shared memory
+__device__ __forceinline__ void load4(const float2 *p, float2 (&v)[4]) {
+    const float4 a = *(const float4 *)p, b = *(const float4 *)(p + 2);
+    v[0] = cf(a.x, a.y);
+    v[1] = cf(a.z, a.w);
+    v[2] = cf(b.x, b.y);
+    v[3] = cf(b.z, b.w);
+}
+__device__ __forceinline__ void load4(const double2 *p, double2 (&v)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) v[i] = p[i];
+}
+
+// 4 x 4 outer products of a 32 (or 64) x 32 tile: rows r0.., columns c0.. of
+// k-major operands
+template <typename T, int PA, int PB>
+__device__ __forceinline__ void tile_fma(const T *A, const T *Bm, int kk, int r0, int c0, T (&acc)[4][4]) {
+#pragma unroll 4
+    for (int q = 0; q < kk; q++) {
+        T a[4], b[4];
+        load4(A + q * PA + r0, a);
+        load4(Bm + q * PB + c0, b);
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) fma_(acc[i][j], a[i], b[j]);
+    }
+}
+
+constexpr int kT = kSubTile;      // 32
+constexpr int kP = kSubTile + 2;  // padded row of an operand tile (16-byte aligned rows)
+
+// ------------------------------------------------------- values and scaling
+// fk: 1/sqrt|diagonal of the area part| (1 on Dirichlet rows); a zero
+// diagonal is error 27 (src/scalab.f90:57-61).  A boundary node whose area
+// part alone is zero while its boundary terms are not keeps scale 1.
+__global__ void k_sub_scale(DevProblem P, DevSub D, const double2 *__restrict__ sigma,
+                            const double *__restrict__ fak_area) {
+    const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= (size_t)P.K * P.n) return;
+    const int k = (int)(g / P.n), i = (int)(g % P.n);
+    double f = fak_area[g];
+    if (P.dirichlet[i]) {
+        f = 1.0;
+    } else if (!(f > 0.0)) {
+        f = 1.0;
+        bool some = false;
+        for (int p = P.rowptr[i]; p < P.rowptr[i + 1]; p++)
+            if (P.col[p] == i)
+                for (int q = P.bnd_ptr[p]; q < P.bnd_ptr[p + 1]; q++) {
+                    const double2 s = sigma[P.brnr[P.bnd_list[q] >> 4]];
+                    some = some || s.x != 0.0 || s.y != 0.0;
+                }
+        if (!some) atomicCAS(&D.kbad[k], 0, 27);
+    }
+    D.fk[g] = f;
+}
+
+__global__ void k_sub_values(DevProblem P, DevSub D, const double2 *__restrict__ adom) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
+    if (p >= P.nnz) return;
+    const int c = P.col[p];
+    double2 v = cz(0.0, 0.0);
+    if (c >= 0) {
+        const int i = P.row[p];
+        if (P.dirichlet[i] || P.dirichlet[c]) {
+            v = i == c ? cz(1.0, 0.0) : cz(0.0, 0.0);
+        } else {
+            const double f = D.fk[(size_t)k * P.n + i] * D.fk[(size_t)k * P.n + c];
+            const double2 a = adom[(size_t)k * P.nnz + p];
+            v = cz(a.x * f, a.y * f);
+        }
+    }
+    D.As[(size_t)k * P.nnz + p] = v;
+}
+
+// the mixed-boundary terms of one entry (rows i, c), scaled by fk
+__device__ __forceinline__ double2 boundary_term(const DevProblem &P, const double *__restrict__ kgl,
+                                                 const double *__restrict__ fk, const double2 *__restrict__ sigma,
+                                                 int code, int i, int c) {
+    const int rb = code >> 4, imn = code & 15;
+    const double f = P.relbg[rb * 3 + imn] * kgl[rb] * fk[i] * fk[c];
+    const double2 s = sigma[P.brnr[rb]];
+    return cz(f * s.x, f * s.y);
+}
+
+// ------------------------------------------------------------ shared factor
+// Assembles a front's F11 (shared memory) and F12 (D.H) from its children's
+// Schur complements and its matrix entries and inverts F11.  The inverse is
+// symmetric up to the sign between swept and unswept rows (Gauss-Jordan
+// sweeps), so only the lower triangle is computed, each entry in a register of
+// its thread; per sweep the pivot row is published twice, raw and divided by
+// the pivot.
+template <typename T, int NT, int NE>
+__global__ __launch_bounds__(NT) void k_sub_pivot(DevSub D, int f0, int nnz) {
+    extern __shared__ __align__(16) unsigned char sm[];
+    T *Fm = (T *)sm;
+    __shared__ T s_raw[2][kSubEMax], s_div[kSubEMax], s_inv[2];
+    const SubFront t = D.fr[f0 + blockIdx.x];
+    const int k = blockIdx.y, e = t.e, r = t.r, ld = e | 1, tid = threadIdx.x;
+    const T *Sk = (const T *)D.S + (size_t)k * D.szS;
+    const double2 *As = D.As + (size_t)k * nnz;
+    T *H = (T *)D.H + (size_t)k * D.szG + t.oG;
+    const SubFront *c0 = t.ch0 >= 0 ? &D.fr[t.ch0] : nullptr, *c1 = t.ch1 >= 0 ? &D.fr[t.ch1] : nullptr;
+    const int r0 = c0 ? c0->r : 0, r1 = c1 ? c1->r : 0;
+    const T *S0 = c0 ? Sk + c0->oS : nullptr, *S1 = c1 ? Sk + c1->oS : nullptr;
+    const int32_t *i0 = D.inv + t.inv0, *i1 = D.inv + t.inv1;
+    auto gathered = [&](int a, int b) {
+        T v = zero_<T>();
+        if (S0) {
+            const int x = i0[a], y = i0[b];
+            if (x >= 0 && y >= 0) v = S0[(size_t)x * r0 + y];
+        }
+        if (S1) {
+            const int x = i1[a], y = i1[b];
+            if (x >= 0 && y >= 0) {
+                const T w = S1[(size_t)x * r1 + y];
+                v.x += w.x;
+                v.y += w.y;
+            }
+        }
+        return v;
+    };
+    for (int q = tid; q < e * e; q += NT) Fm[(q / e) * ld + q % e] = gathered(q / e, q % e);
+    for (int q = tid; q < e * r; q += NT) H[q] = gathered(q / r, e + q % r);
+    __syncthreads();
+    for (int q = tid; q < t.nent; q += NT) {
+        const SubEnt en = D.ent[t.ent0 + q];
+        const T v = from_<T>(As[en.p]);
+        if (en.lc < e) {  // the lower triangle is read below
+            T &d = Fm[en.lc * ld + en.lr];
+            d.x += v.x;
+            d.y += v.y;
+        } else {
+            T &d = H[(size_t)en.lr * r + en.lc - e];
+            d.x += v.x;
+            d.y += v.y;
+        }
+    }
+    __syncthreads();
+    // entries of this thread: q = tid + z NT of the lower triangle, row by row
+    T w[NE];
+    int ri[NE], ci[NE];
+    const int cnt = e * (e + 1) / 2;
+#pragma unroll
+    for (int z = 0; z < NE; z++) {
+        const int q = tid + z * NT;
+        int i = -1, j = -1;
+        w[z] = zero_<T>();
+        if (q < cnt) {
+            i = (int)((sqrtf(8.f * (float)q + 1.f) - 1.f) * 0.5f);
+            while (i * (i + 1) / 2 > q) i--;
+            while ((i + 1) * (i + 2) / 2 <= q) i++;
+            j = q - i * (i + 1) / 2;
+            w[z] = Fm[i * ld + j];
+        }
+        ri[z] = i;
+        ci[z] = j;
+    }
+    bool bad = false;
+    auto publish = [&](int p, int buf) {
+#pragma unroll
+        for (int z = 0; z < NE; z++) {
+            if (ri[z] == p) s_raw[buf][ci[z]] = w[z];
+            else if (ci[z] == p) s_raw[buf][ri[z]] = w[z];
+            if (ri[z] == p && ci[z] == p) {
+                if (is_bad(w[z])) bad = true;
+                s_inv[buf] = rcp_(w[z]);
+            }
+        }
+    };
+    if (e > 0) publish(0, 0);
+    for (int p = 0; p < e; p++) {
+        const int buf = p & 1;
+        __syncthreads();
+        if (tid < e) s_div[tid] = mul_(s_raw[buf][tid], s_inv[buf]);
+        __syncthreads();
+#pragma unroll
+        for (int z = 0; z < NE; z++) {
+            const int i = ri[z], j = ci[z];
+            if (i < 0) continue;
+            if (i == p) {
+                w[z] = j == p ? s_inv[buf] : s_div[j];
+            } else if (j == p) {
+                w[z] = neg_(s_div[i]);
+            } else {
+                // column entry (i, p): minus the stored one where row i is swept already
+                T u = s_raw[buf][i];
+                if (i < p) u = neg_(u);
+                fms_(w[z], u, s_div[j]);
+            }
+        }
+        if (p + 1 < e) publish(p + 1, buf ^ 1);
+    }
+    T *F = (T *)D.F + (size_t)k * D.szF + t.oF;
+#pragma unroll
+    for (int z = 0; z < NE; z++)
+        if (ri[z] >= 0) {
+            F[ri[z] * e + ci[z]] = w[z];
+            F[ci[z] * e + ri[z]] = w[z];
+        }
+    if (bad) atomicCAS(&D.kbad[k], 0, 28);
+}
+
+// 32 rows of `rows` x 32 columns from src (row stride ls) into dst[row][col]
+template <typename T>
+__device__ __forceinline__ void load_tile(T *dst, const T *src, size_t ls, int nr, int nc) {
+    for (int q = threadIdx.x; q < kT * kT; q += 64) {
+        const int a = q / kT, b = q % kT;
+        dst[a * kP + b] = a < nr && b < nc ? src[(size_t)a * ls + b] : zero_<T>();
+    }
+}
+
+// G = F11^-1 F12
+template <typename T>
+__global__ __launch_bounds__(64) void k_sub_g(DevSub D, int t0) {
+    __shared__ __align__(16) T A[kT * kP], Bm[kT * kP];
+    const SubTile tl = D.tG[t0 + blockIdx.x];
+    const SubFront t = D.fr[tl.front];
+    const int k = blockIdx.y, e = t.e, r = t.r, i0 = tl.ti * kT, j0 = tl.tj * kT;
+    const T *F = (const T *)D.F + (size_t)k * D.szF + t.oF, *H = (const T *)D.H + (size_t)k * D.szG + t.oG;
+    T acc[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++) acc[a][b] = zero_<T>();
+    const int tr = (threadIdx.x >> 3) * 4, tc = (threadIdx.x & 7) * 4;
+    for (int p = 0; p < e; p += kT) {
+        const int kk = min(kT, e - p);
+        load_tile(A, F + (size_t)p * e + i0, e, kk, e - i0);  // symmetric: F[p][i]
+        load_tile(Bm, H + (size_t)p * r + j0, r, kk, r - j0);
+        __syncthreads();
+        tile_fma<T, kP, kP>(A, Bm, kk, tr, tc, acc);
+        __syncthreads();
+    }
+    T *G = (T *)D.G + (size_t)k * D.szG + t.oG;
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++)
+            if (i0 + tr + a < e && j0 + tc + b < r) G[(size_t)(i0 + tr + a) * r + j0 + tc + b] = acc[a][b];
+}
+
+// S = (children's complements) - F12^T G, lower tiles, mirrored
+template <typename T>
+__global__ __launch_bounds__(64) void k_sub_s(DevSub D, int t0) {
+    __shared__ __align__(16) T A[kT * kP], Bm[kT * kP];
+    const SubTile tl = D.tS[t0 + blockIdx.x];
+    const SubFront t = D.fr[tl.front];
+    const int k = blockIdx.y, e = t.e, r = t.r, i0 = tl.ti * kT, j0 = tl.tj * kT;
+    const T *H = (const T *)D.H + (size_t)k * D.szG + t.oG, *G = (const T *)D.G + (size_t)k * D.szG + t.oG;
+    T *Sk = (T *)D.S + (size_t)k * D.szS, *S = Sk + t.oS;
+    T acc[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++) acc[a][b] = zero_<T>();
+    const int tr = (threadIdx.x >> 3) * 4, tc = (threadIdx.x & 7) * 4;
+    for (int p = 0; p < e; p += kT) {
+        const int kk = min(kT, e - p);
+        load_tile(A, H + (size_t)p * r + i0, r, kk, r - i0);
+        load_tile(Bm, G + (size_t)p * r + j0, r, kk, r - j0);
+        __syncthreads();
+        tile_fma<T, kP, kP>(A, Bm, kk, tr, tc, acc);
+        __syncthreads();
+    }
+    const SubFront *c0 = t.ch0 >= 0 ? &D.fr[t.ch0] : nullptr, *c1 = t.ch1 >= 0 ? &D.fr[t.ch1] : nullptr;
+    const int r0 = c0 ? c0->r : 0, r1 = c1 ? c1->r : 0;
+    const T *S0 = c0 ? Sk + c0->oS : nullptr, *S1 = c1 ? Sk + c1->oS : nullptr;
+    const int32_t *m0 = D.inv + t.inv0 + e, *m1 = D.inv + t.inv1 + e;
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+            const int i = i0 + tr + a, j = j0 + tc + b;
+            if (i >= r || j > i) continue;
+            T v = neg_(acc[a][b]);
+            if (S0) {
+                const int x = m0[i], y = m0[j];
+                if (x >= 0 && y >= 0) {
+                    const T w = S0[(size_t)x * r0 + y];
+                    v.x += w.x;
+                    v.y += w.y;
+                }
+            }
+            if (S1) {
+                const int x = m1[i], y = m1[j];
+                if (x >= 0 && y >= 0) {
+                    const T w = S1[(size_t)x * r1 + y];
+                    v.x += w.x;
+                    v.y += w.y;
+                }
+            }
+            S[(size_t)i * r + j] = v;
+            S[(size_t)j * r + i] = v;
+        }
+}
+
+// the root's shared part, column-major lower, padded by a unit diagonal:
+// the last front's complement, then the area entries among root nodes
+template <typename T>
+__global__ void k_sub_root_base(DevSub D) {
+    const int c = blockIdx.x, k = blockIdx.y;
+    const T *S = (const T *)D.S + (size_t)k * D.szS + D.root_oS;
+    T *R = (T *)D.R + ((size_t)k * D.mp + c) * D.ldc;
+    const int y = c < D.m ? D.root_inv[c] : -1;
+    for (int i = threadIdx.x; i < D.ldc; i += blockDim.x) {
+        T v = zero_<T>();
+        if (i < D.m && y >= 0) {
+            const int x = D.root_inv[i];
+            if (x >= 0) v = S[(size_t)x * D.root_r + y];
+        }
+        if (i == c && c >= D.m) v.x = 1;
+        R[i] = v;
+    }
+}
+
+template <typename T>
+__global__ void k_sub_root_ent(DevSub D, int nnz) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
+    if (q >= D.n_root_ent) return;
+    const SubEnt en = D.ent[D.root_ent0 + q];
+    const T v = from_<T>(D.As[(size_t)k * nnz + en.p]);
+    T &d = ((T *)D.R)[((size_t)k * D.mp + en.lc) * D.ldc + en.lr];
+    d.x += v.x;
+    d.y += v.y;
+}
+
+// ------------------------------------------------------------- root factor
+// C C^T of one system's root, column-major lower with leading dimension ldc,
+// one block per system, left-looking in 32-column blocks.  A block's rows are
+// worked in tiles of 64: W = M - C C_j^T from the finished columns (cp.async,
+// two chunks of 16 columns in flight), then W C_jj^-T.  The diagonal block is
+// factored and inverted together, one barrier a column; its inverse is stored
+// in its place, which is all that the later solves need.
+constexpr int kRT = 128;   // threads
+constexpr int kRows = 64;  // rows of a tile
+constexpr int kKC = 16;    // columns of a chunk
+
+template <typename T>
+__global__ __launch_bounds__(kRT) void k_sub_root(DevProblem P, DevSub D, SubBatch B,
+                                                  const double2 *__restrict__ sigma) {
+    extern __shared__ __align__(16) unsigned char sm[];
+    constexpr int PX = 34;
+    T *As = (T *)sm;                   // [2][kKC][kRows]; also W of a tile, [32][kRows]
+    T *Bs = As + 2 * kKC * kRows;      // [2][kKC][32]
+    T *Ci = Bs + 2 * kKC * 32;         // [32][PX]: Ci[a][b] = inverse(b, a)
+    __shared__ T col[2][32], inv[2];
+    const int s = blockIdx.x, kk_ = s / B.Lb, k = B.k0 + kk_, l = B.l0 + s % B.Lb;
+    const int mp = D.mp, ldc = D.ldc, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    T *C = (T *)B.C + (size_t)s * mp * ldc;
+    const T *R = (const T *)D.R + (size_t)k * mp * ldc;
+    const double *kgl = P.kg + ((size_t)k * P.eanz + l) * P.relanz;
+    const double *fk = D.fk + (size_t)k * P.n;
+    const int32_t *rnode = D.node + D.nI;
+    const int tr = (tid >> 3) * 4, tc = (tid & 7) * 4;
+    bool bad = false;
+    // pivot-column data of a 32-column block: rows r0.., this thread's 4 x 4 of W
+    for (int j = 0; j < mp; j += 32) {
+        for (int r0 = j; r0 < mp; r0 += kRows) {
+            T acc[4][4];
+#pragma unroll
+            for (int a = 0; a < 4; a++)
+#pragma unroll
+                for (int b = 0; b < 4; b++) acc[a][b] = zero_<T>();
+            const int nch = j / kKC;
+            auto fetch = [&](int ch) {
+                T *a = As + (ch & 1) * kKC * kRows, *b = Bs + (ch & 1) * kKC * 32;
+                constexpr int per = 16 / sizeof(T);
+                for (int q = tid; q < kKC * kRows / per; q += kRT) {
+                    const int c = q / (kRows / per), o = (q % (kRows / per)) * per;
+                    // rows beyond the matrix are not stored: any rows of the column do
+                    const int row = min(r0 + o, ldc - per);
+                    cp_async16(a + c * kRows + o, C + (size_t)(ch * kKC + c) * ldc + row);
+                }
+                for (int q = tid; q < kKC * 32 / per; q += kRT) {
+                    const int c = q / (32 / per), o = (q % (32 / per)) * per;
+                    cp_async16(b + c * 32 + o, C + (size_t)(ch * kKC + c) * ldc + j + o);
+                }
+                cp_commit();
+            };
+            if (nch > 0) fetch(0);
+            for (int ch = 0; ch < nch; ch++) {
+                if (ch + 1 < nch) {
+                    fetch(ch + 1);
+                    cp_wait<1>();
+                } else {
+                    cp_wait<0>();
+                }
+                __syncthreads();
+                tile_fma<T, kRows, 32>(As + (ch & 1) * kKC * kRows, Bs + (ch & 1) * kKC * 32, kKC, tr, tc, acc);
+                __syncthreads();
+            }
+            // W = M - sum, M the wavenumber's part; the electrode's terms follow in shared memory
+#pragma unroll
+            for (int b = 0; b < 4; b++) {
+                const int c = j + tc + b;
+#pragma unroll
+                for (int a = 0; a < 4; a++) {
+                    const int i = min(r0 + tr + a, ldc - 1);
+                    const T m = R[(size_t)c * ldc + i];
+                    As[(tc + b) * kRows + tr + a].x = m.x - acc[a][b].x;
+                    As[(tc + b) * kRows + tr + a].y = m.y - acc[a][b].y;
+                }
+            }
+            __syncthreads();
+            if (tid < 32 && j + tid < D.m) {  // one thread per column: few terms each
+                const int c = j + tid;
+                for (int q = D.root_bptr[c]; q < D.root_bptr[c + 1]; q++) {
+                    const SubEnt en = D.root_bnd[q];
+                    if (en.lr < r0 || en.lr >= r0 + kRows) continue;
+                    const int ni = rnode[en.lr], nc = rnode[c];
+                    if (P.dirichlet[ni] || P.dirichlet[nc]) continue;
+                    const double2 v = boundary_term(P, kgl, fk, sigma, en.p, ni, nc);
+                    T &d = As[tid * kRows + en.lr - r0];
+                    d = from_<T>(cz((double)d.x + v.x, (double)d.y + v.y));
+                }
+            }
+            __syncthreads();
+            if (r0 == j) {
+                // diagonal block: lane = row, warp w the columns w, w + 4, ...
+                T a[8], x[8];
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    a[q] = As[(4 * q + wid) * kRows + lane];
+                    x[q] = zero_<T>();
+                    if (lane == 4 * q + wid) x[q].x = 1;
+                }
+#pragma unroll
+                for (int q = 0; q < 8; q++)
+#pragma unroll
+                    for (int ww = 0; ww < 4; ww++) {
+                        const int p = 4 * q + ww, buf = p & 1;
+                        if (wid == ww) {
+                            const T d = shfl_(a[q], p);
+                            if (is_bad(d)) bad = true;
+                            const T iv = rcp_(sqrt_(d));
+                            col[buf][lane] = lane > p ? mul_(a[q], iv) : zero_<T>();
+                            if (lane == 0) inv[buf] = iv;
+                        }
+                        __syncthreads();
+                        const T cl = col[buf][lane], iv = inv[buf];
+#pragma unroll
+                        for (int z = 0; z < 8; z++) {
+                            const int c = 4 * z + wid;
+                            if (z >= q && c > p) fms_(a[z], cl, col[buf][c]);
+                            if (z <= q) {
+                                const T xp = mul_(shfl_(x[z], p), iv);
+                                if (lane == p) x[z] = xp;
+                                else if (lane > p) fms_(x[z], cl, xp);
+                            }
+                        }
+                    }
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    const int c = 4 * q + wid;
+                    const T v = lane >= c ? x[q] : zero_<T>();
+                    Ci[c * PX + lane] = v;
+                    C[(size_t)(j + c) * ldc + j + lane] = v;
+                }
+                __syncthreads();
+            }
+            // C_ij = W C_jj^-T
+#pragma unroll
+            for (int a = 0; a < 4; a++)
+#pragma unroll
+                for (int b = 0; b < 4; b++) acc[a][b] = zero_<T>();
+            tile_fma<T, kRows, PX>(As, Ci, 32, tr, tc, acc);
+#pragma unroll
+            for (int b = 0; b < 4; b++)
+#pragma unroll
+                for (int a = 0; a < 4; a++) {
+                    const int i = r0 + tr + a;
+                    if (i >= j + 32 && i < mp) C[(size_t)(j + tc + b) * ldc + i] = acc[a][b];
+                }
+            __syncthreads();
+        }
+    }
+    if (D.kbad[k]) {
+        if (tid == 0) atomicCAS(&B.status[s], 0, D.kbad[k]);
+    } else if (bad) {
+        atomicCAS(&B.status[s], 0, 28);
+    }
+}
+
+// ------------------------------------------------------------------- solves
+// x = (C C^T)^-1 u of one system's root, one block per system
+constexpr int kST = 256;
+
+template <typename T>
+__global__ __launch_bounds__(kST) void k_sub_root_solve(DevSub D, SubBatch B, const int *nprev) {
+    extern __shared__ __align__(16) unsigned char sm[];
+    T *v = (T *)sm;            // [mp]
+    __shared__ T t[32];
+    if (nprev && *nprev == 0) return;
+    const int s = blockIdx.x, kk = s / B.Lb, l = s % B.Lb;
+    if (B.kact && !B.kact[kk]) return;
+    const int mp = D.mp, ldc = D.ldc, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const T *C = (const T *)B.C + (size_t)s * mp * ldc;
+    const T *Y = (const T *)B.Y + ((size_t)kk * D.n + D.nI) * B.Lb + l;
+    const T *U = (const T *)B.U + ((size_t)kk * D.szU + D.root_u0) * B.Lb + l;
+    T *Z = (T *)B.Z + ((size_t)kk * D.n + D.nI) * B.Lb + l;
+    for (int i = tid; i < mp; i += kST) {
+        T u = zero_<T>();
+        if (i < D.m) {
+            u = Y[(size_t)i * B.Lb];
+            const int x = D.root_inv[i];
+            if (x >= 0) {
+                const T w = U[(size_t)x * B.Lb];
+                u.x += w.x;
+                u.y += w.y;
+            }
+        }
+        v[i] = u;
+    }
+    __syncthreads();
+    for (int j = 0; j < mp; j += 32) {
+        // y_j = C_jj^-1 v_j: warp w takes 4 columns of the inverse, lane = row
+        T p = zero_<T>();
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int c = wid * 4 + q;
+            if (lane >= c) fma_(p, C[(size_t)(j + c) * ldc + j + lane], v[j + c]);
+        }
+        __shared__ T part[8][33];
+        part[wid][lane] = p;
+        __syncthreads();
+        if (tid < 32) {
+            T y = zero_<T>();
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                y.x += part[q][lane].x;
+                y.y += part[q][lane].y;
+            }
+            v[j + lane] = y;
+            t[lane] = y;
+        }
+        __syncthreads();
+        for (int i = j + 32 + tid; i < mp; i += kST) {
+            T a = v[i];
+#pragma unroll 8
+            for (int c = 0; c < 32; c++) fms_(a, C[(size_t)(j + c) * ldc + i], t[c]);
+            v[i] = a;
+        }
+        __syncthreads();
+    }
+    for (int j = mp - 32; j >= 0; j -= 32) {
+        // t_c = y_c - sum_i C(i, c) x_i: four columns a warp
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int c = wid * 4 + q;
+            T a = zero_<T>();
+            for (int i = j + 32 + lane; i < mp; i += 32) fma_(a, C[(size_t)(j + c) * ldc + i], v[i]);
+            a = warp_sum_(a);
+            if (lane == 0) {
+                t[c].x = v[j + c].x - a.x;
+                t[c].y = v[j + c].y - a.y;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int c = wid * 4 + q;
+            T a = zero_<T>();
+            if (lane >= c) fma_(a, C[(size_t)(j + c) * ldc + j + lane], t[lane]);
+            a = warp_sum_(a);
+            if (lane == 0) v[j + c] = a;
+        }
+        __syncthreads();
+    }
+    for (int i = tid; i < D.m; i += kST) Z[(size_t)i * B.Lb] = v[i];
+}
+
+// Up the tree: b_E (own right-hand sides and the children's updates) goes to
+// W, the update rows U = (children's updates) - G^T b_E to the parent.
+template <typename T>
+__global__ __launch_bounds__(64) void k_sub_up(DevSub D, SubBatch B, int t0, const int *nprev) {
+    __shared__ __align__(16) T A[kT * kP], Bm[kT * kP];
+    if (nprev && *nprev == 0) return;
+    const int kk = blockIdx.z, k = B.k0 + kk;
+    if (B.kact && !B.kact[kk]) return;
+    const SubTile tl = D.tU[t0 + blockIdx.x];
+    const SubFront t = D.fr[tl.front];
+    const int e = t.e, r = t.r, i0 = tl.ti * kT, l0 = blockIdx.y * kT, L = B.Lb, nl = min(kT, L - l0);
+    const T *G = (const T *)D.G + (size_t)k * D.szG + t.oG;
+    const T *Y = (const T *)B.Y + ((size_t)kk * D.n + t.nd0) * L + l0;
+    T *W = (T *)B.W + ((size_t)kk * D.n + t.nd0) * L + l0;
+    T *Uk = (T *)B.U + (size_t)kk * D.szU * L + l0;
+    const T *U0 = t.ch0 >= 0 ? Uk + (size_t)D.fr[t.ch0].u0 * L : nullptr;
+    const T *U1 = t.ch1 >= 0 ? Uk + (size_t)D.fr[t.ch1].u0 * L : nullptr;
+    const int32_t *m0 = D.inv + t.inv0, *m1 = D.inv + t.inv1;
+    auto updates = [&](int row, int c) {
+        T v = zero_<T>();
+        if (U0) {
+            const int x = m0[row];
+            if (x >= 0) v = U0[(size_t)x * L + c];
+        }
+        if (U1) {
+            const int x = m1[row];
+            if (x >= 0) {
+                const T w = U1[(size_t)x * L + c];
+                v.x += w.x;
+                v.y += w.y;
+            }
+        }
+        return v;
+    };
+    T acc[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++) acc[a][b] = zero_<T>();
+    const int tr = (threadIdx.x >> 3) * 4, tc = (threadIdx.x & 7) * 4;
+    for (int p = 0; p < e; p += kT) {
+        const int kc = min(kT, e - p);
+        load_tile(A, G + (size_t)p * r + i0, r, kc, r - i0);
+        for (int q = threadIdx.x; q < kT * kT; q += 64) {
+            const int a = q / kT, c = q % kT;
+            T v = zero_<T>();
+            if (a < kc && c < nl) {
+                v = updates(p + a, c);
+                const T y = Y[(size_t)(p + a) * L + c];
+                v.x += y.x;
+                v.y += y.y;
+                if (tl.ti == 0) W[(size_t)(p + a) * L + c] = v;
+            }
+            Bm[a * kP + c] = v;
+        }
+        __syncthreads();
+        tile_fma<T, kP, kP>(A, Bm, kc, tr, tc, acc);
+        __syncthreads();
+    }
+    T *U = Uk + (size_t)t.u0 * L;
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+        const int i = i0 + tr + a;
+        if (i >= r) continue;
+#pragma unroll
+        for (int b = 0; b < 4; b++)
+            if (tc + b < nl) {
+                T v = updates(e + i, tc + b);
+                v.x -= acc[a][b].x;
+                v.y -= acc[a][b].y;
+                U[(size_t)i * L + tc + b] = v;
+            }
+    }
+}
+
+// Down the tree: x_E = F11^-1 b_E - G x_R
+template <typename T>
+__global__ __launch_bounds__(64) void k_sub_down(DevSub D, SubBatch B, int t0, const int *nprev) {
+    __shared__ __align__(16) T A[kT * kP], Bm[kT * kP];
+    if (nprev && *nprev == 0) return;
+    const int kk = blockIdx.z, k = B.k0 + kk;
+    if (B.kact && !B.kact[kk]) return;
+    const SubTile tl = D.tD[t0 + blockIdx.x];
+    const SubFront t = D.fr[tl.front];
+    const int e = t.e, r = t.r, i0 = tl.ti * kT, l0 = blockIdx.y * kT, L = B.Lb, nl = min(kT, L - l0);
+    const T *F = (const T *)D.F + (size_t)k * D.szF + t.oF, *G = (const T *)D.G + (size_t)k * D.szG + t.oG;
+    const T *W = (const T *)B.W + ((size_t)kk * D.n + t.nd0) * L + l0;
+    T *Zk = (T *)B.Z + (size_t)kk * D.n * L + l0;
+    const int32_t *rows = D.rows + t.rows0;
+    T acc[4][4], acg[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++) acc[a][b] = acg[a][b] = zero_<T>();
+    const int tr = (threadIdx.x >> 3) * 4, tc = (threadIdx.x & 7) * 4;
+    for (int p = 0; p < e; p += kT) {
+        const int kc = min(kT, e - p);
+        load_tile(A, F + (size_t)p * e + i0, e, kc, e - i0);
+        load_tile(Bm, W + (size_t)p * L, L, kc, nl);
+        __syncthreads();
+        tile_fma<T, kP, kP>(A, Bm, kc, tr, tc, acc);
+        __syncthreads();
+    }
+    for (int p = 0; p < r; p += kT) {
+        const int kc = min(kT, r - p);
+        for (int q = threadIdx.x; q < kT * kT; q += 64) {
+            const int a = q / kT, c = q % kT;  // A[column of G][row]: read along the row of G
+            A[c * kP + a] = i0 + a < e && c < kc ? G[(size_t)(i0 + a) * r + p + c] : zero_<T>();
+            Bm[a * kP + c] = a < kc && c < nl ? Zk[(size_t)rows[p + a] * L + c] : zero_<T>();
+        }
+        __syncthreads();
+        tile_fma<T, kP, kP>(A, Bm, kc, tr, tc, acg);
+        __syncthreads();
+    }
+    T *Z = Zk + (size_t)t.nd0 * L;
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++)
+            if (i0 + tr + a < e && tc + b < nl) {
+                T v = acc[a][b];
+                v.x -= acg[a][b].x;
+                v.y -= acg[a][b].y;
+                Z[(size_t)(i0 + tr + a) * L + tc + b] = v;
+            }
+}
+
+// -------------------------------------------------- vectors of a rectangle
+// Right-hand sides, scaled by fk: the unit sink at the electrode and the
+// fictitious sink (src/kompab.f90:180-190), or the rows of src ([eanz][n]).
+template <typename T>
+__global__ void k_sub_rhs(DevProblem P, DevSub D, SubBatch B, int lsink, int nsink,
+                          const double2 *__restrict__ src, int keep) {
+    const int l = blockIdx.y * 32 + (threadIdx.x & 31), p = blockIdx.x * 8 + (threadIdx.x >> 5), kk = blockIdx.z;
+    if (l >= B.Lb || p >= D.n) return;
+    const int i = D.node[p], el = B.l0 + l;
+    double2 v = cz(0.0, 0.0);
+    if (src) v = src[(size_t)el * P.n + i];
+    else {
+        if (i == P.enr0[el]) v = cz(-1.0, 0.0);
+        if (lsink && i == nsink) v = cz(1.0, 0.0);
+    }
+    if (P.dirichlet[i]) v = cz(0.0, 0.0);
+    const double f = D.fk[(size_t)(B.k0 + kk) * P.n + i];
+    v = cz(v.x * f, v.y * f);
+    const size_t at = ((size_t)kk * D.n + p) * B.Lb + l;
+    if (keep) B.Bt[at] = v;
+    ((T *)B.Y)[at] = from_<T>(v);
+}
+
+// Y = b - A x in FP64 (rounded to complex64 at the end): one warp per row, the
+// electrodes across its lanes, so the matrix entries are one broadcast load.
+__global__ __launch_bounds__(256) void k_sub_residual(DevProblem P, DevSub D, SubBatch B,
+                                                      const double2 *__restrict__ sigma, const int *nprev) {
+    if (nprev && *nprev == 0) return;
+    const int kk = blockIdx.z, k = B.k0 + kk, L = B.Lb;
+    if (!B.kact[kk]) return;
+    const int l = blockIdx.y * 32 + (threadIdx.x & 31), p = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (l >= L || p >= D.n) return;
+    const int i = D.node[p];
+    const double2 *As = D.As + (size_t)k * P.nnz;
+    const double2 *X = B.X + (size_t)kk * D.n * L + l;
+    double2 acc = cz(0.0, 0.0);
+    for (int q = P.fptr[i]; q < P.fptr[i + 1]; q++) fma_(acc, As[P.fidx[q]], X[(size_t)D.fcolpos[q] * L]);
+    if (p >= D.nI && !P.dirichlet[i]) {
+        const double *kgl = P.kg + ((size_t)k * P.eanz + B.l0 + l) * P.relanz, *fk = D.fk + (size_t)k * P.n;
+        for (int q = P.fptr[i]; q < P.fptr[i + 1]; q++) {
+            const int e = P.fidx[q], c = P.fcol[q];
+            if (P.dirichlet[c]) continue;
+            for (int z = P.bnd_ptr[e]; z < P.bnd_ptr[e + 1]; z++)
+                fma_(acc, boundary_term(P, kgl, fk, sigma, P.bnd_list[z], i, c), X[(size_t)D.fcolpos[q] * L]);
+        }
+    }
+    const size_t at = ((size_t)kk * D.n + p) * L + l;
+    const double2 b = B.Bt[at];
+    ((float2 *)B.Y)[at] = to_f(cz(b.x - acc.x, b.y - acc.y));
+}
+
+constexpr int kAccRows = 256;
+
+// X (+)= Z with the largest entries of both per system
+__global__ __launch_bounds__(256) void k_sub_accumulate(DevSub D, SubBatch B, int first, const int *nprev) {
+    if (nprev && *nprev == 0) return;
+    const int kk = blockIdx.z, L = B.Lb;
+    if (!first && !B.kact[kk]) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, l = blockIdx.y * 32 + lane;
+    const bool on = l < L && (first || B.active[kk * L + l]);
+    double mz = 0.0, mx = 0.0;
+    if (on) {
+        const size_t base = (size_t)kk * D.n * L + l;
+        const int p1 = min(D.n, (int)(blockIdx.x + 1) * kAccRows);
+        for (int p = blockIdx.x * kAccRows + w; p < p1; p += 8) {
+            const size_t at = base + (size_t)p * L;
+            const double2 z = to_d(((const float2 *)B.Z)[at]);
+            double2 x = z;
+            if (!first) {
+                x = B.X[at];
+                x = cz(x.x + z.x, x.y + z.y);
+            }
+            B.X[at] = x;
+            // a NaN wins every later comparison: fmax would drop it
+            const double az = fmax(fabs(z.x), fabs(z.y)), ax = fmax(fabs(x.x), fabs(x.y));
+            mz = (az > mz || z.x != z.x || z.y != z.y) ? (z.x != z.x || z.y != z.y ? INFINITY : az) : mz;
+            mx = ax > mx ? ax : mx;
+        }
+    }
+    __shared__ double sz[8][32], sx[8][32];
+    sz[w][lane] = mz;
+    sx[w][lane] = mx;
+    __syncthreads();
+    if (w == 0 && on) {
+        for (int q = 1; q < 8; q++) {
+            mz = fmax(mz, sz[q][lane]);
+            mx = fmax(mx, sx[q][lane]);
+        }
+        // bit patterns of non-negative doubles order like the values
+        atomicMax(&B.mz[kk * L + l], (unsigned long long)__double_as_longlong(mz));
+        atomicMax(&B.mx[kk * L + l], (unsigned long long)__double_as_longlong(mx));
+    }
+}
+
+// A system stops once its correction is at most tol times its solution; one
+// block per wavenumber counts those that go on.
+__global__ __launch_bounds__(256) void k_sub_stop(SubBatch B, int first, double tol, const int *nprev, int *nactive,
+                                                  double *zmax) {
+    if (nprev && *nprev == 0) return;
+    const int kk = blockIdx.x, L = B.Lb;
+    int count = 0;
+    if (first || B.kact[kk]) {
+        for (int l = threadIdx.x; l < L; l += blockDim.x) {
+            const int s = kk * L + l;
+            const double mz = __longlong_as_double((long long)B.mz[s]), mx = __longlong_as_double((long long)B.mx[s]);
+            B.mz[s] = 0ull;
+            B.mx[s] = 0ull;
+            int act = first ? 1 : B.active[s];
+            if (!act) continue;
+            if (!first && !(mz > tol * mx)) act = 0;
+            if (!first && zmax && mx > 0.0)
+                atomicMax((unsigned long long *)zmax, (unsigned long long)__double_as_longlong(mz / mx));
+            if (!isfinite(mz) || !isfinite(mx)) {
+                atomicCAS(&B.status[s], 0, 28);
+                act = 0;
+            }
+            B.active[s] = act;
+            count += act;
+        }
+    }
+    __shared__ int tot;
+    if (threadIdx.x == 0) tot = 0;
+    __syncthreads();
+    if (count) atomicAdd(&tot, count);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        B.kact[kk] = tot;
+        if (nactive && tot) atomicAdd(nactive, tot);
+    }
+}
+
+// out[k][l][node] = sign fk x (src/fem.f90:388-389), through shared memory:
+// 32 nodes x 32 electrodes a block; out32 the complex64 hi and lo planes
+template <typename T>
+__global__ __launch_bounds__(256) void k_sub_unpack(DevProblem P, DevSub D, SubBatch B, const T *__restrict__ X,
+                                                    double sign, double2 *out, float2 *out32) {
+    __shared__ double2 tile[32][33];
+    const int kk = blockIdx.z, k = B.k0 + kk, n0 = blockIdx.x * 32, l0 = blockIdx.y * 32;
+    const int a = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int q = w; q < 32; q += 8)
+        if (n0 + q < D.n && l0 + a < B.Lb)
+            tile[q][a] = B.X[((size_t)kk * D.n + D.pos[n0 + q]) * B.Lb + l0 + a];
+    __syncthreads();
+    if (n0 + a >= D.n) return;
+    const double f = sign * D.fk[(size_t)k * P.n + n0 + a];
+    for (int q = w; q < 32; q += 8) {
+        if (l0 + q >= B.Lb) continue;
+        const double2 x = tile[a][q], v = cz(x.x * f, x.y * f);
+        const size_t at = ((size_t)k * P.eanz + B.l0 + l0 + q) * P.n + n0 + a;
+        out[at] = v;
+        if (out32) {
+            const float2 hi = to_f(v);
+            out32[at] = hi;
+            out32[at + (size_t)P.K * P.eanz * P.n] = cf((float)(v.x - (double)hi.x), (float)(v.y - (double)hi.y));
+        }
+    }
+}
+
+inline unsigned nb(size_t n, int t) { return (unsigned)((n + t - 1) / t); }
+
+template <typename T>
+int factor_t(const DevProblem &P, const DevSub &D, const SubPlan &sp, cudaStream_t st) {
+    static std::once_flag once;
+    std::call_once(once, [] {
+        const int most = (int)sizeof(T) * kSubEMax * (kSubEMax | 1);
+        cudaFuncSetAttribute(k_sub_pivot<T, 256, 9>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        cudaFuncSetAttribute(k_sub_pivot<T, 128, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    });
+    int launches = 0;
+    for (int lv = 0; lv < sp.nlevel; lv++) {
+        const int f0 = sp.level[lv], nf = sp.level[lv + 1] - f0;
+        int emax = 1;
+        for (int q = f0; q < f0 + nf; q++) emax = std::max(emax, sp.fronts[q].e);
+        const size_t smem = sizeof(T) * emax * (emax | 1);
+        if (emax * (emax + 1) / 2 <= 128 * 5)
+            k_sub_pivot<T, 128, 5><<<dim3(nf, P.K), 128, smem, st>>>(D, f0, P.nnz);
+        else
+            k_sub_pivot<T, 256, 9><<<dim3(nf, P.K), 256, smem, st>>>(D, f0, P.nnz);
+        const int ng = sp.lG[lv + 1] - sp.lG[lv], ns = sp.lS[lv + 1] - sp.lS[lv];
+        if (ng) k_sub_g<T><<<dim3(ng, P.K), 64, 0, st>>>(D, sp.lG[lv]);
+        if (ns) k_sub_s<T><<<dim3(ns, P.K), 64, 0, st>>>(D, sp.lS[lv]);
+        launches += 1 + (ng > 0) + (ns > 0);
+    }
+    k_sub_root_base<T><<<dim3(D.mp, P.K), 128, 0, st>>>(D);
+    if (D.n_root_ent) k_sub_root_ent<T><<<dim3(nb(D.n_root_ent, 128), P.K), 128, 0, st>>>(D, P.nnz);
+    return launches + 2;
+}
+
+template <typename T>
+size_t root_smem() {
+    return sizeof(T) * (2 * kKC * kRows + 2 * kKC * 32 + 32 * 34);
+}
+
+template <typename T>
+void root_t(const DevProblem &P, const DevSub &D, const SubBatch &B, const double2 *sigma, cudaStream_t st) {
+    static std::once_flag once;
+    std::call_once(once, [] {
+        cudaFuncSetAttribute(k_sub_root<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)root_smem<T>());
+    });
+    k_sub_root<T><<<B.Kb * B.Lb, kRT, root_smem<T>(), st>>>(P, D, B, sigma);
+}
+
+template <typename T>
+int apply_t(const DevSub &D, const SubPlan &sp, const SubBatch &B, const int *nprev, cudaStream_t st) {
+    const int lt = (B.Lb + kT - 1) / kT;
+    for (int lv = 0; lv < sp.nlevel; lv++)
+        k_sub_up<T><<<dim3(sp.lU[lv + 1] - sp.lU[lv], lt, B.Kb), 64, 0, st>>>(D, B, sp.lU[lv], nprev);
+    k_sub_root_solve<T><<<B.Kb * B.Lb, kST, sizeof(T) * D.mp, st>>>(D, B, nprev);
+    int launches = sp.nlevel + 1;
+    for (int lv = sp.nlevel - 1; lv >= 0; lv--) {
+        const int nd = sp.lD[lv + 1] - sp.lD[lv];
+        if (!nd) continue;
+        k_sub_down<T><<<dim3(nd, lt, B.Kb), 64, 0, st>>>(D, B, sp.lD[lv], nprev);
+        launches++;
+    }
+    return launches;
+}
+
+}  // namespace
+
+void sub_launch_values(const DevProblem &P, const DevSub &D, const double2 *sigma, const double2 *adom,
+                       cudaStream_t st) {
+    cudaMemsetAsync(D.kbad, 0, sizeof(int) * P.K, st);
+    const double *fak_area = (const double *)(adom + (size_t)P.K * P.nnz);
+    k_sub_scale<<<nb((size_t)P.K * P.n, 256), 256, 0, st>>>(P, D, sigma, fak_area);
+    k_sub_values<<<dim3(nb(P.nnz, 256), P.K), 256, 0, st>>>(P, D, adom);
+}
+
+int sub_launch_factor(const DevProblem &P, const DevSub &D, const SubPlan &sp, bool mixed, cudaStream_t st) {
+    return mixed ? factor_t<float2>(P, D, sp, st) : factor_t<double2>(P, D, sp, st);
+}
+
+void sub_launch_root(const DevProblem &P, const DevSub &D, const SubBatch &B, const double2 *sigma, bool mixed,
+                     cudaStream_t st) {
+    mixed ? root_t<float2>(P, D, B, sigma, st) : root_t<double2>(P, D, B, sigma, st);
+}
+
+int sub_launch_apply(const DevSub &D, const SubPlan &sp, const SubBatch &B, bool mixed, const int *nprev,
+                     cudaStream_t st) {
+    return mixed ? apply_t<float2>(D, sp, B, nprev, st) : apply_t<double2>(D, sp, B, nprev, st);
+}
+
+void sub_launch_rhs(const DevProblem &P, const DevSub &D, const SubBatch &B, bool mixed, int lsink, int nsink,
+                    const double2 *src, cudaStream_t st) {
+    const dim3 g(nb(D.n, 8), nb(B.Lb, 32), B.Kb);
+    if (mixed) k_sub_rhs<float2><<<g, 256, 0, st>>>(P, D, B, lsink, nsink, src, 1);
+    else k_sub_rhs<double2><<<g, 256, 0, st>>>(P, D, B, lsink, nsink, src, 0);
+}
+
+void sub_launch_residual(const DevProblem &P, const DevSub &D, const SubBatch &B, const double2 *sigma,
+                         const int *nprev, cudaStream_t st) {
+    k_sub_residual<<<dim3(nb(D.n, 8), nb(B.Lb, 32), B.Kb), 256, 0, st>>>(P, D, B, sigma, nprev);
+}
+
+void sub_launch_accumulate(const DevSub &D, const SubBatch &B, bool first, double tol, const int *nprev, int *nactive,
+                           double *zmax, cudaStream_t st) {
+    k_sub_accumulate<<<dim3(nb(D.n, kAccRows), nb(B.Lb, 32), B.Kb), 256, 0, st>>>(D, B, first ? 1 : 0, nprev);
+    k_sub_stop<<<B.Kb, 256, 0, st>>>(B, first ? 1 : 0, tol, nprev, nactive, zmax);
+}
+
+void sub_launch_unpack(const DevProblem &P, const DevSub &D, const SubBatch &B, double sign, double2 *out,
+                       float2 *out32, cudaStream_t st) {
+    k_sub_unpack<double2><<<dim3(nb(D.n, 32), nb(B.Lb, 32), B.Kb), 256, 0, st>>>(P, D, B, B.X, sign, out, out32);
+}
+
+}  // namespace crgpu
