@@ -109,7 +109,7 @@ void free_batch(crgpu_ctx *c) {
 void free_sub_batch(crgpu_ctx *c) {
     drop_graph(c);
     SubBatch &B = c->SB;
-    void *ptrs[] = {B.C,  c->precision == CRGPU_MIXED ? B.X : nullptr, B.Bt, B.Y, B.W, B.Z, B.U, B.status, B.active,
+    void *ptrs[] = {B.C,  B.bval, c->precision == CRGPU_MIXED ? B.X : nullptr, B.Bt, B.Y, B.W, B.Z, B.U, B.status, B.active,
                     B.kact, B.mz};
     for (void *p : ptrs)
         if (p) {
@@ -373,7 +373,7 @@ size_t sub_bytes_per_system(const crgpu_ctx *c) {
     const bool mixed = c->precision == CRGPU_MIXED;
     const size_t n = c->hg.n, esz = mixed ? sizeof(float2) : sizeof(double2);
     return (size_t)c->D.mp * c->D.ldc * esz + n * ((mixed ? 2 : 0) * sizeof(double2) + 3 * esz) +
-           (size_t)c->D.szU * esz + 64;
+           (size_t)c->D.szU * esz + (size_t)c->D.n_be * sizeof(double2) + 64;
 }
 
 // the shared factor's arrays
@@ -410,6 +410,7 @@ int ensure_sub_batch(crgpu_ctx *c, int want) {
     int e = ensure_refine(c);
     e = e ? e : dalloc(c, &C, w * c->D.mp * c->D.ldc * esz);
     B.C = C;
+    e = e ? e : dalloc(c, &B.bval, w * c->D.n_be);
     if (mixed) {
         e = e ? e : dalloc(c, &B.X, w * n);
         e = e ? e : dalloc(c, &B.Bt, w * n);
@@ -463,7 +464,7 @@ int sub_factor_shared(crgpu_ctx *c) {
 int sub_factor_rect(crgpu_ctx *c, const SubBatch &B) {
     CUCHECK(c, cudaMemsetAsync(B.status, 0, sizeof(int) * B.Kb * B.Lb, c->st));
     sub_launch_root(c->P, c->D, B, c->d_sigma, c->precision == CRGPU_MIXED, c->st);
-    c->stats.kernel_launches += 1;
+    c->stats.kernel_launches += 2;
     return 0;
 }
 
@@ -484,7 +485,7 @@ int sub_solve_rect(crgpu_ctx *c, const SubBatch &B, const double2 *src) {
     c->stats.kernel_launches += 2;
     for (int it = 0; it < steps; it++) {
         const int *nprev = it > 0 ? &cnt[it - 1].n : nullptr;
-        sub_launch_residual(c->P, c->D, B, c->d_sigma, nprev, c->st);
+        sub_launch_residual(c->P, c->D, B, nprev, c->st);
         c->stats.kernel_launches += 3 + sub_launch_apply(c->D, c->sp, B, true, nprev, c->st);
         sub_launch_accumulate(c->D, B, false, c->refine_tol, nprev, &cnt[it].n, &cnt[it].z, c->st);
     }
@@ -1035,14 +1036,16 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
         D.n = sp.n;
         D.m = sp.m;
         D.nI = sp.nI;
-        D.mp = (sp.m + 31) & ~31;
-        D.ldc = D.mp + 32;
+        const int nb = sub_root_block(precision == CRGPU_MIXED);
+        D.mp = (sp.m + nb - 1) / nb * nb;
+        D.ldc = D.mp + 64 - nb;  // the last rows' tile of 64 stays inside
         D.szU = sp.szU;
         D.szF = sp.szF;
         D.szG = sp.szG;
         D.szS = sp.szS;
         D.root_ent0 = sp.root_ent0;
         D.n_root_ent = (int)sp.ent.size() - sp.root_ent0;
+        D.n_be = (int)sp.be.size();
         D.root_child = sp.root_child;
         D.root_u0 = sp.fronts[sp.root_child].u0;
         D.root_r = sp.fronts[sp.root_child].r;
@@ -1051,7 +1054,11 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
         for (size_t q = 0; q < fcolpos.size(); q++) fcolpos[q] = sp.pos[c->pat.fcol[q]];
         e = upload(c, &D.fr, sp.fronts);
         if (!e) e = upload(c, &D.ent, sp.ent);
-        if (!e) e = upload(c, &D.root_bnd, sp.root_bnd);
+        if (!e) e = upload(c, &D.be, sp.be);
+        if (!e) e = upload(c, &D.be_ptr, sp.be_ptr);
+        if (!e) e = upload(c, &D.rb_ptr, sp.rb_ptr);
+        if (!e) e = upload(c, &D.rb_ent, sp.rb_ent);
+        if (!e) e = upload(c, &D.rb_pos, sp.rb_pos);
         if (!e) e = upload(c, &D.tG, sp.tG);
         if (!e) e = upload(c, &D.tS, sp.tS);
         if (!e) e = upload(c, &D.tU, sp.tU);
@@ -1061,7 +1068,6 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
         if (!e) e = upload(c, &D.rows, sp.rows);
         if (!e) e = upload(c, &D.inv, sp.inv);
         if (!e) e = upload(c, &D.root_inv, sp.root_inv);
-        if (!e) e = upload(c, &D.root_bptr, sp.root_bptr);
         if (!e) e = upload(c, &D.fcolpos, fcolpos);
         if (e) {
             *out = c;

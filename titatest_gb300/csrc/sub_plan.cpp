@@ -216,13 +216,27 @@ bool build_sub_plan(const HostGrid &hg, const Pattern &pat, SubPlan &sp) {
     for (int p : root_p) {
         const int a = local[pat.row[p]], c = local[pat.col[p]], r = std::max(a, c), l = std::min(a, c);
         sp.ent.push_back({p, r, l});
-        for (int z = pat.bnd_ptr[p]; z < pat.bnd_ptr[p + 1]; z++) cols[l].push_back({pat.bnd_list[z], r, l});
+        if (pat.bnd_ptr[p] < pat.bnd_ptr[p + 1]) cols[l].push_back({p, r, l});
     }
-    sp.root_bptr.assign(1, 0);
+    std::vector<std::vector<std::pair<int32_t, int32_t>>> rowse(sp.m);
+    sp.be_ptr.assign(1, 0);
     for (int c = 0; c < sp.m; c++) {
-        std::stable_sort(cols[c].begin(), cols[c].end(), [](const SubEnt &x, const SubEnt &y) { return x.lr < y.lr; });
-        sp.root_bnd.insert(sp.root_bnd.end(), cols[c].begin(), cols[c].end());
-        sp.root_bptr.push_back((int)sp.root_bnd.size());
+        std::sort(cols[c].begin(), cols[c].end(), [](const SubEnt &x, const SubEnt &y) { return x.lr < y.lr; });
+        for (const SubEnt &en : cols[c]) {
+            const int q = (int)sp.be.size();
+            rowse[en.lr].push_back({q, sp.nI + c});
+            if (en.lr != c) rowse[c].push_back({q, sp.nI + en.lr});
+            sp.be.push_back(en);
+        }
+        sp.be_ptr.push_back((int)sp.be.size());
+    }
+    sp.rb_ptr.assign(1, 0);
+    for (int i = 0; i < sp.m; i++) {
+        for (const auto &x : rowse[i]) {
+            sp.rb_ent.push_back(x.first);
+            sp.rb_pos.push_back(x.second);
+        }
+        sp.rb_ptr.push_back((int)sp.rb_ent.size());
     }
     sp.root_inv.assign(sp.m, -1);
     const std::vector<int32_t> &tr = b.f[order[nf - 1]].R;

@@ -44,8 +44,9 @@ struct SubPlan {
     std::vector<SubEnt> ent;                   // of the fronts, then (from root_ent0) of the root
     int root_ent0 = 0, root_child = -1;
     std::vector<int32_t> root_inv;             // root row -> row of the last front's r rows, or -1
-    std::vector<int32_t> root_bptr;            // mixed-boundary terms of the root entries, by root column:
-    std::vector<SubEnt> root_bnd;              // (boundary line << 4 | imn, row, column)
+    std::vector<SubEnt> be;                    // root entries with mixed-boundary terms, by column (row >= column)
+    std::vector<int32_t> be_ptr;               // m + 1: first of a column
+    std::vector<int32_t> rb_ptr, rb_ent, rb_pos;  // by root row: its entries in be and the other node's position
     // tiles of the four dense products, by level
     std::vector<SubTile> tG, tS, tU, tD;
     std::vector<int32_t> lG, lS, lU, lD;       // nlevel + 1 each

@@ -97,8 +97,8 @@ __device__ __forceinline__ void load4(const double2 *p, double2 (&v)[4]) {
     for (int i = 0; i < 4; i++) v[i] = p[i];
 }
 
-// 4 x 4 outer products of a 32 (or 64) x 32 tile: rows r0.., columns c0.. of
-// k-major operands
+// 4 x 4 outer products of a 32 x 32 tile: rows r0.., columns c0.. of k-major
+// operands
 template <typename T, int PA, int PB>
 __device__ __forceinline__ void tile_fma(const T *A, const T *Bm, int kk, int r0, int c0, T (&acc)[4][4]) {
 #pragma unroll 4
@@ -158,16 +158,6 @@ __global__ void k_sub_values(DevProblem P, DevSub D, const double2 *__restrict__
         }
     }
     D.As[(size_t)k * P.nnz + p] = v;
-}
-
-// the mixed-boundary terms of one entry (rows i, c), scaled by fk
-__device__ __forceinline__ double2 boundary_term(const DevProblem &P, const double *__restrict__ kgl,
-                                                 const double *__restrict__ fk, const double2 *__restrict__ sigma,
-                                                 int code, int i, int c) {
-    const int rb = code >> 4, imn = code & 15;
-    const double f = P.relbg[rb * 3 + imn] * kgl[rb] * fk[i] * fk[c];
-    const double2 s = sigma[P.brnr[rb]];
-    return cz(f * s.x, f * s.y);
 }
 
 // ------------------------------------------------------------ shared factor
@@ -413,55 +403,120 @@ __global__ void k_sub_root_ent(DevSub D, int nnz) {
 }
 
 // ------------------------------------------------------------- root factor
+// The electrodes' boundary terms, summed per root entry in FP64, the
+// electrode fastest: [Kb][n_be][Lb]
+__global__ void k_sub_bval(DevProblem P, DevSub D, SubBatch B, const double2 *__restrict__ sigma) {
+    const int l = blockIdx.y * 32 + (threadIdx.x & 31), q = blockIdx.x * 8 + (threadIdx.x >> 5), kk = blockIdx.z;
+    if (l >= B.Lb || q >= D.n_be) return;
+    const int p = D.be[q].p, i = P.row[p], c = P.col[p], k = B.k0 + kk;
+    double2 v = cz(0.0, 0.0);
+    if (!P.dirichlet[i] && !P.dirichlet[c]) {
+        const double *kgl = P.kg + ((size_t)k * P.eanz + B.l0 + l) * P.relanz, *fk = D.fk + (size_t)k * P.n;
+        const double f = fk[i] * fk[c];
+        for (int z = P.bnd_ptr[p]; z < P.bnd_ptr[p + 1]; z++) {
+            const int rb = P.bnd_list[z] >> 4;
+            const double g = P.relbg[rb * 3 + (P.bnd_list[z] & 15)] * kgl[rb];
+            const double2 sg = sigma[P.brnr[rb]];
+            v = cz(v.x + g * sg.x, v.y + g * sg.y);
+        }
+        v = cz(v.x * f, v.y * f);
+    }
+    B.bval[((size_t)kk * D.n_be + q) * B.Lb + l] = v;
+}
+
 // C C^T of one system's root, column-major lower with leading dimension ldc,
-// one block per system, left-looking in 32-column blocks.  A block's rows are
-// worked in tiles of 64: W = M - C C_j^T from the finished columns (cp.async,
-// two chunks of 16 columns in flight), then W C_jj^-T.  The diagonal block is
-// factored and inverted together, one barrier a column; its inverse is stored
-// in its place, which is all that the later solves need.
+// one block of 128 threads per system, left-looking in NB columns.  A block's
+// rows are worked in tiles of 64, a warp on 16 of them: W = M - C C_j^T from
+// the finished columns (cp.async, two chunks of 16 columns in flight), then
+// W C_jj^-T.  The diagonal block is factored and inverted together, one
+// barrier a column; its inverse is stored in its place, which is all that the
+// later solves need.  Bound by the FP64 pipe in complex128, so NB is 16 there:
+// the panel's products with the full inverse and the upper halves of the
+// diagonal blocks cost m^2 NB / 2 and m^2 NB / 4 beside m^3 / 6.  In complex64
+// the operand traffic counts too and NB is 32.  Warps whose rows lie beyond
+// the matrix skip the products.
 constexpr int kRT = 128;   // threads
 constexpr int kRows = 64;  // rows of a tile
 constexpr int kKC = 16;    // columns of a chunk
 
 template <typename T>
-__global__ __launch_bounds__(kRT) void k_sub_root(DevProblem P, DevSub D, SubBatch B,
-                                                  const double2 *__restrict__ sigma) {
+struct RootShape {
+    static constexpr int NB = sizeof(T) == 8 ? 32 : 16;
+    static constexpr int TR = sizeof(T) == 8 ? 4 : 2;  // rows of a thread; it has 4 columns
+};
+
+template <typename T, int TR>
+__device__ __forceinline__ void load_rows(const T *p, T (&v)[TR]) {
+    if constexpr (sizeof(T) == 8) {
+        const float4 a = *(const float4 *)p, b = *(const float4 *)(p + 2);
+        v[0].x = a.x, v[0].y = a.y, v[1].x = a.z, v[1].y = a.w;
+        v[2].x = b.x, v[2].y = b.y, v[3].x = b.z, v[3].y = b.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < TR; i++) v[i] = p[i];
+    }
+}
+template <typename T, int TR>
+__device__ __forceinline__ void store_rows(T *p, const T (&v)[TR]) {
+    if constexpr (sizeof(T) == 8) {
+        *(float4 *)p = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
+        *(float4 *)(p + 2) = make_float4(v[2].x, v[2].y, v[3].x, v[3].y);
+    } else {
+#pragma unroll
+        for (int i = 0; i < TR; i++) p[i] = v[i];
+    }
+}
+
+// acc[column][row] += A[q][row] B[q][column]
+template <typename T, int TR, int PB>
+__device__ __forceinline__ void root_fma(const T *A, const T *Bm, int kk, int tr, int tc, T (&acc)[4][TR]) {
+#pragma unroll 4
+    for (int q = 0; q < kk; q++) {
+        T a[TR], b[4];
+        load_rows<T, TR>(A + q * kRows + tr, a);
+        load4(Bm + q * PB + tc, b);
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+            for (int i = 0; i < TR; i++) fma_(acc[j][i], a[i], b[j]);
+    }
+}
+
+template <typename T>
+__global__ __launch_bounds__(kRT) void k_sub_root(DevSub D, SubBatch B) {
     extern __shared__ __align__(16) unsigned char sm[];
-    constexpr int PX = 34;
-    T *As = (T *)sm;                   // [2][kKC][kRows]; also W of a tile, [32][kRows]
-    T *Bs = As + 2 * kKC * kRows;      // [2][kKC][32]
-    T *Ci = Bs + 2 * kKC * 32;         // [32][PX]: Ci[a][b] = inverse(b, a)
+    constexpr int NB = RootShape<T>::NB, TR = RootShape<T>::TR, PX = NB + 2, NQ = NB / 4, CT = NB / 4;
+    T *As = (T *)sm;                      // [2][kKC][kRows]; also W of a tile, [NB][kRows]
+    T *Bs = As + 2 * kKC * kRows;         // [2][kKC][NB]
+    T *Ci = Bs + 2 * kKC * NB;            // [NB][PX]: Ci[a][b] = inverse(b, a)
     __shared__ T col[2][32], inv[2];
-    const int s = blockIdx.x, kk_ = s / B.Lb, k = B.k0 + kk_, l = B.l0 + s % B.Lb;
-    const int mp = D.mp, ldc = D.ldc, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int s = blockIdx.x, kk_ = s / B.Lb, k = B.k0 + kk_, l = s % B.Lb;
+    const int mp = D.mp, ldc = D.ldc, m = D.m, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     T *C = (T *)B.C + (size_t)s * mp * ldc;
     const T *R = (const T *)D.R + (size_t)k * mp * ldc;
-    const double *kgl = P.kg + ((size_t)k * P.eanz + l) * P.relanz;
-    const double *fk = D.fk + (size_t)k * P.n;
-    const int32_t *rnode = D.node + D.nI;
-    const int tr = (tid >> 3) * 4, tc = (tid & 7) * 4;
+    const double2 *bval = B.bval + (size_t)kk_ * D.n_be * B.Lb + l;
+    const int tr = tid / CT * TR, tc = tid % CT * 4;
     bool bad = false;
-    // pivot-column data of a 32-column block: rows r0.., this thread's 4 x 4 of W
-    for (int j = 0; j < mp; j += 32) {
+    for (int j = 0; j < mp; j += NB) {
         for (int r0 = j; r0 < mp; r0 += kRows) {
-            T acc[4][4];
+            const bool work = r0 + 16 * wid < m;
+            T acc[4][TR];
 #pragma unroll
-            for (int a = 0; a < 4; a++)
+            for (int b = 0; b < 4; b++)
 #pragma unroll
-                for (int b = 0; b < 4; b++) acc[a][b] = zero_<T>();
+                for (int a = 0; a < TR; a++) acc[b][a] = zero_<T>();
             const int nch = j / kKC;
             auto fetch = [&](int ch) {
-                T *a = As + (ch & 1) * kKC * kRows, *b = Bs + (ch & 1) * kKC * 32;
+                T *a = As + (ch & 1) * kKC * kRows, *b = Bs + (ch & 1) * kKC * NB;
                 constexpr int per = 16 / sizeof(T);
+                // rows beyond the matrix are read (ldc covers them) and not stored
                 for (int q = tid; q < kKC * kRows / per; q += kRT) {
                     const int c = q / (kRows / per), o = (q % (kRows / per)) * per;
-                    // rows beyond the matrix are not stored: any rows of the column do
-                    const int row = min(r0 + o, ldc - per);
-                    cp_async16(a + c * kRows + o, C + (size_t)(ch * kKC + c) * ldc + row);
+                    cp_async16(a + c * kRows + o, C + (size_t)(ch * kKC + c) * ldc + r0 + o);
                 }
-                for (int q = tid; q < kKC * 32 / per; q += kRT) {
-                    const int c = q / (32 / per), o = (q % (32 / per)) * per;
-                    cp_async16(b + c * 32 + o, C + (size_t)(ch * kKC + c) * ldc + j + o);
+                for (int q = tid; q < kKC * NB / per; q += kRT) {
+                    const int c = q / (NB / per), o = (q % (NB / per)) * per;
+                    cp_async16(b + c * NB + o, C + (size_t)(ch * kKC + c) * ldc + j + o);
                 }
                 cp_commit();
             };
@@ -474,46 +529,43 @@ __global__ __launch_bounds__(kRT) void k_sub_root(DevProblem P, DevSub D, SubBat
                     cp_wait<0>();
                 }
                 __syncthreads();
-                tile_fma<T, kRows, 32>(As + (ch & 1) * kKC * kRows, Bs + (ch & 1) * kKC * 32, kKC, tr, tc, acc);
+                if (work)
+                    root_fma<T, TR, NB>(As + (ch & 1) * kKC * kRows, Bs + (ch & 1) * kKC * NB, kKC, tr, tc, acc);
                 __syncthreads();
             }
-            // W = M - sum, M the wavenumber's part; the electrode's terms follow in shared memory
+            // W = M - sum, M the wavenumber's part; then the electrode's terms
 #pragma unroll
             for (int b = 0; b < 4; b++) {
-                const int c = j + tc + b;
+                T w[TR];
+                load_rows<T, TR>(R + (size_t)(j + tc + b) * ldc + r0 + tr, w);
 #pragma unroll
-                for (int a = 0; a < 4; a++) {
-                    const int i = min(r0 + tr + a, ldc - 1);
-                    const T m = R[(size_t)c * ldc + i];
-                    As[(tc + b) * kRows + tr + a].x = m.x - acc[a][b].x;
-                    As[(tc + b) * kRows + tr + a].y = m.y - acc[a][b].y;
+                for (int a = 0; a < TR; a++) {
+                    w[a].x -= acc[b][a].x;
+                    w[a].y -= acc[b][a].y;
                 }
+                store_rows<T, TR>(As + (tc + b) * kRows + tr, w);
             }
             __syncthreads();
-            if (tid < 32 && j + tid < D.m) {  // one thread per column: few terms each
-                const int c = j + tid;
-                for (int q = D.root_bptr[c]; q < D.root_bptr[c + 1]; q++) {
-                    const SubEnt en = D.root_bnd[q];
-                    if (en.lr < r0 || en.lr >= r0 + kRows) continue;
-                    const int ni = rnode[en.lr], nc = rnode[c];
-                    if (P.dirichlet[ni] || P.dirichlet[nc]) continue;
-                    const double2 v = boundary_term(P, kgl, fk, sigma, en.p, ni, nc);
-                    T &d = As[tid * kRows + en.lr - r0];
-                    d = from_<T>(cz((double)d.x + v.x, (double)d.y + v.y));
-                }
+            for (int q = D.be_ptr[min(j, m)] + tid; q < D.be_ptr[min(j + NB, m)]; q += kRT) {
+                const SubEnt en = D.be[q];
+                if (en.lr < r0 || en.lr >= r0 + kRows) continue;
+                const double2 v = bval[(size_t)q * B.Lb];
+                T &d = As[(en.lc - j) * kRows + en.lr - r0];
+                d = from_<T>(cz((double)d.x + v.x, (double)d.y + v.y));
             }
             __syncthreads();
             if (r0 == j) {
                 // diagonal block: lane = row, warp w the columns w, w + 4, ...
-                T a[8], x[8];
+                const int row = NB == 32 ? lane : lane & (NB - 1);
+                T a[NQ], x[NQ];
 #pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    a[q] = As[(4 * q + wid) * kRows + lane];
+                for (int q = 0; q < NQ; q++) {
+                    a[q] = As[(4 * q + wid) * kRows + row];
                     x[q] = zero_<T>();
-                    if (lane == 4 * q + wid) x[q].x = 1;
+                    if (row == 4 * q + wid) x[q].x = 1;
                 }
 #pragma unroll
-                for (int q = 0; q < 8; q++)
+                for (int q = 0; q < NQ; q++)
 #pragma unroll
                     for (int ww = 0; ww < 4; ww++) {
                         const int p = 4 * q + ww, buf = p & 1;
@@ -521,44 +573,44 @@ __global__ __launch_bounds__(kRT) void k_sub_root(DevProblem P, DevSub D, SubBat
                             const T d = shfl_(a[q], p);
                             if (is_bad(d)) bad = true;
                             const T iv = rcp_(sqrt_(d));
-                            col[buf][lane] = lane > p ? mul_(a[q], iv) : zero_<T>();
+                            col[buf][row] = row > p ? mul_(a[q], iv) : zero_<T>();
                             if (lane == 0) inv[buf] = iv;
                         }
                         __syncthreads();
-                        const T cl = col[buf][lane], iv = inv[buf];
+                        const T cl = col[buf][row], iv = inv[buf];
 #pragma unroll
-                        for (int z = 0; z < 8; z++) {
+                        for (int z = 0; z < NQ; z++) {
                             const int c = 4 * z + wid;
                             if (z >= q && c > p) fms_(a[z], cl, col[buf][c]);
                             if (z <= q) {
                                 const T xp = mul_(shfl_(x[z], p), iv);
-                                if (lane == p) x[z] = xp;
-                                else if (lane > p) fms_(x[z], cl, xp);
+                                if (row == p) x[z] = xp;
+                                else if (row > p) fms_(x[z], cl, xp);
                             }
                         }
                     }
+                if (lane < NB) {
 #pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    const int c = 4 * q + wid;
-                    const T v = lane >= c ? x[q] : zero_<T>();
-                    Ci[c * PX + lane] = v;
-                    C[(size_t)(j + c) * ldc + j + lane] = v;
+                    for (int q = 0; q < NQ; q++) {
+                        const int c = 4 * q + wid;
+                        const T v = row >= c ? x[q] : zero_<T>();
+                        Ci[c * PX + row] = v;
+                        C[(size_t)(j + c) * ldc + j + row] = v;
+                    }
                 }
                 __syncthreads();
             }
             // C_ij = W C_jj^-T
+            const int i = r0 + tr;
+            if (r0 + 16 * wid >= j + NB && r0 + 16 * wid < mp) {
 #pragma unroll
-            for (int a = 0; a < 4; a++)
+                for (int b = 0; b < 4; b++)
 #pragma unroll
-                for (int b = 0; b < 4; b++) acc[a][b] = zero_<T>();
-            tile_fma<T, kRows, PX>(As, Ci, 32, tr, tc, acc);
+                    for (int a = 0; a < TR; a++) acc[b][a] = zero_<T>();
+                if (work) root_fma<T, TR, PX>(As, Ci, NB, tr, tc, acc);
 #pragma unroll
-            for (int b = 0; b < 4; b++)
-#pragma unroll
-                for (int a = 0; a < 4; a++) {
-                    const int i = r0 + tr + a;
-                    if (i >= j + 32 && i < mp) C[(size_t)(j + tc + b) * ldc + i] = acc[a][b];
-                }
+                for (int b = 0; b < 4; b++) store_rows<T, TR>(C + (size_t)(j + tc + b) * ldc + i, acc[b]);
+            }
             __syncthreads();
         }
     }
@@ -576,8 +628,9 @@ constexpr int kST = 256;
 template <typename T>
 __global__ __launch_bounds__(kST) void k_sub_root_solve(DevSub D, SubBatch B, const int *nprev) {
     extern __shared__ __align__(16) unsigned char sm[];
-    T *v = (T *)sm;            // [mp]
-    __shared__ T t[32];
+    constexpr int NB = RootShape<T>::NB, CW = NB / 8;  // columns of a warp
+    T *v = (T *)sm;  // [mp]
+    __shared__ T t[NB], part[8][33];
     if (nprev && *nprev == 0) return;
     const int s = blockIdx.x, kk = s / B.Lb, l = s % B.Lb;
     if (B.kact && !B.kact[kk]) return;
@@ -600,18 +653,17 @@ __global__ __launch_bounds__(kST) void k_sub_root_solve(DevSub D, SubBatch B, co
         v[i] = u;
     }
     __syncthreads();
-    for (int j = 0; j < mp; j += 32) {
-        // y_j = C_jj^-1 v_j: warp w takes 4 columns of the inverse, lane = row
+    for (int j = 0; j < mp; j += NB) {
+        // y_j = C_jj^-1 v_j: warp w takes CW columns of the inverse, lane = row
         T p = zero_<T>();
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int c = wid * 4 + q;
-            if (lane >= c) fma_(p, C[(size_t)(j + c) * ldc + j + lane], v[j + c]);
+        for (int q = 0; q < CW; q++) {
+            const int c = wid * CW + q;
+            if (lane >= c && lane < NB) fma_(p, C[(size_t)(j + c) * ldc + j + lane], v[j + c]);
         }
-        __shared__ T part[8][33];
         part[wid][lane] = p;
         __syncthreads();
-        if (tid < 32) {
+        if (tid < NB) {
             T y = zero_<T>();
 #pragma unroll
             for (int q = 0; q < 8; q++) {
@@ -622,21 +674,21 @@ __global__ __launch_bounds__(kST) void k_sub_root_solve(DevSub D, SubBatch B, co
             t[lane] = y;
         }
         __syncthreads();
-        for (int i = j + 32 + tid; i < mp; i += kST) {
+        for (int i = j + NB + tid; i < mp; i += kST) {
             T a = v[i];
 #pragma unroll 8
-            for (int c = 0; c < 32; c++) fms_(a, C[(size_t)(j + c) * ldc + i], t[c]);
+            for (int c = 0; c < NB; c++) fms_(a, C[(size_t)(j + c) * ldc + i], t[c]);
             v[i] = a;
         }
         __syncthreads();
     }
-    for (int j = mp - 32; j >= 0; j -= 32) {
-        // t_c = y_c - sum_i C(i, c) x_i: four columns a warp
+    for (int j = mp - NB; j >= 0; j -= NB) {
+        // t_c = y_c - sum_i C(i, c) x_i: CW columns a warp
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int c = wid * 4 + q;
+        for (int q = 0; q < CW; q++) {
+            const int c = wid * CW + q;
             T a = zero_<T>();
-            for (int i = j + 32 + lane; i < mp; i += 32) fma_(a, C[(size_t)(j + c) * ldc + i], v[i]);
+            for (int i = j + NB + lane; i < mp; i += 32) fma_(a, C[(size_t)(j + c) * ldc + i], v[i]);
             a = warp_sum_(a);
             if (lane == 0) {
                 t[c].x = v[j + c].x - a.x;
@@ -645,10 +697,10 @@ __global__ __launch_bounds__(kST) void k_sub_root_solve(DevSub D, SubBatch B, co
         }
         __syncthreads();
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int c = wid * 4 + q;
+        for (int q = 0; q < CW; q++) {
+            const int c = wid * CW + q;
             T a = zero_<T>();
-            if (lane >= c) fma_(a, C[(size_t)(j + c) * ldc + j + lane], t[lane]);
+            if (lane >= c && lane < NB) fma_(a, C[(size_t)(j + c) * ldc + j + lane], t[lane]);
             a = warp_sum_(a);
             if (lane == 0) v[j + c] = a;
         }
@@ -809,8 +861,7 @@ __global__ void k_sub_rhs(DevProblem P, DevSub D, SubBatch B, int lsink, int nsi
 
 // Y = b - A x in FP64 (rounded to complex64 at the end): one warp per row, the
 // electrodes across its lanes, so the matrix entries are one broadcast load.
-__global__ __launch_bounds__(256) void k_sub_residual(DevProblem P, DevSub D, SubBatch B,
-                                                      const double2 *__restrict__ sigma, const int *nprev) {
+__global__ __launch_bounds__(256) void k_sub_residual(DevProblem P, DevSub D, SubBatch B, const int *nprev) {
     if (nprev && *nprev == 0) return;
     const int kk = blockIdx.z, k = B.k0 + kk, L = B.Lb;
     if (!B.kact[kk]) return;
@@ -821,14 +872,10 @@ __global__ __launch_bounds__(256) void k_sub_residual(DevProblem P, DevSub D, Su
     const double2 *X = B.X + (size_t)kk * D.n * L + l;
     double2 acc = cz(0.0, 0.0);
     for (int q = P.fptr[i]; q < P.fptr[i + 1]; q++) fma_(acc, As[P.fidx[q]], X[(size_t)D.fcolpos[q] * L]);
-    if (p >= D.nI && !P.dirichlet[i]) {
-        const double *kgl = P.kg + ((size_t)k * P.eanz + B.l0 + l) * P.relanz, *fk = D.fk + (size_t)k * P.n;
-        for (int q = P.fptr[i]; q < P.fptr[i + 1]; q++) {
-            const int e = P.fidx[q], c = P.fcol[q];
-            if (P.dirichlet[c]) continue;
-            for (int z = P.bnd_ptr[e]; z < P.bnd_ptr[e + 1]; z++)
-                fma_(acc, boundary_term(P, kgl, fk, sigma, P.bnd_list[z], i, c), X[(size_t)D.fcolpos[q] * L]);
-        }
+    if (p >= D.nI) {
+        const double2 *bv = B.bval + (size_t)kk * D.n_be * L + l;
+        for (int q = D.rb_ptr[p - D.nI]; q < D.rb_ptr[p - D.nI + 1]; q++)
+            fma_(acc, bv[(size_t)D.rb_ent[q] * L], X[(size_t)D.rb_pos[q] * L]);
     }
     const size_t at = ((size_t)kk * D.n + p) * L + l;
     const double2 b = B.Bt[at];
@@ -974,7 +1021,8 @@ int factor_t(const DevProblem &P, const DevSub &D, const SubPlan &sp, cudaStream
 
 template <typename T>
 size_t root_smem() {
-    return sizeof(T) * (2 * kKC * kRows + 2 * kKC * 32 + 32 * 34);
+    constexpr int NB = RootShape<T>::NB;
+    return sizeof(T) * (2 * kKC * kRows + 2 * kKC * NB + NB * (NB + 2));
 }
 
 template <typename T>
@@ -983,7 +1031,8 @@ void root_t(const DevProblem &P, const DevSub &D, const SubBatch &B, const doubl
     std::call_once(once, [] {
         cudaFuncSetAttribute(k_sub_root<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)root_smem<T>());
     });
-    k_sub_root<T><<<B.Kb * B.Lb, kRT, root_smem<T>(), st>>>(P, D, B, sigma);
+    if (D.n_be) k_sub_bval<<<dim3(nb(D.n_be, 8), nb(B.Lb, 32), B.Kb), 256, 0, st>>>(P, D, B, sigma);
+    k_sub_root<T><<<B.Kb * B.Lb, kRT, root_smem<T>(), st>>>(D, B);
 }
 
 template <typename T>
@@ -1012,6 +1061,8 @@ void sub_launch_values(const DevProblem &P, const DevSub &D, const double2 *sigm
     k_sub_values<<<dim3(nb(P.nnz, 256), P.K), 256, 0, st>>>(P, D, adom);
 }
 
+int sub_root_block(bool mixed) { return mixed ? RootShape<float2>::NB : RootShape<double2>::NB; }
+
 int sub_launch_factor(const DevProblem &P, const DevSub &D, const SubPlan &sp, bool mixed, cudaStream_t st) {
     return mixed ? factor_t<float2>(P, D, sp, st) : factor_t<double2>(P, D, sp, st);
 }
@@ -1033,9 +1084,8 @@ void sub_launch_rhs(const DevProblem &P, const DevSub &D, const SubBatch &B, boo
     else k_sub_rhs<double2><<<g, 256, 0, st>>>(P, D, B, lsink, nsink, src, 0);
 }
 
-void sub_launch_residual(const DevProblem &P, const DevSub &D, const SubBatch &B, const double2 *sigma,
-                         const int *nprev, cudaStream_t st) {
-    k_sub_residual<<<dim3(nb(D.n, 8), nb(B.Lb, 32), B.Kb), 256, 0, st>>>(P, D, B, sigma, nprev);
+void sub_launch_residual(const DevProblem &P, const DevSub &D, const SubBatch &B, const int *nprev, cudaStream_t st) {
+    k_sub_residual<<<dim3(nb(D.n, 8), nb(B.Lb, 32), B.Kb), 256, 0, st>>>(P, D, B, nprev);
 }
 
 void sub_launch_accumulate(const DevSub &D, const SubBatch &B, bool first, double tol, const int *nprev, int *nactive,

@@ -15,10 +15,11 @@ struct DevSub {
     int n, m, nI, mp, ldc, szU;
     int64_t szF, szG, szS;
     const SubFront *fr;
-    const SubEnt *ent, *root_bnd;
+    const SubEnt *ent, *be;
     const SubTile *tG, *tS, *tU, *tD;
-    const int32_t *pos, *node, *rows, *inv, *root_inv, *root_bptr, *fcolpos;
-    int root_ent0, n_root_ent, root_child, root_u0, root_r;
+    const int32_t *pos, *node, *rows, *inv, *root_inv, *fcolpos;
+    const int32_t *be_ptr, *rb_ptr, *rb_ent, *rb_pos;
+    int root_ent0, n_root_ent, n_be, root_child, root_u0, root_r;
     int64_t root_oS;
     double2 *As;     // [K][nnz] area parts, scaled by fk on both sides
     double *fk;      // [K][n]   scaling of the area parts' diagonal, by node
@@ -31,12 +32,14 @@ struct DevSub {
 struct SubBatch {
     int k0, Kb, l0, Lb;
     void *C;                        // [Kb * Lb][mp * ldc] root factors
+    double2 *bval;                  // [Kb][n_be][Lb] boundary terms of the root entries
     double2 *X, *Bt;                // solution, right-hand side (scaled by fk)
     void *Y, *W, *Z, *U;            // input, assembled input, output, update rows
     int *status, *active, *kact;    // per system, per system, per wavenumber (null: all)
     unsigned long long *mz, *mx;    // per system: bit patterns of the largest correction and solution
 };
 
+int sub_root_block(bool mixed);  // columns of a block of the root factor
 void sub_launch_values(const DevProblem &P, const DevSub &D, const double2 *sigma, const double2 *adom, cudaStream_t st);
 int sub_launch_factor(const DevProblem &P, const DevSub &D, const SubPlan &sp, bool mixed, cudaStream_t st);
 void sub_launch_root(const DevProblem &P, const DevSub &D, const SubBatch &B, const double2 *sigma, bool mixed,
@@ -45,8 +48,7 @@ int sub_launch_apply(const DevSub &D, const SubPlan &sp, const SubBatch &B, bool
                      cudaStream_t st);
 void sub_launch_rhs(const DevProblem &P, const DevSub &D, const SubBatch &B, bool mixed, int lsink, int nsink,
                     const double2 *src, cudaStream_t st);
-void sub_launch_residual(const DevProblem &P, const DevSub &D, const SubBatch &B, const double2 *sigma,
-                         const int *nprev, cudaStream_t st);
+void sub_launch_residual(const DevProblem &P, const DevSub &D, const SubBatch &B, const int *nprev, cudaStream_t st);
 void sub_launch_accumulate(const DevSub &D, const SubBatch &B, bool first, double tol, const int *nprev, int *nactive,
                            double *zmax, cudaStream_t st);
 void sub_launch_unpack(const DevProblem &P, const DevSub &D, const SubBatch &B, double sign, double2 *out,
