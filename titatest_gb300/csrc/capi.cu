@@ -1030,7 +1030,7 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
             c->sys_l.push_back(0);
         }
     }
-    if (c->nrhs == 1 && build_sub_plan(hg, c->pat, c->sp)) {
+    if (c->nrhs == 1 && build_sub_plan(hg, c->pat, sub_down_rows(precision == CRGPU_MIXED), c->sp)) {
         const SubPlan &sp = c->sp;
         DevSub &D = c->D;
         D.n = sp.n;
@@ -1059,6 +1059,7 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
         if (!e) e = upload(c, &D.rb_ptr, sp.rb_ptr);
         if (!e) e = upload(c, &D.rb_ent, sp.rb_ent);
         if (!e) e = upload(c, &D.rb_pos, sp.rb_pos);
+        if (!e) e = upload(c, &D.tA, sp.tA);
         if (!e) e = upload(c, &D.tG, sp.tG);
         if (!e) e = upload(c, &D.tS, sp.tS);
         if (!e) e = upload(c, &D.tU, sp.tU);

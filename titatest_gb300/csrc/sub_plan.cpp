@@ -14,14 +14,19 @@ namespace crgpu {
 
 namespace {
 
-constexpr int kLeaf = 24;
+// Nodes that are not cut further.  Measured at 16 / 24 / 32 / 48: config-2 mixed
+// forward 13.2 / 12.8 / 12.6 / 12.6 ms, 160x50 quads complex128 39.2 / 39.0 / 38.3
+// / 40.7 ms (smaller leaves store more update rows, larger ones multiply more).
+constexpr int kLeaf = 32;
 
 struct Build {
     const HostGrid &hg;
     const Pattern &pat;
     struct F {
         std::vector<int32_t> E, R;
-        int ch0 = -1, ch1 = -1, lev = 0;
+        std::vector<int> ch;
+        int lev = 0;
+        bool gone = false;  // taken into its parent
     };
     std::vector<F> f;
     std::vector<int32_t> owner;  // front of a node, -1: not eliminated (yet)
@@ -30,16 +35,34 @@ struct Build {
 
     Build(const HostGrid &h, const Pattern &p) : hg(h), pat(p), owner(h.n, -1), mark(h.n, 0) {}
 
-    // eliminates E after the fronts a and b; long lists as a chain
-    int add(const std::vector<int32_t> &E, int a, int b) {
+    // Eliminates E after the fronts of ch; long lists as a chain.  A front that
+    // has children itself is taken into its parent where the two fit one
+    // front: fewer levels, and its update vectors are never stored.
+    int add(std::vector<int32_t> E, std::vector<int> ch) {
+        std::vector<int> up;
+        size_t left = ch.size();
+        for (int c : ch) {
+            left--;
+            F &s = f[c];
+            if (!s.ch.empty() && E.size() + s.E.size() <= (size_t)kSubEMax &&
+                up.size() + s.ch.size() + left <= (size_t)kSubCh) {
+                E.insert(E.begin(), s.E.begin(), s.E.end());
+                up.insert(up.end(), s.ch.begin(), s.ch.end());
+                s.gone = true;
+            } else {
+                up.push_back(c);
+            }
+        }
         const int s = (int)E.size(), parts = std::max(1, (s + kSubEMax - 1) / kSubEMax);
         for (int q = 0; q < parts; q++) {
             F t;
             t.E.assign(E.begin() + (size_t)s * q / parts, E.begin() + (size_t)s * (q + 1) / parts);
-            t.ch0 = a;
-            t.ch1 = b;
+            t.ch = up;
             const int id = (int)f.size();
             for (int v : t.E) owner[v] = id;
+            // the rest of a chain is not eliminated yet
+            if (q == 0)
+                for (size_t z = t.E.size(); z < E.size(); z++) owner[E[z]] = -1;
             const int st = ++stamp;
             auto take = [&](int v) {
                 if (owner[v] < 0 && mark[v] != st) {
@@ -49,14 +72,12 @@ struct Build {
             };
             for (int v : t.E)
                 for (int z = pat.fptr[v]; z < pat.fptr[v + 1]; z++) take(pat.fcol[z]);
-            for (int c : {a, b})
-                if (c >= 0) {
-                    for (int v : f[c].R) take(v);
-                    t.lev = std::max(t.lev, f[c].lev + 1);
-                }
+            for (int c : t.ch) {
+                for (int v : f[c].R) take(v);
+                t.lev = std::max(t.lev, f[c].lev + 1);
+            }
             f.push_back(std::move(t));
-            a = id;
-            b = -1;
+            up.assign(1, id);
         }
         return (int)f.size() - 1;
     }
@@ -78,7 +99,7 @@ struct Build {
     }
 
     int cut(std::vector<int32_t> nodes) {
-        if ((int)nodes.size() <= kLeaf) return add(nodes, -1, -1);
+        if ((int)nodes.size() <= kLeaf) return add(std::move(nodes), {});
         const int h = (int)nodes.size() / 2;
         std::vector<int32_t> best, best_nodes;
         for (int dir = 0; dir < 2; dir++) {
@@ -94,24 +115,24 @@ struct Build {
                 best_nodes = nodes;
             }
         }
-        if (best.size() * 2 >= nodes.size()) return add(nodes, -1, -1);
+        if (best.size() * 2 >= nodes.size()) return add(std::move(nodes), {});
         const int st = ++stamp;
         for (int v : best) mark[v] = st;
         std::vector<int32_t> part[2];
         for (size_t q = 0; q < best_nodes.size(); q++)
             if (mark[best_nodes[q]] != st) part[(int)q >= h].push_back(best_nodes[q]);
-        int ch[2] = {-1, -1};
+        std::vector<int> ch;
         for (int q = 0; q < 2; q++)
-            if (!part[q].empty()) ch[q] = cut(std::move(part[q]));
-        return add(best, ch[0], ch[1]);
+            if (!part[q].empty()) ch.push_back(cut(std::move(part[q])));
+        return add(std::move(best), std::move(ch));
     }
 };
 
-int tiles(int v) { return (v + kSubTile - 1) / kSubTile; }
+int tiles(int v, int edge = kSubTile) { return (v + edge - 1) / edge; }
 
 }  // namespace
 
-bool build_sub_plan(const HostGrid &hg, const Pattern &pat, SubPlan &sp) {
+bool build_sub_plan(const HostGrid &hg, const Pattern &pat, int down_rows, SubPlan &sp) {
     sp = SubPlan();
     const int n = hg.n;
     std::vector<uint8_t> root(n, 0);
@@ -122,14 +143,16 @@ bool build_sub_plan(const HostGrid &hg, const Pattern &pat, SubPlan &sp) {
     if (inner.empty() || outer.empty()) return false;
     Build b(hg, pat);
     b.cut(inner);
-    const int nf = (int)b.f.size();
+    std::vector<int32_t> order;
+    for (int q = 0; q < (int)b.f.size(); q++)
+        if (!b.f[q].gone) order.push_back(q);
+    const int nf = (int)order.size();
     sp.n = n;
     sp.m = (int)outer.size();
     sp.nI = (int)inner.size();
     sp.nfront = nf;
     // fronts by level
-    std::vector<int32_t> order(nf), at(nf);
-    for (int q = 0; q < nf; q++) order[q] = q;
+    std::vector<int32_t> at(b.f.size(), -1);
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return b.f[x].lev < b.f[y].lev; });
     for (int q = 0; q < nf; q++) at[order[q]] = q;
     sp.nlevel = b.f[order[nf - 1]].lev + 1;
@@ -156,9 +179,6 @@ bool build_sub_plan(const HostGrid &hg, const Pattern &pat, SubPlan &sp) {
         t.e = (int)s.E.size();
         t.r = (int)s.R.size();
         t.nd0 = t.e ? sp.pos[s.E[0]] : 0;
-        t.ch0 = s.ch0 >= 0 ? at[s.ch0] : -1;
-        t.ch1 = s.ch1 >= 0 ? at[s.ch1] : -1;
-        t.pad = 0;
         t.rows0 = (int)sp.rows.size();
         for (int v : s.R) sp.rows.push_back(sp.pos[v]);
         t.u0 = sp.szU;
@@ -171,18 +191,22 @@ bool build_sub_plan(const HostGrid &hg, const Pattern &pat, SubPlan &sp) {
         sp.szS += (int64_t)t.r * t.r;
         sp.c_factor += (double)t.e * t.e * t.e + (double)t.e * t.e * t.r + 0.5 * t.e * t.r * (double)t.r;
         sp.c_apply += (double)t.e * (t.e + 2.0 * t.r);
-        auto inverse = [&](int ch) {
-            const int o = (int)sp.inv.size();
-            if (ch < 0) return 0;
-            const std::vector<int32_t> &cr = b.f[order[ch]].R;
-            for (size_t z = 0; z < cr.size(); z++) local[cr[z]] = (int)z;
+        t.nch = (int)s.ch.size();
+        for (int z = 0; z < kSubCh; z++) {
+            t.cr[z] = t.cu[z] = t.inv[z] = 0;
+            t.cS[z] = 0;
+            if (z >= t.nch) continue;
+            const SubFront &u = sp.fronts[at[s.ch[z]]];
+            t.cr[z] = u.r;
+            t.cu[z] = u.u0;
+            t.cS[z] = u.oS;
+            t.inv[z] = (int)sp.inv.size();
+            const std::vector<int32_t> &cr = b.f[s.ch[z]].R;
+            for (size_t y = 0; y < cr.size(); y++) local[cr[y]] = (int)y;
             for (int v : s.E) sp.inv.push_back(local[v]);
             for (int v : s.R) sp.inv.push_back(local[v]);
             for (int v : cr) local[v] = -1;
-            return o;
-        };
-        t.inv0 = inverse(t.ch0);
-        t.inv1 = inverse(t.ch1);
+        }
     }
     // matrix entries, each in the front that eliminates its earlier node
     std::vector<std::vector<int32_t>> own(nf);
@@ -243,20 +267,22 @@ bool build_sub_plan(const HostGrid &hg, const Pattern &pat, SubPlan &sp) {
     for (size_t z = 0; z < tr.size(); z++) sp.root_inv[local[tr[z]]] = (int)z;
     // tiles
     sp.lG.assign(1, 0);
-    sp.lS = sp.lU = sp.lD = sp.lG;
+    sp.lA = sp.lS = sp.lU = sp.lD = sp.lG;
     for (int lv = 0; lv < sp.nlevel; lv++) {
         for (int q = sp.level[lv]; q < sp.level[lv + 1]; q++) {
             const SubFront &t = sp.fronts[q];
             const int te = tiles(t.e), tr2 = tiles(t.r);
             for (int i = 0; i < te; i++) {
-                sp.tD.push_back({q, i, 0});
                 for (int j = 0; j < tr2; j++) sp.tG.push_back({q, i, j});
+                for (int j = 0; t.nch && j < tiles(t.e + t.r); j++) sp.tA.push_back({q, i, j});
             }
+            for (int i = 0; i < tiles(t.e, down_rows); i++) sp.tD.push_back({q, i, 0});
             for (int i = 0; i < tr2; i++) {
                 for (int j = 0; j <= i; j++) sp.tS.push_back({q, i, j});
             }
             for (int i = 0; i < std::max(1, tr2); i++) sp.tU.push_back({q, i, 0});
         }
+        sp.lA.push_back((int)sp.tA.size());
         sp.lG.push_back((int)sp.tG.size());
         sp.lS.push_back((int)sp.tS.size());
         sp.lU.push_back((int)sp.tU.size());

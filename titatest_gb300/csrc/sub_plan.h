@@ -10,18 +10,23 @@
 
 namespace crgpu {
 
+constexpr int kSubTile = 32;   // tile edge of the dense kernels
+constexpr int kSubEMax = 64;   // most nodes one front eliminates
+constexpr int kSubCh = 4;      // most children of a front
+
 // One front: e nodes eliminated here, r nodes it is coupled to (eliminated
 // later, or root nodes).  Local rows 0..e-1 are positions nd0..nd0+e-1, rows
 // e..e+r-1 the positions rows[rows0 .. rows0+r-1].
 struct SubFront {
-    int32_t e, r, nd0;
-    int32_t ch0, ch1;     // children (-1: none)
+    int32_t e, r, nd0, nch;
     int32_t ent0, nent;   // matrix entries assembled here
     int32_t rows0;        // into SubPlan::rows
-    int32_t inv0, inv1;   // into SubPlan::inv: local row -> row of the child's r rows, or -1
     int32_t u0;           // first row of this front's update vectors
-    int32_t pad;
     int64_t oF, oG, oS;   // inverse pivot block (e x e), G (e x r), Schur complement (r x r)
+    // children: their r, first update row and Schur complement, and
+    // (in SubPlan::inv) the row among a child's r rows of every local row, or -1
+    int32_t cr[kSubCh], cu[kSubCh], inv[kSubCh];
+    int64_t cS[kSubCh];
 };
 
 struct SubEnt {
@@ -31,9 +36,6 @@ struct SubEnt {
 struct SubTile {
     int32_t front, ti, tj;
 };
-
-constexpr int kSubTile = 32;   // tile edge of the dense kernels
-constexpr int kSubEMax = 64;   // most nodes one front eliminates
 
 struct SubPlan {
     int n = 0, m = 0, nI = 0, nfront = 0, nlevel = 0;
@@ -47,16 +49,17 @@ struct SubPlan {
     std::vector<SubEnt> be;                    // root entries with mixed-boundary terms, by column (row >= column)
     std::vector<int32_t> be_ptr;               // m + 1: first of a column
     std::vector<int32_t> rb_ptr, rb_ent, rb_pos;  // by root row: its entries in be and the other node's position
-    // tiles of the four dense products, by level
-    std::vector<SubTile> tG, tS, tU, tD;
-    std::vector<int32_t> lG, lS, lU, lD;       // nlevel + 1 each
+    // tiles of a front's gather (e x (e + r)), of G (e x r), of S (r x r, lower)
+    // and row tiles of the solves (r up, e down), by level
+    std::vector<SubTile> tA, tG, tS, tU, tD;
+    std::vector<int32_t> lA, lG, lS, lU, lD;   // nlevel + 1 each
     int64_t szF = 0, szG = 0, szS = 0;         // entries per wavenumber
     int32_t szU = 0;                           // update rows per wavenumber
     double c_factor = 0, c_apply = 0;          // complex multiply-adds: factor per wavenumber, one solve
 };
 
 // The plan for the grid, or false where it has no root (no mixed boundary)
-// or no interior.
-bool build_sub_plan(const HostGrid &hg, const Pattern &pat, SubPlan &sp);
+// or no interior.  down_rows: rows of a tile of the downward solve.
+bool build_sub_plan(const HostGrid &hg, const Pattern &pat, int down_rows, SubPlan &sp);
 
 }  // namespace crgpu

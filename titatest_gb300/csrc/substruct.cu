@@ -97,20 +97,14 @@ __device__ __forceinline__ void load4(const double2 *p, double2 (&v)[4]) {
     for (int i = 0; i < 4; i++) v[i] = p[i];
 }
 
-// 4 x 4 outer products of a 32 x 32 tile: rows r0.., columns c0.. of k-major
-// operands
-template <typename T, int PA, int PB>
-__device__ __forceinline__ void tile_fma(const T *A, const T *Bm, int kk, int r0, int c0, T (&acc)[4][4]) {
-#pragma unroll 4
-    for (int q = 0; q < kk; q++) {
-        T a[4], b[4];
-        load4(A + q * PA + r0, a);
-        load4(Bm + q * PB + c0, b);
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) fma_(acc[i][j], a[i], b[j]);
-    }
+__device__ __forceinline__ void load2(const float2 *p, float2 (&v)[2]) {
+    const float4 a = *(const float4 *)p;
+    v[0] = cf(a.x, a.y);
+    v[1] = cf(a.z, a.w);
+}
+__device__ __forceinline__ void load2(const double2 *p, double2 (&v)[2]) {
+    v[0] = p[0];
+    v[1] = p[1];
 }
 
 constexpr int kT = kSubTile;      // 32
@@ -161,9 +155,54 @@ __global__ void k_sub_values(DevProblem P, DevSub D, const double2 *__restrict__
 }
 
 // ------------------------------------------------------------ shared factor
-// Assembles a front's F11 (shared memory) and F12 (D.H) from its children's
-// Schur complements and its matrix entries and inverts F11.  The inverse is
-// symmetric up to the sign between swept and unswept rows (Gauss-Jordan
+// A front's F11 (into D.F) and F12 (into D.H) from its children's Schur
+// complements, one block per 32 x 32 tile of the e x (e + r) rows.  (Gathered
+// by the pivot kernel's one block per front, the indices and the dependent
+// loads took longer than the elimination: 166 -> 60 us at e = 61, r = 321.)
+template <typename T>
+__global__ __launch_bounds__(256) void k_sub_gather(DevSub D, int t0) {
+    __shared__ int si[kSubCh][kT], sj[kSubCh][kT];
+    const SubTile tl = D.tA[t0 + blockIdx.x];
+    const SubFront &t = D.fr[tl.front];
+    const int k = blockIdx.y, e = t.e, r = t.r, nch = t.nch, i0 = tl.ti * kT, j0 = tl.tj * kT;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int q = w; q < 2 * nch; q += 8) {
+        const int c = q >> 1, o = (q & 1 ? j0 : i0) + lane;
+        const int v = o < ((q & 1) ? e + r : e) ? D.inv[t.inv[c] + o] : -1;
+        (q & 1 ? sj : si)[c][lane] = v;
+    }
+    __syncthreads();
+    const T *Sk = (const T *)D.S + (size_t)k * D.szS;
+    T *F = (T *)D.F + (size_t)k * D.szF + t.oF, *H = (T *)D.H + (size_t)k * D.szG + t.oG;
+    T v[4];
+#pragma unroll
+    for (int z = 0; z < 4; z++) v[z] = zero_<T>();
+    for (int c = 0; c < nch; c++) {
+        const T *S = Sk + t.cS[c];
+        const int cr = t.cr[c], y = sj[c][lane];
+        T g[4];
+#pragma unroll
+        for (int z = 0; z < 4; z++) {
+            const int x = si[c][w + 8 * z];
+            g[z] = x >= 0 && y >= 0 ? S[(size_t)x * cr + y] : zero_<T>();
+        }
+#pragma unroll
+        for (int z = 0; z < 4; z++) {
+            v[z].x += g[z].x;
+            v[z].y += g[z].y;
+        }
+    }
+#pragma unroll
+    for (int z = 0; z < 4; z++) {
+        const int i = i0 + w + 8 * z, j = j0 + lane;
+        if (i >= e || j >= e + r) continue;
+        if (j < e) F[(size_t)i * e + j] = v[z];
+        else H[(size_t)i * r + j - e] = v[z];
+    }
+}
+
+// Adds a front's matrix entries to F11 and F12 and inverts F11.  The inverse
+// is symmetric up to the sign between swept and unswept rows (Gauss-Jordan
 // sweeps), so only the lower triangle is computed, each entry in a register of
 // its thread; per sweep the pivot row is published twice, raw and divided by
 // the pivot.
@@ -172,36 +211,17 @@ __global__ __launch_bounds__(NT) void k_sub_pivot(DevSub D, int f0, int nnz) {
     extern __shared__ __align__(16) unsigned char sm[];
     T *Fm = (T *)sm;
     __shared__ T s_raw[2][kSubEMax], s_div[kSubEMax], s_inv[2];
-    const SubFront t = D.fr[f0 + blockIdx.x];
-    const int k = blockIdx.y, e = t.e, r = t.r, ld = e | 1, tid = threadIdx.x;
-    const T *Sk = (const T *)D.S + (size_t)k * D.szS;
+    const SubFront &t = D.fr[f0 + blockIdx.x];
+    const int k = blockIdx.y, e = t.e, r = t.r, ld = e | 1, tid = threadIdx.x, nent = t.nent, ent0 = t.ent0;
+    const bool leaf = t.nch == 0;
     const double2 *As = D.As + (size_t)k * nnz;
-    T *H = (T *)D.H + (size_t)k * D.szG + t.oG;
-    const SubFront *c0 = t.ch0 >= 0 ? &D.fr[t.ch0] : nullptr, *c1 = t.ch1 >= 0 ? &D.fr[t.ch1] : nullptr;
-    const int r0 = c0 ? c0->r : 0, r1 = c1 ? c1->r : 0;
-    const T *S0 = c0 ? Sk + c0->oS : nullptr, *S1 = c1 ? Sk + c1->oS : nullptr;
-    const int32_t *i0 = D.inv + t.inv0, *i1 = D.inv + t.inv1;
-    auto gathered = [&](int a, int b) {
-        T v = zero_<T>();
-        if (S0) {
-            const int x = i0[a], y = i0[b];
-            if (x >= 0 && y >= 0) v = S0[(size_t)x * r0 + y];
-        }
-        if (S1) {
-            const int x = i1[a], y = i1[b];
-            if (x >= 0 && y >= 0) {
-                const T w = S1[(size_t)x * r1 + y];
-                v.x += w.x;
-                v.y += w.y;
-            }
-        }
-        return v;
-    };
-    for (int q = tid; q < e * e; q += NT) Fm[(q / e) * ld + q % e] = gathered(q / e, q % e);
-    for (int q = tid; q < e * r; q += NT) H[q] = gathered(q / r, e + q % r);
+    T *F = (T *)D.F + (size_t)k * D.szF + t.oF, *H = (T *)D.H + (size_t)k * D.szG + t.oG;
+    for (int q = tid; q < e * e; q += NT) Fm[(q / e) * ld + q % e] = leaf ? zero_<T>() : F[q];
+    if (leaf)
+        for (int q = tid; q < e * r; q += NT) H[q] = zero_<T>();
     __syncthreads();
-    for (int q = tid; q < t.nent; q += NT) {
-        const SubEnt en = D.ent[t.ent0 + q];
+    for (int q = tid; q < nent; q += NT) {
+        const SubEnt en = D.ent[ent0 + q];
         const T v = from_<T>(As[en.p]);
         if (en.lc < e) {  // the lower triangle is read below
             T &d = Fm[en.lc * ld + en.lr];
@@ -268,7 +288,6 @@ __global__ __launch_bounds__(NT) void k_sub_pivot(DevSub D, int f0, int nnz) {
         }
         if (p + 1 < e) publish(p + 1, buf ^ 1);
     }
-    T *F = (T *)D.F + (size_t)k * D.szF + t.oF;
 #pragma unroll
     for (int z = 0; z < NE; z++)
         if (ri[z] >= 0) {
@@ -278,95 +297,141 @@ __global__ __launch_bounds__(NT) void k_sub_pivot(DevSub D, int f0, int nnz) {
     if (bad) atomicCAS(&D.kbad[k], 0, 28);
 }
 
-// 32 rows of `rows` x 32 columns from src (row stride ls) into dst[row][col]
+// Four entries a thread of a 32 x 32 operand tile (rows w, w + 8, ..., column
+// = lane) in registers: the loads of the next chunk are in flight while the
+// present one is multiplied.
 template <typename T>
-__device__ __forceinline__ void load_tile(T *dst, const T *src, size_t ls, int nr, int nc) {
-    for (int q = threadIdx.x; q < kT * kT; q += 64) {
-        const int a = q / kT, b = q % kT;
-        dst[a * kP + b] = a < nr && b < nc ? src[(size_t)a * ls + b] : zero_<T>();
+struct Quad {
+    T v[4];
+    __device__ __forceinline__ void load(const T *src, size_t ls, int nr, int nc) {
+        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+        for (int z = 0; z < 4; z++)
+            v[z] = w + 8 * z < nr && lane < nc ? src[(size_t)(w + 8 * z) * ls + lane] : zero_<T>();
+    }
+    __device__ __forceinline__ void store(T *dst) const {
+        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+        for (int z = 0; z < 4; z++) dst[(w + 8 * z) * kP + lane] = v[z];
+    }
+    __device__ __forceinline__ void store_transposed(T *dst) const {
+        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+        for (int z = 0; z < 4; z++) dst[lane * kP + w + 8 * z] = v[z];
+    }
+};
+
+// 256 threads: RM x 2 outer products of k-major tiles, rows tr.., columns tc..
+template <typename T, int RM>
+__device__ __forceinline__ void tile_fma(const T *A, const T *Bm, int kk, int tr, int tc, T (&acc)[RM][2]) {
+#pragma unroll 8
+    for (int q = 0; q < kk; q++) {
+        T a[RM], b[2];
+        if constexpr (RM == 2) load2(A + q * kP + tr, a);
+        else a[0] = A[q * kP + tr];
+        load2(Bm + q * kP + tc, b);
+#pragma unroll
+        for (int i = 0; i < RM; i++)
+#pragma unroll
+            for (int j = 0; j < 2; j++) fma_(acc[i][j], a[i], b[j]);
     }
 }
 
 // G = F11^-1 F12
 template <typename T>
-__global__ __launch_bounds__(64) void k_sub_g(DevSub D, int t0) {
+__global__ __launch_bounds__(256) void k_sub_g(DevSub D, int t0) {
     __shared__ __align__(16) T A[kT * kP], Bm[kT * kP];
     const SubTile tl = D.tG[t0 + blockIdx.x];
-    const SubFront t = D.fr[tl.front];
+    const SubFront &t = D.fr[tl.front];
     const int k = blockIdx.y, e = t.e, r = t.r, i0 = tl.ti * kT, j0 = tl.tj * kT;
     const T *F = (const T *)D.F + (size_t)k * D.szF + t.oF, *H = (const T *)D.H + (size_t)k * D.szG + t.oG;
-    T acc[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++) acc[a][b] = zero_<T>();
-    const int tr = (threadIdx.x >> 3) * 4, tc = (threadIdx.x & 7) * 4;
+    T *G = (T *)D.G + (size_t)k * D.szG + t.oG;
+    T acc[2][2];
+    acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = zero_<T>();
+    const int tr = (threadIdx.x >> 4) * 2, tc = (threadIdx.x & 15) * 2;
+    const bool work = i0 + (threadIdx.x >> 5) * 4 < e;
+    Quad<T> a, b;
+    a.load(F + i0, e, e, e - i0);  // symmetric: F[p][i]
+    b.load(H + j0, r, e, r - j0);
     for (int p = 0; p < e; p += kT) {
-        const int kk = min(kT, e - p);
-        load_tile(A, F + (size_t)p * e + i0, e, kk, e - i0);  // symmetric: F[p][i]
-        load_tile(Bm, H + (size_t)p * r + j0, r, kk, r - j0);
+        a.store(A);
+        b.store(Bm);
         __syncthreads();
-        tile_fma<T, kP, kP>(A, Bm, kk, tr, tc, acc);
+        if (p + kT < e) {
+            a.load(F + (size_t)(p + kT) * e + i0, e, e - p - kT, e - i0);
+            b.load(H + (size_t)(p + kT) * r + j0, r, e - p - kT, r - j0);
+        }
+        if (work) tile_fma<T, 2>(A, Bm, min(kT, e - p), tr, tc, acc);
         __syncthreads();
     }
-    T *G = (T *)D.G + (size_t)k * D.szG + t.oG;
 #pragma unroll
-    for (int a = 0; a < 4; a++)
+    for (int i = 0; i < 2; i++)
 #pragma unroll
-        for (int b = 0; b < 4; b++)
-            if (i0 + tr + a < e && j0 + tc + b < r) G[(size_t)(i0 + tr + a) * r + j0 + tc + b] = acc[a][b];
+        for (int j = 0; j < 2; j++)
+            if (i0 + tr + i < e && j0 + tc + j < r) G[(size_t)(i0 + tr + i) * r + j0 + tc + j] = acc[i][j];
 }
 
 // S = (children's complements) - F12^T G, lower tiles, mirrored
 template <typename T>
-__global__ __launch_bounds__(64) void k_sub_s(DevSub D, int t0) {
+__global__ __launch_bounds__(256) void k_sub_s(DevSub D, int t0) {
     __shared__ __align__(16) T A[kT * kP], Bm[kT * kP];
+    __shared__ int si[kSubCh][kT], sj[kSubCh][kT];
     const SubTile tl = D.tS[t0 + blockIdx.x];
-    const SubFront t = D.fr[tl.front];
-    const int k = blockIdx.y, e = t.e, r = t.r, i0 = tl.ti * kT, j0 = tl.tj * kT;
+    const SubFront &t = D.fr[tl.front];
+    const int k = blockIdx.y, e = t.e, r = t.r, nch = t.nch, i0 = tl.ti * kT, j0 = tl.tj * kT;
     const T *H = (const T *)D.H + (size_t)k * D.szG + t.oG, *G = (const T *)D.G + (size_t)k * D.szG + t.oG;
     T *Sk = (T *)D.S + (size_t)k * D.szS, *S = Sk + t.oS;
-    T acc[4][4];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    Quad<T> a, b;
+    a.load(H + i0, r, e, r - i0);
+    b.load(G + j0, r, e, r - j0);
+    for (int q = w; q < 2 * nch; q += 8) {
+        const int c = q >> 1, o = (q & 1 ? j0 : i0) + lane;
+        (q & 1 ? sj : si)[c][lane] = o < r ? D.inv[t.inv[c] + e + o] : -1;
+    }
+    __syncthreads();
+    const int tr = (threadIdx.x >> 4) * 2, tc = (threadIdx.x & 15) * 2;
+    const bool work = i0 + w * 4 < r;
+    T sum[2][2], acc[2][2];
 #pragma unroll
-    for (int a = 0; a < 4; a++)
+    for (int i = 0; i < 2; i++)
 #pragma unroll
-        for (int b = 0; b < 4; b++) acc[a][b] = zero_<T>();
-    const int tr = (threadIdx.x >> 3) * 4, tc = (threadIdx.x & 7) * 4;
+        for (int j = 0; j < 2; j++) acc[i][j] = sum[i][j] = zero_<T>();
+    for (int c = 0; c < nch; c++) {
+        const T *Sc = Sk + t.cS[c];
+        const int cr = t.cr[c];
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const int x = si[c][tr + i], y = sj[c][tc + j];
+                if (x >= 0 && y >= 0) {
+                    const T v = Sc[(size_t)x * cr + y];
+                    sum[i][j].x += v.x;
+                    sum[i][j].y += v.y;
+                }
+            }
+    }
     for (int p = 0; p < e; p += kT) {
-        const int kk = min(kT, e - p);
-        load_tile(A, H + (size_t)p * r + i0, r, kk, r - i0);
-        load_tile(Bm, G + (size_t)p * r + j0, r, kk, r - j0);
+        a.store(A);
+        b.store(Bm);
         __syncthreads();
-        tile_fma<T, kP, kP>(A, Bm, kk, tr, tc, acc);
+        if (p + kT < e) {
+            a.load(H + (size_t)(p + kT) * r + i0, r, e - p - kT, r - i0);
+            b.load(G + (size_t)(p + kT) * r + j0, r, e - p - kT, r - j0);
+        }
+        if (work) tile_fma<T, 2>(A, Bm, min(kT, e - p), tr, tc, acc);
         __syncthreads();
     }
-    const SubFront *c0 = t.ch0 >= 0 ? &D.fr[t.ch0] : nullptr, *c1 = t.ch1 >= 0 ? &D.fr[t.ch1] : nullptr;
-    const int r0 = c0 ? c0->r : 0, r1 = c1 ? c1->r : 0;
-    const T *S0 = c0 ? Sk + c0->oS : nullptr, *S1 = c1 ? Sk + c1->oS : nullptr;
-    const int32_t *m0 = D.inv + t.inv0 + e, *m1 = D.inv + t.inv1 + e;
 #pragma unroll
-    for (int a = 0; a < 4; a++)
+    for (int ii = 0; ii < 2; ii++)
 #pragma unroll
-        for (int b = 0; b < 4; b++) {
-            const int i = i0 + tr + a, j = j0 + tc + b;
+        for (int jj = 0; jj < 2; jj++) {
+            const int i = i0 + tr + ii, j = j0 + tc + jj;
             if (i >= r || j > i) continue;
-            T v = neg_(acc[a][b]);
-            if (S0) {
-                const int x = m0[i], y = m0[j];
-                if (x >= 0 && y >= 0) {
-                    const T w = S0[(size_t)x * r0 + y];
-                    v.x += w.x;
-                    v.y += w.y;
-                }
-            }
-            if (S1) {
-                const int x = m1[i], y = m1[j];
-                if (x >= 0 && y >= 0) {
-                    const T w = S1[(size_t)x * r1 + y];
-                    v.x += w.x;
-                    v.y += w.y;
-                }
-            }
+            T v = sum[ii][jj];
+            v.x -= acc[ii][jj].x;
+            v.y -= acc[ii][jj].y;
             S[(size_t)i * r + j] = v;
             S[(size_t)j * r + i] = v;
         }
@@ -710,130 +775,180 @@ __global__ __launch_bounds__(kST) void k_sub_root_solve(DevSub D, SubBatch B, co
 }
 
 // Up the tree: b_E (own right-hand sides and the children's updates) goes to
-// W, the update rows U = (children's updates) - G^T b_E to the parent.
+// W, the update rows U = (children's updates) - G^T b_E to the parent.  One
+// block per 32 update rows x 32 electrodes.
 template <typename T>
-__global__ __launch_bounds__(64) void k_sub_up(DevSub D, SubBatch B, int t0, const int *nprev) {
+__global__ __launch_bounds__(256) void k_sub_up(DevSub D, SubBatch B, int t0, const int *nprev) {
     __shared__ __align__(16) T A[kT * kP], Bm[kT * kP];
+    __shared__ int se[kSubCh][kSubEMax], sr[kSubCh][kT];
     if (nprev && *nprev == 0) return;
     const int kk = blockIdx.z, k = B.k0 + kk;
     if (B.kact && !B.kact[kk]) return;
     const SubTile tl = D.tU[t0 + blockIdx.x];
-    const SubFront t = D.fr[tl.front];
-    const int e = t.e, r = t.r, i0 = tl.ti * kT, l0 = blockIdx.y * kT, L = B.Lb, nl = min(kT, L - l0);
+    const SubFront &t = D.fr[tl.front];
+    const int e = t.e, r = t.r, nch = t.nch, i0 = tl.ti * kT, l0 = blockIdx.y * kT, L = B.Lb, nl = min(kT, L - l0);
     const T *G = (const T *)D.G + (size_t)k * D.szG + t.oG;
-    const T *Y = (const T *)B.Y + ((size_t)kk * D.n + t.nd0) * L + l0;
-    T *W = (T *)B.W + ((size_t)kk * D.n + t.nd0) * L + l0;
+    const T *__restrict__ Y = (const T *)B.Y + ((size_t)kk * D.n + t.nd0) * L + l0;
+    T *__restrict__ W = (T *)B.W + ((size_t)kk * D.n + t.nd0) * L + l0;
     T *Uk = (T *)B.U + (size_t)kk * D.szU * L + l0;
-    const T *U0 = t.ch0 >= 0 ? Uk + (size_t)D.fr[t.ch0].u0 * L : nullptr;
-    const T *U1 = t.ch1 >= 0 ? Uk + (size_t)D.fr[t.ch1].u0 * L : nullptr;
-    const int32_t *m0 = D.inv + t.inv0, *m1 = D.inv + t.inv1;
-    auto updates = [&](int row, int c) {
-        T v = zero_<T>();
-        if (U0) {
-            const int x = m0[row];
-            if (x >= 0) v = U0[(size_t)x * L + c];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int q = threadIdx.x; q < nch * kSubEMax; q += 256) {
+        const int c = q / kSubEMax, o = q % kSubEMax;
+        if (o < e) se[c][o] = D.inv[t.inv[c] + o];
+    }
+    for (int q = threadIdx.x; q < nch * kT; q += 256) {
+        const int c = q / kT, o = q % kT;
+        sr[c][o] = i0 + o < r ? D.inv[t.inv[c] + e + i0 + o] : -1;
+    }
+    __syncthreads();
+    Quad<T> a, b;
+    auto load_b = [&](int p) {
+#pragma unroll
+        for (int z = 0; z < 4; z++) {
+            const int q = p + w + 8 * z;
+            b.v[z] = q < e && lane < nl ? Y[(size_t)q * L + lane] : zero_<T>();
         }
-        if (U1) {
-            const int x = m1[row];
-            if (x >= 0) {
-                const T w = U1[(size_t)x * L + c];
-                v.x += w.x;
-                v.y += w.y;
+        for (int c = 0; c < nch; c++) {
+            const T *U = Uk + (size_t)t.cu[c] * L + lane;
+            T g[4];
+#pragma unroll
+            for (int z = 0; z < 4; z++) {
+                const int q = p + w + 8 * z, x = q < e && lane < nl ? se[c][q] : -1;
+                g[z] = x >= 0 ? U[(size_t)x * L] : zero_<T>();
+            }
+#pragma unroll
+            for (int z = 0; z < 4; z++) {
+                b.v[z].x += g[z].x;
+                b.v[z].y += g[z].y;
             }
         }
-        return v;
     };
-    T acc[4][4];
+    a.load(G + i0, r, e, r - i0);
+    load_b(0);
+    // the children's updates of this thread's four results
+    const int tr = (threadIdx.x >> 4) * 2, tc = (threadIdx.x & 15) * 2;
+    const bool work = i0 + w * 4 < r;
+    T sum[2][2], acc[2][2];
 #pragma unroll
-    for (int a = 0; a < 4; a++)
+    for (int i = 0; i < 2; i++)
 #pragma unroll
-        for (int b = 0; b < 4; b++) acc[a][b] = zero_<T>();
-    const int tr = (threadIdx.x >> 3) * 4, tc = (threadIdx.x & 7) * 4;
+        for (int j = 0; j < 2; j++) acc[i][j] = sum[i][j] = zero_<T>();
+    for (int c = 0; c < nch; c++) {
+        const T *U = Uk + (size_t)t.cu[c] * L;
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int x = sr[c][tr + i];
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+                if (x >= 0 && tc + j < nl) {
+                    const T v = U[(size_t)x * L + tc + j];
+                    sum[i][j].x += v.x;
+                    sum[i][j].y += v.y;
+                }
+        }
+    }
     for (int p = 0; p < e; p += kT) {
-        const int kc = min(kT, e - p);
-        load_tile(A, G + (size_t)p * r + i0, r, kc, r - i0);
-        for (int q = threadIdx.x; q < kT * kT; q += 64) {
-            const int a = q / kT, c = q % kT;
-            T v = zero_<T>();
-            if (a < kc && c < nl) {
-                v = updates(p + a, c);
-                const T y = Y[(size_t)(p + a) * L + c];
-                v.x += y.x;
-                v.y += y.y;
-                if (tl.ti == 0) W[(size_t)(p + a) * L + c] = v;
-            }
-            Bm[a * kP + c] = v;
+        a.store(A);
+        b.store(Bm);
+        if (tl.ti == 0) {
+#pragma unroll
+            for (int z = 0; z < 4; z++)
+                if (p + w + 8 * z < e && lane < nl) W[(size_t)(p + w + 8 * z) * L + lane] = b.v[z];
         }
         __syncthreads();
-        tile_fma<T, kP, kP>(A, Bm, kc, tr, tc, acc);
+        if (p + kT < e) {
+            a.load(G + (size_t)(p + kT) * r + i0, r, e - p - kT, r - i0);
+            load_b(p + kT);
+        }
+        if (work) tile_fma<T, 2>(A, Bm, min(kT, e - p), tr, tc, acc);
         __syncthreads();
     }
     T *U = Uk + (size_t)t.u0 * L;
 #pragma unroll
-    for (int a = 0; a < 4; a++) {
-        const int i = i0 + tr + a;
-        if (i >= r) continue;
+    for (int i = 0; i < 2; i++)
 #pragma unroll
-        for (int b = 0; b < 4; b++)
-            if (tc + b < nl) {
-                T v = updates(e + i, tc + b);
-                v.x -= acc[a][b].x;
-                v.y -= acc[a][b].y;
-                U[(size_t)i * L + tc + b] = v;
+        for (int j = 0; j < 2; j++)
+            if (i0 + tr + i < r && tc + j < nl) {
+                T v = sum[i][j];
+                v.x -= acc[i][j].x;
+                v.y -= acc[i][j].y;
+                U[(size_t)(i0 + tr + i) * L + tc + j] = v;
             }
-    }
 }
 
-// Down the tree: x_E = F11^-1 b_E - G x_R
+// Down the tree: x_E = F11^-1 b_E - G x_R, one block per 16 RM rows x 32
+// electrodes (RM 1 in complex128: the topmost fronts are few, and a tile is
+// bound by its SM's FP64 pipe).
 template <typename T>
-__global__ __launch_bounds__(64) void k_sub_down(DevSub D, SubBatch B, int t0, const int *nprev) {
+struct DownShape {
+    static constexpr int RM = sizeof(T) == 8 ? 2 : 1;
+};
+
+template <typename T>
+__global__ __launch_bounds__(256) void k_sub_down(DevSub D, SubBatch B, int t0, const int *nprev) {
+    constexpr int RM = DownShape<T>::RM, BM = 16 * RM, kIdx = 512;
     __shared__ __align__(16) T A[kT * kP], Bm[kT * kP];
+    __shared__ int sidx[kIdx];
     if (nprev && *nprev == 0) return;
     const int kk = blockIdx.z, k = B.k0 + kk;
     if (B.kact && !B.kact[kk]) return;
     const SubTile tl = D.tD[t0 + blockIdx.x];
-    const SubFront t = D.fr[tl.front];
-    const int e = t.e, r = t.r, i0 = tl.ti * kT, l0 = blockIdx.y * kT, L = B.Lb, nl = min(kT, L - l0);
+    const SubFront &t = D.fr[tl.front];
+    const int e = t.e, r = t.r, i0 = tl.ti * BM, l0 = blockIdx.y * kT, L = B.Lb, nl = min(kT, L - l0);
     const T *F = (const T *)D.F + (size_t)k * D.szF + t.oF, *G = (const T *)D.G + (size_t)k * D.szG + t.oG;
     const T *W = (const T *)B.W + ((size_t)kk * D.n + t.nd0) * L + l0;
     T *Zk = (T *)B.Z + (size_t)kk * D.n * L + l0;
     const int32_t *rows = D.rows + t.rows0;
-    T acc[4][4], acg[4][4];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int tr = (threadIdx.x >> 4) * RM, tc = (threadIdx.x & 15) * 2;
+    const bool work = i0 + w * 2 * RM < e;
+    for (int q = threadIdx.x; q < min(r, kIdx); q += 256) sidx[q] = rows[q];
+    __syncthreads();
+    Quad<T> a, b;
+    // chunks of 32: first the columns of G, then those of F11^-1
+    const int nr = (r + kT - 1) / kT, nc = nr + (e + kT - 1) / kT;
+    auto load = [&](int ch) {
+        if (ch < nr) {
+            const int p = ch * kT;
+            a.load(G + (size_t)i0 * r + p, r, min(BM, e - i0), r - p);  // along the rows of G: transposed below
 #pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++) acc[a][b] = acg[a][b] = zero_<T>();
-    const int tr = (threadIdx.x >> 3) * 4, tc = (threadIdx.x & 7) * 4;
-    for (int p = 0; p < e; p += kT) {
-        const int kc = min(kT, e - p);
-        load_tile(A, F + (size_t)p * e + i0, e, kc, e - i0);
-        load_tile(Bm, W + (size_t)p * L, L, kc, nl);
-        __syncthreads();
-        tile_fma<T, kP, kP>(A, Bm, kc, tr, tc, acc);
-        __syncthreads();
-    }
-    for (int p = 0; p < r; p += kT) {
-        const int kc = min(kT, r - p);
-        for (int q = threadIdx.x; q < kT * kT; q += 64) {
-            const int a = q / kT, c = q % kT;  // A[column of G][row]: read along the row of G
-            A[c * kP + a] = i0 + a < e && c < kc ? G[(size_t)(i0 + a) * r + p + c] : zero_<T>();
-            Bm[a * kP + c] = a < kc && c < nl ? Zk[(size_t)rows[p + a] * L + c] : zero_<T>();
+            for (int z = 0; z < 4; z++) {
+                const int q = p + w + 8 * z;
+                b.v[z] = zero_<T>();
+                if (q < r && lane < nl) b.v[z] = Zk[(size_t)(q < kIdx ? sidx[q] : rows[q]) * L + lane];
+            }
+        } else {
+            const int p = (ch - nr) * kT;
+            a.load(F + (size_t)p * e + i0, e, e - p, min(BM, e - i0));
+            b.load(W + (size_t)p * L, L, e - p, nl);
         }
+    };
+    T acc[RM][2];
+#pragma unroll
+    for (int i = 0; i < RM; i++) acc[i][0] = acc[i][1] = zero_<T>();
+    load(0);
+    for (int ch = 0; ch < nc; ch++) {
+        if (ch < nr) a.store_transposed(A);
+        else a.store(A);
+        b.store(Bm);
         __syncthreads();
-        tile_fma<T, kP, kP>(A, Bm, kc, tr, tc, acg);
+        if (ch + 1 < nc) load(ch + 1);
+        if (ch == nr) {
+#pragma unroll
+            for (int i = 0; i < RM; i++) {
+                acc[i][0] = neg_(acc[i][0]);
+                acc[i][1] = neg_(acc[i][1]);
+            }
+        }
+        if (work) tile_fma<T, RM>(A, Bm, ch < nr ? min(kT, r - ch * kT) : min(kT, e - (ch - nr) * kT), tr, tc, acc);
         __syncthreads();
     }
     T *Z = Zk + (size_t)t.nd0 * L;
 #pragma unroll
-    for (int a = 0; a < 4; a++)
+    for (int i = 0; i < RM; i++)
 #pragma unroll
-        for (int b = 0; b < 4; b++)
-            if (i0 + tr + a < e && tc + b < nl) {
-                T v = acc[a][b];
-                v.x -= acg[a][b].x;
-                v.y -= acg[a][b].y;
-                Z[(size_t)(i0 + tr + a) * L + tc + b] = v;
-            }
+        for (int j = 0; j < 2; j++)
+            if (i0 + tr + i < e && tc + j < nl) Z[(size_t)(i0 + tr + i) * L + tc + j] = acc[i][j];
 }
 
 // -------------------------------------------------- vectors of a rectangle
@@ -1005,14 +1120,15 @@ int factor_t(const DevProblem &P, const DevSub &D, const SubPlan &sp, cudaStream
         int emax = 1;
         for (int q = f0; q < f0 + nf; q++) emax = std::max(emax, sp.fronts[q].e);
         const size_t smem = sizeof(T) * emax * (emax | 1);
+        const int na = sp.lA[lv + 1] - sp.lA[lv], ng = sp.lG[lv + 1] - sp.lG[lv], ns = sp.lS[lv + 1] - sp.lS[lv];
+        if (na) k_sub_gather<T><<<dim3(na, P.K), 256, 0, st>>>(D, sp.lA[lv]);
         if (emax * (emax + 1) / 2 <= 128 * 5)
             k_sub_pivot<T, 128, 5><<<dim3(nf, P.K), 128, smem, st>>>(D, f0, P.nnz);
         else
             k_sub_pivot<T, 256, 9><<<dim3(nf, P.K), 256, smem, st>>>(D, f0, P.nnz);
-        const int ng = sp.lG[lv + 1] - sp.lG[lv], ns = sp.lS[lv + 1] - sp.lS[lv];
-        if (ng) k_sub_g<T><<<dim3(ng, P.K), 64, 0, st>>>(D, sp.lG[lv]);
-        if (ns) k_sub_s<T><<<dim3(ns, P.K), 64, 0, st>>>(D, sp.lS[lv]);
-        launches += 1 + (ng > 0) + (ns > 0);
+        if (ng) k_sub_g<T><<<dim3(ng, P.K), 256, 0, st>>>(D, sp.lG[lv]);
+        if (ns) k_sub_s<T><<<dim3(ns, P.K), 256, 0, st>>>(D, sp.lS[lv]);
+        launches += 1 + (na > 0) + (ng > 0) + (ns > 0);
     }
     k_sub_root_base<T><<<dim3(D.mp, P.K), 128, 0, st>>>(D);
     if (D.n_root_ent) k_sub_root_ent<T><<<dim3(nb(D.n_root_ent, 128), P.K), 128, 0, st>>>(D, P.nnz);
@@ -1039,13 +1155,13 @@ template <typename T>
 int apply_t(const DevSub &D, const SubPlan &sp, const SubBatch &B, const int *nprev, cudaStream_t st) {
     const int lt = (B.Lb + kT - 1) / kT;
     for (int lv = 0; lv < sp.nlevel; lv++)
-        k_sub_up<T><<<dim3(sp.lU[lv + 1] - sp.lU[lv], lt, B.Kb), 64, 0, st>>>(D, B, sp.lU[lv], nprev);
+        k_sub_up<T><<<dim3(sp.lU[lv + 1] - sp.lU[lv], lt, B.Kb), 256, 0, st>>>(D, B, sp.lU[lv], nprev);
     k_sub_root_solve<T><<<B.Kb * B.Lb, kST, sizeof(T) * D.mp, st>>>(D, B, nprev);
     int launches = sp.nlevel + 1;
     for (int lv = sp.nlevel - 1; lv >= 0; lv--) {
         const int nd = sp.lD[lv + 1] - sp.lD[lv];
         if (!nd) continue;
-        k_sub_down<T><<<dim3(nd, lt, B.Kb), 64, 0, st>>>(D, B, sp.lD[lv], nprev);
+        k_sub_down<T><<<dim3(nd, lt, B.Kb), 256, 0, st>>>(D, B, sp.lD[lv], nprev);
         launches++;
     }
     return launches;
@@ -1060,6 +1176,8 @@ void sub_launch_values(const DevProblem &P, const DevSub &D, const double2 *sigm
     k_sub_scale<<<nb((size_t)P.K * P.n, 256), 256, 0, st>>>(P, D, sigma, fak_area);
     k_sub_values<<<dim3(nb(P.nnz, 256), P.K), 256, 0, st>>>(P, D, adom);
 }
+
+int sub_down_rows(bool mixed) { return 16 * (mixed ? DownShape<float2>::RM : DownShape<double2>::RM); }
 
 int sub_root_block(bool mixed) { return mixed ? RootShape<float2>::NB : RootShape<double2>::NB; }
 

@@ -16,7 +16,7 @@ struct DevSub {
     int64_t szF, szG, szS;
     const SubFront *fr;
     const SubEnt *ent, *be;
-    const SubTile *tG, *tS, *tU, *tD;
+    const SubTile *tA, *tG, *tS, *tU, *tD;
     const int32_t *pos, *node, *rows, *inv, *root_inv, *fcolpos;
     const int32_t *be_ptr, *rb_ptr, *rb_ent, *rb_pos;
     int root_ent0, n_root_ent, n_be, root_child, root_u0, root_r;
@@ -39,6 +39,7 @@ struct SubBatch {
     unsigned long long *mz, *mx;    // per system: bit patterns of the largest correction and solution
 };
 
+int sub_down_rows(bool mixed);   // rows of a tile of the downward solve
 int sub_root_block(bool mixed);  // columns of a block of the root factor
 void sub_launch_values(const DevProblem &P, const DevSub &D, const double2 *sigma, const double2 *adom, cudaStream_t st);
 int sub_launch_factor(const DevProblem &P, const DevSub &D, const SubPlan &sp, bool mixed, cudaStream_t st);
