@@ -1030,7 +1030,7 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
             c->sys_l.push_back(0);
         }
     }
-    if (c->nrhs == 1 && build_sub_plan(hg, c->pat, sub_down_rows(precision == CRGPU_MIXED), c->sp)) {
+    if (c->nrhs == 1 && build_sub_plan(hg, c->pat, sub_shape(precision == CRGPU_MIXED), c->sp)) {
         const SubPlan &sp = c->sp;
         DevSub &D = c->D;
         D.n = sp.n;

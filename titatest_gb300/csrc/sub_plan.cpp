@@ -14,14 +14,10 @@ namespace crgpu {
 
 namespace {
 
-// Nodes that are not cut further.  Measured at 16 / 24 / 32 / 48: config-2 mixed
-// forward 13.2 / 12.8 / 12.6 / 12.6 ms, 160x50 quads complex128 39.2 / 39.0 / 38.3
-// / 40.7 ms (smaller leaves store more update rows, larger ones multiply more).
-constexpr int kLeaf = 32;
-
 struct Build {
     const HostGrid &hg;
     const Pattern &pat;
+    const SubShape shape;
     struct F {
         std::vector<int32_t> E, R;
         std::vector<int> ch;
@@ -33,7 +29,8 @@ struct Build {
     std::vector<int32_t> mark;
     int stamp = 0;
 
-    Build(const HostGrid &h, const Pattern &p) : hg(h), pat(p), owner(h.n, -1), mark(h.n, 0) {}
+    Build(const HostGrid &h, const Pattern &p, const SubShape &s)
+        : hg(h), pat(p), shape(s), owner(h.n, -1), mark(h.n, 0) {}
 
     // Eliminates E after the fronts of ch; long lists as a chain.  A front that
     // has children itself is taken into its parent where the two fit one
@@ -44,7 +41,7 @@ struct Build {
         for (int c : ch) {
             left--;
             F &s = f[c];
-            if (!s.ch.empty() && E.size() + s.E.size() <= (size_t)kSubEMax &&
+            if (!s.ch.empty() && E.size() + s.E.size() <= (size_t)shape.emax &&
                 up.size() + s.ch.size() + left <= (size_t)kSubCh) {
                 E.insert(E.begin(), s.E.begin(), s.E.end());
                 up.insert(up.end(), s.ch.begin(), s.ch.end());
@@ -53,7 +50,7 @@ struct Build {
                 up.push_back(c);
             }
         }
-        const int s = (int)E.size(), parts = std::max(1, (s + kSubEMax - 1) / kSubEMax);
+        const int s = (int)E.size(), parts = std::max(1, (s + shape.emax - 1) / shape.emax);
         for (int q = 0; q < parts; q++) {
             F t;
             t.E.assign(E.begin() + (size_t)s * q / parts, E.begin() + (size_t)s * (q + 1) / parts);
@@ -99,7 +96,7 @@ struct Build {
     }
 
     int cut(std::vector<int32_t> nodes) {
-        if ((int)nodes.size() <= kLeaf) return add(std::move(nodes), {});
+        if ((int)nodes.size() <= shape.leaf) return add(std::move(nodes), {});
         const int h = (int)nodes.size() / 2;
         std::vector<int32_t> best, best_nodes;
         for (int dir = 0; dir < 2; dir++) {
@@ -128,11 +125,9 @@ struct Build {
     }
 };
 
-int tiles(int v, int edge = kSubTile) { return (v + edge - 1) / edge; }
-
 }  // namespace
 
-bool build_sub_plan(const HostGrid &hg, const Pattern &pat, int down_rows, SubPlan &sp) {
+bool build_sub_plan(const HostGrid &hg, const Pattern &pat, const SubShape &shape, SubPlan &sp) {
     sp = SubPlan();
     const int n = hg.n;
     std::vector<uint8_t> root(n, 0);
@@ -141,7 +136,7 @@ bool build_sub_plan(const HostGrid &hg, const Pattern &pat, int down_rows, SubPl
     std::vector<int32_t> inner, outer;
     for (int i = 0; i < n; i++) (root[i] ? outer : inner).push_back(i);
     if (inner.empty() || outer.empty()) return false;
-    Build b(hg, pat);
+    Build b(hg, pat, shape);
     b.cut(inner);
     std::vector<int32_t> order;
     for (int q = 0; q < (int)b.f.size(); q++)
@@ -266,6 +261,7 @@ bool build_sub_plan(const HostGrid &hg, const Pattern &pat, int down_rows, SubPl
     const std::vector<int32_t> &tr = b.f[order[nf - 1]].R;
     for (size_t z = 0; z < tr.size(); z++) sp.root_inv[local[tr[z]]] = (int)z;
     // tiles
+    auto tiles = [&](int v) { return (v + shape.tile - 1) / shape.tile; };
     sp.lG.assign(1, 0);
     sp.lA = sp.lS = sp.lU = sp.lD = sp.lG;
     for (int lv = 0; lv < sp.nlevel; lv++) {
@@ -273,10 +269,10 @@ bool build_sub_plan(const HostGrid &hg, const Pattern &pat, int down_rows, SubPl
             const SubFront &t = sp.fronts[q];
             const int te = tiles(t.e), tr2 = tiles(t.r);
             for (int i = 0; i < te; i++) {
+                sp.tD.push_back({q, i, 0});
                 for (int j = 0; j < tr2; j++) sp.tG.push_back({q, i, j});
                 for (int j = 0; t.nch && j < tiles(t.e + t.r); j++) sp.tA.push_back({q, i, j});
             }
-            for (int i = 0; i < tiles(t.e, down_rows); i++) sp.tD.push_back({q, i, 0});
             for (int i = 0; i < tr2; i++) {
                 for (int j = 0; j <= i; j++) sp.tS.push_back({q, i, j});
             }

@@ -10,9 +10,14 @@
 
 namespace crgpu {
 
-constexpr int kSubTile = 32;   // tile edge of the dense kernels
-constexpr int kSubEMax = 64;   // most nodes one front eliminates
+constexpr int kSubEMax = 64;   // most nodes one front may eliminate
 constexpr int kSubCh = 4;      // most children of a front
+
+// What suits a precision (substruct.cu): nodes that are not cut further, most
+// nodes a front eliminates, and the edge of the dense kernels' tiles.
+struct SubShape {
+    int leaf, emax, tile;
+};
 
 // One front: e nodes eliminated here, r nodes it is coupled to (eliminated
 // later, or root nodes).  Local rows 0..e-1 are positions nd0..nd0+e-1, rows
@@ -59,7 +64,7 @@ struct SubPlan {
 };
 
 // The plan for the grid, or false where it has no root (no mixed boundary)
-// or no interior.  down_rows: rows of a tile of the downward solve.
-bool build_sub_plan(const HostGrid &hg, const Pattern &pat, int down_rows, SubPlan &sp);
+// or no interior.
+bool build_sub_plan(const HostGrid &hg, const Pattern &pat, const SubShape &shape, SubPlan &sp);
 
 }  // namespace crgpu

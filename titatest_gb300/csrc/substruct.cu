@@ -45,8 +45,22 @@ __device__ __forceinline__ float2 mul_(float2 a, float2 b) { return cmulf(a, b);
 __device__ __forceinline__ double2 mul_(double2 a, double2 b) { return cmul(a, b); }
 __device__ __forceinline__ float2 rcp_(float2 a) { return crecipf(a); }
 __device__ __forceinline__ double2 rcp_(double2 a) { return crecip(a); }
-__device__ __forceinline__ float2 sqrt_(float2 a) { return csqrtf_(a); }
-__device__ __forceinline__ double2 sqrt_(double2 a) { return csqrtd(a); }
+// 1 / (principal square root).  complex128 without FP64 divisions and roots
+// (about 100 FP64 operations a lane): a complex64 estimate and two Newton steps
+// w <- w (3 - d w^2) / 2, which square its error.
+__device__ __forceinline__ float2 rsqrt_(float2 a) { return crecipf(csqrtf_(a)); }
+__device__ __forceinline__ double2 rsqrt_(double2 d) {
+    const float2 f = to_f(d);
+    const float m = fmaxf(fabsf(f.x), fabsf(f.y));
+    if (!(m > 1e-15f && m < 1e15f)) return crecip(csqrtd(d));
+    double2 w = to_d(crecipf(csqrtf_(f)));
+#pragma unroll
+    for (int it = 0; it < 2; it++) {
+        const double2 h = cmul(d, cmul(w, w));
+        w = cmul(w, cz(1.5 - 0.5 * h.x, -0.5 * h.y));
+    }
+    return w;
+}
 __device__ __forceinline__ float2 neg_(float2 a) { return cf(-a.x, -a.y); }
 __device__ __forceinline__ double2 neg_(double2 a) { return cz(-a.x, -a.y); }
 template <typename T>
@@ -107,8 +121,24 @@ __device__ __forceinline__ void load2(const double2 *p, double2 (&v)[2]) {
     v[1] = p[1];
 }
 
-constexpr int kT = kSubTile;      // 32
-constexpr int kP = kSubTile + 2;  // padded row of an operand tile (16-byte aligned rows)
+constexpr int kKT = 32;  // depth of a chunk of the dense products
+
+// Tile edge of the dense kernels and results a thread: 256 threads own a 32 x
+// 32 tile with 2 x 2 results each in complex64.  In complex128 a tile is bound
+// by its SM's FP64 pipe (32 x 32 x 32 takes 32 us) and the topmost fronts have
+// few tiles, so there it is 16 x 16, one result a thread; and fronts of at most
+// 32 nodes leave more of the elimination to the tiles.  Leaves of 16 / 24 / 32 /
+// 48 nodes: config-2 mixed forward 13.2 / 12.8 / 12.6 / 12.6 ms.
+template <typename T>
+struct Tile;
+template <>
+struct Tile<float2> {
+    static constexpr int E = 32, M = 2, P = 34, leaf = 32, emax = 64;
+};
+template <>
+struct Tile<double2> {
+    static constexpr int E = 16, M = 1, P = 17, leaf = 24, emax = 32;
+};
 
 // ------------------------------------------------------- values and scaling
 // fk: 1/sqrt|diagonal of the area part| (1 on Dirichlet rows); a zero
@@ -161,40 +191,40 @@ __global__ void k_sub_values(DevProblem P, DevSub D, const double2 *__restrict__
 // loads took longer than the elimination: 166 -> 60 us at e = 61, r = 321.)
 template <typename T>
 __global__ __launch_bounds__(256) void k_sub_gather(DevSub D, int t0) {
-    __shared__ int si[kSubCh][kT], sj[kSubCh][kT];
+    constexpr int E = Tile<T>::E, NZ = E * E / 256, RS = 256 / E;
+    __shared__ int si[kSubCh][E], sj[kSubCh][E];
     const SubTile tl = D.tA[t0 + blockIdx.x];
     const SubFront &t = D.fr[tl.front];
-    const int k = blockIdx.y, e = t.e, r = t.r, nch = t.nch, i0 = tl.ti * kT, j0 = tl.tj * kT;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int q = w; q < 2 * nch; q += 8) {
-        const int c = q >> 1, o = (q & 1 ? j0 : i0) + lane;
-        const int v = o < ((q & 1) ? e + r : e) ? D.inv[t.inv[c] + o] : -1;
-        (q & 1 ? sj : si)[c][lane] = v;
+    const int k = blockIdx.y, e = t.e, r = t.r, nch = t.nch, i0 = tl.ti * E, j0 = tl.tj * E;
+    const int col = threadIdx.x % E, row = threadIdx.x / E;
+    for (int q = threadIdx.x; q < 2 * nch * E; q += 256) {
+        const int c = q / (2 * E), b = q / E & 1, o = q % E, at = (b ? j0 : i0) + o;
+        (b ? sj : si)[c][o] = at < (b ? e + r : e) ? D.inv[t.inv[c] + at] : -1;
     }
     __syncthreads();
     const T *Sk = (const T *)D.S + (size_t)k * D.szS;
     T *F = (T *)D.F + (size_t)k * D.szF + t.oF, *H = (T *)D.H + (size_t)k * D.szG + t.oG;
-    T v[4];
+    T v[NZ];
 #pragma unroll
-    for (int z = 0; z < 4; z++) v[z] = zero_<T>();
+    for (int z = 0; z < NZ; z++) v[z] = zero_<T>();
     for (int c = 0; c < nch; c++) {
         const T *S = Sk + t.cS[c];
-        const int cr = t.cr[c], y = sj[c][lane];
-        T g[4];
+        const int cr = t.cr[c], y = sj[c][col];
+        T g[NZ];
 #pragma unroll
-        for (int z = 0; z < 4; z++) {
-            const int x = si[c][w + 8 * z];
+        for (int z = 0; z < NZ; z++) {
+            const int x = si[c][row + RS * z];
             g[z] = x >= 0 && y >= 0 ? S[(size_t)x * cr + y] : zero_<T>();
         }
 #pragma unroll
-        for (int z = 0; z < 4; z++) {
+        for (int z = 0; z < NZ; z++) {
             v[z].x += g[z].x;
             v[z].y += g[z].y;
         }
     }
 #pragma unroll
-    for (int z = 0; z < 4; z++) {
-        const int i = i0 + w + 8 * z, j = j0 + lane;
+    for (int z = 0; z < NZ; z++) {
+        const int i = i0 + row + RS * z, j = j0 + col;
         if (i >= e || j >= e + r) continue;
         if (j < e) F[(size_t)i * e + j] = v[z];
         else H[(size_t)i * r + j - e] = v[z];
@@ -297,141 +327,166 @@ __global__ __launch_bounds__(NT) void k_sub_pivot(DevSub D, int f0, int nnz) {
     if (bad) atomicCAS(&D.kbad[k], 0, 28);
 }
 
-// Four entries a thread of a 32 x 32 operand tile (rows w, w + 8, ..., column
-// = lane) in registers: the loads of the next chunk are in flight while the
-// present one is multiplied.
+// A thread's entries of a kKT x E operand tile (k-major) in registers: the
+// loads of the next chunk are in flight while the present one is multiplied.
 template <typename T>
-struct Quad {
-    T v[4];
+struct Operand {
+    static constexpr int E = Tile<T>::E, P = Tile<T>::P, N = kKT * E / 256;
+    T v[N];
+    // along a row of the tile: column threadIdx % E, rows row(0), row(1), ...
+    __device__ __forceinline__ static int col() { return threadIdx.x % E; }
+    __device__ __forceinline__ static int row(int z) { return threadIdx.x / E + (256 / E) * z; }
     __device__ __forceinline__ void load(const T *src, size_t ls, int nr, int nc) {
-        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
-        for (int z = 0; z < 4; z++)
-            v[z] = w + 8 * z < nr && lane < nc ? src[(size_t)(w + 8 * z) * ls + lane] : zero_<T>();
+        for (int z = 0; z < N; z++) v[z] = row(z) < nr && col() < nc ? src[(size_t)row(z) * ls + col()] : zero_<T>();
     }
     __device__ __forceinline__ void store(T *dst) const {
-        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
-        for (int z = 0; z < 4; z++) dst[(w + 8 * z) * kP + lane] = v[z];
+        for (int z = 0; z < N; z++) dst[row(z) * P + col()] = v[z];
     }
-    __device__ __forceinline__ void store_transposed(T *dst) const {
+    // from the transposed source, E rows of kKT: one warp a row
+    __device__ __forceinline__ void load_t(const T *src, size_t ls, int nr, int nc) {
         const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
-        for (int z = 0; z < 4; z++) dst[lane * kP + w + 8 * z] = v[z];
+        for (int z = 0; z < N; z++)
+            v[z] = w + 8 * z < nr && lane < nc ? src[(size_t)(w + 8 * z) * ls + lane] : zero_<T>();
+    }
+    __device__ __forceinline__ void store_t(T *dst) const {
+        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+        for (int z = 0; z < N; z++) dst[lane * P + w + 8 * z] = v[z];
     }
 };
 
-// 256 threads: RM x 2 outer products of k-major tiles, rows tr.., columns tc..
-template <typename T, int RM>
-__device__ __forceinline__ void tile_fma(const T *A, const T *Bm, int kk, int tr, int tc, T (&acc)[RM][2]) {
-#pragma unroll 8
-    for (int q = 0; q < kk; q++) {
-        T a[RM], b[2];
-        if constexpr (RM == 2) load2(A + q * kP + tr, a);
-        else a[0] = A[q * kP + tr];
-        load2(Bm + q * kP + tc, b);
+// a thread's M x M results of a tile: rows tr.., columns tc..
+template <typename T>
+struct Result {
+    static constexpr int M = Tile<T>::M, E = Tile<T>::E, P = Tile<T>::P;
+    T v[M][M];
+    __device__ __forceinline__ static int tr() { return threadIdx.x / (E / M) * M; }
+    __device__ __forceinline__ static int tc() { return threadIdx.x % (E / M) * M; }
+    // first row of the warp's results
+    __device__ __forceinline__ static int warp_row() { return (threadIdx.x & ~31) / (E / M) * M; }
+    __device__ __forceinline__ void clear() {
 #pragma unroll
-        for (int i = 0; i < RM; i++)
+        for (int i = 0; i < M; i++)
 #pragma unroll
-            for (int j = 0; j < 2; j++) fma_(acc[i][j], a[i], b[j]);
+            for (int j = 0; j < M; j++) v[i][j] = zero_<T>();
     }
-}
+    __device__ __forceinline__ void multiply(const T *A, const T *Bm, int kk) {
+        const int r = tr(), c = tc();
+#pragma unroll 8
+        for (int q = 0; q < kk; q++) {
+            if constexpr (M == 2) {
+                T a[2], b[2];
+                load2(A + q * P + r, a);
+                load2(Bm + q * P + c, b);
+#pragma unroll
+                for (int i = 0; i < 2; i++)
+#pragma unroll
+                    for (int j = 0; j < 2; j++) fma_(v[i][j], a[i], b[j]);
+            } else {
+                fma_(v[0][0], A[q * P + r], Bm[q * P + c]);
+            }
+        }
+    }
+};
 
 // G = F11^-1 F12
 template <typename T>
 __global__ __launch_bounds__(256) void k_sub_g(DevSub D, int t0) {
-    __shared__ __align__(16) T A[kT * kP], Bm[kT * kP];
+    constexpr int E = Tile<T>::E, M = Tile<T>::M, P = Tile<T>::P;
+    __shared__ __align__(16) T A[kKT * P], Bm[kKT * P];
     const SubTile tl = D.tG[t0 + blockIdx.x];
     const SubFront &t = D.fr[tl.front];
-    const int k = blockIdx.y, e = t.e, r = t.r, i0 = tl.ti * kT, j0 = tl.tj * kT;
+    const int k = blockIdx.y, e = t.e, r = t.r, i0 = tl.ti * E, j0 = tl.tj * E;
     const T *F = (const T *)D.F + (size_t)k * D.szF + t.oF, *H = (const T *)D.H + (size_t)k * D.szG + t.oG;
     T *G = (T *)D.G + (size_t)k * D.szG + t.oG;
-    T acc[2][2];
-    acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = zero_<T>();
-    const int tr = (threadIdx.x >> 4) * 2, tc = (threadIdx.x & 15) * 2;
-    const bool work = i0 + (threadIdx.x >> 5) * 4 < e;
-    Quad<T> a, b;
+    Result<T> acc;
+    acc.clear();
+    const bool work = i0 + acc.warp_row() < e;
+    Operand<T> a, b;
     a.load(F + i0, e, e, e - i0);  // symmetric: F[p][i]
     b.load(H + j0, r, e, r - j0);
-    for (int p = 0; p < e; p += kT) {
+    for (int p = 0; p < e; p += kKT) {
         a.store(A);
         b.store(Bm);
         __syncthreads();
-        if (p + kT < e) {
-            a.load(F + (size_t)(p + kT) * e + i0, e, e - p - kT, e - i0);
-            b.load(H + (size_t)(p + kT) * r + j0, r, e - p - kT, r - j0);
+        if (p + kKT < e) {
+            a.load(F + (size_t)(p + kKT) * e + i0, e, e - p - kKT, e - i0);
+            b.load(H + (size_t)(p + kKT) * r + j0, r, e - p - kKT, r - j0);
         }
-        if (work) tile_fma<T, 2>(A, Bm, min(kT, e - p), tr, tc, acc);
+        if (work) acc.multiply(A, Bm, min(kKT, e - p));
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 2; i++)
+    for (int ii = 0; ii < M; ii++)
 #pragma unroll
-        for (int j = 0; j < 2; j++)
-            if (i0 + tr + i < e && j0 + tc + j < r) G[(size_t)(i0 + tr + i) * r + j0 + tc + j] = acc[i][j];
+        for (int jj = 0; jj < M; jj++) {
+            const int i = i0 + acc.tr() + ii, j = j0 + acc.tc() + jj;
+            if (i < e && j < r) G[(size_t)i * r + j] = acc.v[ii][jj];
+        }
 }
 
 // S = (children's complements) - F12^T G, lower tiles, mirrored
 template <typename T>
 __global__ __launch_bounds__(256) void k_sub_s(DevSub D, int t0) {
-    __shared__ __align__(16) T A[kT * kP], Bm[kT * kP];
-    __shared__ int si[kSubCh][kT], sj[kSubCh][kT];
+    constexpr int E = Tile<T>::E, M = Tile<T>::M, P = Tile<T>::P;
+    __shared__ __align__(16) T A[kKT * P], Bm[kKT * P];
+    __shared__ int si[kSubCh][E], sj[kSubCh][E];
     const SubTile tl = D.tS[t0 + blockIdx.x];
     const SubFront &t = D.fr[tl.front];
-    const int k = blockIdx.y, e = t.e, r = t.r, nch = t.nch, i0 = tl.ti * kT, j0 = tl.tj * kT;
+    const int k = blockIdx.y, e = t.e, r = t.r, nch = t.nch, i0 = tl.ti * E, j0 = tl.tj * E;
     const T *H = (const T *)D.H + (size_t)k * D.szG + t.oG, *G = (const T *)D.G + (size_t)k * D.szG + t.oG;
     T *Sk = (T *)D.S + (size_t)k * D.szS, *S = Sk + t.oS;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    Quad<T> a, b;
+    Operand<T> a, b;
     a.load(H + i0, r, e, r - i0);
     b.load(G + j0, r, e, r - j0);
-    for (int q = w; q < 2 * nch; q += 8) {
-        const int c = q >> 1, o = (q & 1 ? j0 : i0) + lane;
-        (q & 1 ? sj : si)[c][lane] = o < r ? D.inv[t.inv[c] + e + o] : -1;
+    for (int q = threadIdx.x; q < 2 * nch * E; q += 256) {
+        const int c = q / (2 * E), bb = q / E & 1, o = q % E, at = (bb ? j0 : i0) + o;
+        (bb ? sj : si)[c][o] = at < r ? D.inv[t.inv[c] + e + at] : -1;
     }
     __syncthreads();
-    const int tr = (threadIdx.x >> 4) * 2, tc = (threadIdx.x & 15) * 2;
-    const bool work = i0 + w * 4 < r;
-    T sum[2][2], acc[2][2];
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int j = 0; j < 2; j++) acc[i][j] = sum[i][j] = zero_<T>();
+    Result<T> acc, sum;
+    acc.clear();
+    sum.clear();
+    const int tr = acc.tr(), tc = acc.tc();
+    const bool work = i0 + acc.warp_row() < r;
     for (int c = 0; c < nch; c++) {
         const T *Sc = Sk + t.cS[c];
         const int cr = t.cr[c];
 #pragma unroll
-        for (int i = 0; i < 2; i++)
+        for (int i = 0; i < M; i++)
 #pragma unroll
-            for (int j = 0; j < 2; j++) {
+            for (int j = 0; j < M; j++) {
                 const int x = si[c][tr + i], y = sj[c][tc + j];
                 if (x >= 0 && y >= 0) {
                     const T v = Sc[(size_t)x * cr + y];
-                    sum[i][j].x += v.x;
-                    sum[i][j].y += v.y;
+                    sum.v[i][j].x += v.x;
+                    sum.v[i][j].y += v.y;
                 }
             }
     }
-    for (int p = 0; p < e; p += kT) {
+    for (int p = 0; p < e; p += kKT) {
         a.store(A);
         b.store(Bm);
         __syncthreads();
-        if (p + kT < e) {
-            a.load(H + (size_t)(p + kT) * r + i0, r, e - p - kT, r - i0);
-            b.load(G + (size_t)(p + kT) * r + j0, r, e - p - kT, r - j0);
+        if (p + kKT < e) {
+            a.load(H + (size_t)(p + kKT) * r + i0, r, e - p - kKT, r - i0);
+            b.load(G + (size_t)(p + kKT) * r + j0, r, e - p - kKT, r - j0);
         }
-        if (work) tile_fma<T, 2>(A, Bm, min(kT, e - p), tr, tc, acc);
+        if (work) acc.multiply(A, Bm, min(kKT, e - p));
         __syncthreads();
     }
 #pragma unroll
-    for (int ii = 0; ii < 2; ii++)
+    for (int ii = 0; ii < M; ii++)
 #pragma unroll
-        for (int jj = 0; jj < 2; jj++) {
+        for (int jj = 0; jj < M; jj++) {
             const int i = i0 + tr + ii, j = j0 + tc + jj;
             if (i >= r || j > i) continue;
-            T v = sum[ii][jj];
-            v.x -= acc[ii][jj].x;
-            v.y -= acc[ii][jj].y;
+            T v = sum.v[ii][jj];
+            v.x -= acc.v[ii][jj].x;
+            v.y -= acc.v[ii][jj].y;
             S[(size_t)i * r + j] = v;
             S[(size_t)j * r + i] = v;
         }
@@ -637,7 +692,7 @@ __global__ __launch_bounds__(kRT) void k_sub_root(DevSub D, SubBatch B) {
                         if (wid == ww) {
                             const T d = shfl_(a[q], p);
                             if (is_bad(d)) bad = true;
-                            const T iv = rcp_(sqrt_(d));
+                            const T iv = rsqrt_(d);
                             col[buf][row] = row > p ? mul_(a[q], iv) : zero_<T>();
                             if (lane == 0) inv[buf] = iv;
                         }
@@ -776,48 +831,45 @@ __global__ __launch_bounds__(kST) void k_sub_root_solve(DevSub D, SubBatch B, co
 
 // Up the tree: b_E (own right-hand sides and the children's updates) goes to
 // W, the update rows U = (children's updates) - G^T b_E to the parent.  One
-// block per 32 update rows x 32 electrodes.
+// block per tile of update rows x electrodes.
 template <typename T>
 __global__ __launch_bounds__(256) void k_sub_up(DevSub D, SubBatch B, int t0, const int *nprev) {
-    __shared__ __align__(16) T A[kT * kP], Bm[kT * kP];
-    __shared__ int se[kSubCh][kSubEMax], sr[kSubCh][kT];
+    constexpr int E = Tile<T>::E, M = Tile<T>::M, P = Tile<T>::P;
+    __shared__ __align__(16) T A[kKT * P], Bm[kKT * P];
+    __shared__ int se[kSubCh][kSubEMax], sr[kSubCh][E];
     if (nprev && *nprev == 0) return;
     const int kk = blockIdx.z, k = B.k0 + kk;
     if (B.kact && !B.kact[kk]) return;
     const SubTile tl = D.tU[t0 + blockIdx.x];
     const SubFront &t = D.fr[tl.front];
-    const int e = t.e, r = t.r, nch = t.nch, i0 = tl.ti * kT, l0 = blockIdx.y * kT, L = B.Lb, nl = min(kT, L - l0);
+    const int e = t.e, r = t.r, nch = t.nch, i0 = tl.ti * E, l0 = blockIdx.y * E, L = B.Lb, nl = min(E, L - l0);
     const T *G = (const T *)D.G + (size_t)k * D.szG + t.oG;
     const T *__restrict__ Y = (const T *)B.Y + ((size_t)kk * D.n + t.nd0) * L + l0;
     T *__restrict__ W = (T *)B.W + ((size_t)kk * D.n + t.nd0) * L + l0;
     T *Uk = (T *)B.U + (size_t)kk * D.szU * L + l0;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int q = threadIdx.x; q < nch * kSubEMax; q += 256) {
         const int c = q / kSubEMax, o = q % kSubEMax;
         if (o < e) se[c][o] = D.inv[t.inv[c] + o];
     }
-    for (int q = threadIdx.x; q < nch * kT; q += 256) {
-        const int c = q / kT, o = q % kT;
+    for (int q = threadIdx.x; q < nch * E; q += 256) {
+        const int c = q / E, o = q % E;
         sr[c][o] = i0 + o < r ? D.inv[t.inv[c] + e + i0 + o] : -1;
     }
     __syncthreads();
-    Quad<T> a, b;
+    Operand<T> a, b;
+    const int col = b.col();
     auto load_b = [&](int p) {
-#pragma unroll
-        for (int z = 0; z < 4; z++) {
-            const int q = p + w + 8 * z;
-            b.v[z] = q < e && lane < nl ? Y[(size_t)q * L + lane] : zero_<T>();
-        }
+        b.load(Y + (size_t)p * L, L, e - p, nl);
         for (int c = 0; c < nch; c++) {
-            const T *U = Uk + (size_t)t.cu[c] * L + lane;
-            T g[4];
+            const T *U = Uk + (size_t)t.cu[c] * L + col;
+            T g[Operand<T>::N];
 #pragma unroll
-            for (int z = 0; z < 4; z++) {
-                const int q = p + w + 8 * z, x = q < e && lane < nl ? se[c][q] : -1;
+            for (int z = 0; z < Operand<T>::N; z++) {
+                const int q = p + b.row(z), x = q < e && col < nl ? se[c][q] : -1;
                 g[z] = x >= 0 ? U[(size_t)x * L] : zero_<T>();
             }
 #pragma unroll
-            for (int z = 0; z < 4; z++) {
+            for (int z = 0; z < Operand<T>::N; z++) {
                 b.v[z].x += g[z].x;
                 b.v[z].y += g[z].y;
             }
@@ -825,130 +877,119 @@ __global__ __launch_bounds__(256) void k_sub_up(DevSub D, SubBatch B, int t0, co
     };
     a.load(G + i0, r, e, r - i0);
     load_b(0);
-    // the children's updates of this thread's four results
-    const int tr = (threadIdx.x >> 4) * 2, tc = (threadIdx.x & 15) * 2;
-    const bool work = i0 + w * 4 < r;
-    T sum[2][2], acc[2][2];
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int j = 0; j < 2; j++) acc[i][j] = sum[i][j] = zero_<T>();
+    // the children's updates of this thread's results
+    Result<T> acc, sum;
+    acc.clear();
+    sum.clear();
+    const int tr = acc.tr(), tc = acc.tc();
+    const bool work = i0 + acc.warp_row() < r;
     for (int c = 0; c < nch; c++) {
         const T *U = Uk + (size_t)t.cu[c] * L;
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
+        for (int i = 0; i < M; i++) {
             const int x = sr[c][tr + i];
 #pragma unroll
-            for (int j = 0; j < 2; j++)
+            for (int j = 0; j < M; j++)
                 if (x >= 0 && tc + j < nl) {
                     const T v = U[(size_t)x * L + tc + j];
-                    sum[i][j].x += v.x;
-                    sum[i][j].y += v.y;
+                    sum.v[i][j].x += v.x;
+                    sum.v[i][j].y += v.y;
                 }
         }
     }
-    for (int p = 0; p < e; p += kT) {
+    for (int p = 0; p < e; p += kKT) {
         a.store(A);
         b.store(Bm);
         if (tl.ti == 0) {
 #pragma unroll
-            for (int z = 0; z < 4; z++)
-                if (p + w + 8 * z < e && lane < nl) W[(size_t)(p + w + 8 * z) * L + lane] = b.v[z];
+            for (int z = 0; z < Operand<T>::N; z++)
+                if (p + b.row(z) < e && col < nl) W[(size_t)(p + b.row(z)) * L + col] = b.v[z];
         }
         __syncthreads();
-        if (p + kT < e) {
-            a.load(G + (size_t)(p + kT) * r + i0, r, e - p - kT, r - i0);
-            load_b(p + kT);
+        if (p + kKT < e) {
+            a.load(G + (size_t)(p + kKT) * r + i0, r, e - p - kKT, r - i0);
+            load_b(p + kKT);
         }
-        if (work) tile_fma<T, 2>(A, Bm, min(kT, e - p), tr, tc, acc);
+        if (work) acc.multiply(A, Bm, min(kKT, e - p));
         __syncthreads();
     }
     T *U = Uk + (size_t)t.u0 * L;
 #pragma unroll
-    for (int i = 0; i < 2; i++)
+    for (int i = 0; i < M; i++)
 #pragma unroll
-        for (int j = 0; j < 2; j++)
+        for (int j = 0; j < M; j++)
             if (i0 + tr + i < r && tc + j < nl) {
-                T v = sum[i][j];
-                v.x -= acc[i][j].x;
-                v.y -= acc[i][j].y;
+                T v = sum.v[i][j];
+                v.x -= acc.v[i][j].x;
+                v.y -= acc.v[i][j].y;
                 U[(size_t)(i0 + tr + i) * L + tc + j] = v;
             }
 }
 
-// Down the tree: x_E = F11^-1 b_E - G x_R, one block per 16 RM rows x 32
-// electrodes (RM 1 in complex128: the topmost fronts are few, and a tile is
-// bound by its SM's FP64 pipe).
-template <typename T>
-struct DownShape {
-    static constexpr int RM = sizeof(T) == 8 ? 2 : 1;
-};
-
+// Down the tree: x_E = F11^-1 b_E - G x_R, one block per tile of rows x
+// electrodes
 template <typename T>
 __global__ __launch_bounds__(256) void k_sub_down(DevSub D, SubBatch B, int t0, const int *nprev) {
-    constexpr int RM = DownShape<T>::RM, BM = 16 * RM, kIdx = 512;
-    __shared__ __align__(16) T A[kT * kP], Bm[kT * kP];
+    constexpr int E = Tile<T>::E, M = Tile<T>::M, P = Tile<T>::P, kIdx = 512;
+    __shared__ __align__(16) T A[kKT * P], Bm[kKT * P];
     __shared__ int sidx[kIdx];
     if (nprev && *nprev == 0) return;
     const int kk = blockIdx.z, k = B.k0 + kk;
     if (B.kact && !B.kact[kk]) return;
     const SubTile tl = D.tD[t0 + blockIdx.x];
     const SubFront &t = D.fr[tl.front];
-    const int e = t.e, r = t.r, i0 = tl.ti * BM, l0 = blockIdx.y * kT, L = B.Lb, nl = min(kT, L - l0);
+    const int e = t.e, r = t.r, i0 = tl.ti * E, l0 = blockIdx.y * E, L = B.Lb, nl = min(E, L - l0);
     const T *F = (const T *)D.F + (size_t)k * D.szF + t.oF, *G = (const T *)D.G + (size_t)k * D.szG + t.oG;
     const T *W = (const T *)B.W + ((size_t)kk * D.n + t.nd0) * L + l0;
     T *Zk = (T *)B.Z + (size_t)kk * D.n * L + l0;
     const int32_t *rows = D.rows + t.rows0;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int tr = (threadIdx.x >> 4) * RM, tc = (threadIdx.x & 15) * 2;
-    const bool work = i0 + w * 2 * RM < e;
     for (int q = threadIdx.x; q < min(r, kIdx); q += 256) sidx[q] = rows[q];
     __syncthreads();
-    Quad<T> a, b;
-    // chunks of 32: first the columns of G, then those of F11^-1
-    const int nr = (r + kT - 1) / kT, nc = nr + (e + kT - 1) / kT;
+    Operand<T> a, b;
+    Result<T> acc;
+    acc.clear();
+    const int tr = acc.tr(), tc = acc.tc();
+    const bool work = i0 + acc.warp_row() < e;
+    // chunks: first the columns of G, then those of F11^-1
+    const int nr = (r + kKT - 1) / kKT, nc = nr + (e + kKT - 1) / kKT;
     auto load = [&](int ch) {
         if (ch < nr) {
-            const int p = ch * kT;
-            a.load(G + (size_t)i0 * r + p, r, min(BM, e - i0), r - p);  // along the rows of G: transposed below
+            const int p = ch * kKT;
+            a.load_t(G + (size_t)i0 * r + p, r, e - i0, r - p);
 #pragma unroll
-            for (int z = 0; z < 4; z++) {
-                const int q = p + w + 8 * z;
+            for (int z = 0; z < Operand<T>::N; z++) {
+                const int q = p + b.row(z);
                 b.v[z] = zero_<T>();
-                if (q < r && lane < nl) b.v[z] = Zk[(size_t)(q < kIdx ? sidx[q] : rows[q]) * L + lane];
+                if (q < r && b.col() < nl) b.v[z] = Zk[(size_t)(q < kIdx ? sidx[q] : rows[q]) * L + b.col()];
             }
         } else {
-            const int p = (ch - nr) * kT;
-            a.load(F + (size_t)p * e + i0, e, e - p, min(BM, e - i0));
+            const int p = (ch - nr) * kKT;
+            a.load(F + (size_t)p * e + i0, e, e - p, e - i0);
             b.load(W + (size_t)p * L, L, e - p, nl);
         }
     };
-    T acc[RM][2];
-#pragma unroll
-    for (int i = 0; i < RM; i++) acc[i][0] = acc[i][1] = zero_<T>();
     load(0);
     for (int ch = 0; ch < nc; ch++) {
-        if (ch < nr) a.store_transposed(A);
+        if (ch < nr) a.store_t(A);
         else a.store(A);
         b.store(Bm);
         __syncthreads();
         if (ch + 1 < nc) load(ch + 1);
         if (ch == nr) {
 #pragma unroll
-            for (int i = 0; i < RM; i++) {
-                acc[i][0] = neg_(acc[i][0]);
-                acc[i][1] = neg_(acc[i][1]);
-            }
+            for (int i = 0; i < M; i++)
+#pragma unroll
+                for (int j = 0; j < M; j++) acc.v[i][j] = neg_(acc.v[i][j]);
         }
-        if (work) tile_fma<T, RM>(A, Bm, ch < nr ? min(kT, r - ch * kT) : min(kT, e - (ch - nr) * kT), tr, tc, acc);
+        if (work) acc.multiply(A, Bm, ch < nr ? min(kKT, r - ch * kKT) : min(kKT, e - (ch - nr) * kKT));
         __syncthreads();
     }
     T *Z = Zk + (size_t)t.nd0 * L;
 #pragma unroll
-    for (int i = 0; i < RM; i++)
+    for (int i = 0; i < M; i++)
 #pragma unroll
-        for (int j = 0; j < 2; j++)
-            if (i0 + tr + i < e && tc + j < nl) Z[(size_t)(i0 + tr + i) * L + tc + j] = acc[i][j];
+        for (int j = 0; j < M; j++)
+            if (i0 + tr + i < e && tc + j < nl) Z[(size_t)(i0 + tr + i) * L + tc + j] = acc.v[i][j];
 }
 
 // -------------------------------------------------- vectors of a rectangle
@@ -1153,7 +1194,7 @@ void root_t(const DevProblem &P, const DevSub &D, const SubBatch &B, const doubl
 
 template <typename T>
 int apply_t(const DevSub &D, const SubPlan &sp, const SubBatch &B, const int *nprev, cudaStream_t st) {
-    const int lt = (B.Lb + kT - 1) / kT;
+    const int lt = (B.Lb + Tile<T>::E - 1) / Tile<T>::E;
     for (int lv = 0; lv < sp.nlevel; lv++)
         k_sub_up<T><<<dim3(sp.lU[lv + 1] - sp.lU[lv], lt, B.Kb), 256, 0, st>>>(D, B, sp.lU[lv], nprev);
     k_sub_root_solve<T><<<B.Kb * B.Lb, kST, sizeof(T) * D.mp, st>>>(D, B, nprev);
@@ -1177,7 +1218,10 @@ void sub_launch_values(const DevProblem &P, const DevSub &D, const double2 *sigm
     k_sub_values<<<dim3(nb(P.nnz, 256), P.K), 256, 0, st>>>(P, D, adom);
 }
 
-int sub_down_rows(bool mixed) { return 16 * (mixed ? DownShape<float2>::RM : DownShape<double2>::RM); }
+SubShape sub_shape(bool mixed) {
+    if (mixed) return {Tile<float2>::leaf, Tile<float2>::emax, Tile<float2>::E};
+    return {Tile<double2>::leaf, Tile<double2>::emax, Tile<double2>::E};
+}
 
 int sub_root_block(bool mixed) { return mixed ? RootShape<float2>::NB : RootShape<double2>::NB; }
 

@@ -39,7 +39,7 @@ struct SubBatch {
     unsigned long long *mz, *mx;    // per system: bit patterns of the largest correction and solution
 };
 
-int sub_down_rows(bool mixed);   // rows of a tile of the downward solve
+SubShape sub_shape(bool mixed);
 int sub_root_block(bool mixed);  // columns of a block of the root factor
 void sub_launch_values(const DevProblem &P, const DevSub &D, const double2 *sigma, const double2 *adom, cudaStream_t st);
 int sub_launch_factor(const DevProblem &P, const DevSub &D, const SubPlan &sp, bool mixed, cudaStream_t st);
