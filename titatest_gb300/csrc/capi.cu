@@ -411,10 +411,7 @@ int ensure_sub_batch(crgpu_ctx *c, int want) {
     e = e ? e : dalloc(c, &C, w * c->D.mp * c->D.ldc * esz);
     B.C = C;
     e = e ? e : dalloc(c, &B.bval, w * c->D.n_be);
-    if (mixed) {
-        e = e ? e : dalloc(c, &B.X, w * n);
-        e = e ? e : dalloc(c, &B.Bt, w * n);
-    }
+    if (mixed) e = e ? e : dalloc(c, &B.X, w * n);
     e = e ? e : dalloc(c, &Y, w * n * esz);
     B.Y = Y;
     e = e ? e : dalloc(c, &W, w * n * esz);
@@ -471,8 +468,13 @@ int sub_factor_rect(crgpu_ctx *c, const SubBatch &B) {
 // Solves the rectangle for the right-hand sides of kompab (src null) or for
 // the rows of src; the solution ends in B.X.  Mixed precision refines as
 // solve_view does: every step is launched without waiting for the host.
-int sub_solve_rect(crgpu_ctx *c, const SubBatch &B, const double2 *src) {
+int sub_solve_rect(crgpu_ctx *c, SubBatch B, const double2 *src) {
     const bool mixed = c->precision == CRGPU_MIXED;
+    if (mixed && src && !c->SB.Bt) {  // the adjoint's right-hand sides are kept for the residuals
+        int e = dalloc(c, &c->SB.Bt, (size_t)c->sub_cap * c->hg.n);
+        if (e) return e;
+    }
+    B.Bt = c->SB.Bt;
     SubBatch B0 = B;
     B0.kact = nullptr;
     sub_launch_rhs(c->P, c->D, B, mixed, c->lsink, c->nsink, src, c->st);
@@ -485,7 +487,7 @@ int sub_solve_rect(crgpu_ctx *c, const SubBatch &B, const double2 *src) {
     c->stats.kernel_launches += 2;
     for (int it = 0; it < steps; it++) {
         const int *nprev = it > 0 ? &cnt[it - 1].n : nullptr;
-        sub_launch_residual(c->P, c->D, B, nprev, c->st);
+        sub_launch_residual(c->P, c->D, B, src == nullptr, c->lsink, c->nsink, nprev, c->st);
         c->stats.kernel_launches += 3 + sub_launch_apply(c->D, c->sp, B, true, nprev, c->st);
         sub_launch_accumulate(c->D, B, false, c->refine_tol, nprev, &cnt[it].n, &cnt[it].z, c->st);
     }

@@ -63,6 +63,30 @@ __device__ __forceinline__ double2 rsqrt_(double2 d) {
 }
 __device__ __forceinline__ float2 neg_(float2 a) { return cf(-a.x, -a.y); }
 __device__ __forceinline__ double2 neg_(double2 a) { return cz(-a.x, -a.y); }
+// float <-> double by their bit fields: the conversion instructions share the
+// FP64 pipe (2 lanes a cycle and SM).  Exact as (double)v; zeros, subnormals,
+// infinities and NaN take the instruction.
+__device__ __forceinline__ double widen(float v) {
+    const unsigned b = __float_as_uint(v), e = (b >> 23) & 255u;
+    if (e - 1u >= 254u) return (double)v;
+    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
+}
+// (float)v, to nearest even
+__device__ __forceinline__ float narrow(double v) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    const unsigned e = (unsigned)(b >> 52) & 2047u;
+    if (e - 897u >= 253u) return (float)v;  // outside the normal floats below their last binade
+    unsigned long long t = (b & 0x7fffffffffffffffull) - (896ull << 52);
+    t += 0x0fffffffull + ((t >> 29) & 1ull);
+    return __uint_as_float((unsigned)(t >> 29) | ((unsigned)(b >> 32) & 0x80000000u));
+}
+__device__ __forceinline__ double2 widen(float2 v) { return cz(widen(v.x), widen(v.y)); }
+__device__ __forceinline__ float2 narrow(double2 v) { return cf(narrow(v.x), narrow(v.y)); }
+// bit pattern of |v|: the patterns of non-negative doubles order like the values
+__device__ __forceinline__ unsigned long long abs_bits(double v) {
+    return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+}
+
 template <typename T>
 __device__ __forceinline__ T from_(double2 v);
 template <>
@@ -993,31 +1017,52 @@ __global__ __launch_bounds__(256) void k_sub_down(DevSub D, SubBatch B, int t0, 
 }
 
 // -------------------------------------------------- vectors of a rectangle
-// Right-hand sides, scaled by fk: the unit sink at the electrode and the
-// fictitious sink (src/kompab.f90:180-190), or the rows of src ([eanz][n]).
+// Right-hand sides from the rows of src ([eanz][n]), scaled by fk
 template <typename T>
-__global__ void k_sub_rhs(DevProblem P, DevSub D, SubBatch B, int lsink, int nsink,
-                          const double2 *__restrict__ src, int keep) {
+__global__ void k_sub_rhs(DevProblem P, DevSub D, SubBatch B, const double2 *__restrict__ src, int keep) {
     const int l = blockIdx.y * 32 + (threadIdx.x & 31), p = blockIdx.x * 8 + (threadIdx.x >> 5), kk = blockIdx.z;
     if (l >= B.Lb || p >= D.n) return;
-    const int i = D.node[p], el = B.l0 + l;
-    double2 v = cz(0.0, 0.0);
-    if (src) v = src[(size_t)el * P.n + i];
-    else {
-        if (i == P.enr0[el]) v = cz(-1.0, 0.0);
-        if (lsink && i == nsink) v = cz(1.0, 0.0);
-    }
-    if (P.dirichlet[i]) v = cz(0.0, 0.0);
-    const double f = D.fk[(size_t)(B.k0 + kk) * P.n + i];
-    v = cz(v.x * f, v.y * f);
+    const int i = D.node[p];
+    double2 v = P.dirichlet[i] ? cz(0.0, 0.0) : src[(size_t)(B.l0 + l) * P.n + i];
     const size_t at = ((size_t)kk * D.n + p) * B.Lb + l;
+    if (v.x != 0.0 || v.y != 0.0) {  // the adjoint sources are zero but at the electrodes
+        const double f = D.fk[(size_t)(B.k0 + kk) * P.n + i];
+        v = cz(v.x * f, v.y * f);
+    }
     if (keep) B.Bt[at] = v;
     ((T *)B.Y)[at] = from_<T>(v);
 }
 
+// kompab's right-hand side of electrode l at node i (src/kompab.f90:180-190):
+// the unit sink at the electrode, the fictitious sink, zero on Dirichlet nodes
+__device__ __forceinline__ double unit_rhs(const DevProblem &P, int el, int i, int lsink, int nsink) {
+    if (P.dirichlet[i]) return 0.0;
+    if (lsink && i == nsink) return 1.0;
+    return i == P.enr0[el] ? -1.0 : 0.0;
+}
+
+// ... scaled by fk, into a zeroed Y: one thread per system
+template <typename T>
+__global__ void k_sub_unit_rhs(DevProblem P, DevSub D, SubBatch B, int lsink, int nsink) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= B.Kb * B.Lb) return;
+    const int kk = s / B.Lb, l = s % B.Lb, el = B.l0 + l;
+    const int nodes[2] = {P.enr0[el], lsink ? nsink : -1};
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        const int i = nodes[q];
+        if (i < 0) continue;
+        const double v = unit_rhs(P, el, i, lsink, nsink) * D.fk[(size_t)(B.k0 + kk) * P.n + i];
+        ((T *)B.Y)[((size_t)kk * D.n + D.pos[i]) * B.Lb + l] = from_<T>(cz(v, 0.0));
+    }
+}
+
 // Y = b - A x in FP64 (rounded to complex64 at the end): one warp per row, the
 // electrodes across its lanes, so the matrix entries are one broadcast load.
-__global__ __launch_bounds__(256) void k_sub_residual(DevProblem P, DevSub D, SubBatch B, const int *nprev) {
+// Bound by the FP64 pipe: 36 fused multiply-adds a node and system.  unit: b
+// is kompab's, else B.Bt.
+__global__ __launch_bounds__(256) void k_sub_residual(DevProblem P, DevSub D, SubBatch B, int unit, int lsink,
+                                                      int nsink, const int *nprev) {
     if (nprev && *nprev == 0) return;
     const int kk = blockIdx.z, k = B.k0 + kk, L = B.Lb;
     if (!B.kact[kk]) return;
@@ -1034,50 +1079,65 @@ __global__ __launch_bounds__(256) void k_sub_residual(DevProblem P, DevSub D, Su
             fma_(acc, bv[(size_t)D.rb_ent[q] * L], X[(size_t)D.rb_pos[q] * L]);
     }
     const size_t at = ((size_t)kk * D.n + p) * L + l;
-    const double2 b = B.Bt[at];
-    ((float2 *)B.Y)[at] = to_f(cz(b.x - acc.x, b.y - acc.y));
+    double2 b = cz(0.0, 0.0);
+    if (!unit) {
+        b = B.Bt[at];
+    } else {
+        const double v = unit_rhs(P, B.l0 + l, i, lsink, nsink);
+        if (v != 0.0) b.x = v * D.fk[(size_t)k * P.n + i];
+    }
+    ((float2 *)B.Y)[at] = narrow(cz(b.x - acc.x, b.y - acc.y));
 }
 
-constexpr int kAccRows = 256;
+constexpr int kAccRows = 128;
 
-// X (+)= Z with the largest entries of both per system
+// X (+)= Z with the largest entries of both per system (as bit patterns)
 __global__ __launch_bounds__(256) void k_sub_accumulate(DevSub D, SubBatch B, int first, const int *nprev) {
     if (nprev && *nprev == 0) return;
     const int kk = blockIdx.z, L = B.Lb;
     if (!first && !B.kact[kk]) return;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, l = blockIdx.y * 32 + lane;
     const bool on = l < L && (first || B.active[kk * L + l]);
-    double mz = 0.0, mx = 0.0;
+    float mz = 0.f;
+    bool nan = false;
+    unsigned long long mx = 0ull;
     if (on) {
-        const size_t base = (size_t)kk * D.n * L + l;
-        const int p1 = min(D.n, (int)(blockIdx.x + 1) * kAccRows);
-        for (int p = blockIdx.x * kAccRows + w; p < p1; p += 8) {
-            const size_t at = base + (size_t)p * L;
-            const double2 z = to_d(((const float2 *)B.Z)[at]);
-            double2 x = z;
-            if (!first) {
-                x = B.X[at];
-                x = cz(x.x + z.x, x.y + z.y);
-            }
-            B.X[at] = x;
-            // a NaN wins every later comparison: fmax would drop it
-            const double az = fmax(fabs(z.x), fabs(z.y)), ax = fmax(fabs(x.x), fabs(x.y));
-            mz = (az > mz || z.x != z.x || z.y != z.y) ? (z.x != z.x || z.y != z.y ? INFINITY : az) : mz;
-            mx = ax > mx ? ax : mx;
+        const float2 *__restrict__ Z = (const float2 *)B.Z + (size_t)kk * D.n * L + l;
+        double2 *__restrict__ X = B.X + (size_t)kk * D.n * L + l;
+        const int p0 = blockIdx.x * kAccRows + w, p1 = min(D.n, (int)(blockIdx.x + 1) * kAccRows);
+        for (int p = p0; p < p1; p += 32) {
+            float2 z[4];
+            double2 x[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (p + 8 * q < p1) {
+                    z[q] = Z[(size_t)(p + 8 * q) * L];
+                    if (!first) x[q] = X[(size_t)(p + 8 * q) * L];
+                }
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (p + 8 * q < p1) {
+                    const double2 zd = widen(z[q]), v = first ? zd : cz(x[q].x + zd.x, x[q].y + zd.y);
+                    X[(size_t)(p + 8 * q) * L] = v;
+                    mz = fmaxf(mz, fmaxf(fabsf(z[q].x), fabsf(z[q].y)));
+                    nan = nan || z[q].x != z[q].x || z[q].y != z[q].y;  // fmaxf drops them
+                    mx = max(mx, max(abs_bits(v.x), abs_bits(v.y)));
+                }
         }
     }
-    __shared__ double sz[8][32], sx[8][32];
-    sz[w][lane] = mz;
+    __shared__ float sz[8][32];
+    __shared__ unsigned long long sx[8][32];
+    sz[w][lane] = nan ? INFINITY : mz;
     sx[w][lane] = mx;
     __syncthreads();
     if (w == 0 && on) {
+        mz = sz[0][lane];
         for (int q = 1; q < 8; q++) {
-            mz = fmax(mz, sz[q][lane]);
-            mx = fmax(mx, sx[q][lane]);
+            mz = fmaxf(mz, sz[q][lane]);
+            mx = max(mx, sx[q][lane]);
         }
-        // bit patterns of non-negative doubles order like the values
-        atomicMax(&B.mz[kk * L + l], (unsigned long long)__double_as_longlong(mz));
-        atomicMax(&B.mx[kk * L + l], (unsigned long long)__double_as_longlong(mx));
+        atomicMax(&B.mz[kk * L + l], abs_bits(widen(mz)));
+        atomicMax(&B.mx[kk * L + l], mx);
     }
 }
 
@@ -1138,9 +1198,10 @@ __global__ __launch_bounds__(256) void k_sub_unpack(DevProblem P, DevSub D, SubB
         const size_t at = ((size_t)k * P.eanz + B.l0 + l0 + q) * P.n + n0 + a;
         out[at] = v;
         if (out32) {
-            const float2 hi = to_f(v);
+            const float2 hi = narrow(v);
+            const double2 h = widen(hi);
             out32[at] = hi;
-            out32[at + (size_t)P.K * P.eanz * P.n] = cf((float)(v.x - (double)hi.x), (float)(v.y - (double)hi.y));
+            out32[at + (size_t)P.K * P.eanz * P.n] = narrow(cz(v.x - h.x, v.y - h.y));
         }
     }
 }
@@ -1241,13 +1302,21 @@ int sub_launch_apply(const DevSub &D, const SubPlan &sp, const SubBatch &B, bool
 
 void sub_launch_rhs(const DevProblem &P, const DevSub &D, const SubBatch &B, bool mixed, int lsink, int nsink,
                     const double2 *src, cudaStream_t st) {
+    if (!src) {
+        const int ns = B.Kb * B.Lb;
+        cudaMemsetAsync(B.Y, 0, (mixed ? sizeof(float2) : sizeof(double2)) * (size_t)ns * D.n, st);
+        if (mixed) k_sub_unit_rhs<float2><<<nb(ns, 128), 128, 0, st>>>(P, D, B, lsink, nsink);
+        else k_sub_unit_rhs<double2><<<nb(ns, 128), 128, 0, st>>>(P, D, B, lsink, nsink);
+        return;
+    }
     const dim3 g(nb(D.n, 8), nb(B.Lb, 32), B.Kb);
-    if (mixed) k_sub_rhs<float2><<<g, 256, 0, st>>>(P, D, B, lsink, nsink, src, 1);
-    else k_sub_rhs<double2><<<g, 256, 0, st>>>(P, D, B, lsink, nsink, src, 0);
+    if (mixed) k_sub_rhs<float2><<<g, 256, 0, st>>>(P, D, B, src, 1);
+    else k_sub_rhs<double2><<<g, 256, 0, st>>>(P, D, B, src, 0);
 }
 
-void sub_launch_residual(const DevProblem &P, const DevSub &D, const SubBatch &B, const int *nprev, cudaStream_t st) {
-    k_sub_residual<<<dim3(nb(D.n, 8), nb(B.Lb, 32), B.Kb), 256, 0, st>>>(P, D, B, nprev);
+void sub_launch_residual(const DevProblem &P, const DevSub &D, const SubBatch &B, bool unit, int lsink, int nsink,
+                         const int *nprev, cudaStream_t st) {
+    k_sub_residual<<<dim3(nb(D.n, 8), nb(B.Lb, 32), B.Kb), 256, 0, st>>>(P, D, B, unit ? 1 : 0, lsink, nsink, nprev);
 }
 
 void sub_launch_accumulate(const DevSub &D, const SubBatch &B, bool first, double tol, const int *nprev, int *nactive,

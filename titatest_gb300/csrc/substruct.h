@@ -33,7 +33,7 @@ struct SubBatch {
     int k0, Kb, l0, Lb;
     void *C;                        // [Kb * Lb][mp * ldc] root factors
     double2 *bval;                  // [Kb][n_be][Lb] boundary terms of the root entries
-    double2 *X, *Bt;                // solution, right-hand side (scaled by fk)
+    double2 *X, *Bt;                // solution; right-hand side of the adjoint (scaled by fk)
     void *Y, *W, *Z, *U;            // input, assembled input, output, update rows
     int *status, *active, *kact;    // per system, per system, per wavenumber (null: all)
     unsigned long long *mz, *mx;    // per system: bit patterns of the largest correction and solution
@@ -49,7 +49,8 @@ int sub_launch_apply(const DevSub &D, const SubPlan &sp, const SubBatch &B, bool
                      cudaStream_t st);
 void sub_launch_rhs(const DevProblem &P, const DevSub &D, const SubBatch &B, bool mixed, int lsink, int nsink,
                     const double2 *src, cudaStream_t st);
-void sub_launch_residual(const DevProblem &P, const DevSub &D, const SubBatch &B, const int *nprev, cudaStream_t st);
+void sub_launch_residual(const DevProblem &P, const DevSub &D, const SubBatch &B, bool unit, int lsink, int nsink,
+                         const int *nprev, cudaStream_t st);
 void sub_launch_accumulate(const DevSub &D, const SubBatch &B, bool first, double tol, const int *nprev, int *nactive,
                            double *zmax, cudaStream_t st);
 void sub_launch_unpack(const DevProblem &P, const DevSub &D, const SubBatch &B, double sign, double2 *out,
