@@ -1040,7 +1040,7 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
         D.nI = sp.nI;
         const int nb = sub_root_block(precision == CRGPU_MIXED);
         D.mp = (sp.m + nb - 1) / nb * nb;
-        D.ldc = D.mp + 64 - nb;  // the last rows' tile of 64 stays inside
+        D.ldc = D.mp + sub_root_rows(precision == CRGPU_MIXED) - nb;  // the last rows' tile stays inside
         D.szU = sp.szU;
         D.szF = sp.szF;
         D.szG = sp.szG;

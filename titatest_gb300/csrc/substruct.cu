@@ -20,6 +20,7 @@
 
 #include "async.cuh"
 #include "kernels.h"
+#include "mixed_common.cuh"
 #include "substruct.h"
 
 namespace crgpu {
@@ -48,7 +49,7 @@ __device__ __forceinline__ double2 rcp_(double2 a) { return crecip(a); }
 // 1 / (principal square root).  complex128 without FP64 divisions and roots
 // (about 100 FP64 operations a lane): a complex64 estimate and two Newton steps
 // w <- w (3 - d w^2) / 2, which square its error.
-__device__ __forceinline__ float2 rsqrt_(float2 a) { return crecipf(csqrtf_(a)); }
+__device__ __forceinline__ float2 rsqrt_(float2 a) { return crecip_fast(csqrt_fast(a)); }
 __device__ __forceinline__ double2 rsqrt_(double2 d) {
     const float2 f = to_f(d);
     const float m = fmaxf(fabsf(f.x), fabsf(f.y));
@@ -122,19 +123,7 @@ __device__ __forceinline__ T zero_() {
 __device__ __forceinline__ bool is_bad(float2 v) { return !(isfinite(v.x) && isfinite(v.y)) || (v.x == 0.f && v.y == 0.f); }
 __device__ __forceinline__ bool is_bad(double2 v) { return !(isfinite(v.x) && isfinite(v.y)) || (v.x == 0.0 && v.y == 0.0); }
 
-// four consecutive entries at a 16-byte boundary of shared memory
-__device__ __forceinline__ void load4(const float2 *p, float2 (&v)[4]) {
-    const float4 a = *(const float4 *)p, b = *(const float4 *)(p + 2);
-    v[0] = cf(a.x, a.y);
-    v[1] = cf(a.z, a.w);
-    v[2] = cf(b.x, b.y);
-    v[3] = cf(b.z, b.w);
-}
-__device__ __forceinline__ void load4(const double2 *p, double2 (&v)[4]) {
-#pragma unroll
-    for (int i = 0; i < 4; i++) v[i] = p[i];
-}
-
+// two consecutive entries at a 16-byte boundary of shared memory
 __device__ __forceinline__ void load2(const float2 *p, float2 (&v)[2]) {
     const float4 a = *(const float4 *)p;
     v[0] = cf(a.x, a.y);
@@ -571,30 +560,41 @@ __global__ void k_sub_bval(DevProblem P, DevSub D, SubBatch B, const double2 *__
 // C C^T of one system's root, column-major lower with leading dimension ldc,
 // one block of 128 threads per system, left-looking in NB columns.  A block's
 // rows are worked in tiles of 64, a warp on 16 of them: W = M - C C_j^T from
-// the finished columns (cp.async, two chunks of 16 columns in flight), then
-// W C_jj^-T.  The diagonal block is factored and inverted together, one
-// barrier a column; its inverse is stored in its place, which is all that the
-// later solves need.  Bound by the FP64 pipe in complex128, so NB is 16 there:
-// the panel's products with the full inverse and the upper halves of the
-// diagonal blocks cost m^2 NB / 2 and m^2 NB / 4 beside m^3 / 6.  In complex64
-// the operand traffic counts too and NB is 32.  Warps whose rows lie beyond
-// the matrix skip the products.
-constexpr int kRT = 128;   // threads
-constexpr int kRows = 64;  // rows of a tile
-constexpr int kKC = 16;    // columns of a chunk
+// the finished columns (cp.async, S chunks of KC columns in flight, one
+// barrier a chunk), then W C_jj^-T.  The diagonal block is factored and
+// inverted together, one barrier a column; its inverse is stored in its place,
+// which is all that the later solves need.  Bound by the FP64 pipe in
+// complex128, so NB is 16 there: the panel's products with the full inverse
+// and the upper halves of the diagonal blocks cost m^2 NB / 2 and m^2 NB / 4
+// beside m^3 / 6.  In complex64 the operand traffic counts too and NB is 32.
+// Five blocks an SM (96 registers): the phases between the products are chains
+// of loads and barriers, which only other blocks fill (at 4 / 5 / 6 the factor
+// of config 2 takes 4.07 / 3.98 / 4.02 ms; tiles of 128 rows with 8 x 4 results a
+// thread were slower).  Warps whose rows lie beyond the matrix skip the
+// products.
+constexpr int kRT = 128;  // threads
 
 template <typename T>
 struct RootShape {
-    static constexpr int NB = sizeof(T) == 8 ? 32 : 16;
-    static constexpr int TR = sizeof(T) == 8 ? 4 : 2;  // rows of a thread; it has 4 columns
+    static constexpr bool F = sizeof(T) == 8;
+    static constexpr int NB = F ? 32 : 16;
+    static constexpr int TR = F ? 4 : 2;            // rows of a thread; it has 4 columns
+    static constexpr int ROWS = kRT / (NB / 4) * TR;  // rows of a tile
+    static constexpr int WR = ROWS / 4;             // rows of a warp
+    static constexpr int KC = F ? 16 : 8;           // columns of a chunk
+    static constexpr int S = 3;                     // chunks in flight
+    static constexpr int AT = S * KC * ROWS, BT = S * KC * NB;  // operand buffers; also W and the block inverse
+    static_assert(AT >= NB * ROWS && BT >= NB * NB, "buffers are used twice");
 };
 
 template <typename T, int TR>
 __device__ __forceinline__ void load_rows(const T *p, T (&v)[TR]) {
     if constexpr (sizeof(T) == 8) {
-        const float4 a = *(const float4 *)p, b = *(const float4 *)(p + 2);
-        v[0].x = a.x, v[0].y = a.y, v[1].x = a.z, v[1].y = a.w;
-        v[2].x = b.x, v[2].y = b.y, v[3].x = b.z, v[3].y = b.w;
+#pragma unroll
+        for (int i = 0; i < TR; i += 2) {
+            const float4 a = *(const float4 *)(p + i);
+            v[i].x = a.x, v[i].y = a.y, v[i + 1].x = a.z, v[i + 1].y = a.w;
+        }
     } else {
 #pragma unroll
         for (int i = 0; i < TR; i++) v[i] = p[i];
@@ -603,22 +603,37 @@ __device__ __forceinline__ void load_rows(const T *p, T (&v)[TR]) {
 template <typename T, int TR>
 __device__ __forceinline__ void store_rows(T *p, const T (&v)[TR]) {
     if constexpr (sizeof(T) == 8) {
-        *(float4 *)p = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
-        *(float4 *)(p + 2) = make_float4(v[2].x, v[2].y, v[3].x, v[3].y);
+#pragma unroll
+        for (int i = 0; i < TR; i += 2) *(float4 *)(p + i) = make_float4(v[i].x, v[i].y, v[i + 1].x, v[i + 1].y);
     } else {
 #pragma unroll
         for (int i = 0; i < TR; i++) p[i] = v[i];
     }
 }
 
+// column of a thread's four: two pairs 16 apart in complex64, so that the
+// warp's 16-byte loads of a pair lie side by side; four in a row in complex128
+template <typename T>
+__device__ __forceinline__ int root_col(int g, int b) {
+    return sizeof(T) == 8 ? 2 * g + (b & 1) + 16 * (b >> 1) : 4 * g + b;
+}
+
 // acc[column][row] += A[q][row] B[q][column]
-template <typename T, int TR, int PB>
-__device__ __forceinline__ void root_fma(const T *A, const T *Bm, int kk, int tr, int tc, T (&acc)[4][TR]) {
+template <typename T, int TR>
+__device__ __forceinline__ void root_fma(const T *A, const T *Bm, int kk, int tr, int g, T (&acc)[4][TR]) {
+    constexpr int NB = RootShape<T>::NB;
 #pragma unroll 4
     for (int q = 0; q < kk; q++) {
         T a[TR], b[4];
-        load_rows<T, TR>(A + q * kRows + tr, a);
-        load4(Bm + q * PB + tc, b);
+        load_rows<T, TR>(A + q * RootShape<T>::ROWS + tr, a);
+        if constexpr (sizeof(T) == 8) {
+            const float4 u = *(const float4 *)(Bm + q * NB + 2 * g), v = *(const float4 *)(Bm + q * NB + 16 + 2 * g);
+            b[0].x = u.x, b[0].y = u.y, b[1].x = u.z, b[1].y = u.w;
+            b[2].x = v.x, b[2].y = v.y, b[3].x = v.z, b[3].y = v.w;
+        } else {
+#pragma unroll
+            for (int z = 0; z < 4; z++) b[z] = Bm[q * NB + 4 * g + z];
+        }
 #pragma unroll
         for (int j = 0; j < 4; j++)
 #pragma unroll
@@ -627,76 +642,90 @@ __device__ __forceinline__ void root_fma(const T *A, const T *Bm, int kk, int tr
 }
 
 template <typename T>
-__global__ __launch_bounds__(kRT) void k_sub_root(DevSub D, SubBatch B) {
+__global__ __launch_bounds__(kRT, 5) void k_sub_root(DevSub D, SubBatch B) {
     extern __shared__ __align__(16) unsigned char sm[];
-    constexpr int NB = RootShape<T>::NB, TR = RootShape<T>::TR, PX = NB + 2, NQ = NB / 4, CT = NB / 4;
-    T *As = (T *)sm;                      // [2][kKC][kRows]; also W of a tile, [NB][kRows]
-    T *Bs = As + 2 * kKC * kRows;         // [2][kKC][NB]
-    T *Ci = Bs + 2 * kKC * NB;            // [NB][PX]: Ci[a][b] = inverse(b, a)
+    using Q = RootShape<T>;
+    constexpr int kRows = Q::ROWS, WR = Q::WR, NB = Q::NB, TR = Q::TR, KC = Q::KC, S = Q::S;
+    constexpr int NQ = NB / 4, CT = NB / 4, per = 16 / sizeof(T);
+    T *As = (T *)sm;       // [S][KC][ROWS]; also W of a tile, [NB][ROWS]
+    T *Bs = As + Q::AT;    // [S][KC][NB]; also the inverse block, Bs[a][b] = inverse(b, a)
     __shared__ T col[2][32], inv[2];
     const int s = blockIdx.x, kk_ = s / B.Lb, k = B.k0 + kk_, l = s % B.Lb;
     const int mp = D.mp, ldc = D.ldc, m = D.m, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     T *C = (T *)B.C + (size_t)s * mp * ldc;
     const T *R = (const T *)D.R + (size_t)k * mp * ldc;
     const double2 *bval = B.bval + (size_t)kk_ * D.n_be * B.Lb + l;
-    const int tr = tid / CT * TR, tc = tid % CT * 4;
+    const int tr = tid / CT * TR, g = tid % CT;
     bool bad = false;
     for (int j = 0; j < mp; j += NB) {
+        // the electrode's terms of these columns: one a thread ahead of the products, the rest when they are added
+        const int be0 = D.be_ptr[min(j, m)], be1 = D.be_ptr[min(j + NB, m)];
+        SubEnt en0{0, -1, 0};
+        double2 bv0 = cz(0.0, 0.0);
+        if (be0 + tid < be1) {
+            en0 = D.be[be0 + tid];
+            bv0 = bval[(size_t)(be0 + tid) * B.Lb];
+        }
         for (int r0 = j; r0 < mp; r0 += kRows) {
-            const bool work = r0 + 16 * wid < m;
+            const bool work = r0 + WR * wid < m;
+            // acc = sum - M, M the wavenumber's part
             T acc[4][TR];
 #pragma unroll
-            for (int b = 0; b < 4; b++)
+            for (int b = 0; b < 4; b++) {
+                load_rows<T, TR>(R + (size_t)(j + root_col<T>(g, b)) * ldc + r0 + tr, acc[b]);
 #pragma unroll
-                for (int a = 0; a < TR; a++) acc[b][a] = zero_<T>();
-            const int nch = j / kKC;
+                for (int a = 0; a < TR; a++) acc[b][a] = neg_(acc[b][a]);
+            }
+            const int nch = j / KC;
             auto fetch = [&](int ch) {
-                T *a = As + (ch & 1) * kKC * kRows, *b = Bs + (ch & 1) * kKC * NB;
-                constexpr int per = 16 / sizeof(T);
-                // rows beyond the matrix are read (ldc covers them) and not stored
-                for (int q = tid; q < kKC * kRows / per; q += kRT) {
-                    const int c = q / (kRows / per), o = (q % (kRows / per)) * per;
-                    cp_async16(a + c * kRows + o, C + (size_t)(ch * kKC + c) * ldc + r0 + o);
-                }
-                for (int q = tid; q < kKC * NB / per; q += kRT) {
-                    const int c = q / (NB / per), o = (q % (NB / per)) * per;
-                    cp_async16(b + c * NB + o, C + (size_t)(ch * kKC + c) * ldc + j + o);
+                if (ch < nch) {
+                    T *a = As + (ch % S) * KC * kRows, *b = Bs + (ch % S) * KC * NB;
+                    const T *src = C + (size_t)ch * KC * ldc;
+                    // rows beyond the matrix are read (ldc covers them) and not stored
+                    for (int q = tid; q < KC * kRows / per; q += kRT) {
+                        const int c = q / (kRows / per), o = (q % (kRows / per)) * per;
+                        cp_async16(a + c * kRows + o, src + (size_t)c * ldc + r0 + o);
+                    }
+                    for (int q = tid; q < KC * NB / per; q += kRT) {
+                        const int c = q / (NB / per), o = (q % (NB / per)) * per;
+                        cp_async16(b + c * NB + o, src + (size_t)c * ldc + j + o);
+                    }
                 }
                 cp_commit();
             };
-            if (nch > 0) fetch(0);
+#pragma unroll
+            for (int q = 0; q < S - 1; q++) fetch(q);
             for (int ch = 0; ch < nch; ch++) {
-                if (ch + 1 < nch) {
-                    fetch(ch + 1);
-                    cp_wait<1>();
-                } else {
-                    cp_wait<0>();
-                }
+                cp_wait<S - 2>();
                 __syncthreads();
-                if (work)
-                    root_fma<T, TR, NB>(As + (ch & 1) * kKC * kRows, Bs + (ch & 1) * kKC * NB, kKC, tr, tc, acc);
-                __syncthreads();
+                fetch(ch + S - 1);  // into the buffer that every warp left before this barrier
+                if (work) root_fma<T, TR>(As + (ch % S) * KC * kRows, Bs + (ch % S) * KC * NB, KC, tr, g, acc);
             }
-            // W = M - sum, M the wavenumber's part; then the electrode's terms
+            cp_wait<0>();
+            __syncthreads();
+            if (r0 != j) {  // the inverse of the diagonal block, for the panel
+                for (int q = tid; q < NB * NB / per; q += kRT) {
+                    const int c = q / (NB / per), o = (q % (NB / per)) * per;
+                    cp_async16(Bs + c * NB + o, C + (size_t)(j + c) * ldc + j + o);
+                }
+                cp_commit();
+            }
+            // W = M - sum, then the electrode's terms
 #pragma unroll
             for (int b = 0; b < 4; b++) {
-                T w[TR];
-                load_rows<T, TR>(R + (size_t)(j + tc + b) * ldc + r0 + tr, w);
 #pragma unroll
-                for (int a = 0; a < TR; a++) {
-                    w[a].x -= acc[b][a].x;
-                    w[a].y -= acc[b][a].y;
-                }
-                store_rows<T, TR>(As + (tc + b) * kRows + tr, w);
+                for (int a = 0; a < TR; a++) acc[b][a] = neg_(acc[b][a]);
+                store_rows<T, TR>(As + root_col<T>(g, b) * kRows + tr, acc[b]);
             }
             __syncthreads();
-            for (int q = D.be_ptr[min(j, m)] + tid; q < D.be_ptr[min(j + NB, m)]; q += kRT) {
-                const SubEnt en = D.be[q];
-                if (en.lr < r0 || en.lr >= r0 + kRows) continue;
-                const double2 v = bval[(size_t)q * B.Lb];
+            auto add_term = [&](const SubEnt &en, double2 v) {
+                if (en.lr < r0 || en.lr >= r0 + kRows) return;
                 T &d = As[(en.lc - j) * kRows + en.lr - r0];
                 d = from_<T>(cz((double)d.x + v.x, (double)d.y + v.y));
-            }
+            };
+            add_term(en0, bv0);
+            for (int q = be0 + kRT + tid; q < be1; q += kRT) add_term(D.be[q], bval[(size_t)q * B.Lb]);
+            cp_wait<0>();
             __syncthreads();
             if (r0 == j) {
                 // diagonal block: lane = row, warp w the columns w, w + 4, ...
@@ -738,22 +767,24 @@ __global__ __launch_bounds__(kRT) void k_sub_root(DevSub D, SubBatch B) {
                     for (int q = 0; q < NQ; q++) {
                         const int c = 4 * q + wid;
                         const T v = row >= c ? x[q] : zero_<T>();
-                        Ci[c * PX + row] = v;
+                        Bs[c * NB + row] = v;
                         C[(size_t)(j + c) * ldc + j + row] = v;
                     }
                 }
                 __syncthreads();
             }
             // C_ij = W C_jj^-T
-            const int i = r0 + tr;
-            if (r0 + 16 * wid >= j + NB && r0 + 16 * wid < mp) {
+            if (r0 + WR * (wid + 1) > j + NB && r0 + WR * wid < mp) {
 #pragma unroll
                 for (int b = 0; b < 4; b++)
 #pragma unroll
                     for (int a = 0; a < TR; a++) acc[b][a] = zero_<T>();
-                if (work) root_fma<T, TR, PX>(As, Ci, NB, tr, tc, acc);
+                if (work) root_fma<T, TR>(As, Bs, NB, tr, g, acc);
+                if (r0 + tr >= j + NB && r0 + tr < mp) {
 #pragma unroll
-                for (int b = 0; b < 4; b++) store_rows<T, TR>(C + (size_t)(j + tc + b) * ldc + i, acc[b]);
+                    for (int b = 0; b < 4; b++)
+                        store_rows<T, TR>(C + (size_t)(j + root_col<T>(g, b)) * ldc + r0 + tr, acc[b]);
+                }
             }
             __syncthreads();
         }
@@ -1239,8 +1270,7 @@ int factor_t(const DevProblem &P, const DevSub &D, const SubPlan &sp, cudaStream
 
 template <typename T>
 size_t root_smem() {
-    constexpr int NB = RootShape<T>::NB;
-    return sizeof(T) * (2 * kKC * kRows + 2 * kKC * NB + NB * (NB + 2));
+    return sizeof(T) * (RootShape<T>::AT + RootShape<T>::BT);
 }
 
 template <typename T>
@@ -1285,6 +1315,7 @@ SubShape sub_shape(bool mixed) {
 }
 
 int sub_root_block(bool mixed) { return mixed ? RootShape<float2>::NB : RootShape<double2>::NB; }
+int sub_root_rows(bool mixed) { return mixed ? RootShape<float2>::ROWS : RootShape<double2>::ROWS; }
 
 int sub_launch_factor(const DevProblem &P, const DevSub &D, const SubPlan &sp, bool mixed, cudaStream_t st) {
     return mixed ? factor_t<float2>(P, D, sp, st) : factor_t<double2>(P, D, sp, st);
