@@ -38,6 +38,13 @@ struct DevProblem {
     const int32_t *enr0;   // eanz: electrode -> node (0-based)
     const int32_t *meas;   // nanz*4: electrodes e1,e2,e3,e4 (0-based, -1 = none)
     const double *strom;   // nanz
+    // sensitivities (post.cu): distinct dipoles (first, second electrode; eanz:
+    // none) of every pass, per measurement the other side's electrodes and its
+    // dipole's place in the table, the passes (first, end, dipoles), row factors
+    const int2 *dip;
+    const int4 *mdip, *spass;
+    int nspass, sens_dips;  // passes; most dipoles of one
+    double2 *sfac;
     const double *kwn, *kwnwi;
     // element matrices (src/precal.f90)
     double *elbg;          // [K][elanz][10]

@@ -1,6 +1,12 @@
 // Wavenumber back-transform, voltages and sensitivities:
 // src/rtrafo.f90:13-92, src/bvolt.f90:7-89, src/bvolti.f90:8-100,
 // src/bsens.f90:23-197, src/bsensi.f90:23-194.
+#include <algorithm>
+#include <mutex>
+#include <unordered_map>
+
+#include "async.cuh"
+#include "convert.cuh"
 #include "device.cuh"
 #include "kernels.h"
 
@@ -81,125 +87,235 @@ void launch_bvolt(const DevProblem &P, const double2 *hpot, int mode, const doub
 //   hsens_k = sum_{m,n} K_k[m][n] (kpot(node_m,e4) - kpot(node_m,e3))
 //                                 (kpot(node_n,e2) - kpot(node_n,e1))
 // with K_k the element matrix elbg; then the quadrature over k.
-// One block per element; the element's kpot values of all electrodes are
-// staged in shared memory one wavenumber at a time, threads run over
-// measurements and keep their k-sums in registers.
+//
+// One block per element.  Per wavenumber the element's potentials of all
+// electrodes are staged in shared memory (cp.async, one wavenumber ahead), the
+// product w_k K_k d is formed once for every distinct dipole d of the side
+// (current or voltage) that has fewer of them, and a measurement is then the
+// other side's difference and one dot product; threads run over measurements
+// and keep their k-sums in registers.  K is symmetric, so either side may take
+// it.  A survey repeats its dipoles: config 2's 4000 measurements have 374
+// voltage dipoles.  Per measurement and wavenumber that leaves 24 operations
+// instead of 66, and the scaling by strom / pi or sigma / (pi V) is a product
+// with a factor formed once per measurement: its six FP64 divisions an entry of
+// J took longer than the whole complex64 contraction.  GB300: bsensi of 4800
+// cells x 2000 in complex128 15.2 -> 6.8 ms (the FP64 pipe bounds it), 12000 x
+// 4000 in complex64 12.8 -> 6.7 ms (shared-memory reads: 12 a measurement and
+// wavenumber, 40 cycles without bank conflicts, 60 measured).
 // ---------------------------------------------------------------------------
 constexpr int kSensThreads = 256;
-constexpr int kSensMPT = 16;  // measurements per thread per pass (4096 per pass)
+constexpr int kSensMPT = 16;    // measurements per thread per pass (4096 per pass)
+constexpr int kSensDip = 1024;  // dipoles of a pass's table (64 KB in complex128: two blocks an SM)
 
+// The measurements in passes of at most kSensThreads * kSensMPT with at most
+// kSensDip distinct dipoles on the side that has the table, whichever side
+// makes the longer pass (the fewer dipoles).  meas: e1..e4 per measurement
+// (-1: none, which becomes the zero entry eanz).
+void host_sens_passes(const std::vector<int32_t> &meas, int nanz, int eanz, std::vector<int2> &dip,
+                      std::vector<int4> &mdip, std::vector<int4> &pass) {
+    auto el = [&](int i, int q) { return meas[(size_t)i * 4 + q] < 0 ? eanz : meas[(size_t)i * 4 + q]; };
+    mdip.resize(nanz);
+    for (int i0 = 0; i0 < nanz;) {
+        int end[2];
+        std::vector<int2> list[2];
+        std::vector<int> at[2];
+        for (int side = 0; side < 2; side++) {
+            std::unordered_map<int64_t, int> seen;
+            int i = i0;
+            for (; i < nanz && i < i0 + kSensThreads * kSensMPT; i++) {
+                const int a = el(i, 2 * side), b = el(i, 2 * side + 1);
+                const int64_t key = (int64_t)a * (eanz + 1) + b;
+                auto it = seen.find(key);
+                if (it == seen.end()) {
+                    if ((int)list[side].size() == kSensDip) break;
+                    it = seen.emplace(key, (int)list[side].size()).first;
+                    list[side].push_back(make_int2(a, b));
+                }
+                at[side].push_back(it->second);
+            }
+            end[side] = i;
+        }
+        const int t = end[1] > end[0] || (end[1] == end[0] && list[1].size() <= list[0].size()) ? 1 : 0;
+        // Threads in an order in which eight neighbours (one shared-memory phase
+        // of 16-byte loads) differ in their electrodes' and dipoles' places modulo
+        // 8, as far as the next 64 measurements allow: fewer bank conflicts (7.1
+        // -> 6.7 ms at 12000 x 4000 in complex64)
+        std::vector<int> wait;
+        int next = i0, used[3] = {0, 0, 0};
+        for (int slot = i0; slot < end[t]; slot++) {
+            if ((slot - i0) % 8 == 0) used[0] = used[1] = used[2] = 0;
+            while (next < end[t] && wait.size() < 64) wait.push_back(next++);
+            size_t best = 0;
+            int cost = 100;
+            for (size_t w = 0; w < wait.size() && cost; w++) {
+                const int i = wait[w], v[3] = {el(i, 2 * (1 - t)), el(i, 2 * (1 - t) + 1), at[t][i - i0]};
+                const int cw = 2 * (used[0] >> (v[0] & 7) & 1) + 2 * (used[1] >> (v[1] & 7) & 1) + (used[2] >> (v[2] & 7) & 1);
+                if (cw < cost) {
+                    cost = cw;
+                    best = w;
+                }
+            }
+            const int i = wait[best];
+            wait.erase(wait.begin() + best);
+            mdip[slot] = make_int4(el(i, 2 * (1 - t)), el(i, 2 * (1 - t) + 1), at[t][i - i0], i);
+            used[0] |= 1 << (mdip[slot].x & 7);
+            used[1] |= 1 << (mdip[slot].y & 7);
+            used[2] |= 1 << (mdip[slot].z & 7);
+        }
+        pass.push_back(make_int4(i0, end[t], (int)dip.size(), (int)list[t].size()));
+        dip.insert(dip.end(), list[t].begin(), list[t].end());
+        i0 = end[t];
+    }
+}
+
+// scaling of row i of J: -strom / pi (mode 0), 1 / (pi V_i) (mode 1; sigma_e is
+// the element's)
+__global__ void k_sens_factor(DevProblem P, const double2 *__restrict__ volt, int mode) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= P.nanz) return;
+    if (mode == 0) {
+        P.sfac[i] = cz(-(P.swrtr ? P.strom[i] / kPi : P.strom[i]), 0.0);
+    } else {
+        double2 v = volt[i];
+        if (P.swrtr) v = cz(kPi * v.x, kPi * v.y);
+        P.sfac[i] = cdiv(cz(1.0, 0.0), v);
+    }
+}
+
+// potentials of one electrode at one node: complex128, or complex64 hi and lo
 template <typename R>
 struct SensT;
 template <>
 struct SensT<double> {
     using C = double2;
+    using S = double2;
     __device__ static C mk(double a, double b) { return cz(a, b); }
+    __device__ static C diff(S a, S b) { return cz(b.x - a.x, b.y - a.y); }
+    __device__ static S none() { return cz(0.0, 0.0); }
 };
 template <>
 struct SensT<float> {
     using C = float2;
+    using S = float4;  // the differences to ~complex64 accuracy of the difference
     __device__ static C mk(float a, float b) { return cf(a, b); }
+    __device__ static C diff(S a, S b) { return cf((b.x - a.x) + (b.z - a.z), (b.y - a.y) + (b.w - a.w)); }
+    __device__ static S none() { return make_float4(0.f, 0.f, 0.f, 0.f); }
 };
+
+__device__ __forceinline__ double2 to_double(double2 v) { return v; }
+__device__ __forceinline__ double2 to_double(float2 v) { return widen(v); }
 
 // MODE 0: src/bsens.f90, MODE 1: src/bsensi.f90.  R: arithmetic type of the
 // element contraction (double: the reference arithmetic, from kpot; float: the
-// mixed mode, from its complex64 copy, with FP64 output).
-template <int MODE, typename R>
-__global__ __launch_bounds__(kSensThreads) void k_bsens(DevProblem P,
-                                                         const typename SensT<R>::C *__restrict__ kpot,
-                                                         const double2 *__restrict__ sigma,
-                                                         const double2 *__restrict__ volt,
-                                                         double2 *__restrict__ sens, int e_first) {
-    using C = typename SensT<R>::C;
-    constexpr bool kTwoPlanes = sizeof(R) == 4;  // complex64: hi and lo planes of kpot
-    extern __shared__ __align__(16) unsigned char kp_raw[];
-    C *kp_sh = (C *)kp_raw;  // [4][eanz]
-    C *kl_sh = kp_sh + 4 * P.eanz;  // [4][eanz] lo plane (complex64 only)
-    const size_t plane = (size_t)P.K * P.eanz * P.n;
-    __shared__ R kel[10];
-    const int e = e_first + blockIdx.x;
-    const int nk = P.etype[e] == 3 ? 3 : 4;
-    int nodes[4];
+// mixed mode, from its complex64 planes, with FP64 output).
+template <int MODE, typename R, int NK>
+__device__ __forceinline__ void sens_element(const DevProblem &P, const typename SensT<R>::C *__restrict__ kpot,
+                                             const double2 *__restrict__ sigma, double2 *__restrict__ sens, int e,
+                                             unsigned char *smem) {
+    using T = SensT<R>;
+    using C = typename T::C;
+    using S = typename T::S;
+    const int eanz = P.eanz, E1 = eanz + 1, tid = threadIdx.x;
+    S *kp = (S *)smem;             // [2][NK][E1], the last entry of a row an absent electrode's zero
+    C *tab = (C *)(kp + 2 * NK * E1);  // [NK][dipoles of the pass]
+    const size_t plane = (size_t)P.K * eanz * P.n;
+    int nodes[NK];
 #pragma unroll
-    for (int q = 0; q < 4; q++) nodes[q] = P.enodes[e * 4 + q];
-    const int eanz = P.eanz;
-    const int4 *meas4 = (const int4 *)P.meas;
-    for (int i0 = 0; i0 < P.nanz; i0 += kSensThreads * kSensMPT) {
+    for (int q = 0; q < NK; q++) nodes[q] = P.enodes[e * 4 + q];
+    if (tid < 2 * NK) kp[tid * E1 + eanz] = T::none();
+    auto fetch = [&](int k, int buf) {
+        for (int t = tid; t < NK * eanz; t += kSensThreads) {
+            const int q = t / eanz, l = t - q * eanz;
+            const C *src = kpot + ((size_t)k * eanz + l) * P.n + nodes[q];
+            S *dst = kp + (buf * NK + q) * E1 + l;
+            if constexpr (sizeof(R) == 8) {
+                cp_async16(dst, src);
+            } else {
+                cp_async8(dst, src);
+                cp_async8((char *)dst + 8, src + plane);
+            }
+        }
+        cp_commit();
+    };
+    const double2 sg = sigma[e];
+    for (int ps = 0; ps < P.nspass; ps++) {
+        const int4 pass = P.spass[ps];
+        const int i0 = pass.x, i1 = pass.y, nd = pass.w;
+        const int2 *dip = P.dip + pass.z;
         C acc[kSensMPT];
 #pragma unroll
-        for (int m = 0; m < kSensMPT; m++) acc[m] = SensT<R>::mk(0, 0);
+        for (int m = 0; m < kSensMPT; m++) acc[m] = T::mk(0, 0);
+        __syncthreads();
+        fetch(0, 0);
         for (int k = 0; k < P.K; k++) {
-            __syncthreads();
-            for (int t = threadIdx.x; t < nk * eanz; t += kSensThreads) {
-                int q = t / eanz, l = t % eanz;
-                const size_t at = ((size_t)k * eanz + l) * P.n + nodes[q];
-                kp_sh[t] = kpot[at];
-                if (kTwoPlanes) kl_sh[t] = kpot[at + plane];
-            }
-            if (threadIdx.x < 10) kel[threadIdx.x] = (R)P.elbg[((size_t)k * P.elanz + e) * 10 + threadIdx.x];
-            __syncthreads();
+            const S *u = kp + (k & 1) * NK * E1;
+            R kel[NK * (NK + 1) / 2];
             const R w = P.swrtr ? (R)P.kwnwi[k] : (R)1;
 #pragma unroll
+            for (int q = 0; q < NK * (NK + 1) / 2; q++)
+                kel[q] = (R)P.elbg[((size_t)k * P.elanz + e) * 10 + q] * w;
+            cp_wait<0>();
+            __syncthreads();
+            if (k + 1 < P.K) fetch(k + 1, (k + 1) & 1);
+            for (int d = tid; d < nd; d += kSensThreads) {
+                const int2 p = dip[d];
+                C v[NK];
+#pragma unroll
+                for (int q = 0; q < NK; q++) v[q] = T::diff(u[q * E1 + p.x], u[q * E1 + p.y]);
+#pragma unroll
+                for (int mi = 0; mi < NK; mi++) {
+                    C s = T::mk(0, 0);
+#pragma unroll
+                    for (int mj = 0; mj < NK; mj++) {
+                        const int hi = mi > mj ? mi : mj, lo = mi < mj ? mi : mj;
+                        const R kk = kel[hi * (hi + 1) / 2 + lo];
+                        s.x = fma(kk, v[mj].x, s.x);
+                        s.y = fma(kk, v[mj].y, s.y);
+                    }
+                    tab[mi * nd + d] = s;
+                }
+            }
+            __syncthreads();
+#pragma unroll
             for (int m = 0; m < kSensMPT; m++) {
-                int i = i0 + m * kSensThreads + threadIdx.x;
-                if (i >= P.nanz) continue;
-                const int4 ee = meas4[i];  // electrodes e1..e4 (-1: none), L1-resident
-                C u[4], v[4];
+                const int i = i0 + m * kSensThreads + tid;
+                if (i >= i1) continue;
+                const int4 md = P.mdip[i];  // L1-resident
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    C s1 = ee.x >= 0 ? kp_sh[q * eanz + ee.x] : SensT<R>::mk(0, 0);
-                    C s2 = ee.y >= 0 ? kp_sh[q * eanz + ee.y] : SensT<R>::mk(0, 0);
-                    C s3 = ee.z >= 0 ? kp_sh[q * eanz + ee.z] : SensT<R>::mk(0, 0);
-                    C s4 = ee.w >= 0 ? kp_sh[q * eanz + ee.w] : SensT<R>::mk(0, 0);
-                    u[q] = SensT<R>::mk(s2.x - s1.x, s2.y - s1.y);
-                    v[q] = SensT<R>::mk(s4.x - s3.x, s4.y - s3.y);
-                    if (kTwoPlanes) {  // the dipole differences to ~complex64 accuracy of the difference
-                        const C z = SensT<R>::mk(0, 0);
-                        C t1 = ee.x >= 0 ? kl_sh[q * eanz + ee.x] : z, t2 = ee.y >= 0 ? kl_sh[q * eanz + ee.y] : z;
-                        C t3 = ee.z >= 0 ? kl_sh[q * eanz + ee.z] : z, t4 = ee.w >= 0 ? kl_sh[q * eanz + ee.w] : z;
-                        u[q] = SensT<R>::mk(u[q].x + (t2.x - t1.x), u[q].y + (t2.y - t1.y));
-                        v[q] = SensT<R>::mk(v[q].x + (t4.x - t3.x), v[q].y + (t4.y - t3.y));
-                    }
-                    if (q >= nk) { u[q] = SensT<R>::mk(0, 0); v[q] = SensT<R>::mk(0, 0); }
+                for (int q = 0; q < NK; q++) {
+                    const C a = T::diff(u[q * E1 + md.x], u[q * E1 + md.y]), b = tab[q * nd + md.z];
+                    acc[m].x = fma(a.x, b.x, acc[m].x);
+                    acc[m].x = fma(-a.y, b.y, acc[m].x);
+                    acc[m].y = fma(a.x, b.y, acc[m].y);
+                    acc[m].y = fma(a.y, b.x, acc[m].y);
                 }
-                C hs = SensT<R>::mk(0, 0);
-#pragma unroll
-                for (int mi = 0; mi < 4; mi++) {
-                    if (mi >= nk) continue;
-                    C ku = SensT<R>::mk(0, 0);
-#pragma unroll
-                    for (int mj = 0; mj < 4; mj++) {
-                        if (mj >= nk) continue;
-                        int imax = mi > mj ? mi : mj, imin = mi < mj ? mi : mj;
-                        R kk = kel[imax * (imax + 1) / 2 + imin];
-                        ku.x = fma(kk, u[mj].x, ku.x);
-                        ku.y = fma(kk, u[mj].y, ku.y);
-                    }
-                    hs.x = fma(v[mi].x, ku.x, hs.x);
-                    hs.x = fma(-v[mi].y, ku.y, hs.x);
-                    hs.y = fma(v[mi].x, ku.y, hs.y);
-                    hs.y = fma(v[mi].y, ku.x, hs.y);
-                }
-                acc[m].x = fma(hs.x, w, acc[m].x);
-                acc[m].y = fma(hs.y, w, acc[m].y);
             }
         }
 #pragma unroll
         for (int m = 0; m < kSensMPT; m++) {
-            int i = i0 + m * kSensThreads + threadIdx.x;
-            if (i >= P.nanz) continue;
-            double2 d = cz((double)acc[m].x, (double)acc[m].y);
-            double2 out;
-            if (MODE == 0) {
-                double f = P.swrtr ? P.strom[i] / kPi : P.strom[i];
-                out = cz(-d.x * f, -d.y * f);
-            } else {
-                if (P.swrtr) d = cz(d.x / kPi, d.y / kPi);
-                out = cdiv(cmul(d, sigma[e]), volt[i]);
-            }
-            sens[(size_t)e * P.nanz + i] = out;
+            if (i0 + m * kSensThreads + tid >= i1) continue;
+            const int i = P.mdip[i0 + m * kSensThreads + tid].w;
+            const double2 d = to_double(acc[m]), f = P.sfac[i];
+            sens[(size_t)e * P.nanz + i] = MODE == 0 ? cz(d.x * f.x, d.y * f.x) : cmul(d, cmul(sg, f));
         }
     }
+}
+
+template <int MODE, typename R>
+__global__ __launch_bounds__(kSensThreads) void k_bsens(DevProblem P,
+                                                        const typename SensT<R>::C *__restrict__ kpot,
+                                                        const double2 *__restrict__ sigma,
+                                                        double2 *__restrict__ sens, int e_first) {
+    extern __shared__ __align__(16) unsigned char kp_raw[];
+    const int e = e_first + blockIdx.x;
+    if (P.etype[e] == 3) sens_element<MODE, R, 3>(P, kpot, sigma, sens, e, kp_raw);
+    else sens_element<MODE, R, 4>(P, kpot, sigma, sens, e, kp_raw);
+}
+
+// the block's shared memory (both element types)
+static size_t sens_smem(const DevProblem &P, bool single) {
+    const size_t c = single ? sizeof(float2) : sizeof(double2);
+    return 2 * 4 * (size_t)(P.eanz + 1) * 16 + 4 * (size_t)P.sens_dips * c;
 }
 
 void launch_bsens(const DevProblem &P, const double2 *kpot, const float2 *kpot32, const double2 *sigma,
@@ -211,14 +327,23 @@ void launch_bsens(const DevProblem &P, const double2 *kpot, const float2 *kpot32
         launch_sens_tc(P, kpot32, sens, st, e_first, e_count);
         return;
     }
+    static std::once_flag once;
+    std::call_once(once, [] {
+        int dev = 0, optin = 48 * 1024;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        for (const void *f : {(const void *)k_bsens<0, float>, (const void *)k_bsens<1, float>,
+                              (const void *)k_bsens<0, double>, (const void *)k_bsens<1, double>})
+            cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    });
+    if (P.nanz > 0) k_sens_factor<<<(P.nanz + 127) / 128, 128, 0, st>>>(P, volt, mode);
+    const size_t smem = sens_smem(P, single);
     if (single) {
-        size_t smem = sizeof(float2) * 8 * P.eanz;  // hi and lo planes
-        if (mode == 0) k_bsens<0, float><<<e_count, kSensThreads, smem, st>>>(P, kpot32, sigma, volt, sens, e_first);
-        else k_bsens<1, float><<<e_count, kSensThreads, smem, st>>>(P, kpot32, sigma, volt, sens, e_first);
+        if (mode == 0) k_bsens<0, float><<<e_count, kSensThreads, smem, st>>>(P, kpot32, sigma, sens, e_first);
+        else k_bsens<1, float><<<e_count, kSensThreads, smem, st>>>(P, kpot32, sigma, sens, e_first);
     } else {
-        size_t smem = sizeof(double2) * 4 * P.eanz;
-        if (mode == 0) k_bsens<0, double><<<e_count, kSensThreads, smem, st>>>(P, kpot, sigma, volt, sens, e_first);
-        else k_bsens<1, double><<<e_count, kSensThreads, smem, st>>>(P, kpot, sigma, volt, sens, e_first);
+        if (mode == 0) k_bsens<0, double><<<e_count, kSensThreads, smem, st>>>(P, kpot, sigma, sens, e_first);
+        else k_bsens<1, double><<<e_count, kSensThreads, smem, st>>>(P, kpot, sigma, sens, e_first);
     }
 }
 
