@@ -1827,7 +1827,7 @@ static int update_common(crgpu_ctx *c, int part, const double *wmatd, const int3
     const size_t o_nb = take(sizeof(int32_t) * (size_t)manz * (maxnk + 1));
     const size_t o_par = take(sizeof(double2) * manz), o_dpar = take(sizeof(double2) * manz);
     const size_t o_cg = take(sizeof(double) * manz);
-    const size_t o_work = take(update_work_bytes(nanz, manz));
+    const size_t o_work = take(update_work_bytes(nanz, manz, ncgmax));
     if (c->upd_bytes < off) {
         if (c->d_upd) cudaFreeAsync(c->d_upd, c->st);
         c->d_upd = nullptr;
@@ -1900,7 +1900,7 @@ int crgpu_blam0_jtj(crgpu_ctx *c, const double *wmatd, const int32_t *wdfak, int
         return o;
     };
     const size_t o_w = take(sizeof(double) * nanz), o_wd = take(sizeof(int32_t) * nanz);
-    const size_t o_cg = take(sizeof(double) * manz), o_work = take(update_work_bytes(nanz, manz));
+    const size_t o_cg = take(sizeof(double) * manz), o_work = take(update_work_bytes(nanz, manz, 0));
     if (c->upd_bytes < off) {
         if (c->d_upd) cudaFreeAsync(c->d_upd, c->st);
         c->d_upd = nullptr;

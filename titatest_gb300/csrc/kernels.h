@@ -138,11 +138,11 @@ struct CGArgs {
     const int32_t *nachbar; // column-major (manz, maxnk+1)
     double2 *par, *dpar;    // in/out model, out update
     double *cgfac;          // out preconditioner
-    double2 *work;          // update_work_bytes(nanz, manz)
+    double2 *work;          // update_work_bytes(nanz, manz, ncgmax)
     int part;               // 0 complex CG; real CG of cjggdc on Re(J): 1 the phases (final phase
                             // improvement, lfpi), 2 the real parts (DC, ldc)
 };
-size_t update_work_bytes(int nanz, int manz);
+size_t update_work_bytes(int nanz, int manz, int ncgmax);
 // runs update + cjggra; cgres (host, ncgmax+2 floats) receives the CG record
 int run_update(const CGArgs &a, cudaStream_t st, int *ncg_out, float *cgres_host);
 // |(J^H W J 1)_j| for the first regularisation parameter (src/blam0.f90); jtj_host: manz doubles
