@@ -4,9 +4,10 @@
 //
 //   ata     = Re(J^H W J) = S^T S               (bata; S = [sqrt(w) Re J; sqrt(w) Im J])
 //   ata_reg = ata + lam R                       (bata_reg)
-//   cov     = ata_reg^-1 = L^-T L^-1            (bmcm: blocked Cholesky, triangular inverse, Y^T Y)
-//   res     = cov ata          -> diag          (bres: row-column dots, O(manz^2))
-//   cov2    = cov ata cov      -> diag          (bmcm2: = (S cov)^T (S cov), column sums of squares)
+//   cov     = ata_reg^-1 = Y^T Y, Y = L^-1      (bmcm: blocked Cholesky, triangular inverse; diagonal:
+//                                                column sums of squares of Y)
+//   res     = cov ata          -> diag          (bres: column sums of G o S, G = S cov = (S Y^T) Y)
+//   cov2    = cov ata cov      -> diag          (bmcm2: = G^T G, column sums of squares)
 //
 // The dense steps are this library's own FP64 kernels (dense.cu); the kernels
 // here form the weighted operand, the regularisation entries and the
@@ -47,25 +48,32 @@ __global__ void k_diag(int n, const double *__restrict__ M, double *__restrict__
     if (i < n) d[i] = M[(size_t)i * n + i];
 }
 
-// ata_reg = ata + lam R for the neighbour regularisation (ltri 1, 2),
-// src/bmcm_mod.f90:357-370 in its order: column by column, the diagonal,
-// then the first nachbar(j, nk+1) neighbour slots (a neighbour in a later
-// slot is not reached, as in the reference), each write mirrored.  One
-// thread: the later column's write of a mirrored pair must win.
+// ata_reg = ata + lam R for the neighbour regularisation (ltri 1, 2), the
+// outcome of src/bmcm_mod.f90:357-370: column by column, the diagonal, then
+// the first nachbar(j, nk+1) neighbour slots (a neighbour in a later slot is
+// not reached, as in the reference), each write mirrored, later writes
+// winning.  One thread per column: it writes a pair unless the other, later
+// column or a later slot of its own writes the same pair (in one thread 4.4 ms
+// for 2400 cells).
 __global__ void k_reg_neighbours(int manz, int nk, double lam, const double *__restrict__ smatm,
                                  const int32_t *__restrict__ nachbar, const double *__restrict__ ata,
                                  double *__restrict__ reg) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    for (int j = 0; j < manz; j++) {
-        reg[(size_t)j * manz + j] = ata[(size_t)j * manz + j] + lam * smatm[(size_t)nk * manz + j];
-        const int cnt = nachbar[(size_t)nk * manz + j];
-        for (int k = 0; k < cnt && k < nk; k++) {
-            const int ik = nachbar[(size_t)k * manz + j];
-            if (ik == 0) continue;
-            const double v = ata[(size_t)j * manz + (ik - 1)] + lam * smatm[(size_t)k * manz + j];
-            reg[(size_t)j * manz + (ik - 1)] = v;
-            reg[(size_t)(ik - 1) * manz + j] = v;
-        }
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= manz) return;
+    auto slots = [&](int c) { return min(nachbar[(size_t)nk * manz + c], nk); };
+    reg[(size_t)j * manz + j] = ata[(size_t)j * manz + j] + lam * smatm[(size_t)nk * manz + j];
+    const int cnt = slots(j);
+    for (int k = 0; k < cnt; k++) {
+        const int o = nachbar[(size_t)k * manz + j] - 1;
+        if (o < 0) continue;
+        bool mine = true;
+        for (int z = k + 1; z < cnt; z++) mine = mine && nachbar[(size_t)z * manz + j] - 1 != o;
+        if (o > j)
+            for (int z = 0, oc = slots(o); z < oc; z++) mine = mine && nachbar[(size_t)z * manz + o] - 1 != j;
+        if (!mine) continue;
+        const double v = ata[(size_t)j * manz + o] + lam * smatm[(size_t)k * manz + j];
+        reg[(size_t)j * manz + o] = v;
+        reg[(size_t)o * manz + j] = v;
     }
 }
 
@@ -154,7 +162,7 @@ void launch_column_sums(int nanz, int manz, const double2 *sens, const double *w
 int run_mcm(const McmArgs &a, cudaStream_t st, std::string &msg) {
     const int n = a.manz, m = a.nanz;
     const size_t nn = (size_t)n * n;
-    double *A = nullptr, *ata = nullptr, *reg = nullptr, *Y = nullptr, *cov = nullptr, *d = nullptr, *work = nullptr;
+    double *A = nullptr, *ata = nullptr, *reg = nullptr, *Y = nullptr, *cov = nullptr, *d = nullptr, *d2 = nullptr, *work = nullptr;
     int *info = nullptr;
     int rc = 0;
     auto fail = [&](int code, const std::string &what) {
@@ -184,42 +192,52 @@ int run_mcm(const McmArgs &a, cudaStream_t st, std::string &msg) {
         if (a.ltri == 0)
             k_reg_stencil<<<nb(n, T), T, 0, st>>>(n, a.nx, a.lam, a.smatm, reg);
         else
-            k_reg_neighbours<<<1, 1, 0, st>>>(n, a.nk, a.lam, a.smatm, a.nachbar, ata, reg);
+            k_reg_neighbours<<<nb(n, 128), 128, 0, st>>>(n, a.nk, a.lam, a.smatm, a.nachbar, ata, reg);
         k_diag<<<nb(n, T), T, 0, st>>>(n, reg, d);
         cudaMemcpyAsync(a.diag_reg, d, sizeof(double) * n, cudaMemcpyDeviceToHost, st);
+    }
+    dal((void **)&Y, sizeof(double) * nn);
+    if (!rc) {
         // bmcm: Cholesky factor L of ata_reg (in place, lower)
         cudaMemsetAsync(info, 0, sizeof(int), st);
-        dense_potrf(n, reg, info, st);
+        dense_potrf(n, reg, Y, info, st);
         int h_info = 0;
         cudaMemcpyAsync(&h_info, info, sizeof(int), cudaMemcpyDeviceToHost, st);
         cudaStreamSynchronize(st);
         if (h_info != 0) fail(108, "CHOLD mcm :: matrix not pos definite..");  // src/bmcm_mod.f90:447-451
     }
-    dal((void **)&Y, sizeof(double) * nn);
-    dal((void **)&cov, sizeof(double) * nn);
+    const bool sums = a.want_res && a.want_cov2;
     if (!rc) {
-        // cov = L^-T L^-1 (lower), then both triangles
-        dense_potri(n, reg, Y, cov, st);
-        k_symmetrize_lower<<<nb(nn, T), T, 0, st>>>(n, cov);
-        k_diag<<<nb(n, T), T, 0, st>>>(n, cov, d);
+        // cov = Y^T Y, Y = L^-1: its diagonal needs Y alone
+        dense_trtri(n, reg, Y, st);
+        dense_lower_col_sq(n, Y, d, st);
         cudaMemcpyAsync(a.diag_cov1, d, sizeof(double) * n, cudaMemcpyDeviceToHost, st);
-        if (a.want_res) {  // bres: diag(cov ata)
+    }
+    if (sums) {
+        // G = S cov without cov: bres diag(cov ata) = sum_l G_lj S_lj, bmcm2
+        // diag(cov ata cov) = sum_l G_lj^2
+        dal((void **)&cov, sizeof(double) * 2 * (size_t)m * n);  // S Y^T
+        dal((void **)&work, sizeof(double) * (size_t)((2 * m + 31) / 32) * 2 * n);
+        dal((void **)&d2, sizeof(double) * n);
+        if (!rc) {
+            dense_product_sums(2 * m, n, A, Y, cov, work, d2, d, st);
+            cudaMemcpyAsync(a.diag_res, d, sizeof(double) * n, cudaMemcpyDeviceToHost, st);
+            cudaMemcpyAsync(a.diag_cov2, d2, sizeof(double) * n, cudaMemcpyDeviceToHost, st);
+        }
+    } else if (a.want_res) {  // bres: diag(cov ata)
+        dal((void **)&cov, sizeof(double) * nn);
+        if (!rc) {
+            dense_lauum_t(n, Y, cov, st);
+            k_symmetrize_lower<<<nb(nn, T), T, 0, st>>>(n, cov);
             k_diag_of_product<<<n, 256, 0, st>>>(n, cov, ata, d);
             cudaMemcpyAsync(a.diag_res, d, sizeof(double) * n, cudaMemcpyDeviceToHost, st);
-        }
-    }
-    if (!rc && a.want_res && a.want_cov2) {  // bmcm2: diag(cov ata cov) = column sums of (S cov)^2
-        dal((void **)&work, sizeof(double) * (size_t)((2 * m + 63) / 64) * n);
-        if (!rc) {
-            dense_col_sq_of_product(2 * m, n, A, 2 * m, cov, work, d, st);
-            cudaMemcpyAsync(a.diag_cov2, d, sizeof(double) * n, cudaMemcpyDeviceToHost, st);
         }
     }
     cudaError_t ce = cudaStreamSynchronize(st);
     if (!rc && ce != cudaSuccess) fail(1000, cudaGetErrorString(ce));
     ce = cudaGetLastError();
     if (!rc && ce != cudaSuccess) fail(1000, cudaGetErrorString(ce));
-    for (void *p : {(void *)A, (void *)ata, (void *)reg, (void *)Y, (void *)cov, (void *)d, (void *)work,
+    for (void *p : {(void *)A, (void *)ata, (void *)reg, (void *)Y, (void *)cov, (void *)d, (void *)d2, (void *)work,
                     (void *)info})
         if (p) cudaFreeAsync(p, st);
     return rc;
