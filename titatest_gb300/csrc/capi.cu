@@ -26,7 +26,7 @@ struct RefineCount {
     double z;  // largest relative correction of the step
 };
 constexpr int kRefineCap = 64;  // refinement steps at most (crgpu_set_refinement)
-constexpr int kRefineSlots = 2;  // counter arrays: the full rounds' solves and the last round's
+constexpr int kRefineSlots = 4;  // counter arrays: one per solve that runs beside others
 
 int fail(crgpu_ctx *c, int code, const std::string &msg) {
     if (c) c->last_error = msg;
@@ -449,63 +449,136 @@ void sub_rect(crgpu_ctx *c, int *kb, int *lb) {
     *lb = bs >= c->eanz ? c->eanz : bs;
 }
 
-int sub_factor_shared(crgpu_ctx *c) {
+// D as seen from wavenumber k0
+DevSub sub_shift(const crgpu_ctx *c, int k0) {
+    DevSub D = c->D;
+    const size_t esz = c->precision == CRGPU_MIXED ? sizeof(float2) : sizeof(double2);
+    D.As += (size_t)k0 * c->pat.nnz;
+    D.fk += (size_t)k0 * c->hg.n;
+    D.kbad += k0;
+    D.F = (char *)D.F + (size_t)k0 * D.szF * esz;
+    D.G = (char *)D.G + (size_t)k0 * D.szG * esz;
+    D.H = (char *)D.H + (size_t)k0 * D.szG * esz;
+    D.S = (char *)D.S + (size_t)k0 * D.szS * esz;
+    D.R = (char *)D.R + (size_t)k0 * D.mp * D.ldc * esz;
+    return D;
+}
+
+// scaled area parts of every wavenumber
+int sub_values(crgpu_ctx *c) {
     int e = ensure_sub_shared(c);
     if (e) return e;
     sub_launch_values(c->P, c->D, c->d_sigma, c->d_adom, c->st);
     c->stats.kernel_launches += 2;
-    c->stats.kernel_launches += sub_launch_factor(c->P, c->D, c->sp, c->precision == CRGPU_MIXED, c->st);
     return 0;
 }
 
-int sub_factor_rect(crgpu_ctx *c, const SubBatch &B) {
-    CUCHECK(c, cudaMemsetAsync(B.status, 0, sizeof(int) * B.Kb * B.Lb, c->st));
-    sub_launch_root(c->P, c->D, B, c->d_sigma, c->precision == CRGPU_MIXED, c->st);
+// shared elimination of the wavenumbers k0 .. k0+kb-1
+void sub_factor_shared(crgpu_ctx *c, int k0, int kb, cudaStream_t st) {
+    c->stats.kernel_launches +=
+        sub_launch_factor(c->P, sub_shift(c, k0), c->sp, kb, c->precision == CRGPU_MIXED, st);
+}
+
+int sub_factor_rect(crgpu_ctx *c, const SubBatch &B, cudaStream_t st) {
+    CUCHECK(c, cudaMemsetAsync(B.status, 0, sizeof(int) * B.Kb * B.Lb, st));
+    sub_launch_root(c->P, c->D, B, c->d_sigma, c->precision == CRGPU_MIXED, st);
     c->stats.kernel_launches += 2;
     return 0;
+}
+
+// the right-hand sides of the adjoint are kept for the residuals
+int ensure_sub_rhs(crgpu_ctx *c) {
+    if (c->precision != CRGPU_MIXED || c->SB.Bt) return 0;
+    return dalloc(c, &c->SB.Bt, (size_t)c->sub_cap * c->hg.n);
 }
 
 // Solves the rectangle for the right-hand sides of kompab (src null) or for
 // the rows of src; the solution ends in B.X.  Mixed precision refines as
-// solve_view does: every step is launched without waiting for the host.
-int sub_solve_rect(crgpu_ctx *c, SubBatch B, const double2 *src) {
+// solve_view does: every step is launched without waiting for the host, with
+// its counters in refinement array `slot`.
+int sub_solve_rect(crgpu_ctx *c, const SubBatch &B, const double2 *src, cudaStream_t st, int slot) {
     const bool mixed = c->precision == CRGPU_MIXED;
-    if (mixed && src && !c->SB.Bt) {  // the adjoint's right-hand sides are kept for the residuals
-        int e = dalloc(c, &c->SB.Bt, (size_t)c->sub_cap * c->hg.n);
-        if (e) return e;
-    }
-    B.Bt = c->SB.Bt;
     SubBatch B0 = B;
     B0.kact = nullptr;
-    sub_launch_rhs(c->P, c->D, B, mixed, c->lsink, c->nsink, src, c->st);
-    c->stats.kernel_launches += 1 + sub_launch_apply(c->D, c->sp, B0, mixed, nullptr, c->st);
+    sub_launch_rhs(c->P, c->D, B, mixed, c->lsink, c->nsink, src, st);
+    c->stats.kernel_launches += 1 + sub_launch_apply(c->D, c->sp, B0, mixed, nullptr, st);
     if (!mixed) return 0;
-    RefineCount *cnt = (RefineCount *)c->d_refine;
+    RefineCount *cnt = (RefineCount *)c->d_refine + (size_t)slot * kRefineCap;
     const int steps = std::min(c->refine_maxit, kRefineCap);
-    CUCHECK(c, cudaMemsetAsync(cnt, 0, sizeof(RefineCount) * kRefineCap, c->st));
-    sub_launch_accumulate(c->D, B, true, c->refine_tol, nullptr, nullptr, nullptr, c->st);
+    CUCHECK(c, cudaMemsetAsync(cnt, 0, sizeof(RefineCount) * kRefineCap, st));
+    sub_launch_accumulate(c->D, B, true, c->refine_tol, nullptr, nullptr, nullptr, st);
     c->stats.kernel_launches += 2;
     for (int it = 0; it < steps; it++) {
         const int *nprev = it > 0 ? &cnt[it - 1].n : nullptr;
-        sub_launch_residual(c->P, c->D, B, src == nullptr, c->lsink, c->nsink, nprev, c->st);
-        c->stats.kernel_launches += 3 + sub_launch_apply(c->D, c->sp, B, true, nprev, c->st);
-        sub_launch_accumulate(c->D, B, false, c->refine_tol, nprev, &cnt[it].n, &cnt[it].z, c->st);
+        sub_launch_residual(c->P, c->D, B, src == nullptr, c->lsink, c->nsink, nprev, st);
+        c->stats.kernel_launches += 3 + sub_launch_apply(c->D, c->sp, B, true, nprev, st);
+        sub_launch_accumulate(c->D, B, false, c->refine_tol, nprev, &cnt[it].n, &cnt[it].z, st);
     }
-    c->refine_used[0] = std::max(c->refine_used[0], steps);
+    c->refine_used[slot] = std::max(c->refine_used[slot], steps);
     return 0;
 }
 
-SubBatch sub_view(const crgpu_ctx *c, int k0, int kb, int l0, int lb) {
+// the rectangle of wavenumbers k0.. x electrodes l0.. on the batch buffers
+// from system s0 on
+SubBatch sub_view(const crgpu_ctx *c, int k0, int kb, int l0, int lb, size_t s0 = 0) {
     SubBatch B = c->SB;
+    const bool mixed = c->precision == CRGPU_MIXED;
+    const size_t n = c->hg.n, esz = mixed ? sizeof(float2) : sizeof(double2);
     B.k0 = k0;
     B.Kb = std::min(kb, c->K - k0);
     B.l0 = l0;
     B.Lb = std::min(lb, c->eanz - l0);
+    B.C = (char *)B.C + s0 * c->D.mp * c->D.ldc * esz;
+    B.bval += s0 * c->D.n_be;
+    B.X += s0 * n;
+    if (B.Bt) B.Bt += s0 * n;
+    B.Y = (char *)B.Y + s0 * n * esz;
+    B.W = (char *)B.W + s0 * n * esz;
+    B.Z = (char *)B.Z + s0 * n * esz;
+    B.U = (char *)B.U + s0 * c->D.szU * esz;
+    B.status += s0;
+    B.active += s0;
+    B.kact += s0 / c->eanz;
+    B.mz += s0;
+    B.mx += s0;
     return B;
 }
 
-// every system of the forward: shared factor, then root factors and solves by
-// rectangles, potentials into d_kpot
+// Groups of wavenumbers whose work is queued on streams of its own.  The
+// phases of a solve are bound by different things (root factor: FP32 issue,
+// residual: FP64 pipe, tree sweeps: memory and launch latency), so groups that
+// are out of step fill each other's gaps.  A small problem's kernels are
+// latency alone, which more launches only add to.  With 1 / 2 / 3 groups: 384
+// thousand unknowns (60x20 quads, 30 electrodes, 10 wavenumbers) 2.11 / 2.30 /
+// 2.54 ms, 15 million (config 2) 12.5 / 11.4 / 11.5, 41 million (300x80, 128)
+// 31.7 / 30.2 / 29.4; three cost an ensemble of contexts 10 %.
+int sub_groups(const crgpu_ctx *c) {
+    return c->K > 1 && c->sys_k.size() * (size_t)c->hg.n >= 4000000 ? 2 : 1;
+}
+
+// Fork and join of the groups around c->st.
+int sub_fork(crgpu_ctx *c, int groups) {
+    if (groups < 2) return 0;
+    if (!c->ev_fork) CUCHECK(c, cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
+    for (int g = 1; g < groups; g++) {
+        if (!c->st_sub[g - 1]) CUCHECK(c, cudaStreamCreateWithFlags(&c->st_sub[g - 1], cudaStreamNonBlocking));
+        if (!c->ev_sub[g - 1]) CUCHECK(c, cudaEventCreateWithFlags(&c->ev_sub[g - 1], cudaEventDisableTiming));
+    }
+    CUCHECK(c, cudaEventRecord(c->ev_fork, c->st));
+    for (int g = 1; g < groups; g++) CUCHECK(c, cudaStreamWaitEvent(c->st_sub[g - 1], c->ev_fork, 0));
+    return 0;
+}
+
+int sub_join(crgpu_ctx *c, int groups) {
+    for (int g = 1; g < groups; g++) {
+        CUCHECK(c, cudaEventRecord(c->ev_sub[g - 1], c->st_sub[g - 1]));
+        CUCHECK(c, cudaStreamWaitEvent(c->st, c->ev_sub[g - 1], 0));
+    }
+    return 0;
+}
+
+// every system of the forward: shared elimination, then root factors and
+// solves by rectangles, potentials into d_kpot
 int forward_sub(crgpu_ctx *c, float *t_factor, float *t_solve) {
     const bool cap = c->capturing;  // recorded, or queued beside other problems: one rectangle, no waiting
     int kb = c->K, lb = c->eanz;
@@ -513,27 +586,38 @@ int forward_sub(crgpu_ctx *c, float *t_factor, float *t_solve) {
     int e = ensure_sub_batch(c, kb * lb);
     if (e) return e;
     c->factors_sub = true;
+    const bool one = kb == c->K && lb == c->eanz;
+    const int groups = one ? sub_groups(c) : 1;
     cudaEvent_t ev[4] = {};
     if (!cap) {
         for (auto &v : ev) cudaEventCreate(&v);
         cudaEventRecord(ev[0], c->st);
     }
-    e = sub_factor_shared(c);
-    if (!cap) cudaEventRecord(ev[1], c->st);
+    e = sub_values(c);
+    if (!e && !one) sub_factor_shared(c, 0, c->K, c->st);
     float shared = 0.f;
     for (int k0 = 0; k0 < c->K && !e; k0 += kb)
         for (int l0 = 0; l0 < c->eanz && !e; l0 += lb) {
-            const SubBatch B = sub_view(c, k0, kb, l0, lb);
-            if (!cap && c->stats.nbatches) cudaEventRecord(ev[1], c->st);
-            e = sub_factor_rect(c, B);
-            if (!cap) cudaEventRecord(ev[2], c->st);
-            if (!e) e = sub_solve_rect(c, B, nullptr);
+            if (!cap) cudaEventRecord(ev[1], c->st);
+            e = sub_fork(c, groups);
+            for (int g = 0; g < groups && !e; g++) {  // one rectangle: groups of its wavenumbers
+                const int ka = one ? c->K * g / groups : k0, kn = one ? c->K * (g + 1) / groups - ka : kb;
+                const cudaStream_t st = g ? c->st_sub[g - 1] : c->st;
+                const SubBatch B = sub_view(c, ka, kn, l0, lb, one ? (size_t)ka * c->eanz : 0);
+                if (one) sub_factor_shared(c, ka, kn, st);
+                e = sub_factor_rect(c, B, st);
+                if (!cap && g == 0) cudaEventRecord(ev[2], c->st);
+                if (!e) e = sub_solve_rect(c, B, nullptr, st, g);
+                if (e) break;
+                sub_launch_unpack(c->P, c->D, B, -1.0, c->d_kpot, c->d_kpot32, st);
+                c->stats.kernel_launches += 1;
+            }
+            if (!e) e = sub_join(c, groups);
             if (e) break;
-            sub_launch_unpack(c->P, c->D, B, -1.0, c->d_kpot, c->d_kpot32, c->st);
-            c->stats.kernel_launches += 1;
             c->stats.nbatches++;
             if (cap) continue;
             cudaEventRecord(ev[3], c->st);
+            const SubBatch B = sub_view(c, k0, kb, l0, lb);
             e = check_device_errors(c, B.status, B.Kb * B.Lb, k0);
             float a = 0.f, b = 0.f;
             if (c->stats.nbatches == 1) cudaEventElapsedTime(&shared, ev[0], ev[1]);
@@ -555,22 +639,35 @@ int adjoint_sub(crgpu_ctx *c) {
     if (!have) {
         sub_rect(c, &kb, &lb);
         e = ensure_sub_batch(c, kb * lb);
-        if (!e) e = sub_factor_shared(c);
+        if (!e) e = sub_values(c);
         if (e) return e;
+        sub_factor_shared(c, 0, c->K, c->st);
         c->factors_sub = true;
     }
+    e = ensure_sub_rhs(c);
+    if (e) return e;
+    const bool one = kb == c->K && lb == c->eanz;
+    const int groups = one ? sub_groups(c) : 1;
     for (int k0 = 0; k0 < c->K; k0 += kb)
         for (int l0 = 0; l0 < c->eanz; l0 += lb) {
-            const SubBatch B = sub_view(c, k0, kb, l0, lb);
-            if (!have) e = sub_factor_rect(c, B);
-            if (!e) e = sub_solve_rect(c, B, c->d_adjsrc);
+            e = sub_fork(c, groups);
+            for (int g = 0; g < groups && !e; g++) {
+                const int ka = one ? c->K * g / groups : k0, kn = one ? c->K * (g + 1) / groups - ka : kb;
+                const cudaStream_t st = g ? c->st_sub[g - 1] : c->st;
+                const SubBatch B = sub_view(c, ka, kn, l0, lb, one ? (size_t)ka * c->eanz : 0);
+                if (!have) e = sub_factor_rect(c, B, st);
+                if (!e) e = sub_solve_rect(c, B, c->d_adjsrc, st, g);
+                if (e) break;
+                sub_launch_unpack(c->P, c->D, B, 1.0, c->d_lambda, nullptr, st);
+                c->stats.kernel_launches += 2;
+            }
+            if (!e) e = sub_join(c, groups);
             if (e) return e;
-            sub_launch_unpack(c->P, c->D, B, 1.0, c->d_lambda, nullptr, c->st);
-            c->stats.kernel_launches += 2;
+            const SubBatch B = sub_view(c, k0, kb, l0, lb);
             e = check_device_errors(c, B.status, B.Kb * B.Lb, k0);
             if (e) return e;
         }
-    c->factors_resident = kb == c->K && lb == c->eanz;
+    c->factors_resident = one;
     return 0;
 }
 
@@ -1110,6 +1207,11 @@ int crgpu_destroy(crgpu_ctx *c) {
     if (c->copy_st) cudaStreamDestroy(c->copy_st);
     if (c->st_hi) cudaStreamDestroy(c->st_hi);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
+    if (c->ev_fork) cudaEventDestroy(c->ev_fork);
+    for (auto s : c->st_sub)
+        if (s) cudaStreamDestroy(s);
+    for (auto v : c->ev_sub)
+        if (v) cudaEventDestroy(v);
     delete c;
     return 0;
 }

@@ -45,13 +45,13 @@ struct crgpu_ctx {
     // refinement step counters on the device, one array per sub-batch of the
     // current batch: {active count, pad, largest relative correction} per step
     void *d_refine = nullptr;
-    int refine_used[2] = {};  // steps launched on each array since the last collection
+    int refine_used[4] = {};  // steps launched on each array since the last collection
     // forward + Jacobian as one CUDA graph (crgpu_forward_sens_graph)
     bool capturing = false;       // recording: no host copies, synchronisation or timing
     cudaGraphExec_t graph = nullptr;
     const void *graph_key[3] = {nullptr, nullptr, nullptr};  // sigma, volt, sens of the recorded graph
     int graph_mode = -1;
-    int graph_refine_used[2] = {};  // refinement steps recorded in the graph per counter array
+    int graph_refine_used[4] = {};  // refinement steps recorded in the graph per counter array
     int64_t mem_budget = 0;
     bool have_forward = false;
     bool factors_resident = false;  // factors of every system still on the device (one batch)
@@ -64,6 +64,8 @@ struct crgpu_ctx {
     crgpu::SubBatch SB{};
     bool sub_shared = false;   // D's numeric arrays are allocated
     int sub_cap = 0;           // systems SB's buffers hold
+    cudaStream_t st_sub[3] = {};  // further groups of wavenumbers beside st
+    cudaEvent_t ev_fork = nullptr, ev_sub[3] = {};
     // adjoint
     double2 *d_lambda = nullptr, *d_adjsrc = nullptr, *d_adjg = nullptr, *d_adjgrad = nullptr;
     const int32_t *d_ebnd_ptr = nullptr, *d_ebnd_list = nullptr;  // element -> mixed boundary elements

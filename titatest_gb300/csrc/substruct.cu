@@ -1222,7 +1222,7 @@ __global__ __launch_bounds__(256) void k_sub_unpack(DevProblem P, DevSub D, SubB
 inline unsigned nb(size_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
 template <typename T>
-int factor_t(const DevProblem &P, const DevSub &D, const SubPlan &sp, cudaStream_t st) {
+int factor_t(const DevProblem &P, const DevSub &D, const SubPlan &sp, int K, cudaStream_t st) {
     static std::once_flag once;
     std::call_once(once, [] {
         const int most = (int)sizeof(T) * kSubEMax * (kSubEMax | 1);
@@ -1236,17 +1236,17 @@ int factor_t(const DevProblem &P, const DevSub &D, const SubPlan &sp, cudaStream
         for (int q = f0; q < f0 + nf; q++) emax = std::max(emax, sp.fronts[q].e);
         const size_t smem = sizeof(T) * emax * (emax | 1);
         const int na = sp.lA[lv + 1] - sp.lA[lv], ng = sp.lG[lv + 1] - sp.lG[lv], ns = sp.lS[lv + 1] - sp.lS[lv];
-        if (na) k_sub_gather<T><<<dim3(na, P.K), 256, 0, st>>>(D, sp.lA[lv]);
+        if (na) k_sub_gather<T><<<dim3(na, K), 256, 0, st>>>(D, sp.lA[lv]);
         if (emax * (emax + 1) / 2 <= 128 * 5)
-            k_sub_pivot<T, 128, 5><<<dim3(nf, P.K), 128, smem, st>>>(D, f0, P.nnz);
+            k_sub_pivot<T, 128, 5><<<dim3(nf, K), 128, smem, st>>>(D, f0, P.nnz);
         else
-            k_sub_pivot<T, 256, 9><<<dim3(nf, P.K), 256, smem, st>>>(D, f0, P.nnz);
-        if (ng) k_sub_g<T><<<dim3(ng, P.K), 256, 0, st>>>(D, sp.lG[lv]);
-        if (ns) k_sub_s<T><<<dim3(ns, P.K), 256, 0, st>>>(D, sp.lS[lv]);
+            k_sub_pivot<T, 256, 9><<<dim3(nf, K), 256, smem, st>>>(D, f0, P.nnz);
+        if (ng) k_sub_g<T><<<dim3(ng, K), 256, 0, st>>>(D, sp.lG[lv]);
+        if (ns) k_sub_s<T><<<dim3(ns, K), 256, 0, st>>>(D, sp.lS[lv]);
         launches += 1 + (na > 0) + (ng > 0) + (ns > 0);
     }
-    k_sub_root_base<T><<<dim3(D.mp, P.K), 128, 0, st>>>(D);
-    if (D.n_root_ent) k_sub_root_ent<T><<<dim3(nb(D.n_root_ent, 128), P.K), 128, 0, st>>>(D, P.nnz);
+    k_sub_root_base<T><<<dim3(D.mp, K), 128, 0, st>>>(D);
+    if (D.n_root_ent) k_sub_root_ent<T><<<dim3(nb(D.n_root_ent, 128), K), 128, 0, st>>>(D, P.nnz);
     return launches + 2;
 }
 
@@ -1299,8 +1299,8 @@ SubShape sub_shape(bool mixed) {
 int sub_root_block(bool mixed) { return mixed ? RootShape<float2>::NB : RootShape<double2>::NB; }
 int sub_root_rows(bool mixed) { return mixed ? RootShape<float2>::ROWS : RootShape<double2>::ROWS; }
 
-int sub_launch_factor(const DevProblem &P, const DevSub &D, const SubPlan &sp, bool mixed, cudaStream_t st) {
-    return mixed ? factor_t<float2>(P, D, sp, st) : factor_t<double2>(P, D, sp, st);
+int sub_launch_factor(const DevProblem &P, const DevSub &D, const SubPlan &sp, int K, bool mixed, cudaStream_t st) {
+    return mixed ? factor_t<float2>(P, D, sp, K, st) : factor_t<double2>(P, D, sp, K, st);
 }
 
 void sub_launch_root(const DevProblem &P, const DevSub &D, const SubBatch &B, const double2 *sigma, bool mixed,
