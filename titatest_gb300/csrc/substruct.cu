@@ -116,6 +116,35 @@ __device__ __forceinline__ void load2(const double2 *p, double2 (&v)[2]) {
     v[1] = p[1];
 }
 
+// Programmatic dependent launch: a forward is a chain of up to 250 short
+// kernels, and the start of each (launch, tables, index loads) overlaps the end
+// of the one before.  Every kernel of the chain waits for its predecessor
+// before it reads or writes anything but the plan's tables, also where it then
+// returns at once, so a kernel's own wait covers all earlier ones.  GB300:
+// 60x20 quads mixed with Jacobian 2.11 -> 1.82 ms, triangle gradient 14.7 -> 13.8
+// ms.  Letting the successor's blocks in before this kernel ends
+// (launch_dependents) cost complex128 3 %: they take the places of its last
+// wave.  In a recorded graph plain edges are the faster ones (9.7 against 10.0
+// ms).
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... P, typename... A>
+void chain_launch(void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(st, &cap);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = cap == cudaStreamCaptureStatusNone ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 constexpr int kKT = 32;  // depth of a chunk of the dense products
 
 // Tile edge of the dense kernels and results a thread: 256 threads own a 32 x
@@ -196,6 +225,7 @@ __global__ __launch_bounds__(256) void k_sub_gather(DevSub D, int t0) {
         const int c = q / (2 * E), b = q / E & 1, o = q % E, at = (b ? j0 : i0) + o;
         (b ? sj : si)[c][o] = at < (b ? e + r : e) ? D.inv[t.inv[c] + at] : -1;
     }
+    chain_wait();
     __syncthreads();
     const T *Sk = (const T *)D.S + (size_t)k * D.szS;
     T *F = (T *)D.F + (size_t)k * D.szF + t.oF, *H = (T *)D.H + (size_t)k * D.szG + t.oG;
@@ -241,6 +271,7 @@ __global__ __launch_bounds__(NT) void k_sub_pivot(DevSub D, int f0, int nnz) {
     const bool leaf = t.nch == 0;
     const double2 *As = D.As + (size_t)k * nnz;
     T *F = (T *)D.F + (size_t)k * D.szF + t.oF, *H = (T *)D.H + (size_t)k * D.szG + t.oG;
+    chain_wait();
     for (int q = tid; q < e * e; q += NT) Fm[(q / e) * ld + q % e] = leaf ? zero_<T>() : F[q];
     if (leaf)
         for (int q = tid; q < e * r; q += NT) H[q] = zero_<T>();
@@ -401,6 +432,7 @@ __global__ __launch_bounds__(256) void k_sub_g(DevSub D, int t0) {
     acc.clear();
     const bool work = i0 + acc.warp_row() < e;
     Operand<T> a, b;
+    chain_wait();
     a.load(F + i0, e, e, e - i0);  // symmetric: F[p][i]
     b.load(H + j0, r, e, r - j0);
     for (int p = 0; p < e; p += kKT) {
@@ -435,12 +467,13 @@ __global__ __launch_bounds__(256) void k_sub_s(DevSub D, int t0) {
     const T *H = (const T *)D.H + (size_t)k * D.szG + t.oG, *G = (const T *)D.G + (size_t)k * D.szG + t.oG;
     T *Sk = (T *)D.S + (size_t)k * D.szS, *S = Sk + t.oS;
     Operand<T> a, b;
-    a.load(H + i0, r, e, r - i0);
-    b.load(G + j0, r, e, r - j0);
     for (int q = threadIdx.x; q < 2 * nch * E; q += 256) {
         const int c = q / (2 * E), bb = q / E & 1, o = q % E, at = (bb ? j0 : i0) + o;
         (bb ? sj : si)[c][o] = at < r ? D.inv[t.inv[c] + e + at] : -1;
     }
+    chain_wait();
+    a.load(H + i0, r, e, r - i0);
+    b.load(G + j0, r, e, r - j0);
     __syncthreads();
     Result<T> acc, sum;
     acc.clear();
@@ -788,6 +821,7 @@ __global__ __launch_bounds__(kST) void k_sub_root_solve(DevSub D, SubBatch B, co
     constexpr int NB = RootShape<T>::NB, CW = NB / 8;  // columns of a warp
     T *v = (T *)sm;  // [mp]
     __shared__ T t[NB], part[8][33];
+    chain_wait();
     if (nprev && *nprev == 0) return;
     const int s = blockIdx.x, kk = s / B.Lb, l = s % B.Lb;
     if (B.kact && !B.kact[kk]) return;
@@ -874,9 +908,7 @@ __global__ __launch_bounds__(256) void k_sub_up(DevSub D, SubBatch B, int t0, co
     constexpr int E = Tile<T>::E, M = Tile<T>::M, P = Tile<T>::P;
     __shared__ __align__(16) T A[kKT * P], Bm[kKT * P];
     __shared__ int se[kSubCh][kSubEMax], sr[kSubCh][E];
-    if (nprev && *nprev == 0) return;
     const int kk = blockIdx.z, k = B.k0 + kk;
-    if (B.kact && !B.kact[kk]) return;
     const SubTile tl = D.tU[t0 + blockIdx.x];
     const SubFront &t = D.fr[tl.front];
     const int e = t.e, r = t.r, nch = t.nch, i0 = tl.ti * E, l0 = blockIdx.y * E, L = B.Lb, nl = min(E, L - l0);
@@ -892,6 +924,9 @@ __global__ __launch_bounds__(256) void k_sub_up(DevSub D, SubBatch B, int t0, co
         const int c = q / E, o = q % E;
         sr[c][o] = i0 + o < r ? D.inv[t.inv[c] + e + i0 + o] : -1;
     }
+    chain_wait();
+    if (nprev && *nprev == 0) return;
+    if (B.kact && !B.kact[kk]) return;
     __syncthreads();
     Operand<T> a, b;
     const int col = b.col();
@@ -970,9 +1005,7 @@ __global__ __launch_bounds__(256) void k_sub_down(DevSub D, SubBatch B, int t0, 
     constexpr int E = Tile<T>::E, M = Tile<T>::M, P = Tile<T>::P, kIdx = 512;
     __shared__ __align__(16) T A[kKT * P], Bm[kKT * P];
     __shared__ int sidx[kIdx];
-    if (nprev && *nprev == 0) return;
     const int kk = blockIdx.z, k = B.k0 + kk;
-    if (B.kact && !B.kact[kk]) return;
     const SubTile tl = D.tD[t0 + blockIdx.x];
     const SubFront &t = D.fr[tl.front];
     const int e = t.e, r = t.r, i0 = tl.ti * E, l0 = blockIdx.y * E, L = B.Lb, nl = min(E, L - l0);
@@ -981,6 +1014,9 @@ __global__ __launch_bounds__(256) void k_sub_down(DevSub D, SubBatch B, int t0, 
     T *Zk = (T *)B.Z + (size_t)kk * D.n * L + l0;
     const int32_t *rows = D.rows + t.rows0;
     for (int q = threadIdx.x; q < min(r, kIdx); q += 256) sidx[q] = rows[q];
+    chain_wait();
+    if (nprev && *nprev == 0) return;
+    if (B.kact && !B.kact[kk]) return;
     __syncthreads();
     Operand<T> a, b;
     Result<T> acc;
@@ -1076,6 +1112,7 @@ __global__ void k_sub_unit_rhs(DevProblem P, DevSub D, SubBatch B, int lsink, in
 // is kompab's, else B.Bt.
 __global__ __launch_bounds__(256) void k_sub_residual(DevProblem P, DevSub D, SubBatch B, int unit, int lsink,
                                                       int nsink, const int *nprev) {
+    chain_wait();
     if (nprev && *nprev == 0) return;
     const int kk = blockIdx.z, k = B.k0 + kk, L = B.Lb;
     if (!B.kact[kk]) return;
@@ -1106,6 +1143,7 @@ constexpr int kAccRows = 128;
 
 // X (+)= Z with the largest entries of both per system (as bit patterns)
 __global__ __launch_bounds__(256) void k_sub_accumulate(DevSub D, SubBatch B, int first, const int *nprev) {
+    chain_wait();
     if (nprev && *nprev == 0) return;
     const int kk = blockIdx.z, L = B.Lb;
     if (!first && !B.kact[kk]) return;
@@ -1158,6 +1196,7 @@ __global__ __launch_bounds__(256) void k_sub_accumulate(DevSub D, SubBatch B, in
 // block per wavenumber counts those that go on.
 __global__ __launch_bounds__(256) void k_sub_stop(SubBatch B, int first, double tol, const int *nprev, int *nactive,
                                                   double *zmax) {
+    chain_wait();
     if (nprev && *nprev == 0) return;
     const int kk = blockIdx.x, L = B.Lb;
     int count = 0;
@@ -1236,13 +1275,13 @@ int factor_t(const DevProblem &P, const DevSub &D, const SubPlan &sp, int K, cud
         for (int q = f0; q < f0 + nf; q++) emax = std::max(emax, sp.fronts[q].e);
         const size_t smem = sizeof(T) * emax * (emax | 1);
         const int na = sp.lA[lv + 1] - sp.lA[lv], ng = sp.lG[lv + 1] - sp.lG[lv], ns = sp.lS[lv + 1] - sp.lS[lv];
-        if (na) k_sub_gather<T><<<dim3(na, K), 256, 0, st>>>(D, sp.lA[lv]);
+        if (na) chain_launch(k_sub_gather<T>, dim3(na, K), 256, 0, st, D, sp.lA[lv]);
         if (emax * (emax + 1) / 2 <= 128 * 5)
-            k_sub_pivot<T, 128, 5><<<dim3(nf, K), 128, smem, st>>>(D, f0, P.nnz);
+            chain_launch(k_sub_pivot<T, 128, 5>, dim3(nf, K), 128, smem, st, D, f0, P.nnz);
         else
-            k_sub_pivot<T, 256, 9><<<dim3(nf, K), 256, smem, st>>>(D, f0, P.nnz);
-        if (ng) k_sub_g<T><<<dim3(ng, K), 256, 0, st>>>(D, sp.lG[lv]);
-        if (ns) k_sub_s<T><<<dim3(ns, K), 256, 0, st>>>(D, sp.lS[lv]);
+            chain_launch(k_sub_pivot<T, 256, 9>, dim3(nf, K), 256, smem, st, D, f0, P.nnz);
+        if (ng) chain_launch(k_sub_g<T>, dim3(ng, K), 256, 0, st, D, sp.lG[lv]);
+        if (ns) chain_launch(k_sub_s<T>, dim3(ns, K), 256, 0, st, D, sp.lS[lv]);
         launches += 1 + (na > 0) + (ng > 0) + (ns > 0);
     }
     k_sub_root_base<T><<<dim3(D.mp, K), 128, 0, st>>>(D);
@@ -1269,13 +1308,13 @@ template <typename T>
 int apply_t(const DevSub &D, const SubPlan &sp, const SubBatch &B, const int *nprev, cudaStream_t st) {
     const int lt = (B.Lb + Tile<T>::E - 1) / Tile<T>::E;
     for (int lv = 0; lv < sp.nlevel; lv++)
-        k_sub_up<T><<<dim3(sp.lU[lv + 1] - sp.lU[lv], lt, B.Kb), 256, 0, st>>>(D, B, sp.lU[lv], nprev);
-    k_sub_root_solve<T><<<B.Kb * B.Lb, kST, sizeof(T) * D.mp, st>>>(D, B, nprev);
+        chain_launch(k_sub_up<T>, dim3(sp.lU[lv + 1] - sp.lU[lv], lt, B.Kb), 256, 0, st, D, B, sp.lU[lv], nprev);
+    chain_launch(k_sub_root_solve<T>, dim3(B.Kb * B.Lb), kST, sizeof(T) * D.mp, st, D, B, nprev);
     int launches = sp.nlevel + 1;
     for (int lv = sp.nlevel - 1; lv >= 0; lv--) {
         const int nd = sp.lD[lv + 1] - sp.lD[lv];
         if (!nd) continue;
-        k_sub_down<T><<<dim3(nd, lt, B.Kb), 256, 0, st>>>(D, B, sp.lD[lv], nprev);
+        chain_launch(k_sub_down<T>, dim3(nd, lt, B.Kb), 256, 0, st, D, B, sp.lD[lv], nprev);
         launches++;
     }
     return launches;
@@ -1329,13 +1368,14 @@ void sub_launch_rhs(const DevProblem &P, const DevSub &D, const SubBatch &B, boo
 
 void sub_launch_residual(const DevProblem &P, const DevSub &D, const SubBatch &B, bool unit, int lsink, int nsink,
                          const int *nprev, cudaStream_t st) {
-    k_sub_residual<<<dim3(nb(D.n, 8), nb(B.Lb, 32), B.Kb), 256, 0, st>>>(P, D, B, unit ? 1 : 0, lsink, nsink, nprev);
+    chain_launch(k_sub_residual, dim3(nb(D.n, 8), nb(B.Lb, 32), B.Kb), 256, 0, st, P, D, B, unit ? 1 : 0, lsink, nsink,
+                 nprev);
 }
 
 void sub_launch_accumulate(const DevSub &D, const SubBatch &B, bool first, double tol, const int *nprev, int *nactive,
                            double *zmax, cudaStream_t st) {
-    k_sub_accumulate<<<dim3(nb(D.n, kAccRows), nb(B.Lb, 32), B.Kb), 256, 0, st>>>(D, B, first ? 1 : 0, nprev);
-    k_sub_stop<<<B.Kb, 256, 0, st>>>(B, first ? 1 : 0, tol, nprev, nactive, zmax);
+    chain_launch(k_sub_accumulate, dim3(nb(D.n, kAccRows), nb(B.Lb, 32), B.Kb), 256, 0, st, D, B, first ? 1 : 0, nprev);
+    chain_launch(k_sub_stop, dim3(B.Kb), 256, 0, st, B, first ? 1 : 0, tol, nprev, nactive, zmax);
 }
 
 void sub_launch_unpack(const DevProblem &P, const DevSub &D, const SubBatch &B, double sign, double2 *out,
