@@ -1618,8 +1618,11 @@ int crgpu_sens(crgpu_ctx *c, int32_t mode, double *sens) {
     cudaEventCreate(&b);
     for (auto &d : done) cudaEventCreateWithFlags(&d, cudaEventDisableTiming);
     cudaEventRecord(a, c->st);
-    const int per = (int)((manz + kChunks - 1) / kChunks);
-    for (int q = 0; q < kChunks; q++) {
+    // chunks of at least 4 MB: a Jacobian of a few MB is one launch and one copy (a
+    // chunk of fewer elements than the GPU has SMs still takes a whole element's time)
+    const int chunks = (int)std::min<size_t>(kChunks, std::max<size_t>(1, cnt * sizeof(double2) >> 22));
+    const int per = (int)((manz + chunks - 1) / chunks);
+    for (int q = 0; q < chunks; q++) {
         const int e0 = q * per, ne = std::min<int>(per, (int)manz - e0);
         if (ne <= 0) break;
         launch_bsens(c->P, c->d_kpot, c->d_kpot32, c->d_sigma, c->d_volt, mode, c->precision == CRGPU_MIXED,
