@@ -45,11 +45,19 @@ __device__ __forceinline__ void fms_(float2 &s, float2 a, float2 b) { s = cfmsf(
 __device__ __forceinline__ void fms_(double2 &s, double2 a, double2 b) { s = cfms(s, a, b); }
 __device__ __forceinline__ float2 mul_(float2 a, float2 b) { return cmulf(a, b); }
 __device__ __forceinline__ double2 mul_(double2 a, double2 b) { return cmul(a, b); }
-__device__ __forceinline__ float2 rcp_(float2 a) { return crecipf(a); }
-__device__ __forceinline__ double2 rcp_(double2 a) { return crecip(a); }
-// 1 / (principal square root).  complex128 without FP64 divisions and roots
-// (about 100 FP64 operations a lane): a complex64 estimate and two Newton steps
-// w <- w (3 - d w^2) / 2, which square its error.
+// reciprocals and inverse roots of pivots.  complex128 without FP64 divisions
+// and roots (about 100 FP64 operations a lane): an FP32 estimate and two Newton
+// steps, which square its error.
+__device__ __forceinline__ float2 rcp_(float2 a) { return crecip_fast(a); }
+__device__ __forceinline__ double2 rcp_(double2 a) {
+    const double m = a.x * a.x + a.y * a.y;
+    if (!(m > 1e-30 && m < 1e30)) return crecip(a);
+    double q = (double)__frcp_rn((float)m);
+#pragma unroll
+    for (int it = 0; it < 2; it++) q = q * (2.0 - m * q);
+    return cz(a.x * q, -a.y * q);
+}
+// 1 / (principal square root); w <- w (3 - d w^2) / 2
 __device__ __forceinline__ float2 rsqrt_(float2 a) { return crecip_fast(csqrt_fast(a)); }
 __device__ __forceinline__ double2 rsqrt_(double2 d) {
     const float2 f = to_f(d);
@@ -256,101 +264,132 @@ __global__ __launch_bounds__(256) void k_sub_gather(DevSub D, int t0) {
     }
 }
 
-// Adds a front's matrix entries to F11 and F12 and inverts F11.  The inverse
-// is symmetric up to the sign between swept and unswept rows (Gauss-Jordan
-// sweeps), so only the lower triangle is computed, each entry in a register of
-// its thread; per sweep the pivot row is published twice, raw and divided by
-// the pivot.
-template <typename T, int NT, int NE>
-__global__ __launch_bounds__(NT) void k_sub_pivot(DevSub D, int f0, int nnz) {
+// In-place inverse of the symmetric h x h matrix M (h <= 32, row stride ld) in
+// shared memory by Gauss-Jordan sweeps: lane = row, warp w the columns w, w + 8,
+// ..., in registers.  Per sweep the pivot's warp publishes its column and the
+// pivot row over the pivot, which is the column again up to the sign between
+// swept and unswept rows; one barrier, and one complex multiply-add an entry.
+// Ends with a barrier.  False where a pivot is zero or not finite.
+template <typename T>
+struct Sweep {
+    T col[2][32], row[2][32];
+};
+
+template <typename T>
+__device__ __forceinline__ bool invert_block(T *M, int ld, int h, Sweep<T> &sw) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    T a[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) a[q] = lane < h && 8 * q + w < h ? M[lane * ld + 8 * q + w] : zero_<T>();
+    bool ok = true;
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+#pragma unroll
+        for (int ww = 0; ww < 8; ww++) {
+            const int p = 8 * q + ww, b = p & 1;
+            if (p >= h) continue;  // the same for all threads
+            if (w == ww) {
+                const T d = shfl_(a[q], p);
+                if (is_bad(d)) ok = false;
+                const T iv = rcp_(d);
+                sw.col[b][lane] = a[q];
+                sw.row[b][lane] = lane == p ? iv : mul_(lane < p ? neg_(a[q]) : a[q], iv);
+                a[q] = zero_<T>();
+            }
+            __syncthreads();
+            const T c = sw.col[b][lane];
+#pragma unroll
+            for (int z = 0; z < 4; z++) {
+                const T t = sw.row[b][8 * z + w];
+                fms_(a[z], c, t);
+                if (lane == p) a[z] = t;
+            }
+        }
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        if (lane < h && 8 * q + w < h) M[lane * ld + 8 * q + w] = a[q];
+    __syncthreads();
+    return ok;
+}
+
+// Adds a front's matrix entries to F11 and F12 and inverts F11, one block of
+// 256 threads.  Beyond 32 nodes by blocks, F11 = [A B; B^T D]: G = A^-1 B, the
+// complement D - B^T G inverted, [A^-1 + K G^T, -K; -K^T, Si] with K = G Si.  (Swept
+// as a whole, lower triangle only, a front of 61 nodes took 114 us: a chain of
+// two barriers and divergent updates a node.)
+template <typename T>
+__global__ __launch_bounds__(256) void k_sub_pivot(DevSub D, int f0, int nnz) {
     extern __shared__ __align__(16) unsigned char sm[];
-    T *Fm = (T *)sm;
-    __shared__ T s_raw[2][kSubEMax], s_div[kSubEMax], s_inv[2];
+    constexpr int H = 32, PH = H + 1;
+    T *Fm = (T *)sm;  // [e][e | 1], then G and K, [32][33] each, beyond 32 nodes
+    __shared__ Sweep<T> sw;
     const SubFront &t = D.fr[f0 + blockIdx.x];
     const int k = blockIdx.y, e = t.e, r = t.r, ld = e | 1, tid = threadIdx.x, nent = t.nent, ent0 = t.ent0;
     const bool leaf = t.nch == 0;
     const double2 *As = D.As + (size_t)k * nnz;
-    T *F = (T *)D.F + (size_t)k * D.szF + t.oF, *H = (T *)D.H + (size_t)k * D.szG + t.oG;
+    T *F = (T *)D.F + (size_t)k * D.szF + t.oF, *Hm = (T *)D.H + (size_t)k * D.szG + t.oG;
     chain_wait();
-    for (int q = tid; q < e * e; q += NT) Fm[(q / e) * ld + q % e] = leaf ? zero_<T>() : F[q];
+    for (int q = tid; q < e * e; q += 256) Fm[(q / e) * ld + q % e] = leaf ? zero_<T>() : F[q];
     if (leaf)
-        for (int q = tid; q < e * r; q += NT) H[q] = zero_<T>();
+        for (int q = tid; q < e * r; q += 256) Hm[q] = zero_<T>();
     __syncthreads();
-    for (int q = tid; q < nent; q += NT) {
+    for (int q = tid; q < nent; q += 256) {
         const SubEnt en = D.ent[ent0 + q];
         const T v = from_<T>(As[en.p]);
-        if (en.lc < e) {  // the lower triangle is read below
-            T &d = Fm[en.lc * ld + en.lr];
+        if (en.lc < e) {
+            T &d = Fm[en.lr * ld + en.lc];
             d.x += v.x;
             d.y += v.y;
+            if (en.lr != en.lc) {
+                T &u = Fm[en.lc * ld + en.lr];
+                u.x += v.x;
+                u.y += v.y;
+            }
         } else {
-            T &d = H[(size_t)en.lr * r + en.lc - e];
+            T &d = Hm[(size_t)en.lr * r + en.lc - e];
             d.x += v.x;
             d.y += v.y;
         }
     }
     __syncthreads();
-    // entries of this thread: q = tid + z NT of the lower triangle, row by row
-    T w[NE];
-    int ri[NE], ci[NE];
-    const int cnt = e * (e + 1) / 2;
-#pragma unroll
-    for (int z = 0; z < NE; z++) {
-        const int q = tid + z * NT;
-        int i = -1, j = -1;
-        w[z] = zero_<T>();
-        if (q < cnt) {
-            i = (int)((sqrtf(8.f * (float)q + 1.f) - 1.f) * 0.5f);
-            while (i * (i + 1) / 2 > q) i--;
-            while ((i + 1) * (i + 2) / 2 <= q) i++;
-            j = q - i * (i + 1) / 2;
-            w[z] = Fm[i * ld + j];
+    bool ok = invert_block(Fm, ld, min(e, H), sw);
+    if (e > H) {
+        const int h = e - H, lane = tid & 31, w = tid >> 5;
+        T *G = Fm + e * ld, *K = G + H * PH;
+        // G = A^-1 B: row = lane, columns w, w + 8, ...
+        for (int c = w; c < h; c += 8) {
+            T s = zero_<T>();
+#pragma unroll 8
+            for (int p = 0; p < H; p++) fma_(s, Fm[lane * ld + p], Fm[p * ld + H + c]);
+            G[lane * PH + c] = s;
         }
-        ri[z] = i;
-        ci[z] = j;
-    }
-    bool bad = false;
-    auto publish = [&](int p, int buf) {
-#pragma unroll
-        for (int z = 0; z < NE; z++) {
-            if (ri[z] == p) s_raw[buf][ci[z]] = w[z];
-            else if (ci[z] == p) s_raw[buf][ri[z]] = w[z];
-            if (ri[z] == p && ci[z] == p) {
-                if (is_bad(w[z])) bad = true;
-                s_inv[buf] = rcp_(w[z]);
-            }
-        }
-    };
-    if (e > 0) publish(0, 0);
-    for (int p = 0; p < e; p++) {
-        const int buf = p & 1;
         __syncthreads();
-        if (tid < e) s_div[tid] = mul_(s_raw[buf][tid], s_inv[buf]);
-        __syncthreads();
-#pragma unroll
-        for (int z = 0; z < NE; z++) {
-            const int i = ri[z], j = ci[z];
-            if (i < 0) continue;
-            if (i == p) {
-                w[z] = j == p ? s_inv[buf] : s_div[j];
-            } else if (j == p) {
-                w[z] = neg_(s_div[i]);
-            } else {
-                // column entry (i, p): minus the stored one where row i is swept already
-                T u = s_raw[buf][i];
-                if (i < p) u = neg_(u);
-                fms_(w[z], u, s_div[j]);
+        if (lane < h)
+            for (int c = w; c < h; c += 8) {
+                T s = Fm[(H + lane) * ld + H + c];
+#pragma unroll 8
+                for (int p = 0; p < H; p++) fms_(s, Fm[(H + lane) * ld + p], G[p * PH + c]);
+                Fm[(H + lane) * ld + H + c] = s;
             }
+        __syncthreads();
+        if (!invert_block(Fm + H * ld + H, ld, h, sw)) ok = false;
+        for (int c = w; c < h; c += 8) {
+            T s = zero_<T>();
+            for (int p = 0; p < h; p++) fma_(s, G[lane * PH + p], Fm[(H + p) * ld + H + c]);
+            K[lane * PH + c] = s;
+            Fm[lane * ld + H + c] = neg_(s);
+            Fm[(H + c) * ld + lane] = neg_(s);
         }
-        if (p + 1 < e) publish(p + 1, buf ^ 1);
+        __syncthreads();
+        for (int c = w; c < H; c += 8) {
+            T s = Fm[lane * ld + c];
+            for (int p = 0; p < h; p++) fma_(s, K[lane * PH + p], G[c * PH + p]);
+            Fm[lane * ld + c] = s;
+        }
+        __syncthreads();
     }
-#pragma unroll
-    for (int z = 0; z < NE; z++)
-        if (ri[z] >= 0) {
-            F[ri[z] * e + ci[z]] = w[z];
-            F[ci[z] * e + ri[z]] = w[z];
-        }
-    if (bad) atomicCAS(&D.kbad[k], 0, 28);
+    for (int q = tid; q < e * e; q += 256) F[q] = Fm[(q / e) * ld + q % e];
+    if (!ok) atomicCAS(&D.kbad[k], 0, 28);
 }
 
 // A thread's entries of a kKT x E operand tile (k-major) in registers: the
@@ -1262,24 +1301,19 @@ inline unsigned nb(size_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
 template <typename T>
 int factor_t(const DevProblem &P, const DevSub &D, const SubPlan &sp, int K, cudaStream_t st) {
+    auto bytes = [](int e) { return sizeof(T) * (e * (e | 1) + (e > 32 ? 2 * 32 * 33 : 0)); };
     static std::once_flag once;
-    std::call_once(once, [] {
-        const int most = (int)sizeof(T) * kSubEMax * (kSubEMax | 1);
-        cudaFuncSetAttribute(k_sub_pivot<T, 256, 9>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        cudaFuncSetAttribute(k_sub_pivot<T, 128, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    std::call_once(once, [&] {
+        cudaFuncSetAttribute(k_sub_pivot<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes(kSubEMax));
     });
     int launches = 0;
     for (int lv = 0; lv < sp.nlevel; lv++) {
         const int f0 = sp.level[lv], nf = sp.level[lv + 1] - f0;
         int emax = 1;
         for (int q = f0; q < f0 + nf; q++) emax = std::max(emax, sp.fronts[q].e);
-        const size_t smem = sizeof(T) * emax * (emax | 1);
         const int na = sp.lA[lv + 1] - sp.lA[lv], ng = sp.lG[lv + 1] - sp.lG[lv], ns = sp.lS[lv + 1] - sp.lS[lv];
         if (na) chain_launch(k_sub_gather<T>, dim3(na, K), 256, 0, st, D, sp.lA[lv]);
-        if (emax * (emax + 1) / 2 <= 128 * 5)
-            chain_launch(k_sub_pivot<T, 128, 5>, dim3(nf, K), 128, smem, st, D, f0, P.nnz);
-        else
-            chain_launch(k_sub_pivot<T, 256, 9>, dim3(nf, K), 256, smem, st, D, f0, P.nnz);
+        chain_launch(k_sub_pivot<T>, dim3(nf, K), 256, bytes(emax), st, D, f0, P.nnz);
         if (ng) chain_launch(k_sub_g<T>, dim3(ng, K), 256, 0, st, D, sp.lG[lv]);
         if (ns) chain_launch(k_sub_s<T>, dim3(ns, K), 256, 0, st, D, sp.lS[lv]);
         launches += 1 + (na > 0) + (ng > 0) + (ns > 0);
