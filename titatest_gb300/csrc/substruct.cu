@@ -703,7 +703,7 @@ __global__ __launch_bounds__(kRT, 5) void k_sub_root(DevSub D, SubBatch B) {
     constexpr int NQ = NB / 4, CT = NB / 4, per = 16 / sizeof(T);
     T *As = (T *)sm;       // [S][KC][ROWS]; also W of a tile, [NB][ROWS]
     T *Bs = As + Q::AT;    // [S][KC][NB]; also the inverse block, Bs[a][b] = inverse(b, a)
-    __shared__ T col[2][32], inv[2];
+    __shared__ T col[2][32], mul[2][32], piv[32];
     const int s = blockIdx.x, kk_ = s / B.Lb, k = B.k0 + kk_, l = s % B.Lb;
     const int mp = D.mp, ldc = D.ldc, m = D.m, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     T *C = (T *)B.C + (size_t)s * mp * ldc;
@@ -782,14 +782,20 @@ __global__ __launch_bounds__(kRT, 5) void k_sub_root(DevSub D, SubBatch B) {
             cp_wait<0>();
             __syncthreads();
             if (r0 == j) {
-                // diagonal block: lane = row, warp w the columns w, w + 4, ...
-                const int row = NB == 32 ? lane : lane & (NB - 1);
-                T a[NQ], x[NQ];
+                // Diagonal block, L D L^T with the inverse of L beside it: per column the
+                // multipliers a_ip / d update both, one barrier; the rows of the inverse
+                // are scaled by 1 / sqrt(d) at the end, all at once.  Warp w has the
+                // columns w, w + 4, ...; lane = row, in complex128 the lower half of the
+                // warp on the block, the upper on the inverse.
+                constexpr bool split = NB == 16;
+                const int row = lane & (NB - 1), half = split ? lane >> 4 : 0;
+                T a[NQ], x[split ? 1 : NQ];
 #pragma unroll
                 for (int q = 0; q < NQ; q++) {
-                    a[q] = As[(4 * q + wid) * kRows + row];
-                    x[q] = zero_<T>();
-                    if (row == 4 * q + wid) x[q].x = 1;
+                    T one = zero_<T>();
+                    if (row == 4 * q + wid) one.x = 1;
+                    a[q] = half ? one : As[(4 * q + wid) * kRows + row];
+                    if constexpr (!split) x[q] = one;
                 }
 #pragma unroll
                 for (int q = 0; q < NQ; q++)
@@ -797,30 +803,37 @@ __global__ __launch_bounds__(kRT, 5) void k_sub_root(DevSub D, SubBatch B) {
                     for (int ww = 0; ww < 4; ww++) {
                         const int p = 4 * q + ww, buf = p & 1;
                         if (wid == ww) {
-                            const T d = shfl_(a[q], p);
+                            const T d = shfl_(a[q], p), raw = split ? shfl_(a[q], row) : a[q];
                             if (is_bad(d)) bad = true;
-                            const T iv = rsqrt_(d);
-                            col[buf][row] = row > p ? mul_(a[q], iv) : zero_<T>();
-                            if (lane == 0) inv[buf] = iv;
+                            const T m1 = mul_(raw, rcp_(d));
+                            if (!half) {
+                                col[buf][row] = raw;
+                                mul[buf][row] = row > p ? m1 : zero_<T>();
+                                if (row == p) piv[p] = d;
+                            }
                         }
                         __syncthreads();
-                        const T cl = col[buf][row], iv = inv[buf];
+                        const T mi = mul[buf][row];
 #pragma unroll
                         for (int z = 0; z < NQ; z++) {
                             const int c = 4 * z + wid;
-                            if (z >= q && c > p) fms_(a[z], cl, col[buf][c]);
-                            if (z <= q) {
-                                const T xp = mul_(shfl_(x[z], p), iv);
-                                if (row == p) x[z] = xp;
-                                else if (row > p) fms_(x[z], cl, xp);
+                            if constexpr (split) {
+                                const T xp = shfl_(a[z], 16 + p);
+                                T f = c > p ? col[buf][c] : zero_<T>();
+                                if (half) f = xp;
+                                fms_(a[z], mi, f);
+                            } else {
+                                if (z >= q && c > p) fms_(a[z], mi, col[buf][c]);
+                                if (z <= q) fms_(x[z], mi, shfl_(x[z], p));
                             }
                         }
                     }
-                if (lane < NB) {
+                const T iv = rsqrt_(piv[row]);
+                if (!split || half) {
 #pragma unroll
                     for (int q = 0; q < NQ; q++) {
                         const int c = 4 * q + wid;
-                        const T v = row >= c ? x[q] : zero_<T>();
+                        const T v = row >= c ? mul_(split ? a[q] : x[split ? 0 : q], iv) : zero_<T>();
                         Bs[c * NB + row] = v;
                         C[(size_t)(j + c) * ldc + j + row] = v;
                     }
