@@ -68,3 +68,21 @@ def test_rectangles_of_a_small_memory_budget(gpu_lib, prec, systems):
         assert m.stats()["nbatches"] > 1
         a2 = m.adjoint(g)
     assert relerr(v2, v1) < 1e-12 and relerr(a2, a1) < 1e-12
+
+
+@pytest.mark.parametrize("where", ["interior", "corner"])
+def test_fictitious_sink_is_a_source(gpu_lib, where):
+    """The right-hand sides with a fictitious sink, inside the mesh and on the
+    mixed boundary (a root node): only fronts above a source take part in
+    their upward sweep."""
+    from titatest_gb300 import MIXED, PLAIN, CRMod
+    s = _case(36, 14, 9)
+    g = s.grid
+    x, y = g.node_xy()
+    nsink = int(np.argmin(np.hypot(x - 18, y + 5)) if where == "interior" else np.argmax(x - y)) + 1
+    P = O.Problem(g, s.survey)
+    kwn, kwnwi = P.rwaven()
+    kp = P.forward(s.sigma, kwn, kwnwi, lsink=True, nsink=nsink)
+    for prec, tol in ((PLAIN, 1e-10), (MIXED, 1e-6)):
+        with CRMod(g, s.survey, kwn, kwnwi, lsink=True, nsink=nsink, precision=prec) as m:
+            assert relerr(m.forward(s.sigma, kpot=True)["kpot"], kp) < tol

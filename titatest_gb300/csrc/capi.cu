@@ -501,7 +501,7 @@ int sub_solve_rect(crgpu_ctx *c, const SubBatch &B, const double2 *src, cudaStre
     SubBatch B0 = B;
     B0.kact = nullptr;
     sub_launch_rhs(c->P, c->D, B, mixed, c->lsink, c->nsink, src, st);
-    c->stats.kernel_launches += 1 + sub_launch_apply(c->D, c->sp, B0, mixed, nullptr, st);
+    c->stats.kernel_launches += 1 + sub_launch_apply(c->D, c->sp, B0, mixed, src == nullptr, nullptr, st);
     if (!mixed) return 0;
     RefineCount *cnt = (RefineCount *)c->d_refine + (size_t)slot * kRefineCap;
     const int steps = std::min(c->refine_maxit, kRefineCap);
@@ -511,7 +511,7 @@ int sub_solve_rect(crgpu_ctx *c, const SubBatch &B, const double2 *src, cudaStre
     for (int it = 0; it < steps; it++) {
         const int *nprev = it > 0 ? &cnt[it - 1].n : nullptr;
         sub_launch_residual(c->P, c->D, B, src == nullptr, c->lsink, c->nsink, nprev, st);
-        c->stats.kernel_launches += 3 + sub_launch_apply(c->D, c->sp, B, true, nprev, st);
+        c->stats.kernel_launches += 3 + sub_launch_apply(c->D, c->sp, B, true, false, nprev, st);
         sub_launch_accumulate(c->D, B, false, c->refine_tol, nprev, &cnt[it].n, &cnt[it].z, st);
     }
     c->refine_used[slot] = std::max(c->refine_used[slot], steps);
@@ -1140,7 +1140,9 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
             c->sys_l.push_back(0);
         }
     }
-    if (c->nrhs == 1 && build_sub_plan(hg, c->pat, sub_shape(precision == CRGPU_MIXED), c->sp)) {
+    std::vector<int32_t> sources(enr0);
+    if (c->nsink >= 0 && c->nsink < hg.n) sources.push_back(c->nsink);
+    if (c->nrhs == 1 && build_sub_plan(hg, c->pat, sub_shape(precision == CRGPU_MIXED), sources, c->sp)) {
         const SubPlan &sp = c->sp;
         DevSub &D = c->D;
         D.n = sp.n;
@@ -1160,6 +1162,7 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
         D.root_u0 = sp.fronts[sp.root_child].u0;
         D.root_r = sp.fronts[sp.root_child].r;
         D.root_oS = sp.fronts[sp.root_child].oS;
+        D.root_live = sp.fronts[sp.root_child].live != 0;
         std::vector<int32_t> fcolpos(c->pat.fcol.size());
         for (size_t q = 0; q < fcolpos.size(); q++) fcolpos[q] = sp.pos[c->pat.fcol[q]];
         e = upload(c, &D.fr, sp.fronts);
@@ -1173,6 +1176,7 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
         if (!e) e = upload(c, &D.tG, sp.tG);
         if (!e) e = upload(c, &D.tS, sp.tS);
         if (!e) e = upload(c, &D.tU, sp.tU);
+        if (!e) e = upload(c, &D.tV, sp.tV);
         if (!e) e = upload(c, &D.tD, sp.tD);
         if (!e) e = upload(c, &D.pos, sp.pos);
         if (!e) e = upload(c, &D.node, sp.node);

@@ -127,7 +127,8 @@ struct Build {
 
 }  // namespace
 
-bool build_sub_plan(const HostGrid &hg, const Pattern &pat, const SubShape &shape, SubPlan &sp) {
+bool build_sub_plan(const HostGrid &hg, const Pattern &pat, const SubShape &shape,
+                    const std::vector<int32_t> &sources, SubPlan &sp) {
     sp = SubPlan();
     const int n = hg.n;
     std::vector<uint8_t> root(n, 0);
@@ -166,6 +167,8 @@ bool build_sub_plan(const HostGrid &hg, const Pattern &pat, const SubShape &shap
     }
     // fronts, their rows and the children's rows in them
     std::vector<int32_t> local(n, -1);
+    std::vector<uint8_t> source(n, 0);
+    for (int v : sources) source[v] = 1;
     sp.fronts.resize(nf);
     for (int q = 0; q < nf; q++) {
         Build::F &s = b.f[order[q]];
@@ -187,6 +190,9 @@ bool build_sub_plan(const HostGrid &hg, const Pattern &pat, const SubShape &shap
         sp.c_factor += (double)t.e * t.e * t.e + (double)t.e * t.e * t.r + 0.5 * t.e * t.r * (double)t.r;
         sp.c_apply += (double)t.e * (t.e + 2.0 * t.r);
         t.nch = (int)s.ch.size();
+        t.live = t.pad = 0;
+        for (int v : s.E)
+            if (source[v]) t.live = 1 << kSubCh;
         for (int z = 0; z < kSubCh; z++) {
             t.cr[z] = t.cu[z] = t.inv[z] = 0;
             t.cS[z] = 0;
@@ -195,6 +201,7 @@ bool build_sub_plan(const HostGrid &hg, const Pattern &pat, const SubShape &shap
             t.cr[z] = u.r;
             t.cu[z] = u.u0;
             t.cS[z] = u.oS;
+            if (u.live) t.live |= 1 << kSubCh | 1 << z;
             t.inv[z] = (int)sp.inv.size();
             const std::vector<int32_t> &cr = b.f[s.ch[z]].R;
             for (size_t y = 0; y < cr.size(); y++) local[cr[y]] = (int)y;
@@ -263,7 +270,7 @@ bool build_sub_plan(const HostGrid &hg, const Pattern &pat, const SubShape &shap
     // tiles
     auto tiles = [&](int v) { return (v + shape.tile - 1) / shape.tile; };
     sp.lG.assign(1, 0);
-    sp.lA = sp.lS = sp.lU = sp.lD = sp.lG;
+    sp.lA = sp.lS = sp.lU = sp.lD = sp.lV = sp.lG;
     for (int lv = 0; lv < sp.nlevel; lv++) {
         for (int q = sp.level[lv]; q < sp.level[lv + 1]; q++) {
             const SubFront &t = sp.fronts[q];
@@ -276,12 +283,16 @@ bool build_sub_plan(const HostGrid &hg, const Pattern &pat, const SubShape &shap
             for (int i = 0; i < tr2; i++) {
                 for (int j = 0; j <= i; j++) sp.tS.push_back({q, i, j});
             }
-            for (int i = 0; i < std::max(1, tr2); i++) sp.tU.push_back({q, i, 0});
+            for (int i = 0; i < std::max(1, tr2); i++) {
+                sp.tU.push_back({q, i, 0});
+                if (t.live) sp.tV.push_back({q, i, 0});
+            }
         }
         sp.lA.push_back((int)sp.tA.size());
         sp.lG.push_back((int)sp.tG.size());
         sp.lS.push_back((int)sp.tS.size());
         sp.lU.push_back((int)sp.tU.size());
+        sp.lV.push_back((int)sp.tV.size());
         sp.lD.push_back((int)sp.tD.size());
     }
     return true;

@@ -24,9 +24,11 @@ struct SubShape {
 // e..e+r-1 the positions rows[rows0 .. rows0+r-1].
 struct SubFront {
     int32_t e, r, nd0, nch;
+    int32_t live;         // bit kSubCh: a source node is eliminated here or below; bit c: ... below child c
     int32_t ent0, nent;   // matrix entries assembled here
     int32_t rows0;        // into SubPlan::rows
     int32_t u0;           // first row of this front's update vectors
+    int32_t pad;
     int64_t oF, oG, oS;   // inverse pivot block (e x e), G (e x r), Schur complement (r x r)
     // children: their r, first update row and Schur complement, and
     // (in SubPlan::inv) the row among a child's r rows of every local row, or -1
@@ -58,13 +60,17 @@ struct SubPlan {
     // and row tiles of the solves (r up, e down), by level
     std::vector<SubTile> tA, tG, tS, tU, tD;
     std::vector<int32_t> lA, lG, lS, lU, lD;   // nlevel + 1 each
+    std::vector<SubTile> tV;                   // those of tU whose front is live
+    std::vector<int32_t> lV;
     int64_t szF = 0, szG = 0, szS = 0;         // entries per wavenumber
     int32_t szU = 0;                           // update rows per wavenumber
     double c_factor = 0, c_apply = 0;          // complex multiply-adds: factor per wavenumber, one solve
 };
 
 // The plan for the grid, or false where it has no root (no mixed boundary)
-// or no interior.
-bool build_sub_plan(const HostGrid &hg, const Pattern &pat, const SubShape &shape, SubPlan &sp);
+// or no interior.  sources: the nodes that kompab's right-hand sides have
+// entries at (electrodes, the fictitious sink).
+bool build_sub_plan(const HostGrid &hg, const Pattern &pat, const SubShape &shape,
+                    const std::vector<int32_t> &sources, SubPlan &sp);
 
 }  // namespace crgpu

@@ -868,7 +868,7 @@ __global__ __launch_bounds__(kRT, 5) void k_sub_root(DevSub D, SubBatch B) {
 constexpr int kST = 256;
 
 template <typename T>
-__global__ __launch_bounds__(kST) void k_sub_root_solve(DevSub D, SubBatch B, const int *nprev) {
+__global__ __launch_bounds__(kST) void k_sub_root_solve(DevSub D, SubBatch B, int unit, const int *nprev) {
     extern __shared__ __align__(16) unsigned char sm[];
     constexpr int NB = RootShape<T>::NB, CW = NB / 8;  // columns of a warp
     T *v = (T *)sm;  // [mp]
@@ -887,7 +887,7 @@ __global__ __launch_bounds__(kST) void k_sub_root_solve(DevSub D, SubBatch B, co
         if (i < D.m) {
             u = Y[(size_t)i * B.Lb];
             const int x = D.root_inv[i];
-            if (x >= 0) {
+            if (x >= 0 && (!unit || D.root_live)) {
                 const T w = U[(size_t)x * B.Lb];
                 u.x += w.x;
                 u.y += w.y;
@@ -954,16 +954,18 @@ __global__ __launch_bounds__(kST) void k_sub_root_solve(DevSub D, SubBatch B, co
 
 // Up the tree: b_E (own right-hand sides and the children's updates) goes to
 // W, the update rows U = (children's updates) - G^T b_E to the parent.  One
-// block per tile of update rows x electrodes.
+// block per tile of update rows x electrodes.  unit: kompab's right-hand sides,
+// zero but at the electrodes, so only the fronts above an electrode take part
+// (config 2: 80 of 300) and the others' rows of W and U are not read.
 template <typename T>
-__global__ __launch_bounds__(256) void k_sub_up(DevSub D, SubBatch B, int t0, const int *nprev) {
+__global__ __launch_bounds__(256) void k_sub_up(DevSub D, SubBatch B, int t0, int unit, const int *nprev) {
     constexpr int E = Tile<T>::E, M = Tile<T>::M, P = Tile<T>::P;
     __shared__ __align__(16) T A[kKT * P], Bm[kKT * P];
     __shared__ int se[kSubCh][kSubEMax], sr[kSubCh][E];
     const int kk = blockIdx.z, k = B.k0 + kk;
-    const SubTile tl = D.tU[t0 + blockIdx.x];
+    const SubTile tl = (unit ? D.tV : D.tU)[t0 + blockIdx.x];
     const SubFront &t = D.fr[tl.front];
-    const int e = t.e, r = t.r, nch = t.nch, i0 = tl.ti * E, l0 = blockIdx.y * E, L = B.Lb, nl = min(E, L - l0);
+    const int e = t.e, r = t.r, nch = t.nch, from = unit ? t.live : -1, i0 = tl.ti * E, l0 = blockIdx.y * E, L = B.Lb, nl = min(E, L - l0);
     const T *G = (const T *)D.G + (size_t)k * D.szG + t.oG;
     const T *__restrict__ Y = (const T *)B.Y + ((size_t)kk * D.n + t.nd0) * L + l0;
     T *__restrict__ W = (T *)B.W + ((size_t)kk * D.n + t.nd0) * L + l0;
@@ -985,6 +987,7 @@ __global__ __launch_bounds__(256) void k_sub_up(DevSub D, SubBatch B, int t0, co
     auto load_b = [&](int p) {
         b.load(Y + (size_t)p * L, L, e - p, nl);
         for (int c = 0; c < nch; c++) {
+            if (!(from >> c & 1)) continue;
             const T *U = Uk + (size_t)t.cu[c] * L + col;
             T g[Operand<T>::N];
 #pragma unroll
@@ -1008,6 +1011,7 @@ __global__ __launch_bounds__(256) void k_sub_up(DevSub D, SubBatch B, int t0, co
     const int tr = acc.tr(), tc = acc.tc();
     const bool work = i0 + acc.warp_row() < r;
     for (int c = 0; c < nch; c++) {
+        if (!(from >> c & 1)) continue;
         const T *U = Uk + (size_t)t.cu[c] * L;
 #pragma unroll
         for (int i = 0; i < M; i++) {
@@ -1053,7 +1057,7 @@ __global__ __launch_bounds__(256) void k_sub_up(DevSub D, SubBatch B, int t0, co
 // Down the tree: x_E = F11^-1 b_E - G x_R, one block per tile of rows x
 // electrodes
 template <typename T>
-__global__ __launch_bounds__(256) void k_sub_down(DevSub D, SubBatch B, int t0, const int *nprev) {
+__global__ __launch_bounds__(256) void k_sub_down(DevSub D, SubBatch B, int t0, int unit, const int *nprev) {
     constexpr int E = Tile<T>::E, M = Tile<T>::M, P = Tile<T>::P, kIdx = 512;
     __shared__ __align__(16) T A[kKT * P], Bm[kKT * P];
     __shared__ int sidx[kIdx];
@@ -1076,7 +1080,7 @@ __global__ __launch_bounds__(256) void k_sub_down(DevSub D, SubBatch B, int t0, 
     const int tr = acc.tr(), tc = acc.tc();
     const bool work = i0 + acc.warp_row() < e;
     // chunks: first the columns of G, then those of F11^-1
-    const int nr = (r + kKT - 1) / kKT, nc = nr + (e + kKT - 1) / kKT;
+    const int nr = (r + kKT - 1) / kKT, nc = nr + (unit && !t.live ? 0 : (e + kKT - 1) / kKT);
     auto load = [&](int ch) {
         if (ch < nr) {
             const int p = ch * kKT;
@@ -1093,7 +1097,7 @@ __global__ __launch_bounds__(256) void k_sub_down(DevSub D, SubBatch B, int t0, 
             b.load(W + (size_t)p * L, L, e - p, nl);
         }
     };
-    load(0);
+    if (nc > 0) load(0);
     for (int ch = 0; ch < nc; ch++) {
         if (ch < nr) a.store_t(A);
         else a.store(A);
@@ -1114,7 +1118,8 @@ __global__ __launch_bounds__(256) void k_sub_down(DevSub D, SubBatch B, int t0, 
     for (int i = 0; i < M; i++)
 #pragma unroll
         for (int j = 0; j < M; j++)
-            if (i0 + tr + i < e && tc + j < nl) Z[(size_t)(i0 + tr + i) * L + tc + j] = acc.v[i][j];
+            if (i0 + tr + i < e && tc + j < nl)
+                Z[(size_t)(i0 + tr + i) * L + tc + j] = nc > nr ? acc.v[i][j] : neg_(acc.v[i][j]);
 }
 
 // -------------------------------------------------- vectors of a rectangle
@@ -1152,7 +1157,7 @@ __global__ void k_sub_unit_rhs(DevProblem P, DevSub D, SubBatch B, int lsink, in
 #pragma unroll
     for (int q = 0; q < 2; q++) {
         const int i = nodes[q];
-        if (i < 0) continue;
+        if (i < 0 || i >= P.n) continue;
         const double v = unit_rhs(P, el, i, lsink, nsink) * D.fk[(size_t)(B.k0 + kk) * P.n + i];
         ((T *)B.Y)[((size_t)kk * D.n + D.pos[i]) * B.Lb + l] = from_<T>(cz(v, 0.0));
     }
@@ -1352,16 +1357,21 @@ void root_t(const DevProblem &P, const DevSub &D, const SubBatch &B, const doubl
 }
 
 template <typename T>
-int apply_t(const DevSub &D, const SubPlan &sp, const SubBatch &B, const int *nprev, cudaStream_t st) {
+int apply_t(const DevSub &D, const SubPlan &sp, const SubBatch &B, bool unit, const int *nprev, cudaStream_t st) {
     const int lt = (B.Lb + Tile<T>::E - 1) / Tile<T>::E;
-    for (int lv = 0; lv < sp.nlevel; lv++)
-        chain_launch(k_sub_up<T>, dim3(sp.lU[lv + 1] - sp.lU[lv], lt, B.Kb), 256, 0, st, D, B, sp.lU[lv], nprev);
-    chain_launch(k_sub_root_solve<T>, dim3(B.Kb * B.Lb), kST, sizeof(T) * D.mp, st, D, B, nprev);
-    int launches = sp.nlevel + 1;
+    const std::vector<int32_t> &up = unit ? sp.lV : sp.lU;
+    int launches = 1;
+    for (int lv = 0; lv < sp.nlevel; lv++) {
+        const int nu = up[lv + 1] - up[lv];
+        if (!nu) continue;
+        chain_launch(k_sub_up<T>, dim3(nu, lt, B.Kb), 256, 0, st, D, B, up[lv], unit ? 1 : 0, nprev);
+        launches++;
+    }
+    chain_launch(k_sub_root_solve<T>, dim3(B.Kb * B.Lb), kST, sizeof(T) * D.mp, st, D, B, unit ? 1 : 0, nprev);
     for (int lv = sp.nlevel - 1; lv >= 0; lv--) {
         const int nd = sp.lD[lv + 1] - sp.lD[lv];
         if (!nd) continue;
-        chain_launch(k_sub_down<T>, dim3(nd, lt, B.Kb), 256, 0, st, D, B, sp.lD[lv], nprev);
+        chain_launch(k_sub_down<T>, dim3(nd, lt, B.Kb), 256, 0, st, D, B, sp.lD[lv], unit ? 1 : 0, nprev);
         launches++;
     }
     return launches;
@@ -1394,9 +1404,9 @@ void sub_launch_root(const DevProblem &P, const DevSub &D, const SubBatch &B, co
     mixed ? root_t<float2>(P, D, B, sigma, st) : root_t<double2>(P, D, B, sigma, st);
 }
 
-int sub_launch_apply(const DevSub &D, const SubPlan &sp, const SubBatch &B, bool mixed, const int *nprev,
+int sub_launch_apply(const DevSub &D, const SubPlan &sp, const SubBatch &B, bool mixed, bool unit, const int *nprev,
                      cudaStream_t st) {
-    return mixed ? apply_t<float2>(D, sp, B, nprev, st) : apply_t<double2>(D, sp, B, nprev, st);
+    return mixed ? apply_t<float2>(D, sp, B, unit, nprev, st) : apply_t<double2>(D, sp, B, unit, nprev, st);
 }
 
 void sub_launch_rhs(const DevProblem &P, const DevSub &D, const SubBatch &B, bool mixed, int lsink, int nsink,

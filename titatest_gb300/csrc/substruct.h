@@ -16,10 +16,10 @@ struct DevSub {
     int64_t szF, szG, szS;
     const SubFront *fr;
     const SubEnt *ent, *be;
-    const SubTile *tA, *tG, *tS, *tU, *tD;
+    const SubTile *tA, *tG, *tS, *tU, *tV, *tD;
     const int32_t *pos, *node, *rows, *inv, *root_inv, *fcolpos;
     const int32_t *be_ptr, *rb_ptr, *rb_ent, *rb_pos;
-    int root_ent0, n_root_ent, n_be, root_child, root_u0, root_r;
+    int root_ent0, n_root_ent, n_be, root_child, root_u0, root_r, root_live;
     int64_t root_oS;
     double2 *As;     // [K][nnz] area parts, scaled by fk on both sides
     double *fk;      // [K][n]   scaling of the area parts' diagonal, by node
@@ -47,7 +47,8 @@ void sub_launch_values(const DevProblem &P, const DevSub &D, const double2 *sigm
 int sub_launch_factor(const DevProblem &P, const DevSub &D, const SubPlan &sp, int K, bool mixed, cudaStream_t st);
 void sub_launch_root(const DevProblem &P, const DevSub &D, const SubBatch &B, const double2 *sigma, bool mixed,
                      cudaStream_t st);
-int sub_launch_apply(const DevSub &D, const SubPlan &sp, const SubBatch &B, bool mixed, const int *nprev,
+// unit: the right-hand sides are kompab's, zero but at the sources of the plan
+int sub_launch_apply(const DevSub &D, const SubPlan &sp, const SubBatch &B, bool mixed, bool unit, const int *nprev,
                      cudaStream_t st);
 void sub_launch_rhs(const DevProblem &P, const DevSub &D, const SubBatch &B, bool mixed, int lsink, int nsink,
                     const double2 *src, cudaStream_t st);
