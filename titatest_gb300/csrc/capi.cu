@@ -1061,14 +1061,13 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
     if (!e) e = upload(c, &P.meas, meas);
     if (!e) e = upload(c, &P.strom, strom);
     {
-        std::vector<int2> dip;
-        std::vector<int4> mdip, pass;
-        host_sens_passes(meas, c->nanz, c->eanz, dip, mdip, pass);
-        P.nspass = (int)pass.size();
-        for (const int4 &p : pass) P.sens_dips = std::max(P.sens_dips, p.w);
-        if (!e) e = upload(c, &P.dip, dip);
-        if (!e) e = upload(c, &P.mdip, mdip);
-        if (!e) e = upload(c, &P.spass, pass);
+        SensPlan sn;
+        host_sens_passes(meas, c->nanz, c->eanz, sn);
+        P.nspass = (int)sn.pass.size();
+        P.sens_dips = sn.most;
+        if (!e) e = upload(c, &P.dip, sn.dip);
+        if (!e) e = upload(c, &P.mdip, sn.slot);
+        if (!e) e = upload(c, &P.spass, sn.pass);
         if (!e) e = dalloc(c, &P.sfac, (size_t)std::max(c->nanz, 1));
     }
     if (!e) e = upload(c, &P.kwn, kwn);

@@ -7,6 +7,12 @@
 
 namespace crgpu {
 
+// One pass over the measurements of an element's sensitivities: slots i0 .. i1-1,
+// those before split with both sides in tables; nd + nd2 dipoles from d0 on.
+struct SensPass {
+    int32_t i0, split, i1, d0, nd, nd2;
+};
+
 struct DevProblem {
     int n, mb, W, elanz, relanz, eanz, nanz, K, nnz, nnz_full;
     int rw;               // padded row width of the lower pattern (row i at i*rw)
@@ -38,11 +44,12 @@ struct DevProblem {
     const int32_t *enr0;   // eanz: electrode -> node (0-based)
     const int32_t *meas;   // nanz*4: electrodes e1,e2,e3,e4 (0-based, -1 = none)
     const double *strom;   // nanz
-    // sensitivities (post.cu): distinct dipoles (first, second electrode; eanz:
-    // none) of every pass, per measurement the other side's electrodes and its
-    // dipole's place in the table, the passes (first, end, dipoles), row factors
+    // sensitivities (post.cu): dipoles (first, second electrode; eanz: none) of the
+    // passes' tables, per slot (the other side's electrodes or place in the second
+    // table, place in the first table, measurement), the passes, row factors
     const int2 *dip;
-    const int4 *mdip, *spass;
+    const int4 *mdip;
+    const SensPass *spass;
     int nspass, sens_dips;  // passes; most dipoles of one
     double2 *sfac;
     const double *kwn, *kwnwi;

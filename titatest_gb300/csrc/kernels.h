@@ -80,8 +80,13 @@ void launch_bvolt(const DevProblem &P, const double2 *hpot, int mode, const doub
 bool sens_tc_supported(const DevProblem &P, int mode);
 void launch_sens_tc(const DevProblem &P, const float2 *kpot32, double2 *sens, cudaStream_t st, int e_first,
                     int e_count);
-void host_sens_passes(const std::vector<int32_t> &meas, int nanz, int eanz, std::vector<int2> &dip,
-                      std::vector<int4> &mdip, std::vector<int4> &pass);
+struct SensPlan {
+    std::vector<int2> dip;
+    std::vector<int4> slot;
+    std::vector<SensPass> pass;
+    int most = 0;
+};
+void host_sens_passes(const std::vector<int32_t> &meas, int nanz, int eanz, SensPlan &sp);
 // single: the complex64 contraction from kpot32 (mixed precision); else the
 // complex128 one from kpot
 void launch_bsens(const DevProblem &P, const double2 *kpot, const float2 *kpot32, const double2 *sigma,

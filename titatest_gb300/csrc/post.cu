@@ -92,29 +92,36 @@ void launch_bvolt(const DevProblem &P, const double2 *hpot, int mode, const doub
 // electrodes are staged in shared memory (cp.async, one wavenumber ahead), the
 // product w_k K_k d is formed once for every distinct dipole d of the side
 // (current or voltage) that has fewer of them, and a measurement is then the
-// other side's difference and one dot product; threads run over measurements
-// and keep their k-sums in registers.  K is symmetric, so either side may take
-// it.  A survey repeats its dipoles: config 2's 4000 measurements have 374
+// other side's difference (from a second table where the pass uses it again) and
+// one dot product; threads run over measurements and keep their k-sums in
+// registers.  K is symmetric, so either side may take it.  A survey repeats its dipoles: config 2's 4000 measurements have 374
 // voltage dipoles.  Per measurement and wavenumber that leaves 24 operations
 // instead of 66, and the scaling by strom / pi or sigma / (pi V) is a product
 // with a factor formed once per measurement: its six FP64 divisions an entry of
 // J took longer than the whole complex64 contraction.  GB300: bsensi of 4800
-// cells x 2000 in complex128 15.2 -> 6.8 ms (the FP64 pipe bounds it), 12000 x
-// 4000 in complex64 12.8 -> 6.7 ms (shared-memory reads: 12 a measurement and
-// wavenumber, 40 cycles without bank conflicts, 60 measured).
+// cells x 2000 in complex128 15.2 -> 6.1 ms (the FP64 pipe bounds it; 6.8 without
+// the second table, whose differences are additions on that pipe), 12000 x 4000 in
+// complex64 12.8 -> 5.0 ms (shared-memory reads; 6.7 without the second table,
+// which leaves 6 of the 9 reads of a measurement and wavenumber).  Blocks an
+// SM: complex64 spends its time waiting on shared memory, and four at 64 registers
+// (100 bytes spilled) do better than the two of 104 registers, 6.4 -> 5.0 ms;
+// complex128 gains nothing beyond two (6.09 and 6.10 ms).
 // ---------------------------------------------------------------------------
 constexpr int kSensThreads = 256;
 constexpr int kSensMPT = 16;    // measurements per thread per pass (4096 per pass)
-constexpr int kSensDip = 1024;  // dipoles of a pass's table (64 KB in complex128: two blocks an SM)
+constexpr int kSensGroup = 2;   // of them taken together (4: 6.5 and 6.0 ms in complex128 and 64, registers)
+constexpr int kSensDip = 1024;  // dipoles of a pass's first table (64 KB in complex128)
+constexpr int kSensDip2 = 512;  // ... of its second table (256: 5.15 ms in complex64, 512 and 1024: 5.0)
 
 // The measurements in passes of at most kSensThreads * kSensMPT with at most
-// kSensDip distinct dipoles on the side that has the table, whichever side
-// makes the longer pass (the fewer dipoles).  meas: e1..e4 per measurement
-// (-1: none, which becomes the zero entry eanz).
-void host_sens_passes(const std::vector<int32_t> &meas, int nanz, int eanz, std::vector<int2> &dip,
-                      std::vector<int4> &mdip, std::vector<int4> &pass) {
+// kSensDip distinct dipoles on the side that has the first table, whichever side
+// makes the longer pass (the fewer dipoles).  The other side's dipoles that the
+// pass uses at least twice go into a second table (their differences alone);
+// measurements with one of those come first.  meas: e1..e4 per measurement (-1:
+// none, which becomes the zero entry eanz).
+void host_sens_passes(const std::vector<int32_t> &meas, int nanz, int eanz, SensPlan &sp) {
     auto el = [&](int i, int q) { return meas[(size_t)i * 4 + q] < 0 ? eanz : meas[(size_t)i * 4 + q]; };
-    mdip.resize(nanz);
+    sp.slot.resize(nanz);
     for (int i0 = 0; i0 < nanz;) {
         int end[2];
         std::vector<int2> list[2];
@@ -135,35 +142,82 @@ void host_sens_passes(const std::vector<int32_t> &meas, int nanz, int eanz, std:
             }
             end[side] = i;
         }
-        const int t = end[1] > end[0] || (end[1] == end[0] && list[1].size() <= list[0].size()) ? 1 : 0;
-        // Threads in an order in which eight neighbours (one shared-memory phase
-        // of 16-byte loads) differ in their electrodes' and dipoles' places modulo
-        // 8, as far as the next 64 measurements allow: fewer bank conflicts (7.1
-        // -> 6.7 ms at 12000 x 4000 in complex64)
-        std::vector<int> wait;
-        int next = i0, used[3] = {0, 0, 0};
-        for (int slot = i0; slot < end[t]; slot++) {
-            if ((slot - i0) % 8 == 0) used[0] = used[1] = used[2] = 0;
-            while (next < end[t] && wait.size() < 64) wait.push_back(next++);
-            size_t best = 0;
-            int cost = 100;
-            for (size_t w = 0; w < wait.size() && cost; w++) {
-                const int i = wait[w], v[3] = {el(i, 2 * (1 - t)), el(i, 2 * (1 - t) + 1), at[t][i - i0]};
-                const int cw = 2 * (used[0] >> (v[0] & 7) & 1) + 2 * (used[1] >> (v[1] & 7) & 1) + (used[2] >> (v[2] & 7) & 1);
-                if (cw < cost) {
-                    cost = cw;
-                    best = w;
-                }
+        const int t = end[1] > end[0] || (end[1] == end[0] && list[1].size() <= list[0].size()) ? 1 : 0, o = 1 - t;
+        const int n = end[t] - i0;
+        // the other side: uses of a dipole, then the second table
+        std::unordered_map<int64_t, int> uses;
+        auto key = [&](int i) { return (int64_t)el(i, 2 * o) * (eanz + 1) + el(i, 2 * o + 1); };
+        for (int i = i0; i < end[t]; i++) uses[key(i)]++;
+        std::unordered_map<int64_t, int> second;
+        std::vector<int2> list2;
+        std::vector<int> order[2];
+        // whole groups of slots (a thread's kSensGroup at a time take the same way)
+        int often = 0, kinds = 0;
+        for (const auto &u : uses)
+            if (u.second > 1 && kinds < kSensDip2) kinds++, often += u.second;
+        for (int i = i0, left = often / (kSensThreads * kSensGroup) * (kSensThreads * kSensGroup); i < end[t]; i++) {
+            const int64_t q = key(i);
+            auto it = second.find(q);
+            if (it == second.end() && left > 0 && uses[q] > 1 && (int)list2.size() < kSensDip2) {
+                it = second.emplace(q, (int)list2.size()).first;
+                list2.push_back(make_int2(el(i, 2 * o), el(i, 2 * o + 1)));
             }
-            const int i = wait[best];
-            wait.erase(wait.begin() + best);
-            mdip[slot] = make_int4(el(i, 2 * (1 - t)), el(i, 2 * (1 - t) + 1), at[t][i - i0], i);
-            used[0] |= 1 << (mdip[slot].x & 7);
-            used[1] |= 1 << (mdip[slot].y & 7);
-            used[2] |= 1 << (mdip[slot].z & 7);
+            const bool in = it != second.end() && left > 0;
+            order[!in].push_back(i);
+            left -= in;
         }
-        pass.push_back(make_int4(i0, end[t], (int)dip.size(), (int)list[t].size()));
-        dip.insert(dip.end(), list[t].begin(), list[t].end());
+        if (order[0].size() % (kSensThreads * kSensGroup)) {  // fewer uses than counted: none
+            order[1].insert(order[1].end(), order[0].begin(), order[0].end());
+            std::sort(order[1].begin(), order[1].end());
+            order[0].clear();
+            list2.clear();
+        }
+        // Threads in an order in which eight neighbours (one shared-memory phase
+        // of 16-byte loads) differ in their places modulo 8, as far as the next 64
+        // measurements allow: fewer bank conflicts
+        int slot = i0;
+        for (int kind = 0; kind < 2; kind++) {
+            std::vector<int4> wait;
+            size_t next = 0;
+            int used[3] = {0, 0, 0}, filled = 0;
+            while (filled < (int)order[kind].size()) {
+                if (filled % 8 == 0) used[0] = used[1] = used[2] = 0;
+                while (next < order[kind].size() && wait.size() < 64) {
+                    const int i = order[kind][next++];
+                    wait.push_back(kind == 0 ? make_int4(second[key(i)], 0, at[t][i - i0], i)
+                                             : make_int4(el(i, 2 * o), el(i, 2 * o + 1), at[t][i - i0], i));
+                }
+                size_t best = 0;
+                int cost = 100;
+                for (size_t w = 0; w < wait.size() && cost; w++) {
+                    const int4 v = wait[w];
+                    const int cw = 2 * (used[0] >> (v.x & 7) & 1) + (kind ? 2 * (used[1] >> (v.y & 7) & 1) : 0) +
+                                   (used[2] >> (v.z & 7) & 1);
+                    if (cw < cost) {
+                        cost = cw;
+                        best = w;
+                    }
+                }
+                const int4 v = wait[best];
+                wait.erase(wait.begin() + best);
+                sp.slot[slot++] = v;
+                used[0] |= 1 << (v.x & 7);
+                used[1] |= 1 << (v.y & 7);
+                used[2] |= 1 << (v.z & 7);
+                filled++;
+            }
+        }
+        SensPass p;
+        p.i0 = i0;
+        p.split = i0 + (int)order[0].size();
+        p.i1 = i0 + n;
+        p.d0 = (int)sp.dip.size();
+        p.nd = (int)list[t].size();
+        p.nd2 = (int)list2.size();
+        sp.pass.push_back(p);
+        sp.dip.insert(sp.dip.end(), list[t].begin(), list[t].end());
+        sp.dip.insert(sp.dip.end(), list2.begin(), list2.end());
+        sp.most = std::max(sp.most, p.nd + p.nd2);
         i0 = end[t];
     }
 }
@@ -217,7 +271,7 @@ __device__ __forceinline__ void sens_element(const DevProblem &P, const typename
     using S = typename T::S;
     const int eanz = P.eanz, E1 = eanz + 1, tid = threadIdx.x;
     S *kp = (S *)smem;             // [2][NK][E1], the last entry of a row an absent electrode's zero
-    C *tab = (C *)(kp + 2 * NK * E1);  // [NK][dipoles of the pass]
+    C *tab = (C *)(kp + 2 * NK * E1);  // [NK][dipoles of the pass], then [NK][those of its second table]
     const size_t plane = (size_t)P.K * eanz * P.n;
     int nodes[NK];
 #pragma unroll
@@ -239,9 +293,10 @@ __device__ __forceinline__ void sens_element(const DevProblem &P, const typename
     };
     const double2 sg = sigma[e];
     for (int ps = 0; ps < P.nspass; ps++) {
-        const int4 pass = P.spass[ps];
-        const int i0 = pass.x, i1 = pass.y, nd = pass.w;
-        const int2 *dip = P.dip + pass.z;
+        const SensPass pass = P.spass[ps];
+        const int i0 = pass.i0, i1 = pass.i1, split = pass.split, nd = pass.nd, nd2 = pass.nd2;
+        const int2 *dip = P.dip + pass.d0;
+        C *tab2 = tab + NK * nd;
         C acc[kSensMPT];
 #pragma unroll
         for (int m = 0; m < kSensMPT; m++) acc[m] = T::mk(0, 0);
@@ -257,11 +312,16 @@ __device__ __forceinline__ void sens_element(const DevProblem &P, const typename
             cp_wait<0>();
             __syncthreads();
             if (k + 1 < P.K) fetch(k + 1, (k + 1) & 1);
-            for (int d = tid; d < nd; d += kSensThreads) {
+            for (int d = tid; d < nd + nd2; d += kSensThreads) {
                 const int2 p = dip[d];
                 C v[NK];
 #pragma unroll
                 for (int q = 0; q < NK; q++) v[q] = T::diff(u[q * E1 + p.x], u[q * E1 + p.y]);
+                if (d >= nd) {
+#pragma unroll
+                    for (int q = 0; q < NK; q++) tab2[q * nd2 + d - nd] = v[q];
+                    continue;
+                }
 #pragma unroll
                 for (int mi = 0; mi < NK; mi++) {
                     C s = T::mk(0, 0);
@@ -277,17 +337,39 @@ __device__ __forceinline__ void sens_element(const DevProblem &P, const typename
             }
             __syncthreads();
 #pragma unroll
-            for (int m = 0; m < kSensMPT; m++) {
-                const int i = i0 + m * kSensThreads + tid;
-                if (i >= i1) continue;
-                const int4 md = P.mdip[i];  // L1-resident
+            for (int m0 = 0; m0 < kSensMPT; m0 += kSensGroup) {
+                const int f = i0 + m0 * kSensThreads;  // the group's first slot
+                if (f >= i1) break;
+                int4 md[kSensGroup];
 #pragma unroll
-                for (int q = 0; q < NK; q++) {
-                    const C a = T::diff(u[q * E1 + md.x], u[q * E1 + md.y]), b = tab[q * nd + md.z];
-                    acc[m].x = fma(a.x, b.x, acc[m].x);
-                    acc[m].x = fma(-a.y, b.y, acc[m].x);
-                    acc[m].y = fma(a.x, b.y, acc[m].y);
-                    acc[m].y = fma(a.y, b.x, acc[m].y);
+                for (int h = 0; h < kSensGroup; h++) {
+                    const int i = f + h * kSensThreads + tid;
+                    md[h] = P.mdip[i < i1 ? i : i1 - 1];  // L1-resident
+                }
+                C a[kSensGroup][NK];
+                if (f < split) {
+#pragma unroll
+                    for (int h = 0; h < kSensGroup; h++)
+#pragma unroll
+                        for (int q = 0; q < NK; q++) a[h][q] = tab2[q * nd2 + md[h].x];
+                } else {
+#pragma unroll
+                    for (int h = 0; h < kSensGroup; h++)
+#pragma unroll
+                        for (int q = 0; q < NK; q++)
+                            a[h][q] = T::diff(u[q * E1 + md[h].x], u[q * E1 + md[h].y]);
+                }
+#pragma unroll
+                for (int h = 0; h < kSensGroup; h++) {
+                    C &s = acc[m0 + h];
+#pragma unroll
+                    for (int q = 0; q < NK; q++) {
+                        const C b = tab[q * nd + md[h].z];
+                        s.x = fma(a[h][q].x, b.x, s.x);
+                        s.x = fma(-a[h][q].y, b.y, s.x);
+                        s.y = fma(a[h][q].x, b.y, s.y);
+                        s.y = fma(a[h][q].y, b.x, s.y);
+                    }
                 }
             }
         }
@@ -302,7 +384,7 @@ __device__ __forceinline__ void sens_element(const DevProblem &P, const typename
 }
 
 template <int MODE, typename R>
-__global__ __launch_bounds__(kSensThreads) void k_bsens(DevProblem P,
+__global__ __launch_bounds__(kSensThreads, sizeof(R) == 4 ? 4 : 2) void k_bsens(DevProblem P,
                                                         const typename SensT<R>::C *__restrict__ kpot,
                                                         const double2 *__restrict__ sigma,
                                                         double2 *__restrict__ sens, int e_first) {
