@@ -86,3 +86,36 @@ def test_fictitious_sink_is_a_source(gpu_lib, where):
     for prec, tol in ((PLAIN, 1e-10), (MIXED, 1e-6)):
         with CRMod(g, s.survey, kwn, kwnwi, lsink=True, nsink=nsink, precision=prec) as m:
             assert relerr(m.forward(s.sigma, kpot=True)["kpot"], kp) < tol
+
+
+@pytest.mark.parametrize("maxit,tol", [(0, 1e-10), (1, 1e-10), (2, 0.0), (8, 1e-2), (8, 1e-10), (64, 1e-10)])
+def test_refinement_stops_alike_on_every_route(gpu_lib, maxit, tol):
+    """Steps launched as the host learns of the systems left (forward, and
+    several contexts in turn) and steps that a graph's loop repeats: the same
+    bits and the same count of steps, from no step at all to the most."""
+    import torch
+
+    from titatest_gb300 import MIXED, CRMod, crmod
+    cases = [_case(30, 30, 16), _case(36, 33, 9, True)]
+    mods = [CRMod(s.grid, s.survey, precision=MIXED) for s in cases]
+    try:
+        for m in mods:
+            m.set_refinement(maxit, tol)
+        one = [(m.forward(s.sigma)["volt"], m.stats()["refine_iterations"]) for m, s in zip(mods, cases)]
+        both = crmod.forward_sens_batch(mods, [s.sigma for s in cases])
+        for m, (v, n), w in zip(mods, one, both):
+            assert np.array_equal(v, w) and m.stats()["refine_iterations"] == n <= maxit
+        s, m = cases[0], mods[0]
+        sig = torch.from_numpy(s.sigma.view(np.float64).copy()).cuda()
+        volt = torch.zeros(2 * s.survey.nanz, dtype=torch.float64, device="cuda")
+        sens = torch.zeros(2 * s.survey.nanz * s.grid.elanz, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        for _ in range(3):  # record, then replay twice
+            volt.zero_()
+            torch.cuda.synchronize()
+            m.forward_sens_graph(sig.data_ptr(), volt.data_ptr(), 0, sens.data_ptr())
+            assert np.array_equal(volt.cpu().numpy().view(np.complex128), one[0][0])
+            assert m.stats()["refine_iterations"] == one[0][1]
+    finally:
+        for m in mods:
+            m.close()

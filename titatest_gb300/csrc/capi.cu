@@ -19,14 +19,8 @@ using namespace crgpu;
 
 namespace {
 
-// counters of one refinement step (written by k_accumulate)
-struct RefineCount {
-    int n;     // items still refining after the step
-    int pad;
-    double z;  // largest relative correction of the step
-};
-constexpr int kRefineCap = 64;  // refinement steps at most (crgpu_set_refinement)
 constexpr int kRefineSlots = 4;  // counter arrays: one per solve that runs beside others
+constexpr int kRefineRow = kRefineCap + 1;  // of one: the steps, and a loop's step number
 
 int fail(crgpu_ctx *c, int code, const std::string &msg) {
     if (c) c->last_error = msg;
@@ -133,10 +127,13 @@ size_t bytes_per_system(const crgpu_ctx *c) {
 
 int ensure_refine(crgpu_ctx *c) {
     if (c->d_refine) return 0;
-    char *cnt = nullptr;  // [kRefineSlots][kRefineCap] steps of {int count, pad, double zmax}
-    int e = dalloc(c, &cnt, kRefineSlots * kRefineCap * sizeof(RefineCount));
+    char *cnt = nullptr;  // [kRefineSlots][kRefineRow]
+    int e = dalloc(c, &cnt, kRefineSlots * kRefineRow * sizeof(RefineCount));
     c->d_refine = cnt;
-    return e;
+    if (e) return e;
+    CUCHECK(c, cudaHostAlloc((void **)&c->refine_left, kRefineSlots * kRefineCap * sizeof(int),
+                             cudaHostAllocPortable | cudaHostAllocMapped));
+    return 0;
 }
 
 int ensure_batch(crgpu_ctx *c, int want) {
@@ -266,7 +263,7 @@ int solve_view(crgpu_ctx *c, const DevBatch &B, bool fused, cudaStream_t st, int
         c->stats.kernel_launches += 1;
         return 0;
     }
-    RefineCount *cnt = (RefineCount *)c->d_refine + (size_t)slot * kRefineCap;
+    RefineCount *cnt = (RefineCount *)c->d_refine + (size_t)slot * kRefineRow;
     const int steps = std::min(c->refine_maxit, kRefineCap);
     CUCHECK(c, cudaMemsetAsync(cnt, 0, sizeof(RefineCount) * kRefineCap, st));
     launch_fill_active(B, nr, st);
@@ -301,7 +298,7 @@ int collect_refine_stats(crgpu_ctx *c) {
         const int used = c->refine_used[slot];
         if (!used) continue;
         std::vector<RefineCount> h(used);
-        CUCHECK(c, cudaMemcpy(h.data(), (RefineCount *)c->d_refine + (size_t)slot * kRefineCap,
+        CUCHECK(c, cudaMemcpy(h.data(), (RefineCount *)c->d_refine + (size_t)slot * kRefineRow,
                               sizeof(RefineCount) * used, cudaMemcpyDeviceToHost));
         int ran = 0;  // step it ran if it was the first or its predecessor left items active
         for (int it = 0; it < used; it++)
@@ -492,29 +489,124 @@ int ensure_sub_rhs(crgpu_ctx *c) {
     return dalloc(c, &c->SB.Bt, (size_t)c->sub_cap * c->hg.n);
 }
 
-// Solves the rectangle for the right-hand sides of kompab (src null) or for
-// the rows of src; the solution ends in B.X.  Mixed precision refines as
-// solve_view does: every step is launched without waiting for the host, with
-// its counters in refinement array `slot`.
-int sub_solve_rect(crgpu_ctx *c, const SubBatch &B, const double2 *src, cudaStream_t st, int slot) {
+// One rectangle's solve for the right-hand sides of kompab (src null) or for the
+// rows of src, queued on st with its counters in refinement array `slot`.
+struct SubJob {
+    crgpu_ctx *c;
+    SubBatch B;
+    const double2 *src;
+    cudaStream_t st;
+    int slot;
+    bool done;
+};
+
+// The first solution, in B.X; mixed precision goes on with sub_refine.
+int sub_solve_rect(SubJob &j) {
+    crgpu_ctx *c = j.c;
     const bool mixed = c->precision == CRGPU_MIXED;
-    SubBatch B0 = B;
+    SubBatch B0 = j.B;
     B0.kact = nullptr;
-    sub_launch_rhs(c->P, c->D, B, mixed, c->lsink, c->nsink, src, st);
-    c->stats.kernel_launches += 1 + sub_launch_apply(c->D, c->sp, B0, mixed, src == nullptr, nullptr, st);
+    sub_launch_rhs(c->P, c->D, j.B, mixed, c->lsink, c->nsink, j.src, j.st);
+    c->stats.kernel_launches += 1 + sub_launch_apply(c->D, c->sp, B0, mixed, j.src == nullptr, nullptr, j.st);
+    j.done = !mixed;
     if (!mixed) return 0;
-    RefineCount *cnt = (RefineCount *)c->d_refine + (size_t)slot * kRefineCap;
-    const int steps = std::min(c->refine_maxit, kRefineCap);
-    CUCHECK(c, cudaMemsetAsync(cnt, 0, sizeof(RefineCount) * kRefineCap, st));
-    sub_launch_accumulate(c->D, B, true, c->refine_tol, nullptr, nullptr, nullptr, st);
+    RefineCount *cnt = (RefineCount *)c->d_refine + (size_t)j.slot * kRefineRow;
+    CUCHECK(c, cudaMemsetAsync(cnt, 0, sizeof(RefineCount) * kRefineRow, j.st));
+    sub_launch_accumulate(c->D, j.B, true, c->refine_tol, nullptr, SubStop{}, j.st);
     c->stats.kernel_launches += 2;
-    for (int it = 0; it < steps; it++) {
-        const int *nprev = it > 0 ? &cnt[it - 1].n : nullptr;
-        sub_launch_residual(c->P, c->D, B, src == nullptr, c->lsink, c->nsink, nprev, st);
-        c->stats.kernel_launches += 3 + sub_launch_apply(c->D, c->sp, B, true, false, nprev, st);
-        sub_launch_accumulate(c->D, B, false, c->refine_tol, nprev, &cnt[it].n, &cnt[it].z, st);
+    return 0;
+}
+
+void sub_refine_step(const SubJob &j, const int *nprev, const SubStop &stop, cudaStream_t st) {
+    crgpu_ctx *c = j.c;
+    sub_launch_residual(c->P, c->D, j.B, j.src == nullptr, c->lsink, c->nsink, nprev, st);
+    c->stats.kernel_launches += 3 + sub_launch_apply(c->D, c->sp, j.B, true, false, nprev, st);
+    sub_launch_accumulate(c->D, j.B, false, c->refine_tol, nprev, stop, st);
+}
+
+// The refinement of a recorded job as a loop node whose body is one step.
+int sub_record_loop(const SubJob &j, RefineCount *cnt, int steps) {
+    crgpu_ctx *c = j.c;
+    cudaStreamCaptureStatus status;
+    cudaGraph_t graph = nullptr;
+    const cudaGraphNode_t *deps = nullptr;
+    const cudaGraphEdgeData *edges = nullptr;
+    size_t nd = 0;
+    CUCHECK(c, cudaStreamGetCaptureInfo(j.st, &status, nullptr, &graph, &deps, &edges, &nd));
+    SubStop stop;
+    stop.cnt = cnt;
+    stop.steps = steps;
+    CUCHECK(c, cudaGraphConditionalHandleCreate(&stop.loop, graph, 1, cudaGraphCondAssignDefault));
+    cudaGraphNodeParams np = {};
+    np.type = cudaGraphNodeTypeConditional;
+    np.conditional.handle = stop.loop;
+    np.conditional.type = cudaGraphCondTypeWhile;
+    np.conditional.size = 1;
+    cudaGraphNode_t node = nullptr;
+    CUCHECK(c, cudaGraphAddNode(&node, graph, deps, edges, nd, &np));
+    cudaGraph_t body = np.conditional.phGraph_out[0];
+    CUCHECK(c, cudaStreamBeginCaptureToGraph(c->st_body, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+    sub_refine_step(j, nullptr, stop, c->st_body);
+    CUCHECK(c, cudaStreamEndCapture(c->st_body, &body));
+    CUCHECK(c, cudaStreamUpdateCaptureDependencies(j.st, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
+    return 0;
+}
+
+// The systems that step `it` of a job has left, as soon as it has counted them.
+int sub_left(const SubJob &j, int it) {
+    const int *f = j.c->refine_left + j.slot * kRefineCap + it;
+    for (;;) {
+        for (int q = 0; q < 256; q++) {
+            const int v = __atomic_load_n(f, __ATOMIC_ACQUIRE);
+            if (v >= 0) return v;
+        }
+        if (cudaStreamQuery(j.st) != cudaErrorNotReady)  // over (or failed, which the caller's check reports)
+            return std::max(__atomic_load_n(f, __ATOMIC_ACQUIRE), 0);
     }
-    c->refine_used[slot] = std::max(c->refine_used[slot], steps);
+}
+
+// Refinement of the jobs, step by step in turn, until none has systems left.
+// Every step used to be queued at once, the later ones to find nothing to do:
+// for config 2, 4 of its 8 with 23 launches each.  Now the host launches a job's
+// step when the one before has left systems over (it learns so from mapped
+// memory, in a few microseconds; other jobs keep the GPU busy meanwhile), and a
+// recorded job is a loop on the device.  A step in hand is worse by
+// 0 to 2 %.  Config 2 forward 10.05 -> 9.48 ms, its replayed graph with Jacobian
+// 8.92 -> 7.90, 300x80 cells with 128 electrodes 26.8 -> 25.5, a 60x20 line with
+// its Jacobian 1.37 -> 1.31, eight 160x50 contexts in turn 24.4 -> 22.8.
+int sub_refine(std::vector<SubJob> &jobs) {
+    size_t open = 0;
+    for (SubJob &j : jobs) {
+        if (j.done) continue;
+        crgpu_ctx *c = j.c;
+        const int steps = std::min(c->refine_maxit, kRefineCap);
+        c->refine_used[j.slot] = std::max(c->refine_used[j.slot], steps);
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        CUCHECK(c, cudaStreamIsCapturing(j.st, &cap));
+        if (cap != cudaStreamCaptureStatusNone) {
+            const int e = steps ? sub_record_loop(j, (RefineCount *)c->d_refine + (size_t)j.slot * kRefineRow, steps) : 0;
+            if (e) return e;
+            j.done = true;
+            continue;
+        }
+        std::fill_n(c->refine_left + j.slot * kRefineCap, kRefineCap, -1);
+        open++;
+    }
+    for (int it = 0; open; it++)
+        for (SubJob &j : jobs) {
+            if (j.done) continue;
+            crgpu_ctx *c = j.c;
+            if (it >= std::min(c->refine_maxit, kRefineCap) || (it > 0 && sub_left(j, it - 1) == 0)) {
+                j.done = true;
+                open--;
+                continue;
+            }
+            RefineCount *cnt = (RefineCount *)c->d_refine + (size_t)j.slot * kRefineRow;
+            SubStop stop;
+            stop.cnt = cnt + it;
+            stop.left = c->refine_left + j.slot * kRefineCap + it;
+            sub_refine_step(j, it > 0 ? &cnt[it - 1].n : nullptr, stop, j.st);
+        }
     return 0;
 }
 
@@ -577,10 +669,17 @@ int sub_join(crgpu_ctx *c, int groups) {
     return 0;
 }
 
+// the potentials of a refined job of the forward
+void sub_finish(const SubJob &j) {
+    sub_launch_unpack(j.c->P, j.c->D, j.B, -1.0, j.c->d_kpot, j.c->d_kpot32, j.st);
+    j.c->stats.kernel_launches += 1;
+}
+
 // every system of the forward: shared elimination, then root factors and
-// solves by rectangles, potentials into d_kpot
-int forward_sub(crgpu_ctx *c, float *t_factor, float *t_solve) {
-    const bool cap = c->capturing;  // recorded, or queued beside other problems: one rectangle, no waiting
+// solves by rectangles, potentials into d_kpot.  later: one rectangle, whose
+// refinement and sub_finish the caller queues (beside other problems').
+int forward_sub(crgpu_ctx *c, float *t_factor, float *t_solve, std::vector<SubJob> *later) {
+    const bool cap = c->capturing || later;  // recorded or queued: one rectangle, no waiting
     int kb = c->K, lb = c->eanz;
     if (!cap) sub_rect(c, &kb, &lb);
     int e = ensure_sub_batch(c, kb * lb);
@@ -599,6 +698,7 @@ int forward_sub(crgpu_ctx *c, float *t_factor, float *t_solve) {
     for (int k0 = 0; k0 < c->K && !e; k0 += kb)
         for (int l0 = 0; l0 < c->eanz && !e; l0 += lb) {
             if (!cap) cudaEventRecord(ev[1], c->st);
+            std::vector<SubJob> jobs;
             e = sub_fork(c, groups);
             for (int g = 0; g < groups && !e; g++) {  // one rectangle: groups of its wavenumbers
                 const int ka = one ? c->K * g / groups : k0, kn = one ? c->K * (g + 1) / groups - ka : kb;
@@ -607,11 +707,17 @@ int forward_sub(crgpu_ctx *c, float *t_factor, float *t_solve) {
                 if (one) sub_factor_shared(c, ka, kn, st);
                 e = sub_factor_rect(c, B, st);
                 if (!cap && g == 0) cudaEventRecord(ev[2], c->st);
-                if (!e) e = sub_solve_rect(c, B, nullptr, st, g);
-                if (e) break;
-                sub_launch_unpack(c->P, c->D, B, -1.0, c->d_kpot, c->d_kpot32, st);
-                c->stats.kernel_launches += 1;
+                jobs.push_back({c, B, nullptr, st, g, false});
+                if (!e) e = sub_solve_rect(jobs.back());
             }
+            if (e) break;
+            if (later) {
+                later->insert(later->end(), jobs.begin(), jobs.end());
+                break;
+            }
+            e = sub_refine(jobs);
+            for (const SubJob &j : jobs)
+                if (!e) sub_finish(j);
             if (!e) e = sub_join(c, groups);
             if (e) break;
             c->stats.nbatches++;
@@ -650,15 +756,20 @@ int adjoint_sub(crgpu_ctx *c) {
     const int groups = one ? sub_groups(c) : 1;
     for (int k0 = 0; k0 < c->K; k0 += kb)
         for (int l0 = 0; l0 < c->eanz; l0 += lb) {
+            std::vector<SubJob> jobs;
             e = sub_fork(c, groups);
             for (int g = 0; g < groups && !e; g++) {
                 const int ka = one ? c->K * g / groups : k0, kn = one ? c->K * (g + 1) / groups - ka : kb;
                 const cudaStream_t st = g ? c->st_sub[g - 1] : c->st;
                 const SubBatch B = sub_view(c, ka, kn, l0, lb, one ? (size_t)ka * c->eanz : 0);
                 if (!have) e = sub_factor_rect(c, B, st);
-                if (!e) e = sub_solve_rect(c, B, c->d_adjsrc, st, g);
+                jobs.push_back({c, B, c->d_adjsrc, st, g, false});
+                if (!e) e = sub_solve_rect(jobs.back());
+            }
+            if (!e) e = sub_refine(jobs);
+            for (const SubJob &j : jobs) {
                 if (e) break;
-                sub_launch_unpack(c->P, c->D, B, 1.0, c->d_lambda, nullptr, st);
+                sub_launch_unpack(c->P, c->D, j.B, 1.0, c->d_lambda, nullptr, j.st);
                 c->stats.kernel_launches += 2;
             }
             if (!e) e = sub_join(c, groups);
@@ -785,7 +896,7 @@ int run_forward(crgpu_ctx *c, const double2 *d_sigma, int volt_mode, const doubl
     }
     c->stats.nsystems = (int)c->sys_k.size();
     float t_factor = 0.f, t_solve = 0.f;
-    int worst = sub_on(c) ? forward_sub(c, &t_factor, &t_solve) : forward_band(c, d_sigma, &t_factor, &t_solve);
+    int worst = sub_on(c) ? forward_sub(c, &t_factor, &t_solve, nullptr) : forward_band(c, d_sigma, &t_factor, &t_solve);
     if (worst) {
         for (auto &ev_ : ev) cudaEventDestroy(ev_);
         return worst;
@@ -1211,6 +1322,8 @@ int crgpu_destroy(crgpu_ctx *c) {
     if (c->st_hi) cudaStreamDestroy(c->st_hi);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
+    if (c->st_body) cudaStreamDestroy(c->st_body);
+    if (c->refine_left) cudaFreeHost(c->refine_left);
     for (auto s : c->st_sub)
         if (s) cudaStreamDestroy(s);
     for (auto v : c->ev_sub)
@@ -1378,6 +1491,7 @@ int crgpu_forward_sens_graph(crgpu_ctx *c, const void *sigma_device, void *volt_
     if (e) return e;
     if (c->stats.nbatches != 1) return 0;
     const crgpu_stats keep = c->stats;  // this call's figures: the recording measures nothing
+    if (!c->st_body) CUCHECK(c, cudaStreamCreateWithFlags(&c->st_body, cudaStreamNonBlocking));
     c->capturing = true;
     cudaGraph_t graph = nullptr;
     cudaError_t ce = cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal);
@@ -1464,6 +1578,7 @@ int crgpu_forward_sens_batch(crgpu_ctx *const *ctxs, int32_t nprob, const double
     std::vector<DevProblem> hp(nprob);
     std::vector<DevBatch> hb(nprob);
     std::vector<int> order(nprob);
+    std::vector<SubJob> jobs;
     for (int p = 0; p < nprob; p++) {  // assembly and right-hand sides, each on its stream
         crgpu_ctx *c = ctxs[p];
         const int ns = (int)c->sys_k.size();
@@ -1476,9 +1591,7 @@ int crgpu_forward_sens_batch(crgpu_ctx *const *ctxs, int32_t nprob, const double
         order[p] = p;
         if (sub_on(c)) {  // potentials queued on its own stream; no part in the band launch
             float t = 0.f;
-            c->capturing = true;
-            const int e = forward_sub(c, &t, &t);
-            c->capturing = false;
+            const int e = forward_sub(c, &t, &t, &jobs);
             if (e) return e;
             c->stats.kernel_launches += 1;
             c->stats.nsystems = ns;
@@ -1498,6 +1611,13 @@ int crgpu_forward_sens_batch(crgpu_ctx *const *ctxs, int32_t nprob, const double
         CUCHECK(c, cudaStreamWaitEvent(st0, c->ev_join, 0));
         hp[p] = c->P;
         hb[p] = B;
+    }
+    if (!jobs.empty()) {
+        int e = sub_refine(jobs);
+        if (e) return e;
+        for (const SubJob &j : jobs) sub_finish(j);
+        for (int p = 0; p < nprob; p++)
+            if (sub_on(ctxs[p]) && (e = sub_join(ctxs[p], sub_groups(ctxs[p])))) return e;
     }
     // the item table, longest systems first
     std::sort(order.begin(), order.end(), [&](int a, int b) { return ctxs[a]->hg.n > ctxs[b]->hg.n; });

@@ -43,8 +43,9 @@ struct crgpu_ctx {
     int refine_maxit = 8;
     double refine_tol = 1e-10;
     // refinement step counters on the device, one array per sub-batch of the
-    // current batch: {active count, pad, largest relative correction} per step
+    // current batch (RefineCount)
     void *d_refine = nullptr;
+    int *refine_left = nullptr;  // mapped host memory: systems each step has left (sub_refine)
     int refine_used[4] = {};  // steps launched on each array since the last collection
     // forward + Jacobian as one CUDA graph (crgpu_forward_sens_graph)
     bool capturing = false;       // recording: no host copies, synchronisation or timing
@@ -64,6 +65,7 @@ struct crgpu_ctx {
     crgpu::SubBatch SB{};
     bool sub_shared = false;   // D's numeric arrays are allocated
     int sub_cap = 0;           // systems SB's buffers hold
+    cudaStream_t st_body = nullptr;  // records a loop's body
     cudaStream_t st_sub[3] = {};  // further groups of wavenumbers beside st
     cudaEvent_t ev_fork = nullptr, ev_sub[3] = {};
     // adjoint

@@ -1250,12 +1250,14 @@ __global__ __launch_bounds__(256) void k_sub_accumulate(DevSub D, SubBatch B, in
 }
 
 // A system stops once its correction is at most tol times its solution; one
-// block per wavenumber counts those that go on.
-__global__ __launch_bounds__(256) void k_sub_stop(SubBatch B, int first, double tol, const int *nprev, int *nactive,
-                                                  double *zmax) {
+// block per wavenumber counts those that go on, the last block passes the sum on
+// (SubStop).
+__global__ __launch_bounds__(256) void k_sub_stop(SubBatch B, int first, double tol, const int *nprev, SubStop stop) {
     chain_wait();
     if (nprev && *nprev == 0) return;
     const int kk = blockIdx.x, L = B.Lb;
+    const int it = stop.steps ? stop.cnt[kRefineCap].n : 0;
+    RefineCount *cnt = stop.cnt ? stop.cnt + it : nullptr;
     int count = 0;
     if (first || B.kact[kk]) {
         for (int l = threadIdx.x; l < L; l += blockDim.x) {
@@ -1266,8 +1268,8 @@ __global__ __launch_bounds__(256) void k_sub_stop(SubBatch B, int first, double 
             int act = first ? 1 : B.active[s];
             if (!act) continue;
             if (!first && !(mz > tol * mx)) act = 0;
-            if (!first && zmax && mx > 0.0)
-                atomicMax((unsigned long long *)zmax, (unsigned long long)__double_as_longlong(mz / mx));
+            if (cnt && mx > 0.0)
+                atomicMax((unsigned long long *)&cnt->z, (unsigned long long)__double_as_longlong(mz / mx));
             if (!isfinite(mz) || !isfinite(mx)) {
                 atomicCAS(&B.status[s], 0, 28);
                 act = 0;
@@ -1281,9 +1283,20 @@ __global__ __launch_bounds__(256) void k_sub_stop(SubBatch B, int first, double 
     __syncthreads();
     if (count) atomicAdd(&tot, count);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        B.kact[kk] = tot;
-        if (nactive && tot) atomicAdd(nactive, tot);
+    if (threadIdx.x != 0) return;
+    B.kact[kk] = tot;
+    if (!cnt) return;
+    if (tot) atomicAdd(&cnt->n, tot);
+    __threadfence();
+    if (atomicAdd(&cnt->ticket, 1) != (int)gridDim.x - 1) return;
+    const int n = atomicAdd(&cnt->n, 0);
+    if (stop.left) {
+        *(volatile int *)stop.left = n;
+        __threadfence_system();
+    }
+    if (stop.steps) {
+        stop.cnt[kRefineCap].n = it + 1;
+        cudaGraphSetConditional(stop.loop, n > 0 && it + 1 < stop.steps ? 1 : 0);
     }
 }
 
@@ -1429,10 +1442,10 @@ void sub_launch_residual(const DevProblem &P, const DevSub &D, const SubBatch &B
                  nprev);
 }
 
-void sub_launch_accumulate(const DevSub &D, const SubBatch &B, bool first, double tol, const int *nprev, int *nactive,
-                           double *zmax, cudaStream_t st) {
+void sub_launch_accumulate(const DevSub &D, const SubBatch &B, bool first, double tol, const int *nprev,
+                           const SubStop &stop, cudaStream_t st) {
     chain_launch(k_sub_accumulate, dim3(nb(D.n, kAccRows), nb(B.Lb, 32), B.Kb), 256, 0, st, D, B, first ? 1 : 0, nprev);
-    chain_launch(k_sub_stop, dim3(B.Kb), 256, 0, st, B, first ? 1 : 0, tol, nprev, nactive, zmax);
+    chain_launch(k_sub_stop, dim3(B.Kb), 256, 0, st, B, first ? 1 : 0, tol, nprev, stop);
 }
 
 void sub_launch_unpack(const DevProblem &P, const DevSub &D, const SubBatch &B, double sign, double2 *out,

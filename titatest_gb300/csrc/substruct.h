@@ -39,6 +39,24 @@ struct SubBatch {
     unsigned long long *mz, *mx;    // per system: bit patterns of the largest correction and solution
 };
 
+// counters of one refinement step
+struct RefineCount {
+    int n;       // systems (band: items) still refining after the step
+    int ticket;  // blocks of k_sub_stop that have counted
+    double z;    // largest relative correction of the step
+};
+constexpr int kRefineCap = 64;  // refinement steps at most (crgpu_set_refinement)
+
+// Where a step counts, and who learns whether systems are left: the host (a word
+// of mapped memory), or the loop node of a graph, whose one recorded step numbers
+// itself (cnt[kRefineCap].n).
+struct SubStop {
+    RefineCount *cnt = nullptr;  // of this step; of step 0 in a loop; null: the first solve
+    int *left = nullptr;
+    cudaGraphConditionalHandle loop = 0;
+    int steps = 0;  // of a loop at most; 0: no loop
+};
+
 SubShape sub_shape(bool mixed);
 int sub_root_block(bool mixed);  // columns of a block of the root factor
 int sub_root_rows(bool mixed);   // rows of one of its tiles
@@ -54,8 +72,8 @@ void sub_launch_rhs(const DevProblem &P, const DevSub &D, const SubBatch &B, boo
                     const double2 *src, cudaStream_t st);
 void sub_launch_residual(const DevProblem &P, const DevSub &D, const SubBatch &B, bool unit, int lsink, int nsink,
                          const int *nprev, cudaStream_t st);
-void sub_launch_accumulate(const DevSub &D, const SubBatch &B, bool first, double tol, const int *nprev, int *nactive,
-                           double *zmax, cudaStream_t st);
+void sub_launch_accumulate(const DevSub &D, const SubBatch &B, bool first, double tol, const int *nprev,
+                           const SubStop &stop, cudaStream_t st);
 void sub_launch_unpack(const DevProblem &P, const DevSub &D, const SubBatch &B, double sign, double2 *out,
                        float2 *out32, cudaStream_t st);
 
