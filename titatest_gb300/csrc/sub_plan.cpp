@@ -26,11 +26,33 @@ struct Build {
     };
     std::vector<F> f;
     std::vector<int32_t> owner;  // front of a node, -1: not eliminated (yet)
-    std::vector<int32_t> mark;
+    std::vector<int32_t> mark, seen;
+    std::vector<int32_t> rank[2], reach[2];  // places across x and across y, the neighbours' last place
     int stamp = 0;
 
     Build(const HostGrid &h, const Pattern &p, const SubShape &s)
-        : hg(h), pat(p), shape(s), owner(h.n, -1), mark(h.n, 0) {}
+        : hg(h), pat(p), shape(s), owner(h.n, -1), mark(h.n, 0), seen(h.n, 0) {}
+
+    // the nodes across x (dir 0) or y, ties by the other coordinate, then by number
+    std::vector<int32_t> sorted(std::vector<int32_t> nodes, int dir) {
+        const std::vector<double> &c0 = dir ? hg.y : hg.x, &c1 = dir ? hg.x : hg.y;
+        struct Key {
+            double a, b;
+            int32_t v;
+            bool operator<(const Key &o) const { return a != o.a ? a < o.a : b != o.b ? b < o.b : v < o.v; }
+        };
+        std::vector<Key> key;
+        key.reserve(nodes.size());
+        for (int v : nodes) key.push_back({c0[v], c1[v], v});
+        if (!std::is_sorted(key.begin(), key.end())) std::sort(key.begin(), key.end());
+        rank[dir].assign(hg.n, -1);
+        for (size_t q = 0; q < key.size(); q++) rank[dir][nodes[q] = key[q].v] = (int)q;
+        reach[dir].assign(hg.n, -1);
+        for (int v : nodes)
+            for (int z = pat.fptr[v]; z < pat.fptr[v + 1]; z++)
+                reach[dir][v] = std::max(reach[dir][v], rank[dir][pat.fcol[z]]);
+        return nodes;
+    }
 
     // Eliminates E after the fronts of ch; long lists as a chain.  A front that
     // has children itself is taken into its parent where the two fit one
@@ -79,48 +101,56 @@ struct Build {
         return (int)f.size() - 1;
     }
 
-    // the smaller of the two vertex separators of the halves nodes[0..h) and nodes[h..)
-    std::vector<int32_t> separator(const std::vector<int32_t> &nodes, int h) {
-        const int lo = ++stamp, hi = ++stamp;
-        for (size_t q = 0; q < nodes.size(); q++) mark[nodes[q]] = (int)q < h ? lo : hi;
+    // The smaller of the two vertex separators of the halves nodes[0..h) and
+    // nodes[h..) of nodes marked st, ordered by rank: only the nodes with a
+    // neighbour ranked beyond the cut are looked at closer.
+    std::vector<int32_t> separator(const std::vector<int32_t> &nodes, int h, int dir, int st) {
+        const std::vector<int32_t> &rk = rank[dir];
+        const int last = rk[nodes[h - 1]], met = ++stamp;
         std::vector<int32_t> a, b;
-        for (size_t q = 0; q < nodes.size(); q++) {
-            const int v = nodes[q], other = (int)q < h ? hi : lo;
-            for (int z = pat.fptr[v]; z < pat.fptr[v + 1]; z++)
-                if (mark[pat.fcol[z]] == other) {
-                    ((int)q < h ? a : b).push_back(v);
-                    break;
-                }
+        for (int q = 0; q < h; q++) {
+            const int v = nodes[q];
+            if (reach[dir][v] <= last) continue;
+            bool cut = false;
+            for (int z = pat.fptr[v]; z < pat.fptr[v + 1]; z++) {
+                const int w = pat.fcol[z];
+                if (mark[w] != st || rk[w] <= last) continue;
+                cut = true;
+                if (seen[w] == met) continue;
+                seen[w] = met;
+                b.push_back(w);
+            }
+            if (cut) a.push_back(v);
         }
-        return a.size() <= b.size() ? a : b;
+        if (a.size() <= b.size()) return a;
+        std::sort(b.begin(), b.end(), [&](int u, int v) { return rk[u] < rk[v]; });
+        return b;
     }
 
-    int cut(std::vector<int32_t> nodes) {
-        if ((int)nodes.size() <= shape.leaf) return add(std::move(nodes), {});
-        const int h = (int)nodes.size() / 2;
-        std::vector<int32_t> best, best_nodes;
-        for (int dir = 0; dir < 2; dir++) {
-            const std::vector<double> &c0 = dir ? hg.y : hg.x, &c1 = dir ? hg.x : hg.y;
-            std::nth_element(nodes.begin(), nodes.begin() + h, nodes.end(), [&](int a, int b) {
-                if (c0[a] != c0[b]) return c0[a] < c0[b];
-                if (c1[a] != c1[b]) return c1[a] < c1[b];
-                return a < b;
-            });
-            std::vector<int32_t> s = separator(nodes, h);
-            if (dir == 0 || s.size() < best.size()) {
-                best = std::move(s);
-                best_nodes = nodes;
-            }
-        }
-        if (best.size() * 2 >= nodes.size()) return add(std::move(nodes), {});
+    // by[0] and by[1]: the same nodes ordered across x and across y
+    int cut(std::vector<int32_t> (&by)[2]) {
+        const int n = (int)by[0].size();
+        if (n <= shape.leaf) return add(std::move(by[1]), {});
+        const int h = n / 2;
         const int st = ++stamp;
-        for (int v : best) mark[v] = st;
-        std::vector<int32_t> part[2];
-        for (size_t q = 0; q < best_nodes.size(); q++)
-            if (mark[best_nodes[q]] != st) part[(int)q >= h].push_back(best_nodes[q]);
+        for (int v : by[0]) mark[v] = st;
+        std::vector<int32_t> best = separator(by[0], h, 0, st), other = separator(by[1], h, 1, st);
+        const int dir = other.size() < best.size() ? 1 : 0;
+        if (dir) best = std::move(other);
+        if (best.size() * 2 >= (size_t)n) return add(std::move(by[dir]), {});
+        const int half = ++stamp, sep = ++stamp;
+        for (int q = 0; q < h; q++) mark[by[dir][q]] = half;
+        for (int v : best) mark[v] = sep;
+        std::vector<int32_t> part[2][2];
+        for (int d = 0; d < 2; d++) {
+            for (auto &p : part) p[d].reserve(n - h);
+            for (int v : by[d])
+                if (mark[v] != sep) part[mark[v] != half][d].push_back(v);
+            by[d] = std::vector<int32_t>();
+        }
         std::vector<int> ch;
-        for (int q = 0; q < 2; q++)
-            if (!part[q].empty()) ch.push_back(cut(std::move(part[q])));
+        for (auto &p : part)
+            if (!p[0].empty()) ch.push_back(cut(p));
         return add(std::move(best), std::move(ch));
     }
 };
@@ -138,7 +168,8 @@ bool build_sub_plan(const HostGrid &hg, const Pattern &pat, const SubShape &shap
     for (int i = 0; i < n; i++) (root[i] ? outer : inner).push_back(i);
     if (inner.empty() || outer.empty()) return false;
     Build b(hg, pat, shape);
-    b.cut(inner);
+    std::vector<int32_t> by[2] = {b.sorted(inner, 0), b.sorted(inner, 1)};
+    b.cut(by);
     std::vector<int32_t> order;
     for (int q = 0; q < (int)b.f.size(); q++)
         if (!b.f[q].gone) order.push_back(q);
@@ -211,24 +242,28 @@ bool build_sub_plan(const HostGrid &hg, const Pattern &pat, const SubShape &shap
         }
     }
     // matrix entries, each in the front that eliminates its earlier node
-    std::vector<std::vector<int32_t>> own(nf);
-    std::vector<int32_t> root_p;
+    std::vector<int32_t> root_p, own(pat.nnz, -1), place(nf + 1, 0);
     for (int p = 0; p < pat.nnz; p++) {
         if (pat.col[p] < 0) continue;
         const int i = pat.row[p], c = pat.col[p];
         const int first = sp.pos[i] < sp.pos[c] ? i : c;
         if (b.owner[first] < 0) root_p.push_back(p);
-        else own[at[b.owner[first]]].push_back(p);
+        else place[(own[p] = at[b.owner[first]]) + 1]++;
     }
+    for (int q = 0; q < nf; q++) place[q + 1] += place[q];
+    std::vector<int32_t> list(place[nf]), next(place.begin(), place.end() - 1);
+    for (int p = 0; p < pat.nnz; p++)
+        if (own[p] >= 0) list[next[own[p]]++] = p;
+    sp.ent.reserve(list.size() + root_p.size());
     for (int q = 0; q < nf; q++) {
         const Build::F &s = b.f[order[q]];
         for (size_t z = 0; z < s.E.size(); z++) local[s.E[z]] = (int)z;
         for (size_t z = 0; z < s.R.size(); z++) local[s.R[z]] = (int)(s.E.size() + z);
         SubFront &t = sp.fronts[q];
         t.ent0 = (int)sp.ent.size();
-        t.nent = (int)own[q].size();
-        for (int p : own[q]) {
-            const int a = local[pat.row[p]], c = local[pat.col[p]];
+        t.nent = place[q + 1] - place[q];
+        for (int z = place[q]; z < place[q + 1]; z++) {
+            const int p = list[z], a = local[pat.row[p]], c = local[pat.col[p]];
             sp.ent.push_back({p, std::min(a, c), std::max(a, c)});
         }
         for (int v : s.E) local[v] = -1;
