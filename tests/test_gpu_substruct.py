@@ -71,6 +71,20 @@ def test_rectangles_of_a_small_memory_budget(gpu_lib, prec, systems):
     assert relerr(v2, v1) < 1e-12 and relerr(a2, a1) < 1e-12
 
 
+@pytest.mark.parametrize("prec", [0, 1])
+def test_memory_need_covers_the_root_factors(gpu_lib, prec):
+    """The bytes a batch would still allocate: the root factors of every
+    system before a forward, the Jacobian alone after it."""
+    from titatest_gb300 import CRMod
+    s = _case(60, 20, 20)
+    with CRMod(s.grid, s.survey, precision=prec) as m:
+        roots = m.kwnanz * 20 * (60 + 2 * 20 + 1) ** 2 * (16 if prec == 0 else 8)
+        sens = s.survey.nanz * s.grid.elanz * 16
+        assert m.memory_need() > roots + sens
+        m.forward(s.sigma)
+        assert m.memory_need() == sens
+
+
 @pytest.mark.parametrize("where", ["interior", "corner"])
 def test_fictitious_sink_is_a_source(gpu_lib, where):
     """The right-hand sides with a fictitious sink, inside the mesh and on the

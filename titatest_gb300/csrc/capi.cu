@@ -438,6 +438,13 @@ size_t sub_bytes_per_system(const crgpu_ctx *c) {
            (size_t)c->D.szU * esz + (size_t)c->D.n_be * sizeof(double2) + 64;
 }
 
+size_t sub_bytes_shared(const crgpu_ctx *c) {
+    const DevSub &D = c->D;
+    const size_t esz = c->precision == CRGPU_MIXED ? sizeof(float2) : sizeof(double2);
+    return c->K * (c->pat.nnz * sizeof(double2) + c->hg.n * sizeof(double) + sizeof(int) +
+                   (D.szF + 2 * D.szG + D.szS + (size_t)D.mp * D.ldc) * esz);
+}
+
 // the shared factor's arrays
 int ensure_sub_shared(crgpu_ctx *c) {
     if (c->sub_shared) return 0;
@@ -1625,7 +1632,13 @@ int crgpu_sens_device(crgpu_ctx *c, int32_t mode, void *sens_device) {
 int crgpu_memory_need(const crgpu_ctx *c, int64_t *bytes) {
     if (!c || !bytes) return ERR_ARG;
     const int nsys = (int)c->sys_k.size();
-    int64_t need = c->batch_cap >= nsys ? 0 : (int64_t)bytes_per_system(c) * nsys;
+    int64_t need = 0;
+    if (sub_on(c)) {
+        if (c->sub_cap < nsys) need += (int64_t)sub_bytes_per_system(c) * nsys;
+        if (!c->sub_shared) need += (int64_t)sub_bytes_shared(c);
+    } else if (c->batch_cap < nsys) {
+        need += (int64_t)bytes_per_system(c) * nsys;
+    }
     if (!c->d_sens) need += (int64_t)c->nanz * c->hg.elanz * (int64_t)sizeof(double2);
     *bytes = need;
     return 0;
