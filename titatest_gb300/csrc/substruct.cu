@@ -1122,6 +1122,168 @@ __global__ __launch_bounds__(256) void k_sub_down(DevSub D, SubBatch B, int t0, 
                 Z[(size_t)(i0 + tr + i) * L + tc + j] = nc > nr ? acc.v[i][j] : neg_(acc.v[i][j]);
 }
 
+// The same two sweeps for the upper levels, whose fronts are too few to fill the
+// chip with tiles: a block has kFewR rows x 32 electrodes, its eight warps take
+// every eighth step of the depth and add up at the end.  No staging of the
+// vectors (a warp reads a row of 32 electrodes once), one barrier before and one
+// after the products, and the factor's rows are read before the chain's wait (they
+// are older than its predecessor).  A tile of 32 x 32 takes ten chunks of the
+// depth one after the other, 2 us each, at the top of config 2's tree (36 tiles).
+constexpr int kFewR = 8, kFewSplit = Tile<float2>::E / kFewR;  // rows, blocks of a tile
+struct Few {
+    static constexpr int D = 128;                    // depth of a piece of the factor's rows in shared memory
+    static constexpr int P = kFewR + 2;              // its pitch
+    float2 a[D * P], red[8][kFewR][32];
+    __device__ __forceinline__ void put(int q, int ri, float2 v) { a[q * P + ri] = v; }
+    // s += (row q of the piece)^T b
+    __device__ __forceinline__ void add(float2 (&s)[kFewR], int q, float2 b) const {
+#pragma unroll
+        for (int ri = 0; ri < kFewR; ri += 2) {
+            float2 v[2];
+            load2(a + q * P + ri, v);
+            fma_(s[ri], v[0], b);
+            fma_(s[ri + 1], v[1], b);
+        }
+    }
+    // the block's sum in row threadIdx / 32
+    __device__ __forceinline__ float2 sum(const float2 (&s)[kFewR]) {
+        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+        for (int ri = 0; ri < kFewR; ri++) red[w][ri][lane] = s[ri];
+        __syncthreads();
+        float2 v = red[0][w][lane];
+#pragma unroll
+        for (int z = 1; z < 8; z++) {
+            v.x += red[z][w][lane].x;
+            v.y += red[z][w][lane].y;
+        }
+        return v;
+    }
+};
+
+__global__ __launch_bounds__(256) void k_sub_up_few(DevSub D, SubBatch B, int t0, int unit, const int *nprev) {
+    constexpr int E = Tile<float2>::E;
+    __shared__ __align__(16) Few sh;
+    __shared__ int se[kSubCh][kSubEMax];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int kk = blockIdx.z, k = B.k0 + kk, L = B.Lb, col = blockIdx.y * 32 + lane;
+    const SubTile tl = (unit ? D.tV : D.tU)[t0 + blockIdx.x / kFewSplit];
+    const SubFront &t = D.fr[tl.front];
+    const int e = t.e, r = t.r, nch = t.nch, from = unit ? t.live : -1;
+    const int i0 = tl.ti * E + blockIdx.x % kFewSplit * kFewR;
+    if (i0 > 0 && i0 >= r) return;
+    const float2 *G = (const float2 *)D.G + (size_t)k * D.szG + t.oG;
+    for (int q = threadIdx.x; q < nch * kSubEMax; q += 256) {
+        const int c = q / kSubEMax, o = q % kSubEMax;
+        if (o < e) se[c][o] = D.inv[t.inv[c] + o];
+    }
+    int x[kSubCh];  // the children's rows of this thread's result
+#pragma unroll
+    for (int c = 0; c < kSubCh; c++) x[c] = c < nch && i0 + w < r && (from >> c & 1) ? D.inv[t.inv[c] + e + i0 + w] : -1;
+    for (int q = threadIdx.x / kFewR; q < e; q += 256 / kFewR) {  // e <= kSubEMax <= Few::D
+        const int ri = threadIdx.x % kFewR;
+        sh.put(q, ri, i0 + ri < r ? G[(size_t)q * r + i0 + ri] : zero_<float2>());
+    }
+    chain_wait();
+    if (nprev && *nprev == 0) return;
+    if (B.kact && !B.kact[kk]) return;
+    __syncthreads();
+    const float2 *Y = (const float2 *)B.Y + ((size_t)kk * D.n + t.nd0) * L + col;
+    float2 *W = (float2 *)B.W + ((size_t)kk * D.n + t.nd0) * L + col;
+    float2 *U = (float2 *)B.U + (size_t)kk * D.szU * L + col;
+    float2 s[kFewR], own = zero_<float2>();
+#pragma unroll
+    for (int ri = 0; ri < kFewR; ri++) s[ri] = zero_<float2>();
+    if (col < L) {
+        constexpr int N = kSubEMax / 8;
+        float2 b[N];
+#pragma unroll
+        for (int z = 0; z < N; z++) b[z] = w + 8 * z < e ? Y[(size_t)(w + 8 * z) * L] : zero_<float2>();
+#pragma unroll
+        for (int c = 0; c < kSubCh; c++) {
+            if (c >= nch || !(from >> c & 1)) continue;
+            const float2 *Uc = U + (size_t)t.cu[c] * L;
+            float2 g[N];
+#pragma unroll
+            for (int z = 0; z < N; z++) {
+                const int y = w + 8 * z < e ? se[c][w + 8 * z] : -1;
+                g[z] = y >= 0 ? Uc[(size_t)y * L] : zero_<float2>();
+            }
+            if (x[c] >= 0) {
+                const float2 v = Uc[(size_t)x[c] * L];
+                own.x += v.x;
+                own.y += v.y;
+            }
+#pragma unroll
+            for (int z = 0; z < N; z++) {
+                b[z].x += g[z].x;
+                b[z].y += g[z].y;
+            }
+        }
+#pragma unroll
+        for (int z = 0; z < N; z++)
+            if (w + 8 * z < e) {
+                if (i0 == 0) W[(size_t)(w + 8 * z) * L] = b[z];
+                sh.add(s, w + 8 * z, b[z]);
+            }
+    }
+    const float2 v = sh.sum(s);
+    if (i0 + w < r && col < L) {
+        own.x -= v.x;
+        own.y -= v.y;
+        U[(size_t)(t.u0 + i0 + w) * L] = own;
+    }
+}
+
+__global__ __launch_bounds__(256) void k_sub_down_few(DevSub D, SubBatch B, int t0, int unit, const int *nprev) {
+    constexpr int E = Tile<float2>::E, N = Few::D / 8;
+    __shared__ __align__(16) Few sh;
+    __shared__ int at[Few::D];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int kk = blockIdx.z, k = B.k0 + kk, L = B.Lb, col = blockIdx.y * 32 + lane;
+    const SubTile tl = D.tD[t0 + blockIdx.x / kFewSplit];
+    const SubFront &t = D.fr[tl.front];
+    const int e = t.e, r = t.r, i0 = tl.ti * E + blockIdx.x % kFewSplit * kFewR;
+    if (i0 >= e) return;
+    const float2 *F = (const float2 *)D.F + (size_t)k * D.szF + t.oF, *G = (const float2 *)D.G + (size_t)k * D.szG + t.oG;
+    const float2 *W = (const float2 *)B.W + ((size_t)kk * D.n + t.nd0) * L + col;
+    float2 *Z = (float2 *)B.Z + (size_t)kk * D.n * L + col;
+    const int32_t *rows = D.rows + t.rows0;
+    const int depth = r + (unit && !t.live ? 0 : e);
+    float2 s[kFewR];
+#pragma unroll
+    for (int ri = 0; ri < kFewR; ri++) s[ri] = zero_<float2>();
+    for (int p = 0; p < depth; p += Few::D) {  // G's columns (negative), then F11^-1's
+        const int n = min(Few::D, depth - p);
+        if (p) __syncthreads();
+        for (int q = lane; q < n; q += 32) {  // one row a warp
+            float2 v = zero_<float2>();
+            if (i0 + w < e) v = p + q < r ? neg_(G[(size_t)(i0 + w) * r + p + q]) : F[(size_t)(i0 + w) * e + p + q - r];
+            sh.put(q, w, v);
+        }
+        for (int q = threadIdx.x; q < n; q += 256)
+            if (p + q < r) at[q] = rows[p + q];
+        if (!p) {
+            chain_wait();
+            if (nprev && *nprev == 0) return;
+            if (B.kact && !B.kact[kk]) return;
+        }
+        __syncthreads();
+        float2 b[N];
+#pragma unroll
+        for (int z = 0; z < N; z++) {
+            const int q = w + 8 * z;
+            b[z] = zero_<float2>();
+            if (q < n && col < L) b[z] = p + q < r ? Z[(size_t)at[q] * L] : W[(size_t)(p + q - r) * L];
+        }
+#pragma unroll
+        for (int z = 0; z < N; z++)
+            if (w + 8 * z < n) sh.add(s, w + 8 * z, b[z]);
+    }
+    const float2 v = sh.sum(s);
+    if (i0 + w < e && col < L) Z[(size_t)(t.nd0 + i0 + w) * L] = v;
+}
+
 // -------------------------------------------------- vectors of a rectangle
 // Right-hand sides from the rows of src ([eanz][n]), scaled by fk
 template <typename T>
@@ -1369,22 +1531,41 @@ void root_t(const DevProblem &P, const DevSub &D, const SubBatch &B, const doubl
     k_sub_root<T><<<B.Kb * B.Lb, kRT, root_smem<T>(), st>>>(D, B);
 }
 
+// Levels with tiles for at most a third of the SMs (48 blocks) take the kernels
+// for few fronts.  Blocks at most against forwards in ms (60x20 line with
+// Jacobian / 200x60 / triangle gradient / 300x80 / eight contexts at once): none
+// 1.31 9.53 12.23 26.1 16.9, 30 1.28 9.54 12.0 26.1 16.9, 48 1.27 9.40 11.84 25.9
+// 16.9, 76 1.25 9.35 11.82 25.9 17.2, 152 1.24 9.35 11.75 25.7 17.2, 608 1.25 9.59
+// 12.07 25.7 18.4: they read the vectors four times as often as the tiles do,
+// which costs where other work could use the chip.  In complex128 every block is
+// FP64-bound and they give nothing (160x50 32.6 -> 32.8), so there the tiles stay.
+constexpr int kFewBlocks = 48;
+
 template <typename T>
 int apply_t(const DevSub &D, const SubPlan &sp, const SubBatch &B, bool unit, const int *nprev, cudaStream_t st) {
-    const int lt = (B.Lb + Tile<T>::E - 1) / Tile<T>::E;
+    const bool few = std::is_same<T, float2>::value;
+    const int lt = nb(B.Lb, Tile<T>::E);
     const std::vector<int32_t> &up = unit ? sp.lV : sp.lU;
     int launches = 1;
     for (int lv = 0; lv < sp.nlevel; lv++) {
         const int nu = up[lv + 1] - up[lv];
         if (!nu) continue;
-        chain_launch(k_sub_up<T>, dim3(nu, lt, B.Kb), 256, 0, st, D, B, up[lv], unit ? 1 : 0, nprev);
+        if (few && nu * lt * B.Kb <= kFewBlocks)
+            chain_launch(k_sub_up_few, dim3(nu * kFewSplit, lt, B.Kb), 256, 0, st, D, B, up[lv], unit ? 1 : 0,
+                         nprev);
+        else
+            chain_launch(k_sub_up<T>, dim3(nu, lt, B.Kb), 256, 0, st, D, B, up[lv], unit ? 1 : 0, nprev);
         launches++;
     }
     chain_launch(k_sub_root_solve<T>, dim3(B.Kb * B.Lb), kST, sizeof(T) * D.mp, st, D, B, unit ? 1 : 0, nprev);
     for (int lv = sp.nlevel - 1; lv >= 0; lv--) {
         const int nd = sp.lD[lv + 1] - sp.lD[lv];
         if (!nd) continue;
-        chain_launch(k_sub_down<T>, dim3(nd, lt, B.Kb), 256, 0, st, D, B, sp.lD[lv], unit ? 1 : 0, nprev);
+        if (few && nd * lt * B.Kb <= kFewBlocks)
+            chain_launch(k_sub_down_few, dim3(nd * kFewSplit, lt, B.Kb), 256, 0, st, D, B, sp.lD[lv],
+                         unit ? 1 : 0, nprev);
+        else
+            chain_launch(k_sub_down<T>, dim3(nd, lt, B.Kb), 256, 0, st, D, B, sp.lD[lv], unit ? 1 : 0, nprev);
         launches++;
     }
     return launches;
