@@ -1053,7 +1053,7 @@ int run_adjoint(crgpu_ctx *c, const double2 *d_g, double2 *d_grad) {
         c->factors_resident = nsys_total <= bs;
     }
     launch_adjoint_grad(P, c->d_kpot, c->d_lambda, c->d_ebnd_ptr, c->d_ebnd_list, d_grad, c->st);
-    c->stats.kernel_launches += 1;
+    c->stats.kernel_launches += 2;
     cudaEventRecord(a1, c->st);
     e = check_device_errors(c, nullptr, 0);
     if (!e) e = collect_refine_stats(c);
