@@ -2287,7 +2287,7 @@ int crgpu_mcm(crgpu_ctx *c, const double *wmatd, const int32_t *wdfak, int32_t l
     a.diag_res = diag_res;
     a.diag_cov2 = diag_cov2;
     std::string msg;
-    const int rc = run_mcm(a, c->st, msg);
+    const int rc = run_mcm(a, c->st, c->st_hi, c->ev_join, msg);
     for (void *p : {(void *)d_w, (void *)d_wd, (void *)d_sm, (void *)d_nb}) {
         if (!p) continue;
         cudaFreeAsync(p, c->st);

@@ -345,41 +345,39 @@ void dense_syrk_t(int n, int k, const double *S, int lds, double *C, cudaStream_
     gemm<true, true>(n, n, k, 1.0, S, lds, S, lds, 0.0, C, n, 1, kDepthAll, nullptr, nullptr, st);
 }
 
-void dense_potrf(int n, double *A, double *Y, int *info_dev, cudaStream_t st) {
+// The factor's chain (a diagonal block on one SM, its panel, the trailing update)
+// runs on hi, and a block row of the inverse follows on st as soon as its panel is
+// there: the inverse's products fill the chip while a diagonal block (0.11 ms, 13 %
+// of the time at n = 2400) or a small trailing update leaves it empty.  Covariance
+// diagonals of 2400 cells x 600 data 32.5 -> 29.3 ms.
+void dense_potrf_inverse(int n, double *A, double *Y, int *info_dev, cudaStream_t st, cudaStream_t hi, cudaEvent_t ev) {
     constexpr int smem = (int)sizeof(double) * 2 * kNB * (kNB + 1);
     static std::once_flag once;
     std::call_once(once, [] { cudaFuncSetAttribute(k_potf2_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
     const int nb = nblk(n);
+    cudaEventRecord(ev, st);
+    cudaStreamWaitEvent(hi, ev, 0);
     for (int b = 0; b < nb; b++) {
-        const int c0 = b * kNB, w = std::min(kNB, n - c0), rest = n - c0 - w;
-        double *Yd = Y + (size_t)c0 * n + c0;
-        k_potf2_inv<<<1, 256, smem, st>>>(n, A, Y, n, c0, info_dev);
-        if (rest <= 0) break;
-        double *X = A + (size_t)c0 * n + c0 + w;
-        k_times_inverse<true><<<(rest + 15) / 16, 256, 0, st>>>(w, Yd, n, X, n, rest);
+        const int c0 = b * kNB, w = std::min(kNB, n - c0), r0 = c0 + w, rest = n - r0;
+        double *Yd = Y + (size_t)c0 * n + c0, *X = A + (size_t)c0 * n + r0;
+        k_potf2_inv<<<1, 256, smem, hi>>>(n, A, Y, n, c0, info_dev);
+        if (rest > 0) k_times_inverse<true><<<(rest + 15) / 16, 256, 0, hi>>>(w, Yd, n, X, n, rest);
+        cudaEventRecord(ev, hi);
         // trailing update A22 -= X X^T, X = the panel (row-index contiguous)
-        double *A22 = A + (size_t)(c0 + w) * n + c0 + w;
-        gemm<false, false>(rest, rest, w, -1.0, X, n, X, n, 1.0, A22, n, 1, kDepthAll, nullptr, nullptr, st);
-    }
-}
-
-void dense_trtri(int n, const double *L, double *Y, cudaStream_t st) {
-    // Y = L^-1 (lower), block row by block row; its diagonal blocks are there
-    const int nb = nblk(n);
-    for (int i = 0; i < nb; i++) {
-        const int c0 = i * kNB, w = std::min(kNB, n - c0);
-        // Y_(i, j) = -Y_ii acc_(i, j), j < i
-        if (i > 0)
-            k_times_inverse<false><<<(c0 + 15) / 16, 256, 0, st>>>(w, Y + (size_t)c0 * n + c0, n, Y + c0, n, c0);
-        const int r0 = c0 + kNB;
-        if (r0 >= n) break;
-        // acc_(i', j) (+)= L_(i', i) Y_(i, j) for the block rows below, j <= i; block
-        // column i begins here
-        if (i > 0)
-            gemm<false, true>(n - r0, c0, w, 1.0, L + (size_t)c0 * n + r0, n, Y + c0, n, 1.0, Y + r0, n, 0, kDepthAll,
-                              nullptr, nullptr, st);
-        gemm<false, true>(n - r0, w, w, 1.0, L + (size_t)c0 * n + r0, n, Y + (size_t)c0 * n + c0, n, 0.0,
-                          Y + (size_t)c0 * n + r0, n, 0, kDepthAll, nullptr, nullptr, st);
+        if (rest > 0)
+            gemm<false, false>(rest, rest, w, -1.0, X, n, X, n, 1.0, A + (size_t)r0 * n + r0, n, 1, kDepthAll, nullptr,
+                               nullptr, hi);
+        // Y = L^-1 (lower), block row by block row; its diagonal blocks are there.
+        // Y_(b, j) = -Y_bb acc_(b, j), j < b
+        cudaStreamWaitEvent(st, ev, 0);
+        if (b > 0) k_times_inverse<false><<<(c0 + 15) / 16, 256, 0, st>>>(w, Yd, n, Y + c0, n, c0);
+        if (rest <= 0) break;
+        // acc_(i, j) (+)= L_(i, b) Y_(b, j) for the block rows below, j <= b; block
+        // column b begins here
+        if (b > 0)
+            gemm<false, true>(rest, c0, w, 1.0, X, n, Y + c0, n, 1.0, Y + r0, n, 0, kDepthAll, nullptr, nullptr, st);
+        gemm<false, true>(rest, w, w, 1.0, X, n, Yd, n, 0.0, Y + (size_t)c0 * n + r0, n, 0, kDepthAll, nullptr, nullptr,
+                          st);
     }
 }
 

@@ -116,19 +116,18 @@ struct McmArgs {
     double *diag_ata, *diag_reg, *diag_cov1, *diag_res, *diag_cov2;
 };
 // dense FP64 kernels (dense.cu), column-major: C (lower) = S^T S for S k x n;
-// the Cholesky factor of A (n x n, lower, in place) with the inverses of its
-// 64-wide diagonal blocks in Y (info_dev: first non-positive pivot, 1-based, 0
-// if none); Y = L^-1 from there; C (lower) = Y^T Y; d_j = sum_i Y_ij^2 of the
+// the Cholesky factor L of A (n x n, lower, in place) and Y = L^-1 (info_dev:
+// first non-positive pivot, 1-based, 0 if none; hi, ev: a stream of high priority
+// and an event that it uses beside st); C (lower) = Y^T Y; d_j = sum_i Y_ij^2 of the
 // lower Y; the sums over l of G_lj^2 and G_lj S_lj for G = S Y^T Y, S m x n, with
 // T (m x n) and work (ceil(m/32) x 2 x n)
 void dense_syrk_t(int n, int k, const double *S, int lds, double *C, cudaStream_t st);
-void dense_potrf(int n, double *A, double *Y, int *info_dev, cudaStream_t st);
-void dense_trtri(int n, const double *L, double *Y, cudaStream_t st);
+void dense_potrf_inverse(int n, double *A, double *Y, int *info_dev, cudaStream_t st, cudaStream_t hi, cudaEvent_t ev);
 void dense_lauum_t(int n, const double *Y, double *C, cudaStream_t st);
 void dense_lower_col_sq(int n, const double *Y, double *d, cudaStream_t st);
 void dense_product_sums(int m, int n, const double *S, const double *Y, double *T, double *work, double *d2, double *dd,
                         cudaStream_t st);
-int run_mcm(const McmArgs &a, cudaStream_t st, std::string &msg);
+int run_mcm(const McmArgs &a, cudaStream_t st, cudaStream_t hi, cudaEvent_t ev, std::string &msg);
 void launch_column_sums(int nanz, int manz, const double2 *sens, const double *wa, const double *wb,
                         const double *wc, double *c1, double *c2, double *c3, cudaStream_t st);
 

@@ -159,7 +159,7 @@ void launch_column_sums(int nanz, int manz, const double2 *sens, const double *w
     if (manz > 0) k_column_sums<<<manz, 256, 0, st>>>(nanz, sens, wa, wb, wc, c1, c2, c3);
 }
 
-int run_mcm(const McmArgs &a, cudaStream_t st, std::string &msg) {
+int run_mcm(const McmArgs &a, cudaStream_t st, cudaStream_t hi, cudaEvent_t ev, std::string &msg) {
     const int n = a.manz, m = a.nanz;
     const size_t nn = (size_t)n * n;
     double *A = nullptr, *ata = nullptr, *reg = nullptr, *Y = nullptr, *cov = nullptr, *d = nullptr, *d2 = nullptr, *work = nullptr;
@@ -198,9 +198,9 @@ int run_mcm(const McmArgs &a, cudaStream_t st, std::string &msg) {
     }
     dal((void **)&Y, sizeof(double) * nn);
     if (!rc) {
-        // bmcm: Cholesky factor L of ata_reg (in place, lower)
+        // bmcm: Cholesky factor L of ata_reg (in place, lower) and Y = L^-1
         cudaMemsetAsync(info, 0, sizeof(int), st);
-        dense_potrf(n, reg, Y, info, st);
+        dense_potrf_inverse(n, reg, Y, info, st, hi, ev);
         int h_info = 0;
         cudaMemcpyAsync(&h_info, info, sizeof(int), cudaMemcpyDeviceToHost, st);
         cudaStreamSynchronize(st);
@@ -208,8 +208,7 @@ int run_mcm(const McmArgs &a, cudaStream_t st, std::string &msg) {
     }
     const bool sums = a.want_res && a.want_cov2;
     if (!rc) {
-        // cov = Y^T Y, Y = L^-1: its diagonal needs Y alone
-        dense_trtri(n, reg, Y, st);
+        // cov = Y^T Y: its diagonal needs Y alone
         dense_lower_col_sq(n, Y, d, st);
         cudaMemcpyAsync(a.diag_cov1, d, sizeof(double) * n, cudaMemcpyDeviceToHost, st);
     }
