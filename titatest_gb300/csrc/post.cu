@@ -269,6 +269,10 @@ __device__ __forceinline__ void sens_element(const DevProblem &P, const typename
     using T = SensT<R>;
     using C = typename T::C;
     using S = typename T::S;
+    // complex64: a wavenumber's sum over the nodes, whose terms nearly cancel, on its
+    // own and the weight afterwards; inside the running sum the rounding of its
+    // terms made J's error 4.9e-6 instead of 3.4e-6 (12000 x 4000)
+    constexpr bool kOwnSum = sizeof(R) == 4;
     const int eanz = P.eanz, E1 = eanz + 1, tid = threadIdx.x;
     S *kp = (S *)smem;             // [2][NK][E1], the last entry of a row an absent electrode's zero
     C *tab = (C *)(kp + 2 * NK * E1);  // [NK][dipoles of the pass], then [NK][those of its second table]
@@ -307,8 +311,10 @@ __device__ __forceinline__ void sens_element(const DevProblem &P, const typename
             R kel[NK * (NK + 1) / 2];
             const R w = P.swrtr ? (R)P.kwnwi[k] : (R)1;
 #pragma unroll
-            for (int q = 0; q < NK * (NK + 1) / 2; q++)
-                kel[q] = (R)P.elbg[((size_t)k * P.elanz + e) * 10 + q] * w;
+            for (int q = 0; q < NK * (NK + 1) / 2; q++) {
+                kel[q] = (R)P.elbg[((size_t)k * P.elanz + e) * 10 + q];
+                if (!kOwnSum) kel[q] *= w;
+            }
             cp_wait<0>();
             __syncthreads();
             if (k + 1 < P.K) fetch(k + 1, (k + 1) & 1);
@@ -361,7 +367,7 @@ __device__ __forceinline__ void sens_element(const DevProblem &P, const typename
                 }
 #pragma unroll
                 for (int h = 0; h < kSensGroup; h++) {
-                    C &s = acc[m0 + h];
+                    C own = T::mk(0, 0), &s = kOwnSum ? own : acc[m0 + h];
 #pragma unroll
                     for (int q = 0; q < NK; q++) {
                         const C b = tab[q * nd + md[h].z];
@@ -369,6 +375,10 @@ __device__ __forceinline__ void sens_element(const DevProblem &P, const typename
                         s.x = fma(-a[h][q].y, b.y, s.x);
                         s.y = fma(a[h][q].x, b.y, s.y);
                         s.y = fma(a[h][q].y, b.x, s.y);
+                    }
+                    if (kOwnSum) {
+                        acc[m0 + h].x = fma(w, own.x, acc[m0 + h].x);
+                        acc[m0 + h].y = fma(w, own.y, acc[m0 + h].y);
                     }
                 }
             }
