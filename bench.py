@@ -94,18 +94,6 @@ class ClockSampler:
                 "reasons": reasons, "samples": len(self.samples)}
 
 
-def tensor_peak_tflops():
-    """Dense tensor peak for a kernel timed inside a long step: the sustained
-    bf16 figure of MEASURED_PEAKS.json (measured on this machine), else
-    the fallback measurement of 1.7 PFLOP/s."""
-    try:
-        with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
-            pk = json.load(f)
-        return float(pk["bf16_tflops_sustained"]), "MEASURED_PEAKS.json bf16_tflops_sustained (of measured)"
-    except (OSError, KeyError, ValueError):
-        return 1700.0, "fallback 1.7 PFLOP/s sustained bf16 (of fallback)"
-
-
 def fp64_dgemm_tflops(stream) -> float:
     """The FP64 rate of this GPU as cuBLAS DGEMM reaches it (4096^3, best of
     3, CUDA events): the denominator of the complex128 factor's roofline."""
@@ -158,30 +146,28 @@ def fp32_sgemm_tflops(stream) -> float:
     return 2.0 * 8192 ** 3 / (best * 1e-3) / 1e12
 
 
-def factored_band(m, g) -> int:
-    """Band width of the matrix a context factors: the grid's, or that of its
-    geometric node order (crgpu_node_order)."""
-    order = np.asarray(m.node_order(), dtype=np.int64) - 1  # grid node at each position
-    pos = np.empty(g.sanz, np.int64)
-    pos[order] = np.arange(g.sanz)
-    area = np.asarray(g.nrel[: g.nelanz[0]], dtype=np.int64) - 1
-    p = pos[area]
-    return int((p.max(axis=1) - p.min(axis=1)).max())
+def root_nodes(g) -> int:
+    """Nodes of the mixed boundary lines (type 11): the order of the dense root
+    that the substructured solver factors for every (wavenumber, electrode)."""
+    rows, i = [], 0
+    for t, cnt in zip(g.typ, g.nelanz):
+        if int(t) == 11:
+            rows.append(np.asarray(g.nrel[i:i + cnt, :2]).ravel())
+        i += int(cnt)
+    return int(np.unique(np.concatenate(rows)).size) if rows else 0
 
 
-FACTOR_KERNELS = {"tensor cores": ("k_factor_tc", "tensor"), "SIMT warp per system": ("k_factor_warp", "fp32"),
-                  "SIMT register tiles": ("k_factor_mixed", "fp32"),
-                  "SIMT shared-memory tiles": ("k_factor_mixed_smem", "fp32")}
-
-
-FACTOR_NOTES = {
-    "k_factor_warp": "latency-bound band factor: a serial chain per column (pivot, reciprocal, rank-1 update of "
-                     "the 64-slot window held in one warp's registers), one system per warp, 12 warps an SM",
-    "k_factor_warp2": "latency-bound band factor, two columns a step (2x2 pivot block, two rank-1 updates of the "
-                      "64-slot window held in one warp's registers), one system per warp, 8 warps an SM; the "
-                      "systems beyond 8 an SM are factored on the tensor cores beside the solves",
-    "k_factor_tc": "latency-bound band factor: each 4-column step is a serial panel plus 4 tf32 MMAs (3 hi/lo "
-                   "products + row injection) on a 128x128 complex window"}
+def factor_phase_ms(m, sigma) -> float:
+    """Device time of the factor phase (shared elimination and root factors) of
+    every system, nothing beside it: two rectangles of systems, whose phases the
+    library times one after the other."""
+    m.set_memory_budget(0)
+    m.set_memory_budget(int(0.6 * m.memory_need()))
+    m.forward(sigma)
+    m.forward(sigma)
+    st = m.stats()
+    m.set_memory_budget(0)
+    return st["ms_factor"] if st["nbatches"] > 1 else float("nan")
 
 
 def read_profile_traffic(name: str):
@@ -257,8 +243,8 @@ def workload_config(cfg: int, s, K: int) -> dict:
     g, sv = s.grid, s.survey
     nsys = K * sv.eanz
     return {"workload": workload_string(cfg, s, K),
-            "l2": "inputs larger than L2: the band factors of all %d systems are %.1f GB in complex64"
-                  % (nsys, nsys * g.sanz * (g.mb + 1) * 8 / 1e9)}
+            "l2": "inputs larger than L2: the potentials of all %d systems are %.2f GB in complex128, the Jacobian "
+                  "%.2f GB" % (nsys, nsys * g.sanz * 16 / 1e9, g.elanz * sv.nanz * 16 / 1e9)}
 
 
 def run_reference(args):
@@ -428,49 +414,28 @@ def run_gpu(args):
     torch.cuda.synchronize()
     plain_ms = p0.elapsed_time(p1) / p_steps
     plain_stats = plain.stats()
+    plain_fac = factor_phase_ms(plain, s.sigma)
     volt_plain = volt_dev.cpu().numpy().view(np.complex128).copy()
     sens_plain = sens_dev.cpu().numpy().view(np.complex128).copy()
     err_v = float(np.abs(volt_mixed - volt_plain).max() / np.abs(volt_plain).max())
     err_j = float(np.abs(sens_mixed - sens_plain).max() / np.abs(sens_plain).max())
     plain.close()
 
-    # ---- roofline of the dominant kernel (the complex64 band factorisation of
-    #      the band the context factors); algorithmic work = complex L L^T of
-    #      every system, 4 n mb^2 flops
-    n, mb = g.sanz, g.mb
-    mb_mixed = factored_band(mixed, g)
-    nsys = K * sv.eanz
-    flops_factor = nsys * 4.0 * n * mb * mb  # the grid's band: the complex128 arm factors it
-    kname, bound = FACTOR_KERNELS.get(tune["factor"], ("k_factor_tc", "tensor"))
-    nsys_main = nsys
-    if kname == "k_factor_warp":
-        # the library's split: up to 8 systems an SM in the timed factor launch,
-        # the excess (at most one an SM) on the tensor cores beside the solves
-        nsm = torch.cuda.get_device_properties(0).multi_processor_count
-        if 0 < nsys - 8 * nsm <= nsm:
-            nsys_main = 8 * nsm
-        if mb_mixed <= 62:
-            kname = "k_factor_warp2"
-    flops_mixed = nsys_main * 4.0 * n * mb_mixed * mb_mixed
-    fp64_peak = fp64_dgemm_tflops(stream)
-    fac_avg_ms = statistics.mean(fac_ms)
-    achieved = flops_mixed / (fac_avg_ms * 1e-3) / 1e12
-    # the same launch on the HBM lens: its algorithmic bytes (the complex64
-    # factor written once, the scaled complex128 pattern rows and the
-    # right-hand side read once) over its time
-    alg_bytes = nsys_main * (n * (mb_mixed + 1) * 8.0 + n * 8.0 + n * 16.0)
+    # ---- roofline of the dominant kernel, the root factor: algorithmic work =
+    #      complex symmetric L D L^T of order m of every system, 4/3 m^3 flops;
+    #      over the whole factor phase (shared elimination included)
+    nsys, m = K * sv.eanz, root_nodes(g)
+    flops_root = nsys * 4.0 / 3.0 * float(m) ** 3
+    fp64_peak, fp32_peak = fp64_dgemm_tflops(stream), fp32_sgemm_tflops(stream)
+    fac_mixed = factor_phase_ms(mixed, s.sigma)
+    achieved = flops_root / (fac_mixed * 1e-3) / 1e12
+    # the same phase on the HBM lens: the lower triangles written once
+    alg_bytes = nsys * 0.5 * m * (m + 1) * 8.0
     hbm_peak, hbm_src = hbm_peak_gbs()
-    hbm_ach = alg_bytes / (fac_avg_ms * 1e-3) / 1e9
+    hbm_ach = alg_bytes / (fac_mixed * 1e-3) / 1e9
     hbm_view = {"bound": "hbm", "achieved": hbm_ach, "peak": hbm_peak, "unit": "GB/s", "frac": hbm_ach / hbm_peak,
-                "peak_source": hbm_src,
-                "algorithmic": "per system: n (mb+1) 8 B of complex64 factor and n 8 B of forward substitution "
-                               "written, n 16 B of right-hand side read (the pattern rows' reads excluded)"}
-    if bound == "tensor":
-        peak, peak_source = tensor_peak_tflops()
-    else:
-        peak = fp32_sgemm_tflops(stream)
-        peak_source = "cuBLAS SGEMM 8192^3, TF32 off, measured in this run (best of 3, CUDA events)"
-    traffic = read_profile_traffic(f"{kname}_cfg2.txt")
+                "peak_source": hbm_src, "algorithmic": "m (m+1) / 2 complex64 entries a system written"}
+    traffic = read_profile_traffic("k_sub_root_cfg2.txt")
     line = {
         "metric": METRIC, "value": value, "unit": "units/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_per_step, "higher_is_better": True, "scaling": "weak",
@@ -489,26 +454,27 @@ def run_gpu(args):
         "plain": {"value": 1e3 / plain_ms, "unit": "units/s", "ms_per_step": plain_ms,
                   "ms_factor": plain_stats["ms_factor"], "ms_solve": plain_stats["ms_solve"],
                   "ms_sens": plain_stats["ms_sens"],
-                  "roofline": {"kernel": "k_factor_plain_reg", "bound": "fp64",
-                               "achieved": flops_factor / (plain_stats["ms_factor"] * 1e-3) / 1e12,
+                  "roofline": {"kernel": "k_sub_root<double2>", "bound": "fp64", "ms_factor_phase": plain_fac,
+                               "achieved": flops_root / (plain_fac * 1e-3) / 1e12,
                                "peak": fp64_peak, "unit": "TFLOP/s",
-                               "frac": flops_factor / (plain_stats["ms_factor"] * 1e-3) / 1e12 / fp64_peak,
+                               "frac": flops_root / (plain_fac * 1e-3) / 1e12 / fp64_peak,
                                "peak_source": "cuBLAS DGEMM 4096^3 measured in this run (best of 3, CUDA events)"}},
         "speedup_mixed_vs_plain": plain_ms / ms_per_step,
         "mixed_vs_plain_rel_err": {"volt": err_v, "jacobian": err_j},
         "accuracy_target": {"volt": 1e-6, "jacobian": 1e-5, "met": bool(err_v < 1e-6 and err_j < 1e-5)},
-        "phases_ms": {"factor": fac_avg_ms, "solve": mixed_stats["ms_solve"],
+        "phases_ms": {"factor": statistics.mean(fac_ms), "solve": mixed_stats["ms_solve"],
                       "forward": mixed_stats["ms_forward"], "sens": statistics.mean(sens_ms)},
-        "factor_band": {"grid_mb": mb, "factored_mb": mb_mixed,
-                        "node_order": "geometric" if mb_mixed != mb else "grid"},
-        "roofline": {"kernel": kname, "bound": bound, "achieved": achieved, "peak": peak,
-                     "unit": "TFLOP/s", "frac": achieved / peak, "traffic": traffic,
-                     "peak_source": peak_source,
-                     "algorithmic": "4*n*mb^2 flops per band system (complex L L^T) at the factored band, "
-                                    "the systems of the timed factor launch",
-                     "systems": nsys_main,
+        "root_order": m,
+        "roofline": {"kernel": "k_sub_root<float2>", "bound": "fp32", "ms_factor_phase": fac_mixed,
+                     "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s", "frac": achieved / fp32_peak,
+                     "traffic": traffic,
+                     "peak_source": "cuBLAS SGEMM 8192^3, TF32 off, measured in this run (best of 3, CUDA events)",
+                     "algorithmic": "4/3 m^3 flops per system (complex symmetric factor of the root of order m), over "
+                                    "the factor phase with the shared elimination",
+                     "systems": nsys,
                      "hbm_view": hbm_view,
-                     "note": FACTOR_NOTES.get(kname, "")},
+                     "note": "one block per system, blocked left-looking factor in 32-column blocks; FP32 FMA issue "
+                             "and the barriers between a block's stages bound it"},
     }
     kwn, kwnwi = mixed.kwn, mixed.kwnwi
     mixed.close()
@@ -560,8 +526,8 @@ def run_ensemble(args):
         "data": "synthetic (seeded meshes 40x15..300x80 quads, 24-128 electrodes, 200-6000 quadrupoles)",
         "config": {"workload": f"config5: {len(probs)} problems, {sum(p.grid.sanz for p in probs)} nodes in total",
                    "workers": args.workers,
-                   "parallelism": ("single GPU, waves of problems: one tensor-core factor launch over all "
-                                   "systems of a wave, the other steps on the problems' streams" if args.ensemble_batched
+                   "parallelism": ("single GPU, waves of problems, each on its own stream, their refinement in "
+                                   "turn" if args.ensemble_batched
                                    else "single GPU, one context per problem on concurrent streams"),
                    "band_order": "geometric node order for mixed bands beyond the tensor-core window"},
         "clocks": clk.summary(),
@@ -674,11 +640,7 @@ def run_case(args):
         if args.autotune_case:
             print("tune", m.autotune(s.sigma), flush=True)
         if args.batch:
-            g = s.grid
-            esz = 8 if prec == MIXED else 16
-            mbf = factored_band(m, g)
-            per = g.sanz * (mbf + 1) * esz + (g.sanz * 12 * 16) + g.sanz * 8 + g.sanz * (3 * 16 + esz) + 64
-            m.set_memory_budget(int(per * args.batch + per // 2))
+            m.set_memory_budget(int(m.memory_need() / (m.kwnanz * s.survey.eanz) * args.batch))
         for _ in range(args.repeat):
             t = time.time()
             out = m.forward(s.sigma)
@@ -730,7 +692,7 @@ def main():
     ap.add_argument("--no-cpu-baseline", dest="cpu_baseline", action="store_false")
     ap.add_argument("--workers", type=int, default=8, help="config 5: concurrent worker streams")
     ap.add_argument("--ensemble-batched", action="store_true",
-                    help="config 5: waves of problems with one factor launch each (crgpu_forward_sens_batch) "
+                    help="config 5: waves of problems (crgpu_forward_sens_batch) "
                          "instead of one context per problem on worker streams")
     ap.add_argument("--ensemble-count", type=int, default=256, help="config 5: number of problems")
     ap.add_argument("--case", action="store_true",

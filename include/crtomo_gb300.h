@@ -140,7 +140,7 @@ int crgpu_set_boundary_values(crgpu_ctx *ctx, int32_t rwdanz, const int32_t *rwd
  * ldc: 0 or 1. */
 int crgpu_set_dc(crgpu_ctx *ctx, int32_t ldc);
 
-/* Upper bound of device memory for the per-system band factors; systems are
+/* Upper bound of device memory for the per-system factors and vectors; systems are
  * processed in batches that fit.  Default: 60% of free device memory. */
 int crgpu_set_memory_budget(crgpu_ctx *ctx, int64_t bytes);
 
@@ -185,10 +185,10 @@ int crgpu_sens_device(crgpu_ctx *ctx, int32_t mode, void *sens_device);
  * The forward of every context (sigma[p] host, elanz complex), its voltages
  * into volt[p] (host, nanz complex: V for volt_mode 0, the CRTomo data for
  * 1) and, for sens_mode 0 or 1, its Jacobian kept on the device (as
- * crgpu_sens(ctx, mode, NULL)); sens_mode -1: none.  The band factors of all
- * problems' systems run in one persistent tensor-core launch over a table of
- * (problem, system) items, longest systems first; assembly and the solves run
- * on each context's own stream.  Every context must be CRGPU_MIXED with a band
+ * crgpu_sens(ctx, mode, NULL)); sens_mode -1: none.  Every context's work is
+ * queued on its own stream, the refinement step by step in turn; contexts on
+ * the band path share one persistent tensor-core factor launch over a table of
+ * (problem, system) items, longest systems first.  Every context must be CRGPU_MIXED with a band
  * that fits the tensor-core window (as created; see crgpu_create2), without
  * singularity removal, DC mode or boundary values, and its systems must fit
  * one batch in device memory (crgpu_memory_need); else 1002 or a CUDA error. */
@@ -233,7 +233,7 @@ int crgpu_factor_system_noalloc(crgpu_ctx *ctx, const void *sigma_device, int32_
  * src/update.f90.  The exact derivative of L = sum_i g_i V_i, the voltages
  * of the last crgpu_forward (V of src/bvolt.f90, before kfak or log), with
  * respect to sigma: one adjoint solve per (k, l) system that reuses the
- * forward's band factors (refactored batch by batch when the systems did not
+ * forward's factors (refactored batch by batch when the systems did not
  * fit in one batch) and an element-wise contraction with the element and
  * mixed-boundary matrices.  V is holomorphic in sigma, so grad_e =
  * sum_i g_i dV_i/dsigma_e.  Not available with singularity removal (1002).
@@ -345,7 +345,13 @@ int crgpu_get_stats(const crgpu_ctx *ctx, crgpu_stats *stats);
 int crgpu_forward_sens_graph(crgpu_ctx *ctx, const void *sigma_device, void *volt_device, int32_t mode,
                              void *sens_device);
 
-/* Autotuner (mixed precision): times the band-factor kernels that can run
+/* With mixed boundaries a forward eliminates the nodes off them once per
+ * wavenumber and factors a dense root per (k, l) system wherever that is
+ * cheaper than the band; the band is factored with singularity removal, in DC
+ * mode, with prescribed Dirichlet values, and where a band kernel is pinned
+ * (crgpu_set_tune).
+ *
+ * Autotuner (mixed precision): times the band-factor kernels that can run
  * this problem (one warp per system; tensor cores; SIMT register tiles at
  * 1, 2 and 4 blocks per SM; SIMT shared-memory tiles) on its first batch of
  * systems, and the two
@@ -364,7 +370,8 @@ int crgpu_autotune(crgpu_ctx *ctx, const double *sigma, int32_t flags);
 int crgpu_get_tune(const crgpu_ctx *ctx, int32_t *out);
 
 /* Sets the launch choices in the layout of crgpu_get_tune (a kernel that
- * cannot run this problem falls back to the default); blocks per SM 0..8. */
+ * cannot run this problem falls back to the default); blocks per SM 0..8.  A
+ * factor kernel other than 0 pins the band path; 0 takes that back. */
 int crgpu_set_tune(crgpu_ctx *ctx, const int32_t *in);
 
 #ifdef __cplusplus

@@ -394,8 +394,8 @@ def run_tomodir(exe_dir: str, precision: int = PLAIN, write: bool = True):
 
 def forward_sens_batch(models, sigmas, sens_mode: int = 0, volt_mode: int = 0):
     """crgpu_forward_sens_batch: the forward of every model (MIXED contexts
-    whose bands fit the tensor-core window), their band factors in one
-    persistent launch; the Jacobians (sens_mode 0 or 1; -1 none) stay on the
+    whose bands fit the tensor-core window), each on its own stream, refined
+    in turn; the Jacobians (sens_mode 0 or 1; -1 none) stay on the
     devices of the contexts.  Returns the voltages, one array per model."""
     n = len(models)
     sig = [np.ascontiguousarray(s, np.complex128) for s in sigmas]

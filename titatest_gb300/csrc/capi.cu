@@ -1649,7 +1649,8 @@ int crgpu_memory_need(const crgpu_ctx *c, int64_t *bytes) {
 // solver takes stay there, the band factors of all others' systems run in one
 // persistent tensor-core launch over a table of (problem, system) items,
 // longest systems first, and each problem's solves, refinement,
-// back-transform, voltages and Jacobian then run on its own stream again.  Every problem must fit one batch (crgpu_memory_need).
+// back-transform, voltages and Jacobian then run on its own stream again.
+// Every problem must fit one batch (crgpu_memory_need).
 int crgpu_forward_sens_batch(crgpu_ctx *const *ctxs, int32_t nprob, const double *const *sigma, int32_t volt_mode,
                              double *const *volt, int32_t sens_mode) {
     if (!ctxs || nprob <= 0 || !sigma || !volt || (sens_mode < -1 || sens_mode > 1)) return ERR_ARG;

@@ -14,7 +14,8 @@
 // Config 2 (12261 nodes, 13 wavenumbers x 96 electrodes, m = 321): 3.9e7
 // complex multiply-adds a wavenumber for the shared part and 5.5e6 a system
 // for the root, against 2.4e7 a system for the band of 62 and 9.0e7 for the
-// grid's band of 121; and 0.4 MB of root factor a system instead of 6.2 (12).
+// grid's band of 121; and a triangle of 0.4 MB a system for the root instead of
+// 6.2 MB (12).
 #include <algorithm>
 #include <mutex>
 
@@ -955,8 +956,8 @@ __global__ __launch_bounds__(kST) void k_sub_root_solve(DevSub D, SubBatch B, in
 // Up the tree: b_E (own right-hand sides and the children's updates) goes to
 // W, the update rows U = (children's updates) - G^T b_E to the parent.  One
 // block per tile of update rows x electrodes.  unit: kompab's right-hand sides,
-// zero but at the electrodes, so only the fronts above an electrode take part
-// (config 2: 80 of 300) and the others' rows of W and U are not read.
+// zero but at the electrodes, so only the fronts above an electrode take part and
+// the others' rows of W and U are not read.
 template <typename T>
 __global__ __launch_bounds__(256) void k_sub_up(DevSub D, SubBatch B, int t0, int unit, const int *nprev) {
     constexpr int E = Tile<T>::E, M = Tile<T>::M, P = Tile<T>::P;

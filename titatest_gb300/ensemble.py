@@ -76,8 +76,8 @@ class Ensemble:
 
     def run_batched(self, sens_mode: Optional[int] = 0, reserve_frac: float = 0.1) -> List[dict]:
         """Runs every problem in waves that fit device memory: per wave one
-        crgpu_forward_sens_batch (all band factors of the wave in one
-        persistent launch, longest systems first).  The contexts of a wave are
+        crgpu_forward_sens_batch (every problem on its own stream, refined in
+        turn).  The contexts of a wave are
         created by the worker threads (the C ABI releases the GIL).  Problems
         the batched call does not take (bands beyond the tensor-core window)
         run one by one."""
