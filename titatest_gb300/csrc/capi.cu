@@ -1320,6 +1320,7 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
             c->sys_l.push_back(0);
         }
     }
+    Block tree;  // its host copy lives until the synchronisation below
     std::vector<int32_t> sources(enr0);
     if (c->nsink >= 0 && c->nsink < hg.n) sources.push_back(c->nsink);
     if (c->nrhs == 1 && build_sub_plan(hg, c->pat, sub_shape(precision == CRGPU_MIXED), sources, c->sp)) {
@@ -1345,7 +1346,6 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
         D.root_live = sp.fronts[sp.root_child].live != 0;
         std::vector<int32_t> fcolpos(c->pat.fcol.size());
         for (size_t q = 0; q < fcolpos.size(); q++) fcolpos[q] = sp.pos[c->pat.fcol[q]];
-        Block tree;
         tree.put(&D.fr, sp.fronts);
         tree.put(&D.ent, sp.ent);
         tree.put(&D.be, sp.be);
