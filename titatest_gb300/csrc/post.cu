@@ -99,7 +99,7 @@ void launch_bvolt(const DevProblem &P, const double2 *hpot, int mode, const doub
 // instead of 66, and the scaling by strom / pi or sigma / (pi V) is a product
 // with a factor formed once per measurement: its six FP64 divisions an entry of
 // J took longer than the whole complex64 contraction.  GB300: bsensi of 4800
-// cells x 2000 in complex128 15.2 -> 6.1 ms (the FP64 pipe bounds it; 6.8 without
+// cells x 2000 in complex128 15.2 -> 5.8 ms (the FP64 pipe bounds it; 0.7 more without
 // the second table, whose differences are additions on that pipe), 12000 x 4000 in
 // complex64 12.8 -> 5.0 ms (shared-memory reads; 6.7 without the second table,
 // which leaves 6 of the 9 reads of a measurement and wavenumber).  Blocks an
@@ -110,6 +110,7 @@ void launch_bvolt(const DevProblem &P, const double2 *hpot, int mode, const doub
 constexpr int kSensThreads = 256;
 constexpr int kSensMPT = 16;    // measurements per thread per pass (4096 per pass)
 constexpr int kSensGroup = 2;   // of them taken together (4: 6.5 and 6.0 ms in complex128 and 64, registers)
+constexpr int kSensK = 160;     // bytes of two element matrices in complex128
 constexpr int kSensDip = 1024;  // dipoles of a pass's first table (64 KB in complex128)
 constexpr int kSensDip2 = 512;  // ... of its second table (256: 5.15 ms in complex64, 512 and 1024: 5.0)
 
@@ -274,7 +275,9 @@ __device__ __forceinline__ void sens_element(const DevProblem &P, const typename
     // terms made J's error 4.9e-6 instead of 3.4e-6 (12000 x 4000)
     constexpr bool kOwnSum = sizeof(R) == 4;
     const int eanz = P.eanz, E1 = eanz + 1, tid = threadIdx.x;
-    S *kp = (S *)smem;             // [2][NK][E1], the last entry of a row an absent electrode's zero
+    constexpr int NM = NK * (NK + 1) / 2;
+    R *ks = (R *)smem;                           // [2][NM], complex128
+    S *kp = (S *)(smem + (kOwnSum ? 0 : kSensK));  // [2][NK][E1], the last entry of a row an absent electrode's zero
     C *tab = (C *)(kp + 2 * NK * E1);  // [NK][dipoles of the pass], then [NK][those of its second table]
     const size_t plane = (size_t)P.K * eanz * P.n;
     int nodes[NK];
@@ -294,6 +297,8 @@ __device__ __forceinline__ void sens_element(const DevProblem &P, const typename
             }
         }
         cp_commit();
+        if (!kOwnSum && tid < NM)  // w_k K_k by one warp: 6.10 -> 5.81 ms against every thread forming it
+            ks[buf * NM + tid] = (R)P.elbg[((size_t)k * P.elanz + e) * 10 + tid] * (P.swrtr ? (R)P.kwnwi[k] : (R)1);
     };
     const double2 sg = sigma[e];
     for (int ps = 0; ps < P.nspass; ps++) {
@@ -308,15 +313,16 @@ __device__ __forceinline__ void sens_element(const DevProblem &P, const typename
         fetch(0, 0);
         for (int k = 0; k < P.K; k++) {
             const S *u = kp + (k & 1) * NK * E1;
-            R kel[NK * (NK + 1) / 2];
+            R kel[NM];
             const R w = P.swrtr ? (R)P.kwnwi[k] : (R)1;
+            if (kOwnSum)
 #pragma unroll
-            for (int q = 0; q < NK * (NK + 1) / 2; q++) {
-                kel[q] = (R)P.elbg[((size_t)k * P.elanz + e) * 10 + q];
-                if (!kOwnSum) kel[q] *= w;
-            }
+                for (int q = 0; q < NM; q++) kel[q] = (R)P.elbg[((size_t)k * P.elanz + e) * 10 + q];
             cp_wait<0>();
             __syncthreads();
+            if (!kOwnSum)
+#pragma unroll
+                for (int q = 0; q < NM; q++) kel[q] = ks[(k & 1) * NM + q];
             if (k + 1 < P.K) fetch(k + 1, (k + 1) & 1);
             for (int d = tid; d < nd + nd2; d += kSensThreads) {
                 const int2 p = dip[d];
@@ -407,7 +413,7 @@ __global__ __launch_bounds__(kSensThreads, sizeof(R) == 4 ? 4 : 2) void k_bsens(
 // the block's shared memory (both element types)
 static size_t sens_smem(const DevProblem &P, bool single) {
     const size_t c = single ? sizeof(float2) : sizeof(double2);
-    return 2 * 4 * (size_t)(P.eanz + 1) * 16 + 4 * (size_t)P.sens_dips * c;
+    return (single ? 0 : kSensK) + 2 * 4 * (size_t)(P.eanz + 1) * 16 + 4 * (size_t)P.sens_dips * c;
 }
 
 void launch_bsens(const DevProblem &P, const double2 *kpot, const float2 *kpot32, const double2 *sigma,
