@@ -134,3 +134,15 @@ def test_refinement_stops_alike_on_every_route(gpu_lib, maxit, tol):
     finally:
         for m in mods:
             m.close()
+
+
+def test_long_mesh_with_a_large_root_matches_the_band(gpu_lib):
+    """2700 x 60 cells in complex128: a root of 2821 nodes is more than its
+    solve's shared memory holds, so the default route is the pinned band's."""
+    from titatest_gb300 import PLAIN, CRMod
+    s = _case(2700, 60, 6)
+    with CRMod(s.grid, s.survey, [0.05], [0.1], precision=PLAIN) as m:
+        v = m.forward(s.sigma)["volt"]
+        m.set_tune(1)  # complex128 has one band factor; any choice pins the band
+        w = m.forward(s.sigma)["volt"]
+    assert np.all(w != 0) and np.array_equal(v, w)

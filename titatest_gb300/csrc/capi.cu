@@ -1370,17 +1370,7 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
             *out = c;
             return e;
         }
-        const double n = hg.n, mb = hg.mb, band = 0.5 * n * mb * mb + 6.0 * n * mb;
-        const double m = sp.m, sub = m * m * m / 6.0 + 4.0 * sp.c_apply + sp.c_factor / c->eanz;
-        // Long, shallow meshes have a narrow band and a large root, but the band
-        // is eliminated column by column, so the root wins beyond equal counts.
-        // Forwards, band -> this solver in ms (sub / band operations): complex64
-        // 300x15 cells 9.4 -> 3.9 (6.7), 200x6 2.5 -> 1.4 (18), 500x12 13.8 -> 7.4
-        // (22), 800x12 21.8 -> 19.7 (52), 1000x10 24 -> 41 (114), 8x4 0.41 -> 0.27
-        // (7.2); complex128 300x15 77 -> 43 (2.4), 400x15 102 -> 82 (3.6), 300x8 37.5
-        // -> 36.3 (9.1), 500x12 95 -> 141 (8.7), and the smallest, all latency, 8x4
-        // 0.29 -> 0.35 (1.9), 12x5 0.39 -> 0.40, 16x6 0.52 -> 0.43.
-        c->sub_fits = precision == CRGPU_MIXED ? sub <= 30.0 * band : sub <= 5.0 * band && n >= 100;
+        c->sub_fits = sub_fits({mixed, hg.n, hg.mb, sp.m, D.mp, sub_root_max(mixed), c->eanz, sp.c_factor, sp.c_apply});
     }
     if (precision == CRGPU_MIXED && !mixed_window_supported(hg.mb + 1)) {
         c->last_error = "mixed precision supports band widths up to 207";

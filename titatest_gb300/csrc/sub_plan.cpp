@@ -333,4 +333,26 @@ bool build_sub_plan(const HostGrid &hg, const Pattern &pat, const SubShape &shap
     return true;
 }
 
+// Long, shallow meshes have a narrow band and a large root, but the band
+// is eliminated column by column, so the root wins beyond equal counts.
+// Forwards, band -> this solver in ms (sub / band operations): complex64
+// 300x15 cells 9.4 -> 3.9 (6.7), 200x6 2.5 -> 1.4 (18), 500x12 13.8 -> 7.4
+// (22), 800x12 21.8 -> 19.7 (52), 1000x10 24 -> 41 (114), 8x4 0.41 -> 0.27
+// (7.2); complex128 300x15 77 -> 43 (2.4), 400x15 102 -> 82 (3.6), 300x8 37.5
+// -> 36.3 (9.1), 500x12 95 -> 141 (8.7), and the smallest, all latency, 8x4
+// 0.29 -> 0.35 (1.9), 12x5 0.39 -> 0.40, 16x6 0.52 -> 0.43.
+bool sub_fits(const SubCost &q) {
+    if (q.mp > q.root_max) return false;  // the root's vector stays in one block's shared memory
+    const double n = q.n, mb = q.mb, m = q.m;
+    const double band = 0.5 * n * mb * mb + 6.0 * n * mb;
+    const double sub = m * m * m / 6.0 + 4.0 * q.c_apply + q.c_factor / q.eanz;
+    return q.mixed ? sub <= 30.0 * band : sub <= 5.0 * band && q.n >= 100;
+}
+
 }  // namespace crgpu
+
+// sub_fits by its numbers, for the tests (not part of the C ABI)
+extern "C" int crgpu_sub_fits(int32_t mixed, int32_t n, int32_t mb, int32_t m, int32_t mp, int32_t root_max, int32_t eanz,
+                              double c_factor, double c_apply) {
+    return crgpu::sub_fits({mixed != 0, n, mb, m, mp, root_max, eanz, c_factor, c_apply});
+}

@@ -73,4 +73,14 @@ struct SubPlan {
 bool build_sub_plan(const HostGrid &hg, const Pattern &pat, const SubShape &shape,
                     const std::vector<int32_t> &sources, SubPlan &sp);
 
+// A problem as the choice between the band and this solver sees it: nodes, band
+// width, nodes of the root, the same padded and the most that k_sub_root_solve
+// holds, electrodes, the plan's complex multiply-adds.
+struct SubCost {
+    bool mixed;
+    int n, mb, m, mp, root_max, eanz;
+    double c_factor, c_apply;
+};
+bool sub_fits(const SubCost &q);
+
 }  // namespace crgpu

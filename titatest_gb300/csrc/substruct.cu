@@ -865,8 +865,14 @@ __global__ __launch_bounds__(kRT, 5) void k_sub_root(DevSub D, SubBatch B) {
 }
 
 // ------------------------------------------------------------------- solves
-// x = (C C^T)^-1 u of one system's root, one block per system
+// x = (C C^T)^-1 u of one system's root, one block per system.  The vector stays in
+// shared memory, which limits the root (root_max): larger ones keep the band.
 constexpr int kST = 256;
+
+template <typename T>
+constexpr int root_max() {  // beside t and part, of the 48 KB that a launch gets without asking
+    return 48 * 1024 / (int)sizeof(T) - RootShape<T>::NB - 8 * 33;
+}
 
 template <typename T>
 __global__ __launch_bounds__(kST) void k_sub_root_solve(DevSub D, SubBatch B, int unit, const int *nprev) {
@@ -1589,6 +1595,8 @@ SubShape sub_shape(bool mixed) {
 
 int sub_root_block(bool mixed) { return mixed ? RootShape<float2>::NB : RootShape<double2>::NB; }
 int sub_root_rows(bool mixed) { return mixed ? RootShape<float2>::ROWS : RootShape<double2>::ROWS; }
+
+int sub_root_max(bool mixed) { return mixed ? root_max<float2>() : root_max<double2>(); }
 
 int sub_launch_factor(const DevProblem &P, const DevSub &D, const SubPlan &sp, int K, bool mixed, cudaStream_t st) {
     return mixed ? factor_t<float2>(P, D, sp, K, st) : factor_t<double2>(P, D, sp, K, st);

@@ -60,6 +60,7 @@ struct SubStop {
 SubShape sub_shape(bool mixed);
 int sub_root_block(bool mixed);  // columns of a block of the root factor
 int sub_root_rows(bool mixed);   // rows of one of its tiles
+int sub_root_max(bool mixed);    // most padded nodes of a root
 void sub_launch_values(const DevProblem &P, const DevSub &D, const double2 *sigma, const double2 *adom, cudaStream_t st);
 // the first K wavenumbers of D's arrays
 int sub_launch_factor(const DevProblem &P, const DevSub &D, const SubPlan &sp, int K, bool mixed, cudaStream_t st);
