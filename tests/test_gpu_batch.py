@@ -54,3 +54,20 @@ def test_forward_sens_batch_rejects_plain_contexts(gpu_lib):
         with pytest.raises(CRGPUError) as ei:
             forward_sens_batch([m], [p.sigma])
         assert ei.value.errnr == 1002
+
+
+def test_forward_sens_batch_reports_refused_launches(gpu_lib):
+    """More wavenumbers than a grid has rows (65535): launches of the chain are
+    refused, and the call says so instead of returning what memory held."""
+    from test_gpu_substruct import _case
+    from titatest_gb300 import MIXED, CRMod
+    from titatest_gb300._lib import CRGPUError
+    from titatest_gb300.crmod import forward_sens_batch
+    s = _case(8, 4, 4)
+    k = 65536 + 64
+    with CRMod(s.grid, s.survey, np.full(k, 0.1), np.full(k, 0.1), precision=MIXED) as m:
+        with pytest.raises(CRGPUError) as ei:
+            forward_sens_batch([m], [s.sigma], sens_mode=-1)
+        assert ei.value.errnr == 1000
+    with CRMod(s.grid, s.survey, precision=MIXED) as m:  # and the next call is not affected
+        assert relerr(forward_sens_batch([m], [s.sigma], sens_mode=-1)[0], m.forward(s.sigma)["volt"]) < 1e-12

@@ -1738,9 +1738,11 @@ int crgpu_forward_sens_batch(crgpu_ctx *const *ctxs, int32_t nprob, const double
             c->last_sens = c->d_sens;
         }
     }
+    // a launch that was refused leaves no status on the device
+    const cudaError_t refused = cudaGetLastError();
+    int worst = refused == cudaSuccess ? 0 : fail(c0, ERR_CUDA, cudaGetErrorString(refused));
     // the voltages once every problem's work is queued (a copy into pageable
     // host memory returns only when it is done)
-    int worst = 0;
     for (int p = 0; p < nprob; p++) {
         crgpu_ctx *c = ctxs[p];
         CUCHECK(c, cudaMemcpyAsync(volt[p], volt_mode == 0 ? c->d_volt : c->d_sigmaa, sizeof(double2) * c->nanz,
@@ -1750,8 +1752,7 @@ int crgpu_forward_sens_batch(crgpu_ctx *const *ctxs, int32_t nprob, const double
         int e = check_device_errors(c, sub ? c->SB.status : hb[p].status, (int)c->sys_k.size());
         if (!e) e = collect_refine_stats(c);
         if (e && !worst) worst = e;
-        c->have_forward = !e;
-        c->factors_resident = !e;
+        c->have_forward = c->factors_resident = !e && refused == cudaSuccess;
         c->stats.nbatches = 1;
     }
     for (void *q : {(void *)dP, (void *)dB, (void *)dI})
