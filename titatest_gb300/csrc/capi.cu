@@ -43,7 +43,10 @@ int dalloc(crgpu_ctx *c, T **p, size_t count) {
     // stream-ordered: no device-wide synchronisation on free, so contexts on
     // different streams (ensembles) do not serialise each other
     cudaError_t e = cudaMallocAsync(&q, count * sizeof(T), c->st);
-    if (e != cudaSuccess) return fail(c, 94, std::string("device allocation: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // reported here, not by the next call's check of its launches
+        return fail(c, 94, std::string("device allocation: ") + cudaGetErrorString(e));
+    }
     c->allocs.push_back(q);
     *p = (T *)q;
     return 0;
