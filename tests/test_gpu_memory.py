@@ -4,7 +4,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
-
+from conftest import relerr
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +52,27 @@ def test_failed_allocation_leaves_no_error_behind(gpu_lib):
                 CRMod(big.grid, big.survey, precision=PLAIN)
             assert ei.value.errnr == 94
             assert np.array_equal(m.forward(small.sigma)["volt"], v)
+
+
+def test_batch_whose_second_problem_does_not_fit(gpu_lib):
+    """The first problem's work on its two streams is over before its buffers
+    are given back: the call fails with 94, and problems that reuse the
+    memory at once get the voltages of a run alone."""
+    from test_gpu_substruct import _case
+    from titatest_gb300 import MIXED, CRMod
+    from titatest_gb300._lib import CRGPUError
+    from titatest_gb300.crmod import forward_sens_batch
+    one, two = _case(200, 50, 48), _case(260, 60, 64)
+    ms = [CRMod(s.grid, s.survey, precision=MIXED) for s in (one, two)]
+    need = ms[0].memory_need()
+    assert ms[1].memory_need() > 1.5 * need
+    with _Short(need + (256 << 20)):
+        with pytest.raises(CRGPUError) as ei:
+            forward_sens_batch(ms, [one.sigma, two.sigma], sens_mode=-1)
+        assert ei.value.errnr == 94
+        ms[0].close()
+        with CRMod(one.grid, one.survey, precision=MIXED) as m:
+            v = m.forward(one.sigma)["volt"]
+    ms[1].close()
+    with CRMod(one.grid, one.survey, precision=MIXED) as m:
+        assert relerr(v, m.forward(one.sigma)["volt"]) < 1e-12

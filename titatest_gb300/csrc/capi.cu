@@ -740,6 +740,22 @@ int sub_join(crgpu_ctx *c, int groups) {
     return 0;
 }
 
+// Problems whose groups are at work: joined by done(), or when the call returns
+// early (another problem's allocation failed).
+struct SubOpen {
+    std::vector<crgpu_ctx *> at;
+    int done() {
+        int e = 0;
+        for (crgpu_ctx *c : at) {
+            const int je = sub_join(c, sub_groups(c));
+            if (!e) e = je;
+        }
+        at.clear();
+        return e;
+    }
+    ~SubOpen() { done(); }
+};
+
 // the potentials of a refined job of the forward
 void sub_finish(const SubJob &j) {
     sub_launch_unpack(j.c->P, j.c->D, j.B, -1.0, j.c->d_kpot, j.c->d_kpot32, j.st);
@@ -781,15 +797,15 @@ int forward_sub(crgpu_ctx *c, float *t_factor, float *t_solve, std::vector<SubJo
                 jobs.push_back({c, B, nullptr, st, g, false});
                 if (!e) e = sub_solve_rect(jobs.back());
             }
-            if (e) break;
-            if (later) {
+            if (later && !e) {
                 later->insert(later->end(), jobs.begin(), jobs.end());
                 break;
             }
-            e = sub_refine(jobs);
+            if (!e) e = sub_refine(jobs);
             for (const SubJob &j : jobs)
                 if (!e) sub_finish(j);
-            if (!e) e = sub_join(c, groups);
+            const int je = sub_join(c, groups);  // after an error too: c->st frees and overwrites the buffers
+            if (!e) e = je;
             if (e) break;
             c->stats.nbatches++;
             if (cap) continue;
@@ -843,7 +859,8 @@ int adjoint_sub(crgpu_ctx *c) {
                 sub_launch_unpack(c->P, c->D, j.B, 1.0, c->d_lambda, nullptr, j.st);
                 c->stats.kernel_launches += 2;
             }
-            if (!e) e = sub_join(c, groups);
+            const int je = sub_join(c, groups);
+            if (!e) e = je;
             if (e) return e;
             const SubBatch B = sub_view(c, k0, kb, l0, lb);
             e = check_device_errors(c, B.status, B.Kb * B.Lb, k0);
@@ -1659,6 +1676,7 @@ int crgpu_forward_sens_batch(crgpu_ctx *const *ctxs, int32_t nprob, const double
     std::vector<DevBatch> hb(nprob);
     std::vector<int> order(nprob);
     std::vector<SubJob> jobs;
+    SubOpen open;
     for (int p = 0; p < nprob; p++) {  // assembly and right-hand sides, each on its stream
         crgpu_ctx *c = ctxs[p];
         const int ns = (int)c->sys_k.size();
@@ -1673,6 +1691,7 @@ int crgpu_forward_sens_batch(crgpu_ctx *const *ctxs, int32_t nprob, const double
             float t = 0.f;
             const int e = forward_sub(c, &t, &t, &jobs);
             if (e) return e;
+            open.at.push_back(c);
             c->stats.kernel_launches += 1;
             c->stats.nsystems = ns;
             continue;
@@ -1696,8 +1715,8 @@ int crgpu_forward_sens_batch(crgpu_ctx *const *ctxs, int32_t nprob, const double
         int e = sub_refine(jobs);
         if (e) return e;
         for (const SubJob &j : jobs) sub_finish(j);
-        for (int p = 0; p < nprob; p++)
-            if (sub_on(ctxs[p]) && (e = sub_join(ctxs[p], sub_groups(ctxs[p])))) return e;
+        e = open.done();
+        if (e) return e;
     }
     // the item table, longest systems first
     std::sort(order.begin(), order.end(), [&](int a, int b) { return ctxs[a]->hg.n > ctxs[b]->hg.n; });
