@@ -195,12 +195,13 @@ size_t bytes_per_system(const crgpu_ctx *c) {
 }
 
 int ensure_refine(crgpu_ctx *c) {
-    if (c->d_refine) return 0;
-    char *cnt = nullptr;  // [kRefineSlots][kRefineRow]
-    int e = dalloc(c, &cnt, kRefineSlots * kRefineRow * sizeof(RefineCount));
-    c->d_refine = cnt;
-    if (e) return e;
-    CUCHECK(c, g_words.take(&c->refine_left));
+    if (!c->d_refine) {
+        char *cnt = nullptr;  // [kRefineSlots][kRefineRow]
+        const int e = dalloc(c, &cnt, kRefineSlots * kRefineRow * sizeof(RefineCount));
+        c->d_refine = cnt;
+        if (e) return e;
+    }
+    if (!c->refine_left) CUCHECK(c, g_words.take(&c->refine_left));
     return 0;
 }
 
