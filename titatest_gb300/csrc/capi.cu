@@ -1391,7 +1391,7 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
             *out = c;
             return e;
         }
-        c->sub_fits = sub_fits({mixed, hg.n, hg.mb, sp.m, D.mp, sub_root_max(mixed), c->eanz, sp.c_factor, sp.c_apply});
+        c->sub_fits = sub_fits({mixed, hg.n, hg.mb, sp.m, D.mp, sub_root_max(mixed), c->eanz, c->K, sp.c_factor, sp.c_apply});
     }
     if (precision == CRGPU_MIXED && !mixed_window_supported(hg.mb + 1)) {
         c->last_error = "mixed precision supports band widths up to 207";

@@ -333,26 +333,68 @@ bool build_sub_plan(const HostGrid &hg, const Pattern &pat, const SubShape &shap
     return true;
 }
 
-// Long, shallow meshes have a narrow band and a large root, but the band
-// is eliminated column by column, so the root wins beyond equal counts.
-// Forwards, band -> this solver in ms (sub / band operations): complex64
-// 300x15 cells 9.4 -> 3.9 (6.7), 200x6 2.5 -> 1.4 (18), 500x12 13.8 -> 7.4
-// (22), 800x12 21.8 -> 19.7 (52), 1000x10 24 -> 41 (114), 8x4 0.41 -> 0.27
-// (7.2); complex128 300x15 77 -> 43 (2.4), 400x15 102 -> 82 (3.6), 300x8 37.5
-// -> 36.3 (9.1), 500x12 95 -> 141 (8.7), and the smallest, all latency, 8x4
-// 0.29 -> 0.35 (1.9), 12x5 0.39 -> 0.40, 16x6 0.52 -> 0.43.
+// The band is eliminated node by node, in mixed precision about as fast for 32
+// systems as for the 1248 that are resident at once (a latency of 1.6 us a node
+// up to the warp kernels' width, 2.35 with all of them at work); in complex128 an
+// SM takes one system at a time, beyond width 126 two.
+double band_us(const SubCost &q) {
+    const double n = q.n, mb = q.mb, systems = (double)q.K * q.eanz, base = 250.0;
+    if (!q.mixed) {
+        if (mb > 126) return base + n * std::max(1.0, systems / 304.0) * 1.4e-3 * mb * mb;
+        return base + n * std::ceil(systems / 152.0) * (2.6 + 0.02 * mb + 3.8e-4 * mb * mb);
+    }
+    const double full = systems / 1248.0;
+    if (mb <= 62) return base + n * std::max(1.0, full) * (1.6 + 0.75 * std::min(1.0, full));
+    return base + n * (1.6 + 2.5e-3 * systems * (mb / 100.0) * (mb <= 124 ? 1.0 : mb / 100.0));
+}
+
+// A root is one block's work, at 215 (complex64) and 6.5 (complex128) GFLOP/s; up
+// to five blocks share an SM, and more systems than SMs do not spread evenly:
+// the second group's blocks come to where the first one's shared elimination has
+// left room, the more so the longer a root takes.  The rest is the shared
+// elimination, the sweeps and residuals, and the chains of the root's solves.
+double sub_us(const SubCost &q) {
+    const double m = q.m, systems = (double)q.K * q.eanz, x = systems / 152.0, flop = 4.0 / 3.0 * m * m * m;
+    const double crowd = q.mixed ? std::min(2.3, std::max(1.3, m / 900.0)) : 1.7;
+    const double load = x <= 1.0 ? 1.0 : std::max(x, std::min(5.0, crowd * x));
+    const double shared = 8.0 * q.K * q.c_factor;
+    if (!q.mixed)
+        return 200.0 + flop / 6.5e3 * load + (shared + 8.0 * systems * q.c_apply) / 0.6e6 + 2e-3 * m * m;
+    return 200.0 + flop / 215e3 * std::max(1.0, 0.82 * load) + shared / 8e6 + 4.5e-4 * q.n * systems + 2.3e-3 * m * m +
+           1.5 * m;
+}
+
+// Long meshes have a narrow band and a large root.  By time, since the two run at
+// very different rates (per counted operation the band is 60 times slower at width
+// 12, 1.4 times at 62).  Forwards, band -> this solver in ms, columns x rows of
+// cells: complex64, 1248 systems 300x10 8.4 -> 4.8, 500x6 8.9 -> 10.8, 500x20 25.7
+// -> 13.9, 700x20 34.9 -> 28.2, 1000x20 50.0 -> 61.1, 2000x20 99 -> 369, 800x30 58.4
+// -> 41.1, 1000x30 73.1 -> 70.1, 1500x30 110 -> 182, 500x60 78.7 -> 26.7, 1250x60
+// 196 -> 139, 1500x60 235 -> 212, 2000x60 313 -> 448, 2000x100 1531 -> 516; 240
+// systems 1000x20 33.8 -> 18.7, 2000x20 67 -> 203, 1500x60 165 -> 112, 2000x60 220
+// -> 243, 2600x60 286 -> 486; 32 systems 2000x60 208 -> 77, 2000x20 63.3 -> 63.8;
+// complex128, 96 systems 200x10 7.2 -> 4.7, 400x10 14.2 -> 21.1, 300x20 25.0 ->
+// 13.2, 600x20 49.7 -> 63.9, 600x30 91 -> 69, 1000x30 151 -> 251, 1500x60 974 ->
+// 845, 2000x60 1298 -> 1819; 384 systems 300x20 69 -> 30, 600x20 137 -> 261, 500x30
+// 213 -> 182, 600x60 1145 -> 367.  Over these and 80 others the choice loses at most
+// 11 % where both were candidates; above 5 ms the band's estimate is 0.63 to 1.22 of
+// its time, this solver's 0.61 to 1.74, both mostly within a fifth.  Beyond the two
+// operation counts the gains are small and not measured over the whole range: those
+// keep the band, as do the smallest complex128 grids, all latency (8x4 cells 0.29 ->
+// 0.35 ms, 16x6 0.52 -> 0.43).
 bool sub_fits(const SubCost &q) {
     if (q.mp > q.root_max) return false;  // the root's vector stays in one block's shared memory
     const double n = q.n, mb = q.mb, m = q.m;
     const double band = 0.5 * n * mb * mb + 6.0 * n * mb;
     const double sub = m * m * m / 6.0 + 4.0 * q.c_apply + q.c_factor / q.eanz;
-    return q.mixed ? sub <= 30.0 * band : sub <= 5.0 * band && q.n >= 100;
+    if (sub > (q.mixed ? 30.0 : 5.0) * band || (!q.mixed && q.n < 100)) return false;
+    return sub_us(q) <= band_us(q);
 }
 
 }  // namespace crgpu
 
 // sub_fits by its numbers, for the tests (not part of the C ABI)
 extern "C" int crgpu_sub_fits(int32_t mixed, int32_t n, int32_t mb, int32_t m, int32_t mp, int32_t root_max, int32_t eanz,
-                              double c_factor, double c_apply) {
-    return crgpu::sub_fits({mixed != 0, n, mb, m, mp, root_max, eanz, c_factor, c_apply});
+                              int32_t K, double c_factor, double c_apply) {
+    return crgpu::sub_fits({mixed != 0, n, mb, m, mp, root_max, eanz, K, c_factor, c_apply});
 }

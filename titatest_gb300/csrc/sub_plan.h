@@ -75,12 +75,16 @@ bool build_sub_plan(const HostGrid &hg, const Pattern &pat, const SubShape &shap
 
 // A problem as the choice between the band and this solver sees it: nodes, band
 // width, nodes of the root, the same padded and the most that k_sub_root_solve
-// holds, electrodes, the plan's complex multiply-adds.
+// holds, electrodes, wavenumbers, the plan's complex multiply-adds.
 struct SubCost {
     bool mixed;
-    int n, mb, m, mp, root_max, eanz;
+    int n, mb, m, mp, root_max, eanz, K;
     double c_factor, c_apply;
 };
+// GB300 times of a forward in microseconds at the default refinement, as
+// sub_fits compares them
+double band_us(const SubCost &q);
+double sub_us(const SubCost &q);
 bool sub_fits(const SubCost &q);
 
 }  // namespace crgpu
