@@ -140,8 +140,11 @@ int crgpu_set_boundary_values(crgpu_ctx *ctx, int32_t rwdanz, const int32_t *rwd
  * ldc: 0 or 1. */
 int crgpu_set_dc(crgpu_ctx *ctx, int32_t ldc);
 
-/* Upper bound of device memory for the per-system factors and vectors; systems are
- * processed in batches that fit.  Default: 60% of free device memory. */
+/* Upper bound of device memory for the factors and vectors of the systems in
+ * work and, on the substructured solver, what a wavenumber's systems share;
+ * systems are processed in batches that fit, of one system at least.  Default:
+ * 60% of free device memory.  Where the device has less room than that, batches
+ * get smaller, and a problem whose shared part does not fit runs on the band. */
 int crgpu_set_memory_budget(crgpu_ctx *ctx, int64_t bytes);
 
 /* No counterpart in the reference.  Free and total memory of the current

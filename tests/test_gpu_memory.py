@@ -76,3 +76,74 @@ def test_batch_whose_second_problem_does_not_fit(gpu_lib):
     ms[1].close()
     with CRMod(one.grid, one.survey, precision=MIXED) as m:
         assert relerr(v, m.forward(one.sigma)["volt"]) < 1e-12
+
+
+class _Peak:
+    """Most bytes that the library's pool had handed out, beyond those at the
+    start of the block."""
+
+    def __enter__(self):
+        self.cu = C.CDLL("libcuda.so.1")
+        dev, self.pool = C.c_int(0), C.c_void_p()
+        assert self.cu.cuDeviceGet(C.byref(dev), 0) == 0
+        assert self.cu.cuDeviceGetDefaultMemPool(C.byref(self.pool), dev) == 0
+        zero = C.c_uint64(0)
+        assert self.cu.cuMemPoolSetAttribute(self.pool, 8, C.byref(zero)) == 0  # USED_MEM_HIGH
+        self.start = self._get(7)  # USED_MEM_CURRENT
+        return self
+
+    def _get(self, attr):
+        v = C.c_uint64(0)
+        assert self.cu.cuMemPoolGetAttribute(self.pool, attr, C.byref(v)) == 0
+        return v.value
+
+    def __exit__(self, *a):
+        self.bytes = self._get(8) - self.start
+
+
+@pytest.mark.parametrize("prec,tol", [(0, 1e-12), (1, 1e-10)])
+@pytest.mark.parametrize("share", [0.6, 0.3])
+def test_memory_budget_holds_the_shared_arrays_too(gpu_lib, prec, tol, share):
+    """Forward and adjoint within a share of what one batch takes: some of the
+    wavenumbers at a time, the results of one batch (tolerance: rounding in
+    complex128, the refinement's in mixed precision)."""
+    from test_gpu_substruct import _case
+    from titatest_gb300 import CRMod
+    s = _case(120, 40, 12)
+    kwn, kwnwi = np.geomspace(0.01, 2.0, 10), np.full(10, 0.1)
+    g = np.random.default_rng(2).normal(size=(s.survey.nanz, 2)) @ np.array([1.0, 1j])
+    with CRMod(s.grid, s.survey, kwn, kwnwi, precision=prec) as m:
+        whole = m.memory_need() - s.survey.nanz * s.grid.elanz * 16
+        v, a = m.forward(s.sigma)["volt"], m.adjoint(g)
+    with CRMod(s.grid, s.survey, kwn, kwnwi, precision=prec) as m:
+        m.set_memory_budget(int(share * whole))
+        with _Peak() as peak:
+            w = m.forward(s.sigma)["volt"]
+        assert m.stats()["nbatches"] > 1
+        b = m.adjoint(g)
+    assert peak.bytes <= share * whole + (1 << 20)  # small change: counters and roundings of the pool
+    assert relerr(w, v) < tol and relerr(b, a) < tol
+
+
+@pytest.mark.parametrize("leave", [0.7, 0.25, 0.05])
+def test_forward_where_memory_is_short(gpu_lib, leave):
+    """Less room than the default budget assumes: rectangles shrink until they
+    fit, and where not even one wavenumber's shared arrays do, the band takes
+    the problem in batches.  Same voltages and gradient."""
+    from test_gpu_substruct import _case
+    from titatest_gb300 import MIXED, CRMod
+    s = _case(900, 60, 8)
+    kwn, kwnwi = np.geomspace(0.01, 2.0, 6), np.full(6, 0.1)
+    g = np.random.default_rng(2).normal(size=(s.survey.nanz, 2)) @ np.array([1.0, 1j])
+    with CRMod(s.grid, s.survey, kwn, kwnwi, precision=MIXED) as m:
+        need = m.memory_need() - s.survey.nanz * s.grid.elanz * 16
+        v, a = m.forward(s.sigma)["volt"], m.adjoint(g)
+    with CRMod(s.grid, s.survey, kwn, kwnwi, precision=MIXED) as m:
+        m.forward(s.sigma)
+        m.adjoint(g)  # the gradient's own arrays are there
+        m.set_memory_budget(0)  # and the solver's are given back
+        with _Short(int(leave * need)):
+            w = m.forward(s.sigma)["volt"]
+            assert m.stats()["nbatches"] > 1
+            b = m.adjoint(g)
+    assert relerr(w, v) < 1e-10 and relerr(b, a) < 1e-9

@@ -124,17 +124,27 @@ void free_batch(crgpu_ctx *c) {
     if (!c->factors_sub) c->factors_resident = false;
 }
 
+void free_array(crgpu_ctx *c, void *p) {
+    if (!p) return;
+    cudaFreeAsync(p, c->st);
+    c->allocs.erase(std::remove(c->allocs.begin(), c->allocs.end(), p), c->allocs.end());
+}
+
 void free_sub_batch(crgpu_ctx *c) {
     drop_graph(c);
     SubBatch &B = c->SB;
-    void *ptrs[] = {B.C, B.Bt};  // C is the first of the batch's block
-    for (void *p : ptrs)
-        if (p) {
-            cudaFreeAsync(p, c->st);
-            c->allocs.erase(std::remove(c->allocs.begin(), c->allocs.end(), p), c->allocs.end());
-        }
+    free_array(c, B.C);  // the first of the batch's block
+    free_array(c, B.Bt);
     B = SubBatch{};
     c->sub_cap = 0;
+    if (c->factors_sub) c->factors_resident = false;
+}
+
+void free_sub_shared(crgpu_ctx *c) {
+    drop_graph(c);
+    free_array(c, c->D.F);  // the first of the block
+    c->D.F = c->D.G = c->D.H = c->D.S = c->D.R = nullptr;
+    c->sub_kcap = 0;
     if (c->factors_sub) c->factors_resident = false;
 }
 
@@ -442,30 +452,42 @@ size_t sub_bytes_per_system(const crgpu_ctx *c) {
            (size_t)c->D.szU * esz + (size_t)c->D.n_be * sizeof(double2) + 64;
 }
 
-size_t sub_bytes_shared(const crgpu_ctx *c) {
+// shared by a wavenumber's systems: the elimination's arrays
+size_t sub_bytes_wavenumber(const crgpu_ctx *c) {
     const DevSub &D = c->D;
     const size_t esz = c->precision == CRGPU_MIXED ? sizeof(float2) : sizeof(double2);
-    return c->K * (c->pat.nnz * sizeof(double2) + c->hg.n * sizeof(double) + sizeof(int) +
-                   (D.szF + 2 * D.szG + D.szS + (size_t)D.mp * D.ldc) * esz);
+    return (D.szF + 2 * D.szG + D.szS + (size_t)D.mp * D.ldc) * esz + 5 * 256;
 }
 
-// the shared factor's arrays
-int ensure_sub_shared(crgpu_ctx *c) {
-    if (c->sub_shared) return 0;
+// ... and of every wavenumber: the scaled matrix
+size_t sub_bytes_values(const crgpu_ctx *c) {
+    return c->K * (c->pat.nnz * sizeof(double2) + c->hg.n * sizeof(double) + sizeof(int)) + 3 * 256;
+}
+
+// the scaled matrices of all wavenumbers, and the elimination's arrays for kcap of them
+int ensure_sub_shared(crgpu_ctx *c, int kcap) {
     DevSub &D = c->D;
     const size_t K = c->K, esz = c->precision == CRGPU_MIXED ? sizeof(float2) : sizeof(double2);
+    if (!D.As) {
+        Block blk;
+        blk.room(&D.As, K * c->pat.nnz);
+        blk.room(&D.fk, K * c->hg.n);
+        blk.room(&D.kbad, K);
+        const int e = blk.make(c);
+        if (e) return e;
+    }
+    if (c->sub_kcap >= kcap) return 0;
+    free_sub_shared(c);
+    const size_t k = kcap;
     Block blk;
-    blk.room(&D.As, K * c->pat.nnz);
-    blk.room(&D.fk, K * c->hg.n);
-    blk.room(&D.kbad, K);
-    blk.room((char **)&D.F, K * D.szF * esz);
-    blk.room((char **)&D.G, K * D.szG * esz);
-    blk.room((char **)&D.H, K * D.szG * esz);
-    blk.room((char **)&D.S, K * D.szS * esz);
-    blk.room((char **)&D.R, K * D.mp * D.ldc * esz);
+    blk.room((char **)&D.F, k * D.szF * esz);
+    blk.room((char **)&D.G, k * D.szG * esz);
+    blk.room((char **)&D.H, k * D.szG * esz);
+    blk.room((char **)&D.S, k * D.szS * esz);
+    blk.room((char **)&D.R, k * D.mp * D.ldc * esz);
     const int e = blk.make(c);
     if (e) return e;
-    c->sub_shared = true;
+    c->sub_kcap = kcap;
     return 0;
 }
 
@@ -497,64 +519,87 @@ int ensure_sub_batch(crgpu_ctx *c, int want) {
     return 0;
 }
 
-// The rectangles of systems that one batch holds: whole wavenumbers, or some
-// of one wavenumber's electrodes where not even those fit the budget.
-void sub_rect(crgpu_ctx *c, int *kb, int *lb) {
-    const int nsys = (int)c->sys_k.size();
-    const size_t per = sub_bytes_per_system(c);
-    int64_t budget = c->mem_budget;
-    if (budget <= 0) {
-        size_t fr = 0, tot = 0;
-        cudaMemGetInfo(&fr, &tot);
-        budget = (int64_t)(0.6 * (double)(fr + (size_t)c->sub_cap * per));
-    }
-    int bs = (int)std::max<int64_t>(1, std::min<int64_t>(nsys, budget / (int64_t)per));
-    if (c->sub_cap >= nsys) bs = nsys;
-    *kb = bs >= c->eanz ? bs / c->eanz : 1;
-    *lb = bs >= c->eanz ? c->eanz : bs;
-}
-
-// D as seen from wavenumber k0
-DevSub sub_shift(const crgpu_ctx *c, int k0) {
-    DevSub D = c->D;
-    const size_t esz = c->precision == CRGPU_MIXED ? sizeof(float2) : sizeof(double2);
-    D.As += (size_t)k0 * c->pat.nnz;
-    D.fk += (size_t)k0 * c->hg.n;
-    D.kbad += k0;
-    D.F = (char *)D.F + (size_t)k0 * D.szF * esz;
-    D.G = (char *)D.G + (size_t)k0 * D.szG * esz;
-    D.H = (char *)D.H + (size_t)k0 * D.szG * esz;
-    D.S = (char *)D.S + (size_t)k0 * D.szS * esz;
-    D.R = (char *)D.R + (size_t)k0 * D.mp * D.ldc * esz;
-    return D;
-}
-
-// scaled area parts of every wavenumber
-int sub_values(crgpu_ctx *c) {
-    int e = ensure_sub_shared(c);
-    if (e) return e;
-    sub_launch_values(c->P, c->D, c->d_sigma, c->d_adom, c->st);
-    c->stats.kernel_launches += 2;
-    return 0;
-}
-
-// shared elimination of the wavenumbers k0 .. k0+kb-1
-void sub_factor_shared(crgpu_ctx *c, int k0, int kb, cudaStream_t st) {
-    c->stats.kernel_launches +=
-        sub_launch_factor(c->P, sub_shift(c, k0), c->sp, kb, c->precision == CRGPU_MIXED, st);
-}
-
-int sub_factor_rect(crgpu_ctx *c, const SubBatch &B, cudaStream_t st) {
-    CUCHECK(c, cudaMemsetAsync(B.status, 0, sizeof(int) * B.Kb * B.Lb, st));
-    sub_launch_root(c->P, c->D, B, c->d_sigma, c->precision == CRGPU_MIXED, st);
-    c->stats.kernel_launches += 2;
-    return 0;
-}
-
 // the right-hand sides of the adjoint are kept for the residuals
 int ensure_sub_rhs(crgpu_ctx *c) {
     if (c->precision != CRGPU_MIXED || c->SB.Bt) return 0;
     return dalloc(c, &c->SB.Bt, (size_t)c->sub_cap * c->hg.n);
+}
+
+// The rectangles of systems that one batch holds: whole wavenumbers with their
+// shared arrays, or some of one wavenumber's electrodes where not even those fit
+// the budget.
+void sub_rect(crgpu_ctx *c, int *kb, int *lb) {
+    const int nsys = (int)c->sys_k.size();
+    const int64_t per = (int64_t)sub_bytes_per_system(c), wave = (int64_t)sub_bytes_wavenumber(c);
+    int64_t budget = c->mem_budget;
+    if (budget <= 0) {
+        size_t fr = 0, tot = 0;
+        cudaMemGetInfo(&fr, &tot);
+        budget = (int64_t)(0.6 * (double)(fr + (size_t)c->sub_cap * per + (size_t)c->sub_kcap * wave +
+                                          (c->D.As ? sub_bytes_values(c) : 0)));
+    }
+    budget -= (int64_t)sub_bytes_values(c);
+    *kb = c->K;
+    *lb = c->eanz;
+    if ((c->sub_cap >= nsys && c->sub_kcap >= c->K) || c->K * wave + nsys * per <= budget) return;
+    *kb = (int)std::max<int64_t>(0, std::min<int64_t>(c->K, budget / (wave + c->eanz * per)));
+    if (*kb > 0) return;
+    *kb = 1;
+    *lb = (int)std::max<int64_t>(1, std::min<int64_t>(c->eanz, (budget - wave) / per));
+}
+
+// Rectangles and their buffers (rhs: the adjoint's), smaller ones where the
+// device has less room than the budget.  94: not even for one system; nothing is
+// queued, and the band takes over.
+int sub_reserve(crgpu_ctx *c, int *kb, int *lb, bool rhs) {
+    sub_rect(c, kb, lb);
+    for (;;) {
+        int e = ensure_sub_shared(c, *kb);
+        if (!e) e = ensure_sub_batch(c, *kb * *lb);
+        if (!e && rhs) e = ensure_sub_rhs(c);
+        if (e != 94) return e;
+        free_sub_batch(c);
+        free_sub_shared(c);
+        if (*kb == 1 && *lb == 1) return e;
+        if (*kb > 1) *kb = (*kb + 1) / 2;
+        else *lb = (*lb + 1) / 2;
+    }
+}
+
+// D whose elimination arrays begin with wavenumber w0, for kernels that count
+// wavenumbers from `first` on (0: as the grid does)
+DevSub sub_window(const crgpu_ctx *c, int w0, int first = 0) {
+    DevSub D = c->D;
+    const int64_t esz = c->precision == CRGPU_MIXED ? sizeof(float2) : sizeof(double2), k = first - w0;
+    auto move = [&](void *p, int64_t entries) { return (void *)((uintptr_t)p + (uintptr_t)(k * entries * esz)); };
+    D.As += (size_t)first * c->pat.nnz;
+    D.fk += (size_t)first * c->hg.n;
+    D.kbad += first;
+    D.F = move(D.F, D.szF);
+    D.G = move(D.G, D.szG);
+    D.H = move(D.H, D.szG);
+    D.S = move(D.S, D.szS);
+    D.R = move(D.R, (int64_t)D.mp * D.ldc);
+    return D;
+}
+
+// scaled area parts of every wavenumber
+void sub_values(crgpu_ctx *c) {
+    sub_launch_values(c->P, c->D, c->d_sigma, c->d_adom, c->st);
+    c->stats.kernel_launches += 2;
+}
+
+// shared elimination of the wavenumbers k0 .. k0+kb-1, arrays from w0 on
+void sub_factor_shared(crgpu_ctx *c, int k0, int kb, int w0, cudaStream_t st) {
+    c->stats.kernel_launches +=
+        sub_launch_factor(c->P, sub_window(c, w0, k0), c->sp, kb, c->precision == CRGPU_MIXED, st);
+}
+
+int sub_factor_rect(crgpu_ctx *c, const SubBatch &B, int w0, cudaStream_t st) {
+    CUCHECK(c, cudaMemsetAsync(B.status, 0, sizeof(int) * B.Kb * B.Lb, st));
+    sub_launch_root(c->P, sub_window(c, w0), B, c->d_sigma, c->precision == CRGPU_MIXED, st);
+    c->stats.kernel_launches += 2;
+    return 0;
 }
 
 // One rectangle's solve for the right-hand sides of kompab (src null) or for the
@@ -565,6 +610,7 @@ struct SubJob {
     const double2 *src;
     cudaStream_t st;
     int slot;
+    int w0;  // first wavenumber that the elimination's arrays hold
     bool done;
 };
 
@@ -575,7 +621,7 @@ int sub_solve_rect(SubJob &j) {
     SubBatch B0 = j.B;
     B0.kact = nullptr;
     sub_launch_rhs(c->P, c->D, j.B, mixed, c->lsink, c->nsink, j.src, j.st);
-    c->stats.kernel_launches += 1 + sub_launch_apply(c->D, c->sp, B0, mixed, j.src == nullptr, nullptr, j.st);
+    c->stats.kernel_launches += 1 + sub_launch_apply(sub_window(c, j.w0), c->sp, B0, mixed, j.src == nullptr, nullptr, j.st);
     j.done = !mixed;
     if (!mixed) return 0;
     RefineCount *cnt = (RefineCount *)c->d_refine + (size_t)j.slot * kRefineRow;
@@ -588,7 +634,7 @@ int sub_solve_rect(SubJob &j) {
 void sub_refine_step(const SubJob &j, const int *nprev, const SubStop &stop, cudaStream_t st) {
     crgpu_ctx *c = j.c;
     sub_launch_residual(c->P, c->D, j.B, j.src == nullptr, c->lsink, c->nsink, nprev, st);
-    c->stats.kernel_launches += 3 + sub_launch_apply(c->D, c->sp, j.B, true, false, nprev, st);
+    c->stats.kernel_launches += 3 + sub_launch_apply(sub_window(c, j.w0), c->sp, j.B, true, false, nprev, st);
     sub_launch_accumulate(c->D, j.B, false, c->refine_tol, nprev, stop, st);
 }
 
@@ -769,8 +815,8 @@ void sub_finish(const SubJob &j) {
 int forward_sub(crgpu_ctx *c, float *t_factor, float *t_solve, std::vector<SubJob> *later) {
     const bool cap = c->capturing || later;  // recorded or queued: one rectangle, no waiting
     int kb = c->K, lb = c->eanz;
-    if (!cap) sub_rect(c, &kb, &lb);
-    int e = ensure_sub_batch(c, kb * lb);
+    int e = cap ? ensure_sub_shared(c, kb) : sub_reserve(c, &kb, &lb, false);
+    if (!e && cap) e = ensure_sub_batch(c, kb * lb);
     if (e) return e;
     c->factors_sub = true;
     const bool one = kb == c->K && lb == c->eanz;
@@ -780,8 +826,7 @@ int forward_sub(crgpu_ctx *c, float *t_factor, float *t_solve, std::vector<SubJo
         for (auto &v : ev) cudaEventCreate(&v);
         cudaEventRecord(ev[0], c->st);
     }
-    e = sub_values(c);
-    if (!e && !one) sub_factor_shared(c, 0, c->K, c->st);
+    sub_values(c);
     float shared = 0.f;
     for (int k0 = 0; k0 < c->K && !e; k0 += kb)
         for (int l0 = 0; l0 < c->eanz && !e; l0 += lb) {
@@ -792,10 +837,10 @@ int forward_sub(crgpu_ctx *c, float *t_factor, float *t_solve, std::vector<SubJo
                 const int ka = one ? c->K * g / groups : k0, kn = one ? c->K * (g + 1) / groups - ka : kb;
                 const cudaStream_t st = g ? c->st_sub[g - 1] : c->st;
                 const SubBatch B = sub_view(c, ka, kn, l0, lb, one ? (size_t)ka * c->eanz : 0);
-                if (one) sub_factor_shared(c, ka, kn, st);
-                e = sub_factor_rect(c, B, st);
+                if (l0 == 0) sub_factor_shared(c, ka, B.Kb, k0, st);
+                e = sub_factor_rect(c, B, k0, st);
                 if (!cap && g == 0) cudaEventRecord(ev[2], c->st);
-                jobs.push_back({c, B, nullptr, st, g, false});
+                jobs.push_back({c, B, nullptr, st, g, k0, false});
                 if (!e) e = sub_solve_rect(jobs.back());
             }
             if (later && !e) {
@@ -828,18 +873,16 @@ int forward_sub(crgpu_ctx *c, float *t_factor, float *t_solve, std::vector<SubJo
 
 // lambda_(k,l) of run_adjoint
 int adjoint_sub(crgpu_ctx *c) {
-    const bool have = c->factors_resident && c->factors_sub;
+    // where the right-hand sides do not fit beside resident factors, smaller rectangles of both
+    const bool have = c->factors_resident && c->factors_sub && ensure_sub_rhs(c) == 0;
     int kb = c->K, lb = c->eanz, e = 0;
     if (!have) {
-        sub_rect(c, &kb, &lb);
-        e = ensure_sub_batch(c, kb * lb);
-        if (!e) e = sub_values(c);
+        e = sub_reserve(c, &kb, &lb, true);
         if (e) return e;
-        sub_factor_shared(c, 0, c->K, c->st);
         c->factors_sub = true;
+        c->factors_resident = false;
+        sub_values(c);
     }
-    e = ensure_sub_rhs(c);
-    if (e) return e;
     const bool one = kb == c->K && lb == c->eanz;
     const int groups = one ? sub_groups(c) : 1;
     for (int k0 = 0; k0 < c->K; k0 += kb)
@@ -850,8 +893,9 @@ int adjoint_sub(crgpu_ctx *c) {
                 const int ka = one ? c->K * g / groups : k0, kn = one ? c->K * (g + 1) / groups - ka : kb;
                 const cudaStream_t st = g ? c->st_sub[g - 1] : c->st;
                 const SubBatch B = sub_view(c, ka, kn, l0, lb, one ? (size_t)ka * c->eanz : 0);
-                if (!have) e = sub_factor_rect(c, B, st);
-                jobs.push_back({c, B, c->d_adjsrc, st, g, false});
+                if (!have && l0 == 0) sub_factor_shared(c, ka, B.Kb, k0, st);
+                if (!have) e = sub_factor_rect(c, B, k0, st);
+                jobs.push_back({c, B, c->d_adjsrc, st, g, k0, false});
                 if (!e) e = sub_solve_rect(jobs.back());
             }
             if (!e) e = sub_refine(jobs);
@@ -985,7 +1029,10 @@ int run_forward(crgpu_ctx *c, const double2 *d_sigma, int volt_mode, const doubl
     }
     c->stats.nsystems = (int)c->sys_k.size();
     float t_factor = 0.f, t_solve = 0.f;
-    int worst = sub_on(c) ? forward_sub(c, &t_factor, &t_solve, nullptr) : forward_band(c, d_sigma, &t_factor, &t_solve);
+    // recording: on the route that the ordinary run took
+    const bool sub = sub_on(c) && (!cap || c->factors_sub);
+    int worst = sub ? forward_sub(c, &t_factor, &t_solve, nullptr) : forward_band(c, d_sigma, &t_factor, &t_solve);
+    if (sub && worst == 94) worst = forward_band(c, d_sigma, &t_factor, &t_solve);
     if (worst) {
         for (auto &ev_ : ev) cudaEventDestroy(ev_);
         return worst;
@@ -1039,10 +1086,16 @@ int run_adjoint(crgpu_ctx *c, const double2 *d_g, double2 *d_grad) {
     const int nsys_total = (int)c->sys_k.size();
     const int nr = c->nrhs;
     int e = 0;
-    if (sub_on(c)) {
+    const bool band_resident = c->factors_resident && !c->factors_sub;
+    bool sub = sub_on(c) && !band_resident;
+    if (sub) {
         e = adjoint_sub(c);
-        if (e) return e;
-    } else if (c->factors_resident && !c->factors_sub) {
+        if (e && e != 94) return e;
+        sub = e == 0;
+    }
+    if (sub) {
+        // lambda is there
+    } else if (band_resident) {
         DevBatch B = batch_view(c, nsys_total);
         launch_adjoint_rhs(P, B, nr, c->d_adjsrc, c->st);
         e = solve_batch(c, nsys_total, false);
@@ -1052,7 +1105,7 @@ int run_adjoint(crgpu_ctx *c, const double2 *d_g, double2 *d_grad) {
         e = check_device_errors(c, B.status, nsys_total);
         if (e) return e;
     } else {
-        if (c->batch_cap == 0) e = ensure_batch(c, batch_size(c));
+        e = c->batch_cap == 0 ? ensure_batch(c, batch_size(c)) : 0;
         if (e) return e;
         const int bs = c->batch_cap;
         c->factors_sub = false;
@@ -1487,6 +1540,7 @@ int crgpu_set_memory_budget(crgpu_ctx *c, int64_t bytes) {
     c->mem_budget = bytes;
     free_batch(c);
     free_sub_batch(c);
+    free_sub_shared(c);
     return 0;
 }
 
@@ -1646,7 +1700,8 @@ int crgpu_memory_need(const crgpu_ctx *c, int64_t *bytes) {
     int64_t need = 0;
     if (sub_on(c)) {
         if (c->sub_cap < nsys) need += (int64_t)sub_bytes_per_system(c) * nsys;
-        if (!c->sub_shared) need += (int64_t)sub_bytes_shared(c);
+        if (c->sub_kcap < c->K) need += (int64_t)sub_bytes_wavenumber(c) * c->K;
+        if (!c->D.As) need += (int64_t)sub_bytes_values(c);
     } else if (c->batch_cap < nsys) {
         need += (int64_t)bytes_per_system(c) * nsys;
     }

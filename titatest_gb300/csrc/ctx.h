@@ -63,7 +63,7 @@ struct crgpu_ctx {
     crgpu::SubPlan sp;
     crgpu::DevSub D{};
     crgpu::SubBatch SB{};
-    bool sub_shared = false;   // D's numeric arrays are allocated
+    int sub_kcap = 0;          // wavenumbers that D's elimination arrays hold
     int sub_cap = 0;           // systems SB's buffers hold
     cudaStream_t st_body = nullptr;  // records a loop's body
     cudaStream_t st_sub[3] = {};  // further groups of wavenumbers beside st
