@@ -374,7 +374,8 @@ int crgpu_get_tune(const crgpu_ctx *ctx, int32_t *out);
 
 /* Sets the launch choices in the layout of crgpu_get_tune (a kernel that
  * cannot run this problem falls back to the default); blocks per SM 0..8.  A
- * factor kernel other than 0 pins the band path; 0 takes that back. */
+ * factor kernel other than 0 pins the band path; 0 takes that back; the one that
+ * crgpu_get_tune reports (the autotuner's, say) leaves the path as it is. */
 int crgpu_set_tune(crgpu_ctx *ctx, const int32_t *in);
 
 #ifdef __cplusplus

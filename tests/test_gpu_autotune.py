@@ -51,3 +51,27 @@ def test_autotune_wide_band_matches_plain(gpu_lib):
         assert t["factor"] == "SIMT shared-memory tiles" and t["factor_blocks_per_sm"] in (1, 2)
         vm = m.forward(sig)["volt"]
     assert relerr(vm, vp) < 1e-6
+
+
+def test_tune_read_and_given_back_keeps_the_solver(gpu_lib):
+    """crgpu_get_tune's values given to crgpu_set_tune change nothing, on a
+    context whose forwards do not run on the tuned band kernel; another choice
+    pins the band, and 0 takes that back (the buffers a forward still needs tell
+    which solver is next)."""
+    from titatest_gb300 import MIXED, CRMod, synth
+    s = synth.config1()
+    with CRMod(s.grid, s.survey, precision=MIXED) as m:
+        m.autotune(s.sigma, force=True)
+        v, need = m.forward(s.sigma)["volt"], m.memory_need()
+        t = m.tune()
+        kind = {"tensor cores": 1, "SIMT register tiles": 2, "SIMT shared-memory tiles": 3,
+                "SIMT warp per system": 4}[t["factor"]]
+        jac = {"default": 0, "tensor cores": 1, "SIMT": 2}[t["jacobian"]]
+        m.set_tune(kind, t["factor_blocks_per_sm"], jac)
+        assert m.memory_need() == need and m.tune() == t
+        assert np.array_equal(m.forward(s.sigma)["volt"], v)
+        m.set_tune(3 - kind if kind < 3 else 1, 0, jac)
+        assert m.memory_need() > need
+        assert relerr(m.forward(s.sigma)["volt"], v) < 1e-6
+        m.set_tune(0, 0, jac)
+        assert m.memory_need() == need

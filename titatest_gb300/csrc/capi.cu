@@ -2161,7 +2161,7 @@ int crgpu_autotune(crgpu_ctx *c, const double *sigma, int32_t flags) {
 int crgpu_set_tune(crgpu_ctx *c, const int32_t *in) {
     if (!c || !in || in[0] < 0 || in[0] > 4 || in[1] < 0 || in[1] > 8 || in[2] < 0 || in[2] > 2) return ERR_ARG;
     drop_graph(c);
-    c->band_pinned = in[0] != 0;
+    if (in[0] != c->P.tune_factor) c->band_pinned = in[0] != 0;  // a choice given back unchanged pins nothing
     c->P.tune_factor = in[0];
     c->P.tune_ctas = in[1];
     c->P.tune_sens = in[2];
