@@ -147,3 +147,18 @@ def test_forward_where_memory_is_short(gpu_lib, leave):
             assert m.stats()["nbatches"] > 1
             b = m.adjoint(g)
     assert relerr(w, v) < 1e-10 and relerr(b, a) < 1e-9
+
+
+def test_singularity_removal_keeps_no_elimination_plan(gpu_lib):
+    """Forwards with singularity removal run on the band, so such a context
+    has no tables of the dissection."""
+    from test_gpu_substruct import _case
+    from titatest_gb300 import PLAIN, CRMod
+    s = _case(120, 40, 12)
+    held = []
+    for lsr in (False, True):
+        with _Peak() as peak:
+            with CRMod(s.grid, s.survey, lsr=lsr, precision=PLAIN):
+                pass
+        held.append(peak.bytes)
+    assert held[1] < held[0] - 4 * s.grid.sanz  # one position a node at least

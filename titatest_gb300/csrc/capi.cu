@@ -1394,10 +1394,15 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
             c->sys_l.push_back(0);
         }
     }
+    if (precision == CRGPU_MIXED && !mixed_window_supported(hg.mb + 1)) {
+        c->last_error = "mixed precision supports band widths up to 207";
+        *out = c;
+        return ERR_UNSUPPORTED;
+    }
     Block tree;  // its host copy lives until the synchronisation below
     std::vector<int32_t> sources(enr0);
     if (c->nsink >= 0 && c->nsink < hg.n) sources.push_back(c->nsink);
-    if (c->nrhs == 1 && build_sub_plan(hg, c->pat, sub_shape(precision == CRGPU_MIXED), sources, c->sp)) {
+    if (c->nrhs == 1 && !c->lsr && build_sub_plan(hg, c->pat, sub_shape(precision == CRGPU_MIXED), sources, c->sp)) {
         const SubPlan &sp = c->sp;
         DevSub &D = c->D;
         D.n = sp.n;
@@ -1445,11 +1450,6 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
             return e;
         }
         c->sub_fits = sub_fits({mixed, hg.n, hg.mb, sp.m, D.mp, sub_root_max(mixed), c->eanz, c->K, sp.c_factor, sp.c_apply});
-    }
-    if (precision == CRGPU_MIXED && !mixed_window_supported(hg.mb + 1)) {
-        c->last_error = "mixed precision supports band widths up to 207";
-        *out = c;
-        return ERR_UNSUPPORTED;
     }
     int ce2 = check_device_errors(c, nullptr, 0);
     *out = c;
