@@ -44,3 +44,39 @@ def test_sensitivities_match_oracle(gpu_lib, ne, nanz, poles, tri):
             v = np.abs(volt)[:, None]
             assert relerr(m.bsens(), ref[0]) < tol
             assert relerr(m.bsensi() * v, ref[1] * v) < tol
+
+
+@pytest.mark.parametrize("ne,parts,poles", [(90, (1300, 1500, 2300), False), (70, (2100,), True), (90, (33, 4096), False)])
+def test_passes_with_and_without_tables_match_oracle(gpu_lib, ne, parts, poles):
+    """Surveys that repeat their dipoles in parts only: stretches of random
+    configurations (passes without tables) between stretches of 40 dipoles
+    (passes with tables), and lengths around a pass and a warp."""
+    from titatest_gb300 import MIXED, PLAIN, CRMod, formats
+    from test_gpu_substruct import _case
+    s = _case(100, 4, ne)
+    rng = np.random.default_rng(8)
+    st, vn = [], []
+    for q, n in enumerate(parts):
+        a, b = _survey(ne, n, poles, 5 + q)
+        if q % 2:
+            a, b = rng.choice(a[:40], n), rng.choice(b[:40], n)
+            same = {(x, y) for x, y in zip(a, b) if {x // 10000, x % 10000} & {y // 10000, y % 10000} - {0}}
+            keep = np.array([(x, y) not in same for x, y in zip(a, b)])  # no shared electrode
+            a, b = a[keep], b[keep]
+        st.append(a)
+        vn.append(b)
+    st, vn = np.concatenate(st).astype(np.int32), np.concatenate(vn).astype(np.int32)
+    sv = formats.Survey(enr=s.survey.enr, strnr=st, vnr=vn, strom=np.linspace(0.5, 2.0, len(st)))
+    P = O.Problem(s.grid, sv)
+    kwn, kwnwi = np.array([0.02, 0.1, 0.5]), np.array([0.1, 0.2, 0.3])
+    kp = P.forward(s.sigma, kwn, kwnwi)
+    volt, _ = P.bvolt(P.rtrafo(kp, kwnwi), 0, None)
+    ref = [P.bsens(kp, kwn, kwnwi, s.sigma, volt, mode=m) for m in (0, 1)]
+    v = np.abs(volt)[:, None]
+    for prec, tol in ((PLAIN, 1e-10), (MIXED, 1e-5)):
+        with CRMod(s.grid, sv, kwn, kwnwi, precision=prec) as m:
+            if prec == MIXED:
+                m.set_tune(0, 0, 2)  # the direct form
+            m.forward(s.sigma)
+            assert relerr(m.bsens(), ref[0]) < tol
+            assert relerr(m.bsensi() * v, ref[1] * v) < tol

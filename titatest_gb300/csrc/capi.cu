@@ -1316,9 +1316,11 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
     blk.put(&P.strom, strom);
     {
         SensPlan sn;
-        host_sens_passes(meas, c->nanz, c->eanz, sn);
+        host_sens_passes(meas, c->nanz, c->eanz, mixed, sn);
         P.nspass = (int)sn.pass.size();
+        P.nsdirect = (int)sn.direct.size();
         P.sens_dips = sn.most;
+        sn.pass.insert(sn.pass.end(), sn.direct.begin(), sn.direct.end());
         blk.put(&P.dip, sn.dip);
         blk.put(&P.mdip, sn.slot);
         blk.put(&P.spass, sn.pass);

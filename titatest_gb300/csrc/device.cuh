@@ -50,7 +50,7 @@ struct DevProblem {
     const int2 *dip;
     const int4 *mdip;
     const SensPass *spass;
-    int nspass, sens_dips;  // passes; most dipoles of one
+    int nspass, nsdirect, sens_dips;  // passes with tables, then those without; most dipoles of one
     double2 *sfac;
     const double *kwn, *kwnwi;
     // element matrices (src/precal.f90)

@@ -83,10 +83,11 @@ void launch_sens_tc(const DevProblem &P, const float2 *kpot32, double2 *sens, cu
 struct SensPlan {
     std::vector<int2> dip;
     std::vector<int4> slot;
-    std::vector<SensPass> pass;
+    std::vector<SensPass> pass, direct;
     int most = 0;
 };
-void host_sens_passes(const std::vector<int32_t> &meas, int nanz, int eanz, SensPlan &sp);
+// single: for the complex64 contraction
+void host_sens_passes(const std::vector<int32_t> &meas, int nanz, int eanz, bool single, SensPlan &sp);
 // single: the complex64 contraction from kpot32 (mixed precision); else the
 // complex128 one from kpot
 void launch_bsens(const DevProblem &P, const double2 *kpot, const float2 *kpot32, const double2 *sigma,

@@ -120,7 +120,17 @@ constexpr int kSensDip2 = 512;  // ... of its second table (256: 5.15 ms in comp
 // pass uses at least twice go into a second table (their differences alone);
 // measurements with one of those come first.  meas: e1..e4 per measurement (-1:
 // none, which becomes the zero entry eanz).
-void host_sens_passes(const std::vector<int32_t> &meas, int nanz, int eanz, SensPlan &sp) {
+//
+// Without tables where the survey hardly repeats its dipoles: a table then has an
+// entry nearly for every measurement, and its capacity cuts the pass, which
+// stages the same potentials again.  Random four-electrode surveys of 4000
+// measurements, bsensi in ms, tables -> none (measurements a dipole of a full
+// table): complex64, 3000 cells, 40 electrodes 2.64 -> 2.72 (1.6), 50 2.98 -> 2.81 (1.3),
+// 64 3.33 -> 3.08 (1.15); 5400 cells, 150 electrodes 12.0 -> 6.6 (1.02), and a pass that is
+// not cut 2.82 -> 2.01 (1000 measurements).  complex128 is bound by its operations,
+// which tables save from the first repetition on: 64 electrodes 20.0 -> 21.4, 110 46.4
+// -> 42.6, 150 47.2 -> 42.9, not cut 10.4 -> 11.8.
+void host_sens_passes(const std::vector<int32_t> &meas, int nanz, int eanz, bool single, SensPlan &sp) {
     auto el = [&](int i, int q) { return meas[(size_t)i * 4 + q] < 0 ? eanz : meas[(size_t)i * 4 + q]; };
     sp.slot.resize(nanz);
     for (int i0 = 0; i0 < nanz;) {
@@ -145,6 +155,16 @@ void host_sens_passes(const std::vector<int32_t> &meas, int nanz, int eanz, Sens
         }
         const int t = end[1] > end[0] || (end[1] == end[0] && list[1].size() <= list[0].size()) ? 1 : 0, o = 1 - t;
         const int n = end[t] - i0;
+        const bool cut = end[t] < nanz && n < kSensThreads * kSensMPT;
+        const double repeat = single ? 1.5 : cut ? 1.12 : 0.0;
+        if (n < repeat * (double)list[t].size()) {  // without tables, in the survey's order
+            for (int i = i0; i < end[t]; i++) sp.slot[i] = make_int4(el(i, 0), el(i, 1), el(i, 2), el(i, 3));
+            SensPass *last = sp.direct.empty() ? nullptr : &sp.direct.back();
+            if (last && last->i1 == i0 && end[t] - last->i0 <= kSensThreads * kSensMPT) last->i1 = end[t];
+            else sp.direct.push_back({i0, i0, end[t], 0, 0, 0});
+            i0 = end[t];
+            continue;
+        }
         // the other side: uses of a dipole, then the second table
         std::unordered_map<int64_t, int> uses;
         auto key = [&](int i) { return (int64_t)el(i, 2 * o) * (eanz + 1) + el(i, 2 * o + 1); };
@@ -260,6 +280,25 @@ struct SensT<float> {
 __device__ __forceinline__ double2 to_double(double2 v) { return v; }
 __device__ __forceinline__ double2 to_double(float2 v) { return widen(v); }
 
+// the potentials of wavenumber k at an element's nodes, all electrodes, to dst [NK][eanz + 1]
+template <typename R, int NK>
+__device__ __forceinline__ void sens_stage(const DevProblem &P, const typename SensT<R>::C *__restrict__ kpot,
+                                           const int (&nodes)[NK], int k, typename SensT<R>::S *dst) {
+    const size_t plane = (size_t)P.K * P.eanz * P.n;
+    for (int t = threadIdx.x; t < NK * P.eanz; t += kSensThreads) {
+        const int q = t / P.eanz, l = t - q * P.eanz;
+        const auto *src = kpot + ((size_t)k * P.eanz + l) * P.n + nodes[q];
+        char *to = (char *)(dst + q * (P.eanz + 1) + l);
+        if constexpr (sizeof(R) == 8) {
+            cp_async16(to, src);
+        } else {
+            cp_async8(to, src);
+            cp_async8(to + 8, src + plane);
+        }
+    }
+    cp_commit();
+}
+
 // MODE 0: src/bsens.f90, MODE 1: src/bsensi.f90.  R: arithmetic type of the
 // element contraction (double: the reference arithmetic, from kpot; float: the
 // mixed mode, from its complex64 planes, with FP64 output).
@@ -279,24 +318,12 @@ __device__ __forceinline__ void sens_element(const DevProblem &P, const typename
     R *ks = (R *)smem;                           // [2][NM], complex128
     S *kp = (S *)(smem + (kOwnSum ? 0 : kSensK));  // [2][NK][E1], the last entry of a row an absent electrode's zero
     C *tab = (C *)(kp + 2 * NK * E1);  // [NK][dipoles of the pass], then [NK][those of its second table]
-    const size_t plane = (size_t)P.K * eanz * P.n;
     int nodes[NK];
 #pragma unroll
     for (int q = 0; q < NK; q++) nodes[q] = P.enodes[e * 4 + q];
     if (tid < 2 * NK) kp[tid * E1 + eanz] = T::none();
     auto fetch = [&](int k, int buf) {
-        for (int t = tid; t < NK * eanz; t += kSensThreads) {
-            const int q = t / eanz, l = t - q * eanz;
-            const C *src = kpot + ((size_t)k * eanz + l) * P.n + nodes[q];
-            S *dst = kp + (buf * NK + q) * E1 + l;
-            if constexpr (sizeof(R) == 8) {
-                cp_async16(dst, src);
-            } else {
-                cp_async8(dst, src);
-                cp_async8((char *)dst + 8, src + plane);
-            }
-        }
-        cp_commit();
+        sens_stage<R, NK>(P, kpot, nodes, k, kp + buf * NK * E1);
         if (!kOwnSum && tid < NM)  // w_k K_k by one warp: 6.10 -> 5.81 ms against every thread forming it
             ks[buf * NM + tid] = (R)P.elbg[((size_t)k * P.elanz + e) * 10 + tid] * (P.swrtr ? (R)P.kwnwi[k] : (R)1);
     };
@@ -351,7 +378,7 @@ __device__ __forceinline__ void sens_element(const DevProblem &P, const typename
 #pragma unroll
             for (int m0 = 0; m0 < kSensMPT; m0 += kSensGroup) {
                 const int f = i0 + m0 * kSensThreads;  // the group's first slot
-                if (f >= i1) break;
+                if (f + (tid & ~31) >= i1) break;  // the warp has no more
                 int4 md[kSensGroup];
 #pragma unroll
                 for (int h = 0; h < kSensGroup; h++) {
@@ -399,6 +426,100 @@ __device__ __forceinline__ void sens_element(const DevProblem &P, const typename
     }
 }
 
+// The passes without tables: both differences and the product with K of every
+// measurement on its own, rows of J in the survey's order.
+template <int MODE, typename R, int NK>
+__device__ __forceinline__ void sens_direct(const DevProblem &P, const typename SensT<R>::C *__restrict__ kpot,
+                                            const double2 *__restrict__ sigma, double2 *__restrict__ sens, int e,
+                                            unsigned char *smem) {
+    using T = SensT<R>;
+    using C = typename T::C;
+    using S = typename T::S;
+    constexpr bool kOwnSum = sizeof(R) == 4;  // as in sens_element
+    constexpr int NM = NK * (NK + 1) / 2;
+    const int E1 = P.eanz + 1, tid = threadIdx.x;
+    R *ks = (R *)smem;                             // [2][NM], complex128: w_k K_k
+    S *kp = (S *)(smem + (kOwnSum ? 0 : kSensK));  // [2][NK][E1]
+    int nodes[NK];
+#pragma unroll
+    for (int q = 0; q < NK; q++) nodes[q] = P.enodes[e * 4 + q];
+    if (tid < 2 * NK) kp[tid * E1 + P.eanz] = T::none();
+    auto fetch = [&](int k, int buf) {
+        sens_stage<R, NK>(P, kpot, nodes, k, kp + buf * NK * E1);
+        if (!kOwnSum && tid < NM)
+            ks[buf * NM + tid] = (R)P.elbg[((size_t)k * P.elanz + e) * 10 + tid] * (P.swrtr ? (R)P.kwnwi[k] : (R)1);
+    };
+    const double2 sg = sigma[e];
+    for (int ps = P.nspass; ps < P.nspass + P.nsdirect; ps++) {
+        const int i0 = P.spass[ps].i0, i1 = P.spass[ps].i1;
+        C acc[kSensMPT];
+#pragma unroll
+        for (int m = 0; m < kSensMPT; m++) acc[m] = T::mk(0, 0);
+        __syncthreads();
+        fetch(0, 0);
+        for (int k = 0; k < P.K; k++) {
+            const S *u = kp + (k & 1) * NK * E1;
+            R kel[NM];
+            const R w = P.swrtr ? (R)P.kwnwi[k] : (R)1;
+            if (kOwnSum)
+#pragma unroll
+                for (int q = 0; q < NM; q++) kel[q] = (R)P.elbg[((size_t)k * P.elanz + e) * 10 + q];
+            cp_wait<0>();
+            __syncthreads();
+            if (!kOwnSum)
+#pragma unroll
+                for (int q = 0; q < NM; q++) kel[q] = ks[(k & 1) * NM + q];
+            if (k + 1 < P.K) fetch(k + 1, (k + 1) & 1);
+#pragma unroll
+            for (int m = 0; m < kSensMPT; m++) {
+                const int f = i0 + m * kSensThreads;
+                if (f + (tid & ~31) >= i1) break;  // the warp has no more
+                const int4 el = P.mdip[min(f + tid, i1 - 1)];
+                C a[NK], own = T::mk(0, 0), &s = kOwnSum ? own : acc[m];
+#pragma unroll
+                for (int q = 0; q < NK; q++) a[q] = T::diff(u[q * E1 + el.x], u[q * E1 + el.y]);
+#pragma unroll
+                for (int mi = 0; mi < NK; mi++) {
+                    C b = T::mk(0, 0);
+#pragma unroll
+                    for (int mj = 0; mj < NK; mj++) {
+                        const int hi = mi > mj ? mi : mj, lo = mi < mj ? mi : mj;
+                        const R kk = kel[hi * (hi + 1) / 2 + lo];
+                        b.x = fma(kk, a[mj].x, b.x);
+                        b.y = fma(kk, a[mj].y, b.y);
+                    }
+                    const C v = T::diff(u[mi * E1 + el.z], u[mi * E1 + el.w]);
+                    s.x = fma(v.x, b.x, s.x);
+                    s.x = fma(-v.y, b.y, s.x);
+                    s.y = fma(v.x, b.y, s.y);
+                    s.y = fma(v.y, b.x, s.y);
+                }
+                if (kOwnSum) {
+                    acc[m].x = fma(w, own.x, acc[m].x);
+                    acc[m].y = fma(w, own.y, acc[m].y);
+                }
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < kSensMPT; m++) {
+            const int i = i0 + m * kSensThreads + tid;
+            if (i >= i1) continue;
+            const double2 d = to_double(acc[m]), f = P.sfac[i];
+            sens[(size_t)e * P.nanz + i] = MODE == 0 ? cz(d.x * f.x, d.y * f.x) : cmul(d, cmul(sg, f));
+        }
+    }
+}
+
+template <int MODE, typename R>
+__global__ __launch_bounds__(kSensThreads, sizeof(R) == 4 ? 4 : 1) void k_bsens_direct(
+    DevProblem P, const typename SensT<R>::C *__restrict__ kpot, const double2 *__restrict__ sigma,
+    double2 *__restrict__ sens, int e_first) {
+    extern __shared__ __align__(16) unsigned char kp_raw[];
+    const int e = e_first + blockIdx.x;
+    if (P.etype[e] == 3) sens_direct<MODE, R, 3>(P, kpot, sigma, sens, e, kp_raw);
+    else sens_direct<MODE, R, 4>(P, kpot, sigma, sens, e, kp_raw);
+}
+
 template <int MODE, typename R>
 __global__ __launch_bounds__(kSensThreads, sizeof(R) == 4 ? 4 : 2) void k_bsens(DevProblem P,
                                                         const typename SensT<R>::C *__restrict__ kpot,
@@ -410,10 +531,10 @@ __global__ __launch_bounds__(kSensThreads, sizeof(R) == 4 ? 4 : 2) void k_bsens(
     else sens_element<MODE, R, 4>(P, kpot, sigma, sens, e, kp_raw);
 }
 
-// the block's shared memory (both element types)
-static size_t sens_smem(const DevProblem &P, bool single) {
+// the block's shared memory (both element types) with tables of dips dipoles
+static size_t sens_smem(const DevProblem &P, bool single, int dips) {
     const size_t c = single ? sizeof(float2) : sizeof(double2);
-    return (single ? 0 : kSensK) + 2 * 4 * (size_t)(P.eanz + 1) * 16 + 4 * (size_t)P.sens_dips * c;
+    return (single ? 0 : kSensK) + 2 * 4 * (size_t)(P.eanz + 1) * 16 + 4 * (size_t)dips * c;
 }
 
 void launch_bsens(const DevProblem &P, const double2 *kpot, const float2 *kpot32, const double2 *sigma,
@@ -431,17 +552,23 @@ void launch_bsens(const DevProblem &P, const double2 *kpot, const float2 *kpot32
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         for (const void *f : {(const void *)k_bsens<0, float>, (const void *)k_bsens<1, float>,
-                              (const void *)k_bsens<0, double>, (const void *)k_bsens<1, double>})
+                              (const void *)k_bsens<0, double>, (const void *)k_bsens<1, double>,
+                              (const void *)k_bsens_direct<0, float>, (const void *)k_bsens_direct<1, float>,
+                              (const void *)k_bsens_direct<0, double>, (const void *)k_bsens_direct<1, double>})
             cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
     });
     if (P.nanz > 0) k_sens_factor<<<(P.nanz + 127) / 128, 128, 0, st>>>(P, volt, mode);
-    const size_t smem = sens_smem(P, single);
+    const size_t smem = sens_smem(P, single, P.sens_dips), direct_smem = sens_smem(P, single, 0);
+    auto run = [&](auto table, auto direct, const auto *pot) {
+        if (P.nspass) table<<<e_count, kSensThreads, smem, st>>>(P, pot, sigma, sens, e_first);
+        if (P.nsdirect) direct<<<e_count, kSensThreads, direct_smem, st>>>(P, pot, sigma, sens, e_first);
+    };
     if (single) {
-        if (mode == 0) k_bsens<0, float><<<e_count, kSensThreads, smem, st>>>(P, kpot32, sigma, sens, e_first);
-        else k_bsens<1, float><<<e_count, kSensThreads, smem, st>>>(P, kpot32, sigma, sens, e_first);
+        if (mode == 0) run(k_bsens<0, float>, k_bsens_direct<0, float>, kpot32);
+        else run(k_bsens<1, float>, k_bsens_direct<1, float>, kpot32);
     } else {
-        if (mode == 0) k_bsens<0, double><<<e_count, kSensThreads, smem, st>>>(P, kpot, sigma, sens, e_first);
-        else k_bsens<1, double><<<e_count, kSensThreads, smem, st>>>(P, kpot, sigma, sens, e_first);
+        if (mode == 0) run(k_bsens<0, double>, k_bsens_direct<0, double>, kpot);
+        else run(k_bsens<1, double>, k_bsens_direct<1, double>, kpot);
     }
 }
 
