@@ -80,3 +80,37 @@ def test_passes_with_and_without_tables_match_oracle(gpu_lib, ne, parts, poles):
             m.forward(s.sigma)
             assert relerr(m.bsens(), ref[0]) < tol
             assert relerr(m.bsensi() * v, ref[1] * v) < tol
+
+
+def test_jacobian_to_pinned_memory_leaves_the_updates_jacobian(gpu_lib):
+    """CRMod's Jacobian into page-locked memory, in chunks of a buffer beside the
+    device array: the bits of the pageable one, and crgpu_update still reads the
+    Jacobian of log V that the device holds."""
+    import ctypes as C
+
+    import torch
+
+    from titatest_gb300 import MIXED, CRMod
+    from test_gpu_substruct import _case
+    s = _case(200, 30, 150)
+    nanz, manz = s.survey.nanz, s.grid.elanz
+    assert nanz * manz * 16 > 3 * (4 << 20)  # several chunks
+    with CRMod(s.grid, s.survey, precision=MIXED) as m:
+        m.set_tune(0, 0, 2)  # the direct form, with tables
+        v = m.forward(s.sigma)["volt"]
+        ref = m.bsens()
+        reg = np.zeros((3, manz))  # smatm(manz, 3), column-major
+        reg[0] = 1.0
+
+        def update():
+            return m.update(np.ones(nanz), np.ones(nanz, np.int32), -np.log(v) * 1.01, -np.log(v), 0,
+                            reg, nx=200, lam=300.0, ncgmax=5)
+
+        m.bsensi()
+        before = update()
+        host = torch.zeros(2 * nanz * manz, dtype=torch.float64).pin_memory()
+        assert gpu_lib.crgpu_sens(m._h, 0, C.cast(host.data_ptr(), C.POINTER(C.c_double))) == 0
+        got = host.numpy().view(np.complex128).reshape(manz, nanz).T
+        assert np.array_equal(got, ref)
+        for x, y in zip(before, update()):
+            assert np.array_equal(np.asarray(x), np.asarray(y))

@@ -1870,10 +1870,27 @@ int crgpu_sens(crgpu_ctx *c, int32_t mode, double *sens) {
     }
     // CRMod sensitivities into pinned (page-locked) host memory are written by
     // the kernel itself, over the host link, while it computes; otherwise
-    // chunked copies of the device array (which crgpu_update reads for mode 1)
+    // chunked copies of the device array (which crgpu_update reads for mode 1).
+    // The complex64 kernel with tables writes a row of J here and a row there (its
+    // measurements are ordered for shared memory), which the link takes at half its
+    // rate: there chunks of a buffer beside the device array, which stays as it is.
+    // 4800 cells x 2780 written by the kernel 2.65 ms, in chunks 1.65; 5720 data 4.57, 2.86.
     cudaPointerAttributes pa{};
-    if (mode == 0 && cudaPointerGetAttributes(&pa, sens) == cudaSuccess && pa.type == cudaMemoryTypeHost &&
-        pa.devicePointer) {
+    const bool pinned = mode == 0 && cudaPointerGetAttributes(&pa, sens) == cudaSuccess &&
+                        pa.type == cudaMemoryTypeHost && pa.devicePointer;
+    const bool scattered = c->precision == CRGPU_MIXED && c->P.nspass > 0 &&
+                           !(sens_tc_supported(c->P, mode) && c->P.tune_sens != 2);
+    // chunks of at least 4 MB: a Jacobian of a few MB is one launch and one copy (a
+    // chunk of fewer elements than the GPU has SMs still takes a whole element's time)
+    constexpr int kChunks = 8;
+    const int chunks = (int)std::min<size_t>(kChunks, std::max<size_t>(1, cnt * sizeof(double2) >> 22));
+    const int per = (int)((manz + chunks - 1) / chunks);
+    double2 *ring = nullptr;  // two chunks
+    if (pinned && scattered &&
+        cudaMallocAsync((void **)&ring, sizeof(double2) * 2 * per * nanz, c->st) != cudaSuccess)
+        ring = nullptr;
+    if (pinned && !ring) {
+        cudaGetLastError();
         cudaEvent_t a, b;
         cudaEventCreate(&a);
         cudaEventCreate(&b);
@@ -1893,27 +1910,25 @@ int crgpu_sens(crgpu_ctx *c, int32_t mode, double *sens) {
     }
     cudaGetLastError();  // a pageable pointer is not an error
     if (!c->copy_st) CUCHECK(c, cudaStreamCreateWithFlags(&c->copy_st, cudaStreamNonBlocking));
-    constexpr int kChunks = 8;
-    cudaEvent_t a, b, done[kChunks];
+    cudaEvent_t a, b, done[kChunks], copied[kChunks];
     cudaEventCreate(&a);
     cudaEventCreate(&b);
     for (auto &d : done) cudaEventCreateWithFlags(&d, cudaEventDisableTiming);
+    for (auto &d : copied) cudaEventCreateWithFlags(&d, cudaEventDisableTiming);
     cudaEventRecord(a, c->st);
-    // chunks of at least 4 MB: a Jacobian of a few MB is one launch and one copy (a
-    // chunk of fewer elements than the GPU has SMs still takes a whole element's time)
-    const int chunks = (int)std::min<size_t>(kChunks, std::max<size_t>(1, cnt * sizeof(double2) >> 22));
-    const int per = (int)((manz + chunks - 1) / chunks);
     for (int q = 0; q < chunks; q++) {
         const int e0 = q * per, ne = std::min<int>(per, (int)manz - e0);
         if (ne <= 0) break;
+        double2 *at = ring ? ring + (size_t)(q & 1) * per * nanz : c->d_sens + (size_t)e0 * nanz;
+        if (ring && q > 1) CUCHECK(c, cudaStreamWaitEvent(c->st, copied[q - 2], 0));
         launch_bsens(c->P, c->d_kpot, c->d_kpot32, c->d_sigma, c->d_volt, mode, c->precision == CRGPU_MIXED,
-                     c->d_sens, c->st, e0,
-                     ne);
+                     at - (size_t)e0 * nanz, c->st, e0, ne);
         c->stats.kernel_launches += 1;
         CUCHECK(c, cudaEventRecord(done[q], c->st));
         CUCHECK(c, cudaStreamWaitEvent(c->copy_st, done[q], 0));
-        CUCHECK(c, cudaMemcpyAsync(sens + 2 * (size_t)e0 * nanz, c->d_sens + (size_t)e0 * nanz,
-                                   (size_t)ne * nanz * sizeof(double2), cudaMemcpyDeviceToHost, c->copy_st));
+        CUCHECK(c, cudaMemcpyAsync(sens + 2 * (size_t)e0 * nanz, at, (size_t)ne * nanz * sizeof(double2),
+                                   cudaMemcpyDeviceToHost, c->copy_st));
+        CUCHECK(c, cudaEventRecord(copied[q], c->copy_st));
     }
     cudaEventRecord(b, c->st);
     CUCHECK(c, cudaStreamSynchronize(c->copy_st));
@@ -1924,7 +1939,9 @@ int crgpu_sens(crgpu_ctx *c, int32_t mode, double *sens) {
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     for (auto &d : done) cudaEventDestroy(d);
-    c->last_sens = c->d_sens;
+    for (auto &d : copied) cudaEventDestroy(d);
+    if (ring) cudaFreeAsync(ring, c->st);
+    else c->last_sens = c->d_sens;
     CUCHECK(c, cudaGetLastError());
     return 0;
 }
