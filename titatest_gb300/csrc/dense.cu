@@ -36,7 +36,7 @@ __device__ __forceinline__ double opnd(const double *__restrict__ A, int ld, int
 // lower), kDepthFromCol at the block column's (B(j, k) is 0 for k < j),
 // kDepthToCol ends with it (0 for k > j).  sq: instead of storing C, store the
 // sums over each tile's rows of the squared entries and of the entries times
-// D(i, j), sq[(2 bi) * N + j] and sq[(2 bi + 1) * N + j] (the diagonals of G^T G
+// D(i, j) (leading dimension ldc), sq[(2 bi) * N + j] and sq[(2 bi + 1) * N + j] (the diagonals of G^T G
 // and G^T D).
 enum { kDepthAll = 0, kDepthLower, kDepthFromCol, kDepthToCol };
 
@@ -97,7 +97,7 @@ __global__ __launch_bounds__(kGT) void k_gemm(int M, int N, int K, double alpha,
                 const int i = i0 + ty + 16 * a;
                 if (i >= M) continue;
                 s = fma(acc[a][b], acc[a][b], s);
-                if (D && j < N) t = fma(acc[a][b], D[(size_t)j * M + i], t);
+                if (D && j < N) t = fma(acc[a][b], D[(size_t)j * ldc + i], t);
             }
             red[0][ty][tx + 16 * b] = s;
             red[1][ty][tx + 16 * b] = t;
@@ -307,12 +307,12 @@ __global__ __launch_bounds__(256) void k_lower_col_sq(int n, const double *__res
     }
 }
 
-// the sums over the row blocks of sq (nblk x 2 x n), in block order
+// d2 and dd += the sums over the row blocks of sq (nblk x 2 x n), in block order
 __global__ void k_sum_blocks(int nblk, int n, const double *__restrict__ sq, double *__restrict__ d2,
                              double *__restrict__ dd) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
-    double s = 0.0, t = 0.0;
+    double s = d2[j], t = dd[j];
     for (int b = 0; b < nblk; b++) {
         s += sq[(size_t)(2 * b) * n + j];
         t += sq[(size_t)(2 * b + 1) * n + j];
@@ -390,13 +390,27 @@ void dense_lower_col_sq(int n, const double *Y, double *d, cudaStream_t st) {
     if (n > 0) k_lower_col_sq<<<n, 256, 0, st>>>(n, Y, d);
 }
 
+int dense_product_rows(int m, int n) {
+    // whole where T takes 32 MB at most or no more than a matrix of n x n; at least a tile
+    const int rows = std::max(n, (4 << 20) / std::max(n, 1));
+    return std::min(m, std::max(kTS, rows / kTS * kTS));
+}
+
+size_t dense_product_work(int rows, int n) { return (size_t)ntile(rows) * 2 * n; }
+
 void dense_product_sums(int m, int n, const double *S, const double *Y, double *T, double *work, double *d2, double *dd,
                         cudaStream_t st) {
-    // T = S Y^T: T(l, j) = sum_{p <= j} S(l, p) Y(j, p), then G = T Y: G(l, j) =
+    // By chunks of rows: T = S Y^T: T(l, j) = sum_{p <= j} S(l, p) Y(j, p), then G = T Y: G(l, j) =
     // sum_{p >= j} T(l, p) Y(p, j), kept as per-row-block partial sums in work
-    gemm<false, false>(m, n, n, 1.0, S, m, Y, n, 0.0, T, m, 0, kDepthToCol, nullptr, nullptr, st);
-    gemm<false, true>(m, n, n, 1.0, T, m, Y, n, 0.0, nullptr, 0, 0, kDepthFromCol, S, work, st);
-    k_sum_blocks<<<(n + 255) / 256, 256, 0, st>>>(ntile(m), n, work, d2, dd);
+    const int rows = dense_product_rows(m, n);
+    cudaMemsetAsync(d2, 0, sizeof(double) * n, st);
+    cudaMemsetAsync(dd, 0, sizeof(double) * n, st);
+    for (int r0 = 0; r0 < m; r0 += rows) {
+        const int r = std::min(rows, m - r0);
+        gemm<false, false>(r, n, n, 1.0, S + r0, m, Y, n, 0.0, T, r, 0, kDepthToCol, nullptr, nullptr, st);
+        gemm<false, true>(r, n, n, 1.0, T, r, Y, n, 0.0, nullptr, m, 0, kDepthFromCol, S + r0, work, st);
+        k_sum_blocks<<<(n + 255) / 256, 256, 0, st>>>(ntile(r), n, work, d2, dd);
+    }
 }
 
 }  // namespace crgpu

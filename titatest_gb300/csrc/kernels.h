@@ -120,12 +120,14 @@ struct McmArgs {
 // the Cholesky factor L of A (n x n, lower, in place) and Y = L^-1 (info_dev:
 // first non-positive pivot, 1-based, 0 if none; hi, ev: a stream of high priority
 // and an event that it uses beside st); C (lower) = Y^T Y; d_j = sum_i Y_ij^2 of the
-// lower Y; the sums over l of G_lj^2 and G_lj S_lj for G = S Y^T Y, S m x n, with
-// T (m x n) and work (ceil(m/32) x 2 x n)
+// lower Y; the sums over l of G_lj^2 and G_lj S_lj for G = S Y^T Y, S m x n, by
+// chunks of dense_product_rows rows, with T (rows x n) and work (dense_product_work)
 void dense_syrk_t(int n, int k, const double *S, int lds, double *C, cudaStream_t st);
 void dense_potrf_inverse(int n, double *A, double *Y, int *info_dev, cudaStream_t st, cudaStream_t hi, cudaEvent_t ev);
 void dense_lauum_t(int n, const double *Y, double *C, cudaStream_t st);
 void dense_lower_col_sq(int n, const double *Y, double *d, cudaStream_t st);
+int dense_product_rows(int m, int n);
+size_t dense_product_work(int rows, int n);
 void dense_product_sums(int m, int n, const double *S, const double *Y, double *T, double *work, double *d2, double *dd,
                         cudaStream_t st);
 int run_mcm(const McmArgs &a, cudaStream_t st, cudaStream_t hi, cudaEvent_t ev, std::string &msg);

@@ -215,8 +215,11 @@ int run_mcm(const McmArgs &a, cudaStream_t st, cudaStream_t hi, cudaEvent_t ev, 
     if (sums) {
         // G = S cov without cov: bres diag(cov ata) = sum_l G_lj S_lj, bmcm2
         // diag(cov ata cov) = sum_l G_lj^2
-        dal((void **)&cov, sizeof(double) * 2 * (size_t)m * n);  // S Y^T
-        dal((void **)&work, sizeof(double) * (size_t)((2 * m + 31) / 32) * 2 * n);
+        const int rows = dense_product_rows(2 * m, n);  // of S at a time
+        cudaFreeAsync(reg, st);
+        reg = nullptr;
+        dal((void **)&cov, sizeof(double) * (size_t)rows * n);  // S Y^T
+        dal((void **)&work, sizeof(double) * dense_product_work(rows, n));
         dal((void **)&d2, sizeof(double) * n);
         if (!rc) {
             dense_product_sums(2 * m, n, A, Y, cov, work, d2, d, st);
