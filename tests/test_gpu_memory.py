@@ -162,3 +162,17 @@ def test_singularity_removal_keeps_no_elimination_plan(gpu_lib):
                 pass
         held.append(peak.bytes)
     assert held[1] < held[0] - 4 * s.grid.sanz  # one position a node at least
+
+
+def test_refused_context_takes_no_device_memory(gpu_lib):
+    """A mixed context in a band of 258 is refused (1002) before its arrays are
+    allocated and filled."""
+    from test_gpu_substruct import _case
+    from titatest_gb300 import MIXED, CRMod
+    from titatest_gb300._lib import CRGPUError
+    s = _case(160, 150, 8)
+    assert s.grid.mb > 207
+    with _Peak() as peak:
+        with pytest.raises(CRGPUError) as ei:
+            CRMod(s.grid, s.survey, precision=MIXED, band_order=0)
+    assert ei.value.errnr == 1002 and peak.bytes == 0

@@ -1292,6 +1292,11 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
     std::vector<double> strom(c->nanz, 1.0), kwn(sv->kwn, sv->kwn + c->K), kwnwi(sv->kwnwi, sv->kwnwi + c->K);
     if (sv->strom)
         for (int i = 0; i < c->nanz; i++) strom[i] = sv->strom[i];
+    if (mixed && !mixed_window_supported(hg.mb + 1)) {
+        c->last_error = "mixed precision supports band widths up to 207";
+        *out = c;
+        return ERR_UNSUPPORTED;
+    }
     Block blk;
     blk.put(&P.x, hg.x);
     blk.put(&P.y, hg.y);
@@ -1396,11 +1401,6 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
             c->sys_l.push_back(0);
         }
     }
-    if (precision == CRGPU_MIXED && !mixed_window_supported(hg.mb + 1)) {
-        c->last_error = "mixed precision supports band widths up to 207";
-        *out = c;
-        return ERR_UNSUPPORTED;
-    }
     Block tree;  // its host copy lives until the synchronisation below
     std::vector<int32_t> sources(enr0);
     if (c->nsink >= 0 && c->nsink < hg.n) sources.push_back(c->nsink);
@@ -1448,6 +1448,7 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
         tree.put(&D.fcolpos, fcolpos);
         e = tree.make(c);
         if (e) {
+            cudaStreamSynchronize(c->st);  // blk's copy may still read its host memory
             *out = c;
             return e;
         }
