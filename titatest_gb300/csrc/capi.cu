@@ -253,6 +253,7 @@ int check_device_errors(crgpu_ctx *c, const int *d_status, int nsys, int k0 = -1
     std::vector<int> st(nsys > 0 ? nsys : 0);
     if (nsys > 0) CUCHECK(c, cudaMemcpyAsync(st.data(), d_status, sizeof(int) * nsys, cudaMemcpyDeviceToHost, c->st));
     CUCHECK(c, cudaStreamSynchronize(c->st));
+    c->left_open = false;
     if (h_err) return fail(c, h_err, "device reported error " + std::to_string(h_err));
     for (int s = 0; s < nsys; s++)
         if (st[s]) {
@@ -694,6 +695,8 @@ int sub_left(const SubJob &j, int it) {
 // its Jacobian 1.37 -> 1.31, eight 160x50 contexts in turn 24.4 -> 22.8.
 int sub_refine(std::vector<SubJob> &jobs) {
     size_t open = 0;
+    for (const SubJob &j : jobs)  // a call that failed may have left steps that write the same words
+        if (!j.done && j.c->left_open) CUCHECK(j.c, cudaStreamSynchronize(j.st));
     for (SubJob &j : jobs) {
         if (j.done) continue;
         crgpu_ctx *c = j.c;
@@ -708,6 +711,7 @@ int sub_refine(std::vector<SubJob> &jobs) {
             continue;
         }
         std::fill_n(c->refine_left + j.slot * kRefineCap, kRefineCap, -1);
+        c->left_open = true;
         open++;
     }
     for (int it = 0; open; it++)
@@ -1462,6 +1466,9 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
 int crgpu_destroy(crgpu_ctx *c) {
     if (!c) return 0;
     drop_graph(c);
+    // after a call that failed with refinement steps queued: they write the words
+    // that the next context gets
+    if (c->left_open) cudaStreamSynchronize(c->st);
     for (void *p : c->allocs) cudaFreeAsync(p, c->st);
     if (c->d_upd) cudaFreeAsync(c->d_upd, c->st);
     if (c->own_st) cudaStreamDestroy(c->own_st);

@@ -46,6 +46,7 @@ struct crgpu_ctx {
     // current batch (RefineCount)
     void *d_refine = nullptr;
     int *refine_left = nullptr;  // mapped host memory: systems each step has left (sub_refine)
+    bool left_open = false;      // steps that write it may still be queued
     int refine_used[4] = {};  // steps launched on each array since the last collection
     // forward + Jacobian as one CUDA graph (crgpu_forward_sens_graph)
     bool capturing = false;       // recording: no host copies, synchronisation or timing
