@@ -540,9 +540,7 @@ void sub_rect(crgpu_ctx *c, int *kb, int *lb) {
                                           (c->D.As ? sub_bytes_values(c) : 0)));
     }
     budget -= (int64_t)sub_bytes_values(c);
-    *kb = c->K;
-    *lb = c->eanz;
-    if ((c->sub_cap >= nsys && c->sub_kcap >= c->K) || c->K * wave + nsys * per <= budget) return;
+    if (c->K * wave + nsys * per <= budget) return;
     *kb = (int)std::max<int64_t>(0, std::min<int64_t>(c->K, budget / (wave + c->eanz * per)));
     if (*kb > 0) return;
     *kb = 1;
@@ -1918,11 +1916,13 @@ int crgpu_sens(crgpu_ctx *c, int32_t mode, double *sens) {
     }
     cudaGetLastError();  // a pageable pointer is not an error
     if (!c->copy_st) CUCHECK(c, cudaStreamCreateWithFlags(&c->copy_st, cudaStreamNonBlocking));
-    cudaEvent_t a, b, done[kChunks], copied[kChunks];
+    cudaEvent_t a, b, done[kChunks] = {}, copied[kChunks] = {};
     cudaEventCreate(&a);
     cudaEventCreate(&b);
-    for (auto &d : done) cudaEventCreateWithFlags(&d, cudaEventDisableTiming);
-    for (auto &d : copied) cudaEventCreateWithFlags(&d, cudaEventDisableTiming);
+    for (int q = 0; q < chunks; q++) {
+        cudaEventCreateWithFlags(&done[q], cudaEventDisableTiming);
+        if (ring) cudaEventCreateWithFlags(&copied[q], cudaEventDisableTiming);
+    }
     cudaEventRecord(a, c->st);
     for (int q = 0; q < chunks; q++) {
         const int e0 = q * per, ne = std::min<int>(per, (int)manz - e0);
@@ -1936,7 +1936,7 @@ int crgpu_sens(crgpu_ctx *c, int32_t mode, double *sens) {
         CUCHECK(c, cudaStreamWaitEvent(c->copy_st, done[q], 0));
         CUCHECK(c, cudaMemcpyAsync(sens + 2 * (size_t)e0 * nanz, at, (size_t)ne * nanz * sizeof(double2),
                                    cudaMemcpyDeviceToHost, c->copy_st));
-        CUCHECK(c, cudaEventRecord(copied[q], c->copy_st));
+        if (ring) CUCHECK(c, cudaEventRecord(copied[q], c->copy_st));
     }
     cudaEventRecord(b, c->st);
     CUCHECK(c, cudaStreamSynchronize(c->copy_st));
@@ -1946,8 +1946,10 @@ int crgpu_sens(crgpu_ctx *c, int32_t mode, double *sens) {
     c->stats.ms_sens = ms;
     cudaEventDestroy(a);
     cudaEventDestroy(b);
-    for (auto &d : done) cudaEventDestroy(d);
-    for (auto &d : copied) cudaEventDestroy(d);
+    for (int q = 0; q < chunks; q++) {
+        cudaEventDestroy(done[q]);
+        if (ring) cudaEventDestroy(copied[q]);
+    }
     if (ring) cudaFreeAsync(ring, c->st);
     else c->last_sens = c->d_sens;
     CUCHECK(c, cudaGetLastError());

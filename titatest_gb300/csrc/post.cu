@@ -378,7 +378,7 @@ __device__ __forceinline__ void sens_element(const DevProblem &P, const typename
 #pragma unroll
             for (int m0 = 0; m0 < kSensMPT; m0 += kSensGroup) {
                 const int f = i0 + m0 * kSensThreads;  // the group's first slot
-                if (f + (tid & ~31) >= i1) break;  // the warp has no more
+                if (f + (kOwnSum ? 0 : tid & ~31) >= i1) break;  // complex128 (FP64 pipe): warp by warp
                 int4 md[kSensGroup];
 #pragma unroll
                 for (int h = 0; h < kSensGroup; h++) {
