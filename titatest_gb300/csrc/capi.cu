@@ -532,6 +532,9 @@ int ensure_sub_rhs(crgpu_ctx *c) {
 void sub_rect(crgpu_ctx *c, int *kb, int *lb) {
     const int nsys = (int)c->sys_k.size();
     const int64_t per = (int64_t)sub_bytes_per_system(c), wave = (int64_t)sub_bytes_wavenumber(c);
+    *kb = c->K;
+    *lb = c->eanz;
+    if (c->sub_cap >= nsys && c->sub_kcap >= c->K) return;
     int64_t budget = c->mem_budget;
     if (budget <= 0) {
         size_t fr = 0, tot = 0;
@@ -682,15 +685,15 @@ int sub_left(const SubJob &j, int it) {
     }
 }
 
-// Refinement of the jobs, step by step in turn, until none has systems left.
-// Every step used to be queued at once, the later ones to find nothing to do:
-// for config 2, 4 of its 8 with 23 launches each.  Now the host launches a job's
-// step when the one before has left systems over (it learns so from mapped
-// memory, in a few microseconds; other jobs keep the GPU busy meanwhile), and a
-// recorded job is a loop on the device.  A step in hand is worse by
-// 0 to 2 %.  Config 2 forward 10.05 -> 9.48 ms, its replayed graph with Jacobian
-// 8.92 -> 7.90, 300x80 cells with 128 electrodes 26.8 -> 25.5, a 60x20 line with
-// its Jacobian 1.37 -> 1.31, eight 160x50 contexts in turn 24.4 -> 22.8.
+// Refinement of the jobs, step by step in turn, until none has systems left.  The
+// host launches a job's step when the one before has left systems over (it learns
+// so from mapped memory, in a few microseconds; other jobs keep the GPU busy
+// meanwhile), and a recorded job is a loop on the device.  Against all steps queued
+// at once, where the later ones find nothing to do (4 of config 2's 8, with 23
+// launches each): config 2 forward 10.05 -> 9.48 ms, its replayed graph with
+// Jacobian 8.92 -> 7.90, 300x80 cells with 128 electrodes 26.8 -> 25.5, a 60x20 line
+// with its Jacobian 1.37 -> 1.31, eight 160x50 contexts in turn 24.4 -> 22.8.  A step
+// queued ahead is worse by 0 to 2 %.
 int sub_refine(std::vector<SubJob> &jobs) {
     size_t open = 0;
     for (const SubJob &j : jobs)  // a call that failed may have left steps that write the same words
@@ -1422,11 +1425,11 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
         D.root_ent0 = sp.root_ent0;
         D.n_root_ent = (int)sp.ent.size() - sp.root_ent0;
         D.n_be = (int)sp.be.size();
-        D.root_child = sp.root_child;
-        D.root_u0 = sp.fronts[sp.root_child].u0;
-        D.root_r = sp.fronts[sp.root_child].r;
-        D.root_oS = sp.fronts[sp.root_child].oS;
-        D.root_live = sp.fronts[sp.root_child].live != 0;
+        const SubFront &top = sp.fronts.back();
+        D.root_u0 = top.u0;
+        D.root_r = top.r;
+        D.root_oS = top.oS;
+        D.root_live = top.live != 0;
         std::vector<int32_t> fcolpos(c->pat.fcol.size());
         for (size_t q = 0; q < fcolpos.size(); q++) fcolpos[q] = sp.pos[c->pat.fcol[q]];
         tree.put(&D.fr, sp.fronts);

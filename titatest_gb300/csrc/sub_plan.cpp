@@ -221,7 +221,7 @@ bool build_sub_plan(const HostGrid &hg, const Pattern &pat, const SubShape &shap
         sp.c_factor += (double)t.e * t.e * t.e + (double)t.e * t.e * t.r + 0.5 * t.e * t.r * (double)t.r;
         sp.c_apply += (double)t.e * (t.e + 2.0 * t.r);
         t.nch = (int)s.ch.size();
-        t.live = t.pad = 0;
+        t.live = 0;
         for (int v : s.E)
             if (source[v]) t.live = 1 << kSubCh;
         for (int z = 0; z < kSubCh; z++) {
@@ -271,7 +271,6 @@ bool build_sub_plan(const HostGrid &hg, const Pattern &pat, const SubShape &shap
     }
     // the root: its entries, the last front's rows in it, the boundary terms by column
     sp.root_ent0 = (int)sp.ent.size();
-    sp.root_child = nf - 1;
     for (int v : outer) local[v] = sp.pos[v] - sp.nI;
     std::vector<std::vector<SubEnt>> cols(sp.m);
     for (int p : root_p) {
@@ -379,7 +378,7 @@ double sub_us(const SubCost &q) {
 // 213 -> 182, 600x60 1145 -> 367.  Over these and 80 others the choice loses at most
 // 11 % where both were candidates; above 5 ms the band's estimate is 0.63 to 1.22 of
 // its time, this solver's 0.61 to 1.74, both mostly within a fifth.  Beyond the two
-// operation counts the gains are small and not measured over the whole range: those
+// operation counts the choice is not measured over the whole range: those problems
 // keep the band, as do the smallest complex128 grids, all latency (8x4 cells 0.29 ->
 // 0.35 ms, 16x6 0.52 -> 0.43).
 bool sub_fits(const SubCost &q) {

@@ -28,7 +28,6 @@ struct SubFront {
     int32_t ent0, nent;   // matrix entries assembled here
     int32_t rows0;        // into SubPlan::rows
     int32_t u0;           // first row of this front's update vectors
-    int32_t pad;
     int64_t oF, oG, oS;   // inverse pivot block (e x e), G (e x r), Schur complement (r x r)
     // children: their r, first update row and Schur complement, and
     // (in SubPlan::inv) the row among a child's r rows of every local row, or -1
@@ -51,7 +50,7 @@ struct SubPlan {
     std::vector<int32_t> level;                // nlevel + 1: first front of a level
     std::vector<int32_t> rows, inv;
     std::vector<SubEnt> ent;                   // of the fronts, then (from root_ent0) of the root
-    int root_ent0 = 0, root_child = -1;
+    int root_ent0 = 0;
     std::vector<int32_t> root_inv;             // root row -> row of the last front's r rows, or -1
     std::vector<SubEnt> be;                    // root entries with mixed-boundary terms, by column (row >= column)
     std::vector<int32_t> be_ptr;               // m + 1: first of a column

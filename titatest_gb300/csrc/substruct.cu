@@ -127,9 +127,10 @@ __device__ __forceinline__ void load2(const double2 *p, double2 (&v)[2]) {
 
 // Programmatic dependent launch: a forward is a chain of up to 250 short
 // kernels, and the start of each (launch, tables, index loads) overlaps the end
-// of the one before.  Every kernel of the chain waits for its predecessor
-// before it reads or writes anything but the plan's tables, also where it then
-// returns at once, so a kernel's own wait covers all earlier ones.  GB300:
+// of the one before.  A kernel waits for its predecessor before it reads or writes
+// anything but the plan's tables and what is older than that predecessor.  A block
+// may return without the wait, but of every grid at least one block waits, so a
+// grid ends only after all earlier ones and its successor's wait covers them.  GB300:
 // 60x20 quads mixed with Jacobian 2.11 -> 1.82 ms, triangle gradient 14.7 -> 13.8
 // ms.  Letting the successor's blocks in before this kernel ends
 // (launch_dependents) cost complex128 3 %: they take the places of its last
@@ -354,7 +355,7 @@ __global__ __launch_bounds__(256) void k_sub_pivot(DevSub D, int f0, int nnz) {
     }
     __syncthreads();
     bool ok = invert_block(Fm, ld, min(e, H), sw);
-    if (e > H) {
+    if (Tile<T>::emax > H && e > H) {
         const int h = e - H, lane = tid & 31, w = tid >> 5;
         T *G = Fm + e * ld, *K = G + H * PH;
         // G = A^-1 B: row = lane, columns w, w + 8, ...
@@ -1471,9 +1472,8 @@ __global__ __launch_bounds__(256) void k_sub_stop(SubBatch B, int first, double 
 
 // out[k][l][node] = sign fk x (src/fem.f90:388-389), through shared memory:
 // 32 nodes x 32 electrodes a block; out32 the complex64 hi and lo planes
-template <typename T>
-__global__ __launch_bounds__(256) void k_sub_unpack(DevProblem P, DevSub D, SubBatch B, const T *__restrict__ X,
-                                                    double sign, double2 *out, float2 *out32) {
+__global__ __launch_bounds__(256) void k_sub_unpack(DevProblem P, DevSub D, SubBatch B, double sign, double2 *out,
+                                                    float2 *out32) {
     __shared__ double2 tile[32][33];
     const int kk = blockIdx.z, k = B.k0 + kk, n0 = blockIdx.x * 32, l0 = blockIdx.y * 32;
     const int a = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1504,7 +1504,7 @@ int factor_t(const DevProblem &P, const DevSub &D, const SubPlan &sp, int K, cud
     auto bytes = [](int e) { return sizeof(T) * (e * (e | 1) + (e > 32 ? 2 * 32 * 33 : 0)); };
     static std::once_flag once;
     std::call_once(once, [&] {
-        cudaFuncSetAttribute(k_sub_pivot<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes(kSubEMax));
+        cudaFuncSetAttribute(k_sub_pivot<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes(Tile<T>::emax));
     });
     int launches = 0;
     for (int lv = 0; lv < sp.nlevel; lv++) {
@@ -1538,7 +1538,7 @@ void root_t(const DevProblem &P, const DevSub &D, const SubBatch &B, const doubl
     k_sub_root<T><<<B.Kb * B.Lb, kRT, root_smem<T>(), st>>>(D, B);
 }
 
-// Levels with tiles for at most a third of the SMs (48 blocks) take the kernels
+// Levels with tiles for at most 48 blocks (a third of the 152 SMs) take the kernels
 // for few fronts.  Blocks at most against forwards in ms (60x20 line with
 // Jacobian / 200x60 / triangle gradient / 300x80 / eight contexts at once): none
 // 1.31 9.53 12.23 26.1 16.9, 30 1.28 9.54 12.0 26.1 16.9, 48 1.27 9.40 11.84 25.9
@@ -1640,7 +1640,7 @@ void sub_launch_accumulate(const DevSub &D, const SubBatch &B, bool first, doubl
 
 void sub_launch_unpack(const DevProblem &P, const DevSub &D, const SubBatch &B, double sign, double2 *out,
                        float2 *out32, cudaStream_t st) {
-    k_sub_unpack<double2><<<dim3(nb(D.n, 32), nb(B.Lb, 32), B.Kb), 256, 0, st>>>(P, D, B, B.X, sign, out, out32);
+    k_sub_unpack<<<dim3(nb(D.n, 32), nb(B.Lb, 32), B.Kb), 256, 0, st>>>(P, D, B, sign, out, out32);
 }
 
 }  // namespace crgpu

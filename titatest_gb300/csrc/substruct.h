@@ -19,7 +19,7 @@ struct DevSub {
     const SubTile *tA, *tG, *tS, *tU, *tV, *tD;
     const int32_t *pos, *node, *rows, *inv, *root_inv, *fcolpos;
     const int32_t *be_ptr, *rb_ptr, *rb_ent, *rb_pos;
-    int root_ent0, n_root_ent, n_be, root_child, root_u0, root_r, root_live;
+    int root_ent0, n_root_ent, n_be, root_u0, root_r, root_live;
     int64_t root_oS;
     double2 *As;     // [K][nnz] area parts, scaled by fk on both sides
     double *fk;      // [K][n]   scaling of the area parts' diagonal, by node
