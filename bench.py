@@ -446,7 +446,7 @@ def run_gpu(args):
         "launch": "forward + Jacobian calls" if args.no_graph else
                   "forward + Jacobian as one CUDA graph (crgpu_forward_sens_graph)",
         "refinement": {"maxit": args.refine_maxit, "tol": args.refine_tol, "iterations": statistics.mean(iters)},
-        "autotuned_kernels": tune,
+        "autotuned_kernels": dict(tune, factor_applies_to="the band path; here the root factor below runs instead"),
         "clocks": clk.summary(),
         "gpu_launches": int(launches),
         "e2e": {"value": 1e3 / e2e_ms, "unit": "units/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
