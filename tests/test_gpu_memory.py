@@ -149,19 +149,22 @@ def test_forward_where_memory_is_short(gpu_lib, leave):
     assert relerr(w, v) < 1e-10 and relerr(b, a) < 1e-9
 
 
-def test_singularity_removal_keeps_no_elimination_plan(gpu_lib):
+@pytest.mark.parametrize("nx,nz,same", [(120, 40, False), (400, 10, True)])
+def test_contexts_on_the_band_keep_no_elimination_plan(gpu_lib, nx, nz, same):
     """Forwards with singularity removal run on the band, so such a context
-    has no tables of the dissection."""
+    has no tables of the dissection; nor has one that the rule leaves on the
+    band (400 x 10 cells in complex128)."""
     from test_gpu_substruct import _case
     from titatest_gb300 import PLAIN, CRMod
-    s = _case(120, 40, 12)
+    s = _case(nx, nz, 12)
+    kwn, kwnwi = np.geomspace(0.01, 2.0, 4), np.full(4, 0.1)
     held = []
     for lsr in (False, True):
         with _Peak() as peak:
-            with CRMod(s.grid, s.survey, lsr=lsr, precision=PLAIN):
+            with CRMod(s.grid, s.survey, kwn, kwnwi, lsr=lsr, precision=PLAIN):
                 pass
         held.append(peak.bytes)
-    assert held[1] < held[0] - 4 * s.grid.sanz  # one position a node at least
+    assert held[1] == held[0] if same else held[1] < held[0] - 4 * s.grid.sanz  # one position a node at least
 
 
 def test_refused_context_takes_no_device_memory(gpu_lib):

@@ -1409,15 +1409,21 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
     Block tree;  // its host copy lives until the synchronisation below
     std::vector<int32_t> sources(enr0);
     if (c->nsink >= 0 && c->nsink < hg.n) sources.push_back(c->nsink);
-    if (c->nrhs == 1 && !c->lsr && build_sub_plan(hg, c->pat, sub_shape(precision == CRGPU_MIXED), sources, c->sp)) {
+    if (c->nrhs == 1 && !c->lsr && build_sub_plan(hg, c->pat, sub_shape(mixed), sources, c->sp)) {
+        const int nb = sub_root_block(mixed), m = c->sp.m;
+        c->D.mp = (m + nb - 1) / nb * nb;
+        c->sub_fits = sub_fits({mixed, hg.n, hg.mb, m, c->D.mp, sub_root_max(mixed), c->eanz, c->K, c->sp.c_factor,
+                                c->sp.c_apply});
+    }
+    if (!c->sub_fits) {
+        c->sp = SubPlan();
+    } else {
         const SubPlan &sp = c->sp;
         DevSub &D = c->D;
         D.n = sp.n;
         D.m = sp.m;
         D.nI = sp.nI;
-        const int nb = sub_root_block(precision == CRGPU_MIXED);
-        D.mp = (sp.m + nb - 1) / nb * nb;
-        D.ldc = D.mp + sub_root_rows(precision == CRGPU_MIXED) - nb;  // the last rows' tile stays inside
+        D.ldc = D.mp + sub_root_rows(mixed) - sub_root_block(mixed);  // the last rows' tile stays inside
         D.szU = sp.szU;
         D.szF = sp.szF;
         D.szG = sp.szG;
@@ -1457,7 +1463,6 @@ int crgpu_create2(const crgpu_grid *grid, const crgpu_survey *sv, int32_t precis
             *out = c;
             return e;
         }
-        c->sub_fits = sub_fits({mixed, hg.n, hg.mb, sp.m, D.mp, sub_root_max(mixed), c->eanz, c->K, sp.c_factor, sp.c_apply});
     }
     int ce2 = check_device_errors(c, nullptr, 0);
     *out = c;
