@@ -34,7 +34,7 @@ MEASURED = [
     (1, 1000, 20, 96, 13, 22, 1.07e8, 2.14e6, 50.0, 61.1), (1, 500, 20, 96, 13, 22, 3.75e7, 1.03e6, 25.7, 13.9),
     (1, 1500, 30, 96, 13, 32, 2.39e8, 4.94e6, 110, 182), (1, 800, 30, 96, 13, 32, 1.22e8, 2.64e6, 58.4, 41.1),
     (1, 2000, 60, 96, 13, 62, 8.32e8, 1.48e7, 313, 448), (1, 1250, 60, 96, 13, 62, 4.4e8, 9.0e6, 196, 139),
-    (1, 2600, 60, 24, 10, 62, 1.08e9, 1.92e7, 286, 486), (1, 2000, 60, 8, 4, 62, 8.32e8, 1.48e7, 208, 77),
+    (1, 2600, 60, 24, 10, 62, 1.08e9, 1.92e7, 286, 486), (1, 2000, 60, 24, 10, 62, 8.32e8, 1.48e7, 220, 243), (1, 2000, 60, 8, 4, 62, 8.32e8, 1.48e7, 208, 77),
     (1, 2000, 100, 96, 13, 102, 1.57e9, 2.57e7, 1531, 516), (1, 200, 60, 96, 13, 62, 3.9e7, 1.36e6, 32.0, 9.6),
     (0, 600, 20, 24, 4, 41, 2.81e7, 1.03e6, 49.7, 63.9), (0, 300, 20, 24, 4, 41, 1.17e7, 4.98e5, 25.0, 13.2),
     (0, 1000, 30, 24, 10, 61, 1.04e8, 2.97e6, 287, 766), (0, 600, 30, 24, 4, 61, 5.12e7, 1.70e6, 91, 69),

@@ -354,7 +354,7 @@ double band_us(const SubCost &q) {
 // elimination, the sweeps and residuals, and the chains of the root's solves.
 double sub_us(const SubCost &q) {
     const double m = q.m, systems = (double)q.K * q.eanz, x = systems / 152.0, flop = 4.0 / 3.0 * m * m * m;
-    const double crowd = q.mixed ? std::min(2.3, std::max(1.3, m / 900.0)) : 1.7;
+    const double crowd = q.mixed ? std::min(2.9, std::max(1.3, m / 700.0)) : 1.7;
     const double load = x <= 1.0 ? 1.0 : std::max(x, std::min(5.0, crowd * x));
     const double shared = 8.0 * q.K * q.c_factor;
     if (!q.mixed)
@@ -375,12 +375,12 @@ double sub_us(const SubCost &q) {
 // complex128, 96 systems 200x10 7.2 -> 4.7, 400x10 14.2 -> 21.1, 300x20 25.0 ->
 // 13.2, 600x20 49.7 -> 63.9, 600x30 91 -> 69, 1000x30 151 -> 251, 1500x60 974 ->
 // 845, 2000x60 1298 -> 1819; 384 systems 300x20 69 -> 30, 600x20 137 -> 261, 500x30
-// 213 -> 182, 600x60 1145 -> 367.  Over these and 80 others the choice loses at most
-// 11 % where both were candidates; above 5 ms the band's estimate is 0.63 to 1.22 of
-// its time, this solver's 0.61 to 1.74, both mostly within a fifth.  Beyond the two
-// operation counts the choice is not measured over the whole range: those problems
-// keep the band, as do the smallest complex128 grids, all latency (8x4 cells 0.29 ->
-// 0.35 ms, 16x6 0.52 -> 0.43).
+// 213 -> 182, 600x60 1145 -> 367.  Over these and 80 others the band is kept at most
+// where it costs 11 % more, and never left where it is the faster one; above 5 ms
+// the band's estimate is 0.63 to 1.22 of its time, this solver's 0.71 to 2.14, nine
+// tenths of both 0.8 to 1.25.  Beyond the two operation counts the choice is not
+// measured over the whole range: those problems keep the band, as do the smallest
+// complex128 grids, all latency (8x4 cells 0.29 -> 0.35 ms, 16x6 0.52 -> 0.43).
 bool sub_fits(const SubCost &q) {
     if (q.mp > q.root_max) return false;  // the root's vector stays in one block's shared memory
     const double n = q.n, mb = q.mb, m = q.m;
